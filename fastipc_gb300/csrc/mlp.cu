@@ -3,11 +3,13 @@
 // Network: 55 inputs (padded to 64) -> 128 -> 128 -> 128 -> 3 (padded to 4), GELU after each
 // hidden layer.  Rows are vertices; parameters are one flat FP32 array:
 //   W1 [128][64], b1 [128], W2 [128][128], b2 [128], W3 [128][128], b3 [128], W4 [4][128], b4 [4].
-// The layer products run on a tiled FP32 SGEMM (64x64 output tiles, 16-deep K slices in shared
-// memory, 4x4 outputs per thread); every output element sums its K range in a fixed order, so
-// forward and backward results are reproducible.  No counterpart in the reference: this is the
+// The forward pass is one kernel over tiles of rows; the backward pass alternates data-gradient
+// tiles and weight-gradient chunks of rows.  FP32 FMAs throughout; every output element sums its K
+// range in a fixed order, so forward and backward results are reproducible.  No counterpart in the reference: this is the
 // learned warm start the task adds beside the drop-in path.
 #include <cuda_runtime.h>
+
+#include <initializer_list>
 
 #include "ctx.cuh"
 
@@ -18,94 +20,358 @@ constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + MLP_H * MLP_IN, OFF_W2 = OFF_B1 + ML
               OFF_W3 = OFF_B2 + MLP_H, OFF_B3 = OFF_W3 + MLP_H * MLP_H, OFF_W4 = OFF_B3 + MLP_H,
               OFF_B4 = OFF_W4 + MLP_OUT * MLP_H, MLP_NPARAM = OFF_B4 + MLP_OUT;
 
-// C[M][N] (ldc) = alpha * op(A)[M][K] * op(B)[K][N] + beta * C.  op(A) = A[M][K] (lda) or, when
-// ta, A stored [K][M]; op(B) = B[K][N] (ldb) or, when tb, B stored [N][K].
-constexpr int TM = 64, TN = 64, TK = 16;
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, float alpha, const float* __restrict__ A, int lda, int ta,
-                                               const float* __restrict__ B, int ldb, int tb, float beta, float* __restrict__ C,
-                                               int ldc) {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        // 64 x 16 tile of op(A) and 16 x 64 tile of op(B), 4 elements per thread each
-        for (int e = threadIdx.x; e < TM * TK; e += 256) {
-            const int mm = e / TK, kk = e % TK;
-            const int gm = m0 + mm, gk = k0 + kk;
-            float va = 0.f;
-            if (gm < M && gk < K) va = ta ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            As[kk][mm] = va;
+// ---------------------------------------------------------------- tiles
+// A CTA holds a tile of R rows in shared memory, k-major (Hs[k][row]), and multiplies it with a
+// 128-column weight matrix whose K slices of 32 pass through a double buffer Ws.  Thread (tx, ty)
+// of 16 x 16 owns R/16 consecutive rows and the columns 4 tx .. 4 tx + 3 and 64 + 4 tx ..; per k
+// it loads its rows and two float4 of weights for (R/16) x 8 FMAs.  FP32 FMA issue binds: at
+// R = 128 a k step is 64 FMAs per thread against 4 shared-memory loads.  Rows are swizzled by the
+// column group (row ^ 4 ((k / 4) % 8)) so that the transposed store of a layer's output, which
+// strides by columns, meets distinct banks while the row loads stay aligned.  Every output sums
+// its K range in ascending order in one FMA chain.
+// R = 128 needs n >= 2 x 152 such tiles to fill the GPU; below that R = 64, then 32, keep more SMs
+// busy.  Measured on a GB300, forward pass: 176,841 rows 1.19 ms as separate 64 x 64 products with
+// bias and activation passes, 0.50 ms here; a training step of 8,192 rows 5.3 ms, of
+// which 97% were products (the weight gradients, 128 x 128 outputs over all rows, ran on 2 to 4
+// CTAs), 0.17 ms here.
+constexpr int MLP_THREADS = 256, KS = 32, WLD = MLP_H + 4;
+
+// four consecutive floats of global memory: one 16-byte access when every array of the call is
+// 16-byte aligned (al), else four (callers may pass any float address)
+__device__ __forceinline__ float4 ld4(const float* p, bool al) {
+    return al ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+__device__ __forceinline__ void st4(float* p, float4 v, bool al) {
+    if (al) {
+        *reinterpret_cast<float4*>(p) = v;
+    } else {
+        p[0] = v.x;
+        p[1] = v.y;
+        p[2] = v.z;
+        p[3] = v.w;
+    }
+}
+
+template <int R>
+__device__ __forceinline__ int hs_at(int k, int row) {
+    return k * R + (row ^ (((k >> 2) & 7) << 2));
+}
+
+// rows [r0, r0 + R) of src [n][K] into Hs, zeros past n; a lane takes one row's float4 at a time
+template <int R>
+__device__ __forceinline__ void load_rows(float* Hs, const float* __restrict__ src, int K, int r0, int n, bool al) {
+    for (int e = threadIdx.x; e < R * (K / 4); e += MLP_THREADS) {
+        const int row = e % R, k = 4 * (e / R);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r0 + row < n) v = ld4(src + (size_t)(r0 + row) * K + k, al);
+        Hs[hs_at<R>(k, row)] = v.x;
+        Hs[hs_at<R>(k + 1, row)] = v.y;
+        Hs[hs_at<R>(k + 2, row)] = v.z;
+        Hs[hs_at<R>(k + 3, row)] = v.w;
+    }
+}
+
+// one K slice of the weights, held in registers between its load and its store to shared memory:
+// T (transposed): W [128][K], slice[kk][c] = W[c][k0 + kk];  else W [K][128], slice[kk][c] = W[k0 + kk][c]
+template <bool T>
+__device__ __forceinline__ void fetch_slice(float4 (&w)[4], const float* __restrict__ W, int K, int k0, bool al) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int e = threadIdx.x + q * MLP_THREADS;
+        if (T) w[q] = ld4(W + (size_t)(e % MLP_H) * K + k0 + 4 * (e / MLP_H), al);
+        else w[q] = ld4(W + (size_t)(k0 + e / 32) * MLP_H + 4 * (e % 32), al);
+    }
+}
+template <bool T>
+__device__ __forceinline__ void store_slice(float* Ws, const float4 (&w)[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int e = threadIdx.x + q * MLP_THREADS;
+        if (T) {
+            float* p = Ws + 4 * (e / MLP_H) * WLD + e % MLP_H;
+            p[0] = w[q].x;
+            p[WLD] = w[q].y;
+            p[2 * WLD] = w[q].z;
+            p[3 * WLD] = w[q].w;
+        } else {
+            *reinterpret_cast<float4*>(Ws + (e / 32) * WLD + 4 * (e % 32)) = w[q];
         }
-        for (int e = threadIdx.x; e < TK * TN; e += 256) {
-            const int kk = e / TN, nn = e % TN;
-            const int gk = k0 + kk, gn = n0 + nn;
-            float vb = 0.f;
-            if (gk < K && gn < N) vb = tb ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-            Bs[kk][nn] = vb;
+    }
+}
+
+// acc[i][j] = sum_k Hs[k][row i] W(k, col j) for the thread's rows and columns; Hs complete on entry
+template <int R, bool T>
+__device__ __forceinline__ void tile_product(float (&acc)[R / 16][8], const float* Hs, float* Ws, const float* __restrict__ W, int K,
+                                             bool al) {
+    constexpr int TR = R / 16;
+    const int tx = threadIdx.x % 16, row0 = (threadIdx.x / 16) * TR;
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    float4 w[4];
+    fetch_slice<T>(w, W, K, 0, al);
+    store_slice<T>(Ws, w);
+    __syncthreads();
+    for (int k0 = 0, buf = 0; k0 < K; k0 += KS, buf ^= 1) {
+        const bool more = k0 + KS < K;
+        if (more) fetch_slice<T>(w, W, K, k0 + KS, al);
+        const float* Wb = Ws + buf * KS * WLD + 4 * tx;
+#pragma unroll 8
+        for (int kk = 0; kk < KS; ++kk) {
+            const float* h = Hs + (k0 + kk) * R;
+            const int s = (((k0 + kk) >> 2) & 7) << 2;
+            float a[TR];
+            if (TR == 2) {
+                const float2 v = *reinterpret_cast<const float2*>(h + (row0 ^ s));
+                a[0] = v.x;
+                a[TR - 1] = v.y;
+            } else {
+#pragma unroll
+                for (int i = 0; i + 3 < TR; i += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(h + ((row0 + i) ^ s));
+                    a[i] = v.x;
+                    a[i + 1] = v.y;
+                    a[i + 2] = v.z;
+                    a[i + 3] = v.w;
+                }
+            }
+            const float4 b0 = *reinterpret_cast<const float4*>(Wb + kk * WLD), b1 = *reinterpret_cast<const float4*>(Wb + kk * WLD + 64);
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (int i = 0; i < TR; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
+        if (more) store_slice<T>(Ws + (buf ^ 1) * KS * WLD, w);
         __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gm = m0 + ty * 4 + i, gn = n0 + tx * 4 + j;
-            if (gm < M && gn < N) {
-                float* c = C + (size_t)gm * ldc + gn;
-                *c = alpha * acc[i][j] + (beta != 0.f ? beta * *c : 0.f);
-            }
-        }
 }
+__device__ __forceinline__ int tile_col(int j) { return 4 * (threadIdx.x % 16) + (j & 3) + 64 * (j >> 2); }
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float z) {
     return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-// Z += bias (row broadcast); A = gelu(Z) when act, else A = Z
-__global__ void k_bias_act(int rows, int cols, float* __restrict__ Z, const float* __restrict__ bias, float* __restrict__ A, int act) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * cols) return;
-    const float z = Z[i] + bias[i % cols];
-    Z[i] = z;
-    A[i] = act ? gelu(z) : z;
+template <int R>
+constexpr int tile_smem() {
+    return 4 * (MLP_H * R + 2 * KS * WLD);
 }
 
-// dZ = dA * gelu'(Z), in place on dA
-__global__ void k_gelu_back(int rows, int cols, const float* __restrict__ Z, float* __restrict__ dA) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * cols) return;
-    dA[i] *= gelu_grad(Z[i]);
-}
-
-// db[c] = sum over rows of dZ[r][c]: one block per column, fixed-order strides + tree
-__global__ void k_bias_grad(int rows, int cols, const float* __restrict__ dZ, float* __restrict__ db) {
-    __shared__ float sh[256];
-    const int c = blockIdx.x;
-    float a = 0.f;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) a += dZ[(size_t)r * cols + c];
-    sh[threadIdx.x] = a;
+// the whole forward pass of R rows in one CTA: the activations stay in shared memory from layer to
+// layer (overwritten in place once a layer's sums are in registers); Z and A are written for the
+// backward pass.  One launch instead of eight.
+template <int R>
+__global__ void __launch_bounds__(MLP_THREADS, 2) k_mlp_forward(int n, const float* __restrict__ X, const float* __restrict__ P,
+                                                                float* __restrict__ Z, float* __restrict__ A, float* __restrict__ out, bool al) {
+    extern __shared__ float4 smem4[];
+    float* Hs = reinterpret_cast<float*>(smem4);
+    float* Ws = Hs + MLP_H * R;
+    constexpr int TR = R / 16;
+    const int r0 = blockIdx.x * R, row0 = (threadIdx.x / 16) * TR;
+    load_rows<R>(Hs, X, MLP_IN, r0, n, al);
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
+#pragma unroll 1
+    for (int l = 0; l < 3; ++l) {
+        const int K = l == 0 ? MLP_IN : MLP_H;
+        const float* W = P + (l == 0 ? OFF_W1 : (l == 1 ? OFF_W2 : OFF_W3));
+        const float* bias = P + (l == 0 ? OFF_B1 : (l == 1 ? OFF_B2 : OFF_B3));
+        float acc[TR][8];
+        tile_product<R, true>(acc, Hs, Ws, W, K, al);
+        float* Zl = Z + (size_t)l * n * MLP_H;
+        float* Al = A + (size_t)l * n * MLP_H;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 bb = ld4(bias + tile_col(4 * h), al);
+            const float bv[4] = {bb.x, bb.y, bb.z, bb.w};
+#pragma unroll
+            for (int i = 0; i < TR; ++i) {
+                float z[4], a[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    z[j] = acc[i][4 * h + j] + bv[j];
+                    a[j] = gelu(z[j]);
+                    acc[i][4 * h + j] = a[j];
+                }
+                const int r = r0 + row0 + i;
+                if (r < n) {
+                    const size_t o = (size_t)r * MLP_H + tile_col(4 * h);
+                    st4(Zl + o, make_float4(z[0], z[1], z[2], z[3]), al);
+                    st4(Al + o, make_float4(a[0], a[1], a[2], a[3]), al);
+                }
+            }
+        }
+        // tile_product ended with a barrier: every thread is done with the old activations
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (TR == 2) {
+                *reinterpret_cast<float2*>(Hs + hs_at<R>(tile_col(j), row0)) = make_float2(acc[0][j], acc[TR - 1][j]);
+            } else {
+#pragma unroll
+                for (int i = 0; i + 3 < TR; i += 4)
+                    *reinterpret_cast<float4*>(Hs + hs_at<R>(tile_col(j), row0 + i)) = make_float4(acc[i][j], acc[i + 1][j], acc[i + 2][j], acc[i + 3][j]);
+            }
+        }
         __syncthreads();
     }
-    if (threadIdx.x == 0) db[c] = sh[0];
+    for (int e = threadIdx.x; e < R * MLP_OUT; e += MLP_THREADS) {
+        const int row = e % R, o = e / R;
+        const float* w = P + OFF_W4 + o * MLP_H;
+        float s = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < MLP_H; ++k) s = fmaf(Hs[hs_at<R>(k, row)], __ldg(w + k), s);
+        if (r0 + row < n) out[(size_t)(r0 + row) * MLP_OUT + o] = s + __ldg(P + OFF_B4 + o);
+    }
+}
+
+// gradient of a layer's input: din = (d W) gelu'(Z), d [n][128], W [128][128]
+template <int R>
+__global__ void __launch_bounds__(MLP_THREADS, 2) k_mlp_data_grad(int n, const float* __restrict__ d, const float* __restrict__ W,
+                                                                  const float* __restrict__ Z, float* __restrict__ din, bool al) {
+    extern __shared__ float4 smem4[];
+    float* Hs = reinterpret_cast<float*>(smem4);
+    float* Ws = Hs + MLP_H * R;
+    constexpr int TR = R / 16;
+    const int r0 = blockIdx.x * R, row0 = (threadIdx.x / 16) * TR;
+    load_rows<R>(Hs, d, MLP_H, r0, n, al);
+    __syncthreads();
+    float acc[TR][8];
+    tile_product<R, false>(acc, Hs, Ws, W, MLP_H, al);
+#pragma unroll
+    for (int i = 0; i < TR; ++i) {
+        const int r = r0 + row0 + i;
+        if (r >= n) break;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const size_t o = (size_t)r * MLP_H + tile_col(4 * h);
+            const float4 z = ld4(Z + o, al);
+            st4(din + o, make_float4(acc[i][4 * h] * gelu_grad(z.x), acc[i][4 * h + 1] * gelu_grad(z.y),
+                                     acc[i][4 * h + 2] * gelu_grad(z.z), acc[i][4 * h + 3] * gelu_grad(z.w)), al);
+        }
+    }
+}
+
+// the last layer's backward over one chunk of rows: d3 = (dout W4) gelu'(Z3) for its rows, and the
+// chunk's sums of dout^T A3 [4][128] and of dout [4] into part (MLP_LAST floats per chunk).  Thread
+// (c, h): column c, rows of parity h; the two halves are added at the end, rows in ascending order.
+constexpr int MLP_LAST = MLP_OUT * MLP_H + MLP_OUT;
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_last_grad(int n, int chunk, const float* __restrict__ dout,
+                                                               const float* __restrict__ W4, const float* __restrict__ A3,
+                                                               const float* __restrict__ Z3, float* __restrict__ d3,
+                                                               float* __restrict__ part, bool al) {
+    __shared__ float sh[MLP_OUT + 1][MLP_H];
+    const int c = threadIdx.x % MLP_H, h = threadIdx.x / MLP_H;
+    const int r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
+    float w[MLP_OUT], g[MLP_OUT] = {}, b = 0.f;
+#pragma unroll
+    for (int o = 0; o < MLP_OUT; ++o) w[o] = __ldg(W4 + o * MLP_H + c);
+#pragma unroll 4
+    for (int r = r0 + h; r < r1; r += 2) {
+        const float4 q = ld4(dout + (size_t)r * MLP_OUT, al);
+        const float a = __ldg(A3 + (size_t)r * MLP_H + c), z = __ldg(Z3 + (size_t)r * MLP_H + c);
+        g[0] = fmaf(q.x, a, g[0]);
+        g[1] = fmaf(q.y, a, g[1]);
+        g[2] = fmaf(q.z, a, g[2]);
+        g[3] = fmaf(q.w, a, g[3]);
+        if (c < MLP_OUT) b += c == 0 ? q.x : (c == 1 ? q.y : (c == 2 ? q.z : q.w));
+        const float d = fmaf(q.w, w[3], fmaf(q.z, w[2], fmaf(q.y, w[1], q.x * w[0])));
+        d3[(size_t)r * MLP_H + c] = d * gelu_grad(z);
+    }
+    if (h == 1) {
+#pragma unroll
+        for (int o = 0; o < MLP_OUT; ++o) sh[o][c] = g[o];
+        sh[MLP_OUT][c] = b;
+    }
+    __syncthreads();
+    if (h == 1) return;
+    float* p = part + (size_t)blockIdx.x * MLP_LAST;
+#pragma unroll
+    for (int o = 0; o < MLP_OUT; ++o) p[o * MLP_H + c] = g[o] + sh[o][c];
+    if (c < MLP_OUT) p[MLP_OUT * MLP_H + c] = b + sh[MLP_OUT][c];
+}
+
+// weight gradient of a layer over one chunk of rows: part [128][DIN] = sum_r d[r]^T in[r] and the
+// bias gradient sum_r d[r] behind it (128 DIN + 128 floats per chunk).  The rows are the product's
+// K range, so both operands load into shared memory as they lie.  blockIdx.y takes 64 of the 128
+// output rows.
+template <int DIN>
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_weight_grad(int n, int chunk, const float* __restrict__ d,
+                                                                 const float* __restrict__ in, float* __restrict__ part, bool al) {
+    constexpr int KT = 16, TC = DIN / 16;
+    __shared__ __align__(16) float Ds[2][KT][64], Is[2][KT][DIN];
+    const int r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk), m0 = 64 * blockIdx.y;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    float acc[4][TC] = {}, bsum[4] = {};
+    float4 dv, iv[DIN / 64];
+    auto fetch = [&](int r) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        {
+            const int q = r + threadIdx.x / 16;
+            dv = q < r1 ? ld4(d + (size_t)q * MLP_H + m0 + 4 * (threadIdx.x % 16), al) : zero;
+        }
+#pragma unroll
+        for (int k = 0; k < DIN / 64; ++k) {
+            const int e = threadIdx.x + k * MLP_THREADS, q = r + e / (DIN / 4);
+            iv[k] = q < r1 ? ld4(in + (size_t)q * DIN + 4 * (e % (DIN / 4)), al) : zero;
+        }
+    };
+    auto store = [&](int b) {
+        *reinterpret_cast<float4*>(&Ds[b][threadIdx.x / 16][4 * (threadIdx.x % 16)]) = dv;
+#pragma unroll
+        for (int k = 0; k < DIN / 64; ++k) {
+            const int e = threadIdx.x + k * MLP_THREADS;
+            *reinterpret_cast<float4*>(&Is[b][e / (DIN / 4)][4 * (e % (DIN / 4))]) = iv[k];
+        }
+    };
+    fetch(r0);
+    store(0);
+    __syncthreads();
+    for (int r = r0, buf = 0; r < r1; r += KT, buf ^= 1) {
+        const bool more = r + KT < r1;
+        if (more) fetch(r + KT);
+#pragma unroll
+        for (int k = 0; k < KT; ++k) {
+            const float4 a4 = *reinterpret_cast<const float4*>(&Ds[buf][k][4 * ty]);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+            float b[TC];
+#pragma unroll
+            for (int j = 0; j < TC; j += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(&Is[buf][k][4 * tx + 16 * j]);
+                b[j] = v.x;
+                b[j + 1] = v.y;
+                b[j + 2] = v.z;
+                b[j + 3] = v.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                bsum[i] += a[i];
+#pragma unroll
+                for (int j = 0; j < TC; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            }
+        }
+        if (more) store(buf ^ 1);
+        __syncthreads();
+    }
+    float* p = part + (size_t)blockIdx.x * (MLP_H * DIN + MLP_H);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int m = m0 + 4 * ty + i;
+#pragma unroll
+        for (int j = 0; j < TC; j += 4)
+            st4(p + (size_t)m * DIN + 4 * tx + 16 * j, make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]), al);
+        if (tx == 0) p[MLP_H * DIN + m] = bsum[i];
+    }
+}
+
+// g[e] = sum of part[q][e] over the chunks, chunks in ascending order
+__global__ void k_mlp_sum_chunks(int nchunk, int size, const float* __restrict__ part, float* __restrict__ g) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= size) return;
+    float s = 0.f;
+#pragma unroll 8
+    for (int q = 0; q < nchunk; ++q) s += __ldg(part + (size_t)q * size + e);
+    g[e] = s;
 }
 
 // mean squared error over the first 3 outputs: dout = 2 (out - target) / (3 n), loss partials
@@ -162,15 +428,46 @@ __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g
 namespace fipc {
 static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
-static void sgemm(cudaStream_t s, int M, int N, int K, const float* A, int lda, int ta, const float* B, int ldb, int tb, float beta,
-                  float* C, int ldc) {
-    dim3 grid(nblk(N, TN), nblk(M, TM));
-    k_sgemm<<<grid, 256, 0, s>>>(M, N, K, 1.f, A, lda, ta, B, ldb, tb, beta, C, ldc);
+// rows per tile: the largest that still gives every SM two CTAs (R = 128) or most SMs one (R = 64)
+static int tile_rows(int n) { return n >= 128 * 304 ? 128 : (n >= 64 * 96 ? 64 : 32); }
+
+template <int R>
+static int launch_forward(int n, const float* X, const float* P, float* Z, float* A, float* out, bool al, cudaStream_t s) {
+    FIPC_CUDA(cudaFuncSetAttribute(k_mlp_forward<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem<R>()));
+    k_mlp_forward<R><<<nblk(n, R), MLP_THREADS, tile_smem<R>(), s>>>(n, X, P, Z, A, out, al);
     FIPC_LAUNCHED();
+    return FIPC_OK;
 }
-static void bias_act(cudaStream_t s, int rows, int cols, float* Z, const float* b, float* A, int act) {
-    k_bias_act<<<nblk((long long)rows * cols, 256), 256, 0, s>>>(rows, cols, Z, b, A, act);
+template <int R>
+static int launch_data_grad(int n, const float* d, const float* W, const float* Z, float* din, bool al, cudaStream_t s) {
+    FIPC_CUDA(cudaFuncSetAttribute(k_mlp_data_grad<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem<R>()));
+    k_mlp_data_grad<R><<<nblk(n, R), MLP_THREADS, tile_smem<R>(), s>>>(n, d, W, Z, din, al);
     FIPC_LAUNCHED();
+    return FIPC_OK;
+}
+
+static bool aligned16(std::initializer_list<const void*> ps) {
+    for (const void* p : ps)
+        if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+    return true;
+}
+
+// weight and bias gradient of one layer.  The chunks' partial sums go to scratch (n x 128 floats,
+// free at that time): a chunk takes at least 192 rows and at most 128 x 129 floats, so they fit; at
+// most 152 chunks (two CTAs each).  One chunk writes the gradients directly.
+template <int DIN>
+static void weight_grad(int n, const float* d, const float* in, float* scratch, float* G, bool al, cudaStream_t s) {
+    constexpr int size = MLP_H * DIN + MLP_H;
+    int nc = n / 192;
+    nc = nc < 1 ? 1 : (nc > 152 ? 152 : nc);
+    const int chunk = (n + nc - 1) / nc;
+    nc = nblk(n, chunk);
+    k_mlp_weight_grad<DIN><<<dim3(nc, 2), MLP_THREADS, 0, s>>>(n, chunk, d, in, nc > 1 ? scratch : G, al);
+    FIPC_LAUNCHED();
+    if (nc > 1) {
+        k_mlp_sum_chunks<<<nblk(size, 128), 128, 0, s>>>(nc, size, scratch, G);
+        FIPC_LAUNCHED();
+    }
 }
 }  // namespace fipc
 
@@ -186,22 +483,18 @@ int fipc_mlp_forward(int n, const float* X, const float* params, float* Z, float
     if (n < 0 || !X || !params || !Z || !A || !out) return FIPC_ERR_ARGUMENT;
     if (n == 0) return FIPC_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t L = (size_t)n * MLP_H;
-    const float* P = params;
-    sgemm(s, n, MLP_H, MLP_IN, X, MLP_IN, 0, P + OFF_W1, MLP_IN, 1, 0.f, Z, MLP_H);
-    bias_act(s, n, MLP_H, Z, P + OFF_B1, A, 1);
-    sgemm(s, n, MLP_H, MLP_H, A, MLP_H, 0, P + OFF_W2, MLP_H, 1, 0.f, Z + L, MLP_H);
-    bias_act(s, n, MLP_H, Z + L, P + OFF_B2, A + L, 1);
-    sgemm(s, n, MLP_H, MLP_H, A + L, MLP_H, 0, P + OFF_W3, MLP_H, 1, 0.f, Z + 2 * L, MLP_H);
-    bias_act(s, n, MLP_H, Z + 2 * L, P + OFF_B3, A + 2 * L, 1);
-    sgemm(s, n, MLP_OUT, MLP_H, A + 2 * L, MLP_H, 0, P + OFF_W4, MLP_H, 1, 0.f, out, MLP_OUT);
-    bias_act(s, n, MLP_OUT, out, P + OFF_B4, out, 0);
+    const int R = tile_rows(n);
+    const bool al = aligned16({X, params, Z, A, out});
+    const int st = R == 128 ? launch_forward<128>(n, X, params, Z, A, out, al, s)
+                            : (R == 64 ? launch_forward<64>(n, X, params, Z, A, out, al, s) : launch_forward<32>(n, X, params, Z, A, out, al, s));
+    if (st) return st;
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
 }
 
 // parameter gradients (grads, same layout as params) of sum(dout . out) for the forward pass
-// that produced Z, A; dA: scratch [2][n][128]
+// that produced Z, A; dA: scratch [2][n][128].  One half of dA holds the current layer's output
+// gradient, the other its weight gradient's partial sums until the next layer's gradient overwrites it.
 int fipc_mlp_backward(int n, const float* X, const float* params, const float* Z, const float* A, const float* dout, float* grads,
                       float* dA, void* stream) {
     if (n <= 0 || !X || !params || !Z || !A || !dout || !grads || !dA) return FIPC_ERR_ARGUMENT;
@@ -210,24 +503,27 @@ int fipc_mlp_backward(int n, const float* X, const float* params, const float* Z
     const float* P = params;
     float* G = grads;
     float *d0 = dA, *d1 = dA + L;
-    // layer 4 (linear)
-    sgemm(s, MLP_OUT, MLP_H, n, dout, MLP_OUT, 1, A + 2 * L, MLP_H, 0, 0.f, G + OFF_W4, MLP_H);
-    k_bias_grad<<<MLP_OUT, 256, 0, s>>>(n, MLP_OUT, dout, G + OFF_B4);
-    FIPC_LAUNCHED();
-    sgemm(s, n, MLP_H, MLP_OUT, dout, MLP_OUT, 0, P + OFF_W4, MLP_H, 0, 0.f, d0, MLP_H);
-    // layers 3, 2, 1 (GELU)
-    const int offW[3] = {OFF_W3, OFF_W2, OFF_W1}, offB[3] = {OFF_B3, OFF_B2, OFF_B1};
-    for (int l = 2; l >= 0; --l) {
-        const int k = 2 - l;
-        k_gelu_back<<<nblk((long long)L, 256), 256, 0, s>>>(n, MLP_H, Z + l * L, d0);
+    const bool al = aligned16({X, params, Z, A, dout, grads, dA});
+    {   // layer 4 (linear): at least 64 rows a chunk (MLP_LAST / 64 < 8.1 floats a row)
+        const int chunk = n > 64 * 304 ? (n + 303) / 304 : 64, nc = nblk(n, chunk);
+        float* part = nc > 1 ? d1 : G + OFF_W4;
+        k_mlp_last_grad<<<nc, MLP_THREADS, 0, s>>>(n, chunk, dout, P + OFF_W4, A + 2 * L, Z + 2 * L, d0, part, al);
         FIPC_LAUNCHED();
-        const float* in = l > 0 ? A + (l - 1) * L : X;
-        const int din = l > 0 ? MLP_H : MLP_IN;
-        sgemm(s, MLP_H, din, n, d0, MLP_H, 1, in, din, 0, 0.f, G + offW[k], din);
-        k_bias_grad<<<MLP_H, 256, 0, s>>>(n, MLP_H, d0, G + offB[k]);
-        FIPC_LAUNCHED();
+        if (nc > 1) {
+            k_mlp_sum_chunks<<<nblk(MLP_LAST, 32), 32, 0, s>>>(nc, MLP_LAST, part, G + OFF_W4);
+            FIPC_LAUNCHED();
+        }
+    }
+    const int R = tile_rows(n);
+    for (int l = 2; l >= 0; --l) {   // layers 3, 2, 1
+        const int offW = l == 2 ? OFF_W3 : (l == 1 ? OFF_W2 : OFF_W1);
+        if (l > 0) weight_grad<MLP_H>(n, d0, A + (l - 1) * L, d1, G + offW, al, s);
+        else weight_grad<MLP_IN>(n, d0, X, d1, G + offW, al, s);
         if (l > 0) {
-            sgemm(s, n, MLP_H, MLP_H, d0, MLP_H, 0, P + offW[k], MLP_H, 0, 0.f, d1, MLP_H);
+            const float* Zl = Z + (l - 1) * L;
+            const int st = R == 128 ? launch_data_grad<128>(n, d0, P + offW, Zl, d1, al, s)
+                                    : (R == 64 ? launch_data_grad<64>(n, d0, P + offW, Zl, d1, al, s) : launch_data_grad<32>(n, d0, P + offW, Zl, d1, al, s));
+            if (st) return st;
             float* t = d0;
             d0 = d1;
             d1 = t;
