@@ -33,8 +33,7 @@ int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_
 int contact_reduce(fipc_ctx* c, const TypeTable& tt, int nrows, long long nent, cudaStream_t s);
 int assemble_elastic(fipc_ctx* c, cudaStream_t s);
 int cs_offsets(fipc_ctx* c, const double* x, cudaStream_t s);
-int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* diag_pos, double rtol, int maxit, double* sol, int* iters,
-              cudaStream_t s);
+int pcg_solve(fipc_ctx* c, const unsigned char* fixed, int guess, double rtol, int maxit, double* sol, int* iters, cudaStream_t s);
 
 // The reference's local loops run until the step is small.  A row whose Hessian (unprojected,
 // as the reference takes it) is indefinite gets a huge regularised step that the halving cuts
@@ -580,7 +579,7 @@ int fipc_admm_global(fipc_ctx* c, const double* xtilde, const double* W, const d
         if (st) return st;
     }
     FIPC_CUDA(cudaGetLastError());
-    return pcg_solve(c, fixed, nullptr, rtol, maxit, x, iters_h, s);
+    return pcg_solve(c, fixed, 1, rtol, maxit, x, iters_h, s);
 }
 
 int fipc_admm_local(fipc_ctx* c, const double* x, const double* W, double* z, const double* u, double* y, const double* r,

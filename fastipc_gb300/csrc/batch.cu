@@ -258,14 +258,13 @@ __global__ void __launch_bounds__(TR) k_bpcg_start(BPCG a, const double* __restr
             if (i < a.voff[sr + 1]) a.m.x[3 * i] = a.m.x[3 * i + 1] = a.m.x[3 * i + 2] = 0.0;
             continue;
         }
-        double rr = 0.0, bb = 0.0;
+        double rr = 0.0, bb = 0.0, y0, y1, y2;
+        row_apply<3>(a.m, i, i < a.voff[s + 1], a.m.x, y0, y1, y2);
         if (i < a.voff[s + 1]) {
             double Mi[9];
             const bool fx = a.m.fixed[i] != 0;
             jacobi_block_inverse(a.m, i, fx, Mi);
             for (int k = 0; k < 9; ++k) a.m.minv[9 * (size_t)i + k] = Mi[k];
-            double y0, y1, y2;
-            row_apply<3>(a.m, i, a.m.x, y0, y1, y2);
             const double r0 = fx ? 0.0 : rhs[3 * i] - y0, r1 = fx ? 0.0 : rhs[3 * i + 1] - y1, r2 = fx ? 0.0 : rhs[3 * i + 2] - y2;
             a.m.r[3 * i] = r0;
             a.m.r[3 * i + 1] = r1;
@@ -306,10 +305,9 @@ __global__ void __launch_bounds__(TR) k_bpcg_spmv(BPCG a) {
         const int s = a.dry ? a.tile_scene[t] : tile_scene_live<TR>(a, t);
         if (s < 0) continue;
         const int i = a.tile_row0[t] + threadIdx.x;
-        double g = 0.0, dl = 0.0, rr = 0.0;
+        double g = 0.0, dl = 0.0, rr = 0.0, y0, y1, y2;
+        row_apply<4>(a.m, i, i < a.voff[s + 1] && !a.m.fixed[i], a.m.u, y0, y1, y2);
         if (i < a.voff[s + 1]) {
-            double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-            if (!a.m.fixed[i]) row_apply<4>(a.m, i, a.m.u, y0, y1, y2);
             a.m.w[3 * i] = y0;
             a.m.w[3 * i + 1] = y1;
             a.m.w[3 * i + 2] = y2;

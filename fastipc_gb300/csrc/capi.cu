@@ -18,8 +18,7 @@ int ensure_row_capacity(fipc_ctx* c, int cap);
 int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, cudaStream_t s);
 int check_collision(fipc_ctx* c, const double* x, int* hit_h, cudaStream_t s);
 int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t s);
-int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* diag_pos, double rtol, int maxit, double* sol, int* iters,
-              cudaStream_t s);
+int pcg_solve(fipc_ctx* c, const unsigned char* fixed, int guess, double rtol, int maxit, double* sol, int* iters, cudaStream_t s);
 int sell_to_bsr(fipc_ctx* c, double* out, cudaStream_t s);
 int launch_energy(const fipc_ctx* c, const double* x, const double* xt, const int* const* rows, const int* counts, double* part,
                   double* out, cudaStream_t s);
@@ -434,7 +433,7 @@ int fipc_solve_system(fipc_ctx* c, const unsigned char* fixed, double rtol, int 
                       void* stream) {
     if (!c || !fixed || !sol || maxit <= 0 || !(rtol >= 0)) return FIPC_ERR_ARGUMENT;
     if (!use_guess) FIPC_CUDA(cudaMemsetAsync(sol, 0, sizeof(double) * 3ull * c->nV, (cudaStream_t)stream));
-    return pcg_solve(c, fixed, c->diag_pos, rtol, maxit, sol, iters_h, (cudaStream_t)stream);
+    return pcg_solve(c, fixed, use_guess != 0, rtol, maxit, sol, iters_h, (cudaStream_t)stream);
 }
 
 int fipc_output_residual(fipc_ctx* c, const double* sol, double* res_h, void* stream) {

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "ctx.cuh"
+#include "mg_node.cuh"
 #include "mg_plan.h"
 #include "pcg.cuh"
 
@@ -321,11 +322,10 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_power0(PCGArgs a, const doubl
                                                           double* __restrict__ vout, double* __restrict__ part) {
     __shared__ double sh[MG_THREADS];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double s = 0.0;
+    double s = 0.0, y[3];
+    row_apply<4>(a, i, i < a.nV && !a.fixed[i], vin, y[0], y[1], y[2]);
     if (i < a.nV) {
-        double y[3] = {0.0, 0.0, 0.0};
         if (!a.fixed[i]) {
-            row_apply<4>(a, i, vin, y[0], y[1], y[2]);
             const double sc = 1.0 / nrm[0];
             for (int k = 0; k < 3; ++k) y[k] *= sc;
         }
@@ -345,42 +345,6 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_power0(PCGArgs a, const doubl
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// y_p = (A v)_{I,p} at level >= 1 (both patterns), one warp per node: lane = 6 kk + p (kk < 5;
-// lanes 30, 31 idle) takes output p of the row's blocks kk, kk + 5, ...; the five partial sums of
-// each output are added in a fixed order.  Every lane returns y for its p = lane % 6.
-__device__ __forceinline__ double mg_row_warp(const MgLev& L, int I, const double* __restrict__ v, int lane) {
-    const int kk = lane / 6, p = lane % 6;
-    double y = 0.0;
-    if (lane < 30) {
-        for (int pass = 0; pass < 2; ++pass) {
-            const int* rp = pass ? L.c_rp : L.s_rp;
-            if (!rp) continue;
-            const int* ci = pass ? L.c_ci : L.s_ci;
-            const double* val = pass ? L.c_val : L.s_val;
-            for (int k = rp[I] + kk; k < rp[I + 1]; k += 5) {
-                const double* B = val + 36 * (size_t)k + 6 * p;
-                const double* x = v + 6 * (size_t)ci[k];
-#pragma unroll
-                for (int q = 0; q < 6; ++q) y = fma(__ldg(B + q), x[q], y);
-            }
-        }
-    }
-    const unsigned full = 0xffffffffu;
-    const double y1 = __shfl_sync(full, y, p + 6), y2 = __shfl_sync(full, y, p + 12), y3 = __shfl_sync(full, y, p + 18),
-                 y4 = __shfl_sync(full, y, p + 24);
-    const double y0 = __shfl_sync(full, y, p);
-    return ((y0 + y1) + (y2 + y3)) + y4;
-}
-
-// z_p = w sum_q M_pq s_q for the lane's p, with s_q held by lane q (q < 6)
-__device__ __forceinline__ double mg_minv_warp(const double* __restrict__ M, double s, double w, int lane) {
-    const int p = lane % 6;
-    double z = 0.0;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) z = fma(__ldg(M + 6 * p + q), __shfl_sync(0xffffffffu, s, q), z);
-    return w * z;
-}
-
 // level l >= 1: vout = D_l^-1 A_l (vin / |vin|), one warp per node
 __global__ void __launch_bounds__(MG_THREADS) k_mg_powerl(MgLev L, const double* __restrict__ vin, const double* __restrict__ nrm,
                                                           double* __restrict__ vout, double* __restrict__ part) {
@@ -388,8 +352,15 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_powerl(MgLev L, const double*
     const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     double s = 0.0;
     if (I < L.n) {
-        const double y = mg_row_warp(L, I, vin, lane) * (1.0 / nrm[0]);
-        const double z = mg_minv_warp(L.minv + 36 * (size_t)I, y, 1.0, lane);
+        double y = 0.0;
+        if (lane < 30) {
+            NodeCursor<2> c;
+            c.open(L, I, lane / 6, 5);
+            y = node_row<false>(L, c, vin, lane % 6, 5);
+        }
+        __syncwarp();
+        y = node_gather(y, lane % 6) * (1.0 / nrm[0]);
+        const double z = node_minv(L.minv + 36 * (size_t)I, y, 1.0, 0, lane % 6);
         if (lane < 6) {
             vout[6 * (size_t)I + lane] = z;
             s = z * z;
@@ -436,10 +407,10 @@ __global__ void k_mg_to_f32(long long n, const double* __restrict__ in, float* _
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_res0(PCGArgs a, const double* __restrict__ z0, double* __restrict__ t0) {
     if (*(volatile int*)&a.flag[0]) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool fx = i < a.nV && a.fixed[i];
+    double y0, y1, y2;
+    row_apply<4>(a, i, i < a.nV && !fx, z0, y0, y1, y2);
     if (i >= a.nV) return;
-    double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-    const bool fx = a.fixed[i];
-    if (!fx) row_apply<4>(a, i, z0, y0, y1, y2);
     t0[3 * (size_t)i] = fx ? 0.0 : a.r[3 * (size_t)i] - y0;
     t0[3 * (size_t)i + 1] = fx ? 0.0 : a.r[3 * (size_t)i + 1] - y1;
     t0[3 * (size_t)i + 2] = fx ? 0.0 : a.r[3 * (size_t)i + 2] - y2;
@@ -450,73 +421,92 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_res0_f32(PCGArgs a, const fl
                                                              const float4* __restrict__ z0f, double* __restrict__ t0) {
     if (*(volatile int*)&a.flag[0]) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool fx = i < a.nV && a.fixed[i];
+    float y0, y1, y2;
+    row_apply_f32(a, v32, c32, i, i < a.nV && !fx, z0f, y0, y1, y2);
     if (i >= a.nV) return;
-    float y0 = 0.f, y1 = 0.f, y2 = 0.f;
-    const bool fx = a.fixed[i];
-    if (!fx) row_apply_f32(a, v32, c32, i, z0f, y0, y1, y2);
     t0[3 * (size_t)i] = fx ? 0.0 : a.r[3 * (size_t)i] - (double)y0;
     t0[3 * (size_t)i + 1] = fx ? 0.0 : a.r[3 * (size_t)i + 1] - (double)y1;
     t0[3 * (size_t)i + 2] = fx ? 0.0 : a.r[3 * (size_t)i + 2] - (double)y2;
 }
 
 // restriction of the finer residual t (vertices: stride 3, Dirichlet vertices skipped; nodes:
-// stride 6) into level L, one warp per node: lanes take members lane, lane + 32, ... and the six
-// sums are added by a fixed shuffle tree; below the coarsest also z = w D^-1 g
+// stride 6) into level L; below the coarsest also z = w D^-1 g.  Eight lanes per node take its
+// members in turn, and the six sums are added by the halving exchange of reduce8: FP64 issue binds
+// (a warp-wide FP64 instruction takes an SM's pipe for some 19 clocks whatever its active lanes), and
+// a warp per node spent 30 adds on a node's sums alone.  960k-tet bar, the three restrictions of a
+// cycle: 39 us before, 26 us (ncu).
 __global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(PCGArgs a, MgLev L, const double* __restrict__ t, int from_vertices,
                                                             const double* __restrict__ omega, int coarsest) {
     if (*(volatile int*)&a.flag[0]) return;
-    const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (I >= L.n) return;
-    double g[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x, I = gt >> 3, sub = gt & 7;
+    if ((gt >> 5) * 4 >= L.n) return;   // the whole warp is past the last node
+    double g[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     const int st = from_vertices ? 3 : 6;
-    for (int k = L.mem_ptr[I] + lane; k < L.mem_ptr[I + 1]; k += 32) {
-        const int i = L.mem[k];
-        if (from_vertices && a.fixed[i]) continue;
-        const double t0 = t[(size_t)st * i], t1 = t[(size_t)st * i + 1], t2 = t[(size_t)st * i + 2];
-        const double d0 = L.d[3 * (size_t)i], d1 = L.d[3 * (size_t)i + 1], d2 = L.d[3 * (size_t)i + 2];
-        g[0] += t0;
-        g[1] += t1;
-        g[2] += t2;
-        g[3] += d1 * t2 - d2 * t1;
-        g[4] += d2 * t0 - d0 * t2;
-        g[5] += d0 * t1 - d1 * t0;
-        if (!from_vertices) {
-            g[3] += t[6 * (size_t)i + 3];
-            g[4] += t[6 * (size_t)i + 4];
-            g[5] += t[6 * (size_t)i + 5];
+    if (I < L.n) {
+#pragma unroll 2
+        for (int k = L.mem_ptr[I] + sub; k < L.mem_ptr[I + 1]; k += 8) {
+            const int i = L.mem[k];
+            if (from_vertices && a.fixed[i]) continue;
+            const double t0 = t[(size_t)st * i], t1 = t[(size_t)st * i + 1], t2 = t[(size_t)st * i + 2];
+            const double d0 = L.d[3 * (size_t)i], d1 = L.d[3 * (size_t)i + 1], d2 = L.d[3 * (size_t)i + 2];
+            g[0] += t0;
+            g[1] += t1;
+            g[2] += t2;
+            if (!from_vertices) {
+                g[3] += t[6 * (size_t)i + 3];
+                g[4] += t[6 * (size_t)i + 4];
+                g[5] += t[6 * (size_t)i + 5];
+            }
+            g[3] = fma(d1, t2, fma(-d2, t1, g[3]));
+            g[4] = fma(d2, t0, fma(-d0, t2, g[4]));
+            g[5] = fma(d0, t1, fma(-d1, t0, g[5]));
         }
     }
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) g[q] += __shfl_down_sync(0xffffffffu, g[q], o);
-        g[q] = __shfl_sync(0xffffffffu, g[q], 0);
-    }
-    const int p = lane % 6;
-    double gp = g[0];
-#pragma unroll
-    for (int q = 1; q < 6; ++q)
-        if (p == q) gp = g[q];
-    if (lane < 6) L.g[6 * (size_t)I + lane] = gp;
+    __syncwarp();
+    const double gp = reduce8(g, sub);
+    const bool live = I < L.n && sub < 6;
+    if (live) L.g[6 * (size_t)I + sub] = gp;
     if (!coarsest) {
-        const double z = mg_minv_warp(L.minv + 36 * (size_t)I, gp, omega[0], lane);
-        if (lane < 6) L.z[6 * (size_t)I + lane] = z;
+        const int p = sub < 6 ? sub : 0;
+        const double z = node_minv(L.minv + 36 * (size_t)(I < L.n ? I : 0), gp, omega[0], threadIdx.x & 24, p);
+        if (live) L.z[6 * (size_t)I + sub] = z;
     }
 }
 
-// level >= 1, one warp per node: post = 0: t = g - A z;  post = 1: z2 = z + w D^-1 (g - A z)
-__global__ void __launch_bounds__(MG_THREADS) k_mg_smooth(PCGArgs a, MgLev L, const double* __restrict__ omega, int post) {
+// level >= 1: POST = false: t = g - A z;  POST = true: z2 = z + w D^-1 (g - A z).  One node per warp,
+// or (FIVE) five: lane = 6 n + p takes output p of node n's whole row, a third fewer FP64
+// instructions per node; taken for levels with enough nodes to fill the GPU with such warps.
+template <bool POST, bool FIVE>
+__global__ void __launch_bounds__(MG_THREADS) k_mg_smooth(PCGArgs a, MgLev L, const double* __restrict__ omega) {
     if (*(volatile int*)&a.flag[0]) return;
-    const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (I >= L.n) return;
-    const int p = lane % 6;
-    const double r = L.g[6 * (size_t)I + p] - mg_row_warp(L, I, L.z, lane);
-    if (!post) {
-        if (lane < 6) L.t[6 * (size_t)I + lane] = r;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, p = lane % 6;
+    const int n = FIVE ? lane / 6 : 0, I = FIVE ? 5 * w + n : w;
+    if ((FIVE ? 5 * w : w) >= L.n) return;
+    const bool live = FIVE ? n < 5 && I < L.n : lane < 6;
+    double y = 0.0;
+    if (FIVE ? live : lane < 30) {
+        NodeCursor<FIVE ? 4 : 2> c;
+        c.open(L, I, FIVE ? 0 : lane / 6, FIVE ? 1 : 5);
+        y = node_row<false>(L, c, L.z, p, FIVE ? 1 : 5);
+    }
+    __syncwarp();
+    if (!FIVE) y = node_gather(y, p);
+    const int J = FIVE ? (live ? I : 0) : I;
+    const double r = L.g[6 * (size_t)J + p] - y;
+    if (!POST) {
+        if (live) L.t[6 * (size_t)I + p] = r;
         return;
     }
-    const double z = mg_minv_warp(L.minv + 36 * (size_t)I, r, omega[0], lane);
-    if (lane < 6) L.z2[6 * (size_t)I + lane] = L.z[6 * (size_t)I + lane] + z;
+    const double z = node_minv(L.minv + 36 * (size_t)J, r, omega[0], FIVE ? 6 * (n < 5 ? n : 0) : 0, p);
+    if (live) L.z2[6 * (size_t)I + p] = L.z[6 * (size_t)I + p] + z;
+}
+constexpr int MG_FIVE_MIN = 2432;   // nodes from which five share a warp
+
+template <bool POST>
+static void launch_smooth(const PCGArgs& a, const MgLev& L, const double* omega, cudaStream_t s) {
+    if (L.n >= MG_FIVE_MIN) k_mg_smooth<POST, true><<<nblk_m(32ll * ((L.n + 4) / 5), MG_THREADS), MG_THREADS, 0, s>>>(a, L, omega);
+    else k_mg_smooth<POST, false><<<nblk_m(32ll * L.n, MG_THREADS), MG_THREADS, 0, s>>>(a, L, omega);
 }
 
 // coarsest: z = D^-1 g (dense, row stride ld), one warp per row, fixed-order lane sums and
@@ -569,13 +559,14 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_prolong(PCGArgs a, MgLev L, c
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_post0(PCGArgs a, const double* __restrict__ z0, const double* __restrict__ omega) {
     if (*(volatile int*)&a.flag[0]) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool fx = i < a.nV && a.fixed[i];
+    double y0, y1, y2;
+    row_apply<4>(a, i, i < a.nV && !fx, z0, y0, y1, y2);
     if (i >= a.nV) return;
-    if (a.fixed[i]) {
+    if (fx) {
         a.u[4 * (size_t)i] = a.u[4 * (size_t)i + 1] = a.u[4 * (size_t)i + 2] = 0.0;
         return;
     }
-    double y0, y1, y2;
-    row_apply<4>(a, i, z0, y0, y1, y2);
     const double s0 = a.r[3 * (size_t)i] - y0, s1 = a.r[3 * (size_t)i + 1] - y1, s2 = a.r[3 * (size_t)i + 2] - y2;
     const double* M = a.minv + 9 * (size_t)i;
     const double w = omega[0];
@@ -590,13 +581,14 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_post0_f32(PCGArgs a, const f
                                                               const double* __restrict__ omega) {
     if (*(volatile int*)&a.flag[0]) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool fx = i < a.nV && a.fixed[i];
+    float y0, y1, y2;
+    row_apply_f32(a, v32, c32, i, i < a.nV && !fx, z0f, y0, y1, y2);
     if (i >= a.nV) return;
-    if (a.fixed[i]) {
+    if (fx) {
         a.u[4 * (size_t)i] = a.u[4 * (size_t)i + 1] = a.u[4 * (size_t)i + 2] = 0.0;
         return;
     }
-    float y0, y1, y2;
-    row_apply_f32(a, v32, c32, i, z0f, y0, y1, y2);
     const double s0 = a.r[3 * (size_t)i] - (double)y0, s1 = a.r[3 * (size_t)i + 1] - (double)y1, s2 = a.r[3 * (size_t)i + 2] - (double)y2;
     const double* M = a.minv + 9 * (size_t)i;
     const double w = omega[0];
@@ -718,10 +710,12 @@ int mg_prepare(fipc_ctx* c, const unsigned char* fixed, PCGArgs& a, cudaStream_t
     // contact patterns of every level
     if (c->c_nnzb > 0) {
         std::vector<int> crp(nV + 1), cci(c->c_nnzb);
+        std::vector<unsigned char> fx(nV);
+        FIPC_CUDA(cudaMemcpyAsync(fx.data(), fixed, nV, cudaMemcpyDeviceToHost, s));
         FIPC_CUDA(cudaMemcpyAsync(crp.data(), c->c_rowptr.p, 4ll * (nV + 1), cudaMemcpyDeviceToHost, s));
         FIPC_CUDA(cudaMemcpyAsync(cci.data(), c->c_col.p, 4ll * c->c_nnzb, cudaMemcpyDeviceToHost, s));
         FIPC_CUDA(cudaStreamSynchronize(s));
-        mg_contact(M->plan, nV, crp.data(), cci.data());
+        mg_contact(M->plan, nV, crp.data(), cci.data(), fx.data());
         M->contact_empty = false;
         for (int l = 1; l < NL; ++l) {
             const MgPattern& C = M->plan.L[l].C;
@@ -850,6 +844,19 @@ int mg_prepare(fipc_ctx* c, const unsigned char* fixed, PCGArgs& a, cudaStream_t
     return FIPC_OK;
 }
 
+// the V-cycle's arguments for the solve that mg_prepare set up, and the power iterations' vectors
+int mg_loop_args(fipc_ctx* c, MgArgs* m, double** omega, double** pv0, double** pv1) {
+    MgState* M = state(c);
+    if (!M) return FIPC_ERR_ARGUMENT;
+    *m = M->args;
+    *omega = M->omega.as<double>();
+    for (int l = 0; l < M->plan.levels; ++l) {
+        pv0[l] = M->B[l].pv0.as<double>();
+        pv1[l] = M->B[l].pv1.as<double>();
+    }
+    return FIPC_OK;
+}
+
 // smoother weights (power iteration: level 0 needs the block-Jacobi inverse of the PCG's start
 // kernel), then z0 = w0 D^-1 r0 and the first V-cycle
 int mg_start(fipc_ctx* c, const PCGArgs& a, cudaStream_t s) {
@@ -896,9 +903,9 @@ void mg_vcycle(const fipc_ctx* c, const PCGArgs& a, cudaStream_t s) {
     else k_mg_res0<<<nb0, PCG_THREADS, 0, s>>>(a, m.z0, m.t0);
     for (int l = 1; l < NL; ++l) {
         const MgLev& L = m.L[l];
-        k_mg_restrict<<<nblk_m(32ll * L.n, MG_THREADS), MG_THREADS, 0, s>>>(a, L, l == 1 ? m.t0 : m.L[l - 1].t, l == 1, m.omega + l,
+        k_mg_restrict<<<nblk_m(8ll * L.n, MG_THREADS), MG_THREADS, 0, s>>>(a, L, l == 1 ? m.t0 : m.L[l - 1].t, l == 1, m.omega + l,
                                                                             l == NL - 1);
-        if (l < NL - 1) k_mg_smooth<<<nblk_m(32ll * L.n, MG_THREADS), MG_THREADS, 0, s>>>(a, L, m.omega + l, 0);
+        if (l < NL - 1) launch_smooth<false>(a, L, m.omega + l, s);
     }
     k_mg_coarsest<<<nblk_m(32ll * m.n_dense, MG_THREADS), MG_THREADS, 0, s>>>(a, m.L[NL - 1], m.dense, m.n_dense, m.ld_dense);
     for (int l = NL - 1; l >= 1; --l) {
@@ -906,7 +913,7 @@ void mg_vcycle(const fipc_ctx* c, const PCGArgs& a, cudaStream_t s) {
         const int nf = l == 1 ? nV : m.L[l - 1].n;
         k_mg_prolong<<<nblk_m(nf, MG_THREADS), MG_THREADS, 0, s>>>(a, L, l == NL - 1 ? L.z : L.z2, l == 1 ? m.z0 : m.L[l - 1].z, nf,
                                                                     l == 1);
-        if (l - 1 >= 1) k_mg_smooth<<<nblk_m(32ll * nf, MG_THREADS), MG_THREADS, 0, s>>>(a, m.L[l - 1], m.omega + (l - 1), 1);
+        if (l - 1 >= 1) launch_smooth<true>(a, m.L[l - 1], m.omega + (l - 1), s);
     }
     if (m.z0f) k_mg_post0_f32<<<nb0, PCG_THREADS, 0, s>>>(a, m.v32, m.c32, reinterpret_cast<const float4*>(m.z0f), m.z0, m.omega);
     else k_mg_post0<<<nb0, PCG_THREADS, 0, s>>>(a, m.z0, m.omega);

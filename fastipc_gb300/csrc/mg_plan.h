@@ -53,7 +53,9 @@ struct MgPlan {
 namespace mg_detail {
 
 // pattern of the aggregated level and its contribution lists from a finer pattern (rp, ci)
-inline void galerkin_pattern(int n_fine, const int* rp, const int* ci, const std::vector<int>& agg_of, int n_coarse, MgPattern& out) {
+// (fixed, may be null: fine rows and columns to leave out)
+inline void galerkin_pattern(int n_fine, const int* rp, const int* ci, const std::vector<int>& agg_of, int n_coarse, MgPattern& out,
+                             const unsigned char* fixed = nullptr) {
     struct E {
         long long key;
         int src, r, c;
@@ -64,6 +66,7 @@ inline void galerkin_pattern(int n_fine, const int* rp, const int* ci, const std
         for (int i = 0; i < n_fine; ++i)
             for (int k = rp[i]; k < rp[i + 1]; ++k) {
                 const int j = ci[k];
+                if (fixed && (fixed[i] || fixed[j])) continue;
                 e.push_back({(long long)agg_of[i] * n_coarse + agg_of[j], k, i, j});
             }
     std::sort(e.begin(), e.end(), [](const E& a, const E& b) { return a.key < b.key || (a.key == b.key && a.src < b.src); });
@@ -208,8 +211,10 @@ inline void mg_build(int nV, const double* x0, const int* rp, const int* ci, dou
 }
 
 // Per-level contact patterns from the system's contact block pattern (crp, cci over vertices;
-// null or empty: no contact).  Level 0's contact pattern is the system's own.
-inline void mg_contact(MgPlan& P, int nV, const int* crp, const int* cci) {
+// null or empty: no contact).  Level 0's contact pattern is the system's own.  Blocks of Dirichlet
+// vertices (fixed, may be null) contribute nothing to a coarse matrix and are left out: a ground
+// body's few nodes would otherwise couple, through zero blocks, with every node that rests on it.
+inline void mg_contact(MgPlan& P, int nV, const int* crp, const int* cci, const unsigned char* fixed = nullptr) {
     MgLevelPlan& l0 = P.L[0];
     l0.C = MgPattern();
     if (crp && crp[nV] > 0) {
@@ -221,7 +226,7 @@ inline void mg_contact(MgPlan& P, int nV, const int* crp, const int* cci) {
         MgLevelPlan& c = P.L[l];
         c.C = MgPattern();
         if (f.C.nnz() == 0) continue;
-        mg_detail::galerkin_pattern(f.n, f.C.rp.data(), f.C.ci.data(), c.agg_of, c.n, c.C);
+        mg_detail::galerkin_pattern(f.n, f.C.rp.data(), f.C.ci.data(), c.agg_of, c.n, c.C, l == 1 ? fixed : nullptr);
     }
 }
 

@@ -81,11 +81,74 @@ __device__ __forceinline__ void load_v(const double* __restrict__ v, int j, doub
     }
 }
 
-template <int ST>
-__device__ __forceinline__ void row_apply(const PCGArgs& a, int i, const double* __restrict__ v, double& y0, double& y1, double& y2) {
+// position of the r-th set bit of mask (r counts from 0)
+__device__ __forceinline__ int nth_bit(unsigned mask, int r) {
+    int pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const int c = __popc((mask >> pos) & ((1u << w) - 1u));
+        if (r >= c) {
+            r -= c;
+            pos += w;
+        }
+    }
+    return pos;
+}
+
+// the contact part of y = A v for the rows of one warp (row(i) per lane, act: the lane has one), all
+// lanes together: groups of 8 lanes take one row with contact each, lane q of a group its blocks q,
+// q + 8, ..., and the group's sums go back to the row's lane.  (One lane per row waited for some 20
+// dependent loads of its row while the lanes of rows without contact idled.)
+template <class T, class LOAD>
+__device__ __forceinline__ void contact_rows(const int* __restrict__ crp, const int* __restrict__ cci, const T* __restrict__ cva, int i,
+                                             bool act, LOAD load, T& y0, T& y1, T& y2) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    const int b = act ? __ldg(crp + i) : 0, e = act ? __ldg(crp + i + 1) : 0;
+    const unsigned mask = __ballot_sync(full, e > b);
+    const int n = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u));
+    for (int r0 = 0; r0 < n; r0 += 4) {
+        const int r = r0 + (lane >> 3), row = nth_bit(mask, r < n ? r : 0);
+        const int eb = __shfl_sync(full, b, row), ee = __shfl_sync(full, e, row);
+        T s[3] = {T(0), T(0), T(0)};
+        if (r < n) {
+#pragma unroll 2
+            for (int k = eb + sub; k < ee; k += 8) {
+                const T* B = cva + 9 * (size_t)k;
+                T v0, v1, v2, m[9];
+                load(__ldg(cci + k), v0, v1, v2);
+#pragma unroll
+                for (int q = 0; q < 9; ++q) m[q] = __ldg(B + q);
+                s[0] = fma(m[0], v0, fma(m[1], v1, fma(m[2], v2, s[0])));
+                s[1] = fma(m[3], v0, fma(m[4], v1, fma(m[5], v2, s[1])));
+                s[2] = fma(m[6], v0, fma(m[7], v1, fma(m[8], v2, s[2])));
+            }
+        }
+        __syncwarp();
+        const bool mine = e > b && rank >= r0 && rank < r0 + 4;
+        const int src = mine ? 8 * (rank - r0) : lane;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s[c] += __shfl_xor_sync(full, s[c], o);
+            s[c] = __shfl_sync(full, s[c], src);
+        }
+        if (mine) {
+            y0 += s[0];
+            y1 += s[1];
+            y2 += s[2];
+        }
+    }
+}
+
+// act: the lane has a row; all lanes of a warp call.  WIDE: contact blocks by groups of lanes, else each
+// row's by its own lane in order (scenes below 1000 vertices, where a warp's rows hold few of them)
+template <int ST, bool WIDE = true>
+__device__ __forceinline__ void row_apply(const PCGArgs& a, int i, bool act, const double* __restrict__ v, double& y0, double& y1,
+                                          double& y2) {
     y0 = y1 = y2 = 0.0;
     const int sl = i >> 5, lane = i & 31;
-    const int base = a.soff[sl], len = a.rlen[i];
+    const int base = act ? a.soff[sl] : 0, len = act ? a.rlen[i] : 0;
     int k = 0;
     // two blocks per trip: their index, value and vector loads are independent
     for (; k + 1 < len; k += 2) {
@@ -120,24 +183,31 @@ __device__ __forceinline__ void row_apply(const PCGArgs& a, int i, const double*
         y1 = fma(__ldg(B + 96), p0, fma(__ldg(B + 128), p1, fma(__ldg(B + 160), p2, y1)));
         y2 = fma(__ldg(B + 192), p0, fma(__ldg(B + 224), p1, fma(__ldg(B + 256), p2, y2)));
     }
-    for (int e = a.crp[i]; e < a.crp[i + 1]; ++e) {
-        const int j = a.cci[e];
-        const double* B = a.cva + 9 * (size_t)e;
-        double v0, v1, v2;
-        load_v<ST>(v, j, v0, v1, v2);
-        y0 = fma(B[0], v0, fma(B[1], v1, fma(B[2], v2, y0)));
-        y1 = fma(B[3], v0, fma(B[4], v1, fma(B[5], v2, y1)));
-        y2 = fma(B[6], v0, fma(B[7], v1, fma(B[8], v2, y2)));
+    if (!WIDE) {
+        if (act)
+            for (int e = a.crp[i]; e < a.crp[i + 1]; ++e) {
+                const int j = a.cci[e];
+                const double* B = a.cva + 9 * (size_t)e;
+                double v0, v1, v2;
+                load_v<ST>(v, j, v0, v1, v2);
+                y0 = fma(B[0], v0, fma(B[1], v1, fma(B[2], v2, y0)));
+                y1 = fma(B[3], v0, fma(B[4], v1, fma(B[5], v2, y1)));
+                y2 = fma(B[6], v0, fma(B[7], v1, fma(B[8], v2, y2)));
+            }
+        return;
     }
+    __syncwarp();
+    contact_rows<double>(a.crp, a.cci, a.cva, i, act, [&](int j, double& v0, double& v1, double& v2) { load_v<ST>(v, j, v0, v1, v2); },
+                         y0, y1, y2);
 }
 
 // y = A v with FP32 copies of the values (v32: the sliced-ELL layout of sval; c32: the contact
 // blocks) and an FP32 vector (stride 4), accumulated in FP32: the multigrid's smoothing products
 __device__ __forceinline__ void row_apply_f32(const PCGArgs& a, const float* __restrict__ v32, const float* __restrict__ c32, int i,
-                                              const float4* __restrict__ v, float& y0, float& y1, float& y2) {
+                                              bool act, const float4* __restrict__ v, float& y0, float& y1, float& y2) {
     y0 = y1 = y2 = 0.f;
     const int sl = i >> 5, lane = i & 31;
-    const int base = a.soff[sl], len = a.rlen[i];
+    const int base = act ? a.soff[sl] : 0, len = act ? a.rlen[i] : 0;
     int k = 0;
     for (; k + 1 < len; k += 2) {
         const size_t s0 = (size_t)(base + k), s1 = s0 + 1;
@@ -167,13 +237,13 @@ __device__ __forceinline__ void row_apply_f32(const PCGArgs& a, const float* __r
         y1 = fmaf(__ldg(B + 96), p.x, fmaf(__ldg(B + 128), p.y, fmaf(__ldg(B + 160), p.z, y1)));
         y2 = fmaf(__ldg(B + 192), p.x, fmaf(__ldg(B + 224), p.y, fmaf(__ldg(B + 256), p.z, y2)));
     }
-    for (int e = a.crp[i]; e < a.crp[i + 1]; ++e) {
-        const float* B = c32 + 9 * (size_t)e;
-        const float4 p = __ldg(v + a.cci[e]);
-        y0 = fmaf(B[0], p.x, fmaf(B[1], p.y, fmaf(B[2], p.z, y0)));
-        y1 = fmaf(B[3], p.x, fmaf(B[4], p.y, fmaf(B[5], p.z, y1)));
-        y2 = fmaf(B[6], p.x, fmaf(B[7], p.y, fmaf(B[8], p.z, y2)));
-    }
+    __syncwarp();
+    contact_rows<float>(a.crp, a.cci, c32, i, act, [&](int j, float& v0, float& v1, float& v2) {
+        const float4 p = __ldg(v + j);
+        v0 = p.x;
+        v1 = p.y;
+        v2 = p.z;
+    }, y0, y1, y2);
 }
 
 // block sums of NV per-thread values into the shared array out[NV] (valid in every thread on
@@ -245,9 +315,16 @@ __device__ __forceinline__ void jacobi_block_inverse(const PCGArgs& a, int i, bo
         double D[9];
         const double* E = a.sval + (size_t)(a.diag_spos[i] >> 5) * 288 + (a.diag_spos[i] & 31);
         for (int k = 0; k < 9; ++k) D[k] = E[32 * k];
-        for (int k = a.crp[i]; k < a.crp[i + 1]; ++k)
-            if (a.cci[k] == i)
-                for (int q = 0; q < 9; ++q) D[q] += a.cva[9 * (size_t)k + q];
+        // the row's contact columns ascend
+        int lo = a.crp[i], hi = a.crp[i + 1];
+        const int end = hi;
+        while (lo < hi) {
+            const int m = (lo + hi) >> 1;
+            if (a.cci[m] < i) lo = m + 1;
+            else hi = m;
+        }
+        if (lo < end && a.cci[lo] == i)
+            for (int q = 0; q < 9; ++q) D[q] += a.cva[9 * (size_t)lo + q];
         const double c00 = D[4] * D[8] - D[5] * D[7], c01 = D[5] * D[6] - D[3] * D[8], c02 = D[3] * D[7] - D[4] * D[6];
         const double id = 1.0 / (D[0] * c00 + D[1] * c01 + D[2] * c02);
         Mi[0] = c00 * id;

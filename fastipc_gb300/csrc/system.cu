@@ -217,16 +217,16 @@ __device__ __forceinline__ void final_sums(const PCGArgs& a, double (&out)[NV]) 
 }
 
 // residual of the initial guess, block-Jacobi inverse, u = M^-1 r; partials of (r,r)
+template <bool WIDE>
 __global__ void __launch_bounds__(PCG_THREADS) k_pcg_start(PCGArgs a, const double* __restrict__ rhs, double rtol, int maxit) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double rr = 0.0, bb = 0.0, r3[3] = {0.0, 0.0, 0.0};
+    double rr = 0.0, bb = 0.0, r3[3] = {0.0, 0.0, 0.0}, y0, y1, y2;
+    row_apply<3, WIDE>(a, i, i < a.nV, a.x, y0, y1, y2);
     if (i < a.nV) {
         double Mi[9];
         const bool fx = a.fixed[i] != 0;
         jacobi_block_inverse(a, i, fx, Mi);
         for (int k = 0; k < 9; ++k) a.minv[9 * (size_t)i + k] = Mi[k];
-        double y0, y1, y2;
-        row_apply<3>(a, i, a.x, y0, y1, y2);
         const double r0 = fx ? 0.0 : rhs[3 * i] - y0, r1 = fx ? 0.0 : rhs[3 * i + 1] - y1, r2 = fx ? 0.0 : rhs[3 * i + 2] - y2;
         a.r[3 * i] = r0;
         a.r[3 * i + 1] = r1;
@@ -270,13 +270,13 @@ __global__ void __launch_bounds__(PCG_THREADS) k_pcg_start(PCGArgs a, const doub
 
 // iteration k (= flag[3], kept on the device so that a captured chunk of iterations replays
 // unchanged), part 1: w = A u and the dot products; the last block derives alpha, beta
+template <bool WIDE>
 __global__ void __launch_bounds__(PCG_THREADS) k_pcg_spmv(PCGArgs a) {
     if (*(volatile int*)&a.flag[0]) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double g = 0.0, dl = 0.0, rr = 0.0;
+    double g = 0.0, dl = 0.0, rr = 0.0, y0, y1, y2;
+    row_apply<4, WIDE>(a, i, i < a.nV && !a.fixed[i], a.u, y0, y1, y2);
     if (i < a.nV) {
-        double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-        if (!a.fixed[i]) row_apply<4>(a, i, a.u, y0, y1, y2);
         a.w[3 * i] = y0;
         a.w[3 * i + 1] = y1;
         a.w[3 * i + 2] = y2;
@@ -387,6 +387,13 @@ int mg_prepare(fipc_ctx* c, const unsigned char* fixed, PCGArgs& a, cudaStream_t
 int mg_start(fipc_ctx* c, const PCGArgs& a, cudaStream_t s);
 void mg_vcycle(const fipc_ctx* c, const PCGArgs& a, cudaStream_t s);
 int mg_launches_per_cycle(int levels);
+int pcg_mg_run(fipc_ctx* c, const PCGArgs& a, double rtol, int maxit, int guess, int* iters, cudaStream_t s);
+// Up to this many vertices a multigrid-preconditioned solve is one cooperative launch (pcg_mg.cu);
+// above, the kernel chain below, whose level-0 kernels fill the GPU, is faster.  Per PCG iteration,
+// chain against one launch: 46 us
+// against 29 us on 1,458 vertices, 79 / 49 us on 1,736 with 608 contact rows, 74 / 57 us on 13,832 with
+// 4,932, 69 / 63 us on 25,704 without, but 113 / 133 us on 58,089.
+constexpr int PCG_RUN_MAX_VERTICES = 32768;
 
 int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_out, cudaStream_t s);
 
@@ -511,7 +518,8 @@ int sell_to_bsr(fipc_ctx* c, double* out, cudaStream_t s) {
     return FIPC_OK;
 }
 
-// The single-scene PCG replays from one captured graph per solve: a while-loop (conditional)
+// The single-scene PCG of larger scenes, and without the multigrid preconditioner of any, replays from
+// one captured graph per solve: a while-loop (conditional)
 // node whose body holds PCG3_BODY iterations (SpMV, update, preconditioner) and a one-thread
 // kernel that keeps the loop going while the solve has not converged and another body fits the
 // iteration budget.  Convergence is decided on the device; the host launches the graph once and
@@ -527,6 +535,11 @@ __global__ void k_pcg_continue(const int* __restrict__ flag, cudaGraphConditiona
     const volatile int* f = flag;
     const bool go = f[0] == 0 && f[3] + PCG3_BODY <= f[4];
     cudaGraphSetConditional(h, go ? 1u : 0u);
+}
+
+static void launch_spmv(const PCGArgs& a, int nb, cudaStream_t s) {
+    if (a.mg) k_pcg_spmv<true><<<nb, PCG_THREADS, 0, s>>>(a);
+    else k_pcg_spmv<false><<<nb, PCG_THREADS, 0, s>>>(a);
 }
 
 // drops the captured PCG graph (its kernels hold the preconditioner's buffers)
@@ -571,7 +584,7 @@ static bool pcg3_graph(fipc_ctx* c, const PCGArgs& a) {
         const long long counted = g_launches.load();   // captured launches run (and count) at replay
         if (cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess) break;
         for (int k = 0; k < PCG3_BODY; ++k) {
-            k_pcg_spmv<<<nb, PCG_THREADS, 0, cs>>>(a);
+            launch_spmv(a, nb, cs);
             k_pcg_update<<<nb, PCG_THREADS, 0, cs>>>(a);
             if (a.mg) mg_vcycle(c, a, cs);
             else if (a.cs_blocks) cs_apply(c, a, cs);
@@ -591,10 +604,9 @@ static bool pcg3_graph(fipc_ctx* c, const PCGArgs& a) {
     return ok;
 }
 
-// solve_system (NEWTON_IPC.py:750-777) by block-Jacobi PCG; sol: device [3 nV] holding the
-// initial guess on entry (zero for the reference's semantics) and the solution on return
-int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* /*diag_pos*/, double rtol, int maxit, double* sol, int* iters,
-              cudaStream_t s) {
+// solve_system (NEWTON_IPC.py:750-777) by PCG; sol: device [3 nV] holding the initial guess on
+// entry (all zero, the reference's semantics, when guess = 0) and the solution on return
+int pcg_solve(fipc_ctx* c, const unsigned char* fixed, int guess, double rtol, int maxit, double* sol, int* iters, cudaStream_t s) {
     const long long n3 = 3ll * c->nV;
     const int nb = nblk(c->nV, PCG_THREADS);
     if (c->pcg_vec.ensure(8 * (n3 * 4 + 13ll * c->nV) + 64) || c->pcg_part.ensure(8ll * (3 * nb + SC_COUNT) + 64) || c->scal.ensure(80))
@@ -628,6 +640,9 @@ int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* /*diag_pos*/, 
     int st = c->mg ? mg_prepare(c, fixed, a, s) : cs_prepare(c, fixed, a, s);
     if (st) return st;
     if (a.mg) a.cs_blocks = 0;
+    const int pk = profile_kernel();
+    const bool timed = pk == PK_PCG_SPMV || pk == PK_PCG_UPDATE;
+    if (a.mg && c->nV <= PCG_RUN_MAX_VERTICES && !timed) return pcg_mg_run(c, a, rtol, maxit, guess, iters, s);
     // traffic model per launch: matrix blocks and column ids once (padding slots included),
     // row data, the gathered vector once, w written, r read
     const double slots = 32.0 * (double)c->n_slots, nv = (double)c->nV, cn = (double)c->c_nnzb;
@@ -635,7 +650,8 @@ int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* /*diag_pos*/, 
     const double spmv_flops = (double)(c->nnzb + c->c_nnzb) * 18.0 + nv * 18.0;
     const double upd_bytes = nv * (32.0 * 2 + 24.0 * 2 * 4 + 24.0 + 72.0);
     const double upd_flops = nv * 36.0;
-    k_pcg_start<<<nb, PCG_THREADS, 0, s>>>(a, c->rhs, rtol, maxit);
+    if (a.mg) k_pcg_start<true><<<nb, PCG_THREADS, 0, s>>>(a, c->rhs, rtol, maxit);
+    else k_pcg_start<false><<<nb, PCG_THREADS, 0, s>>>(a, c->rhs, rtol, maxit);
     FIPC_LAUNCHED();
     if (a.mg) {
         st = mg_start(c, a, s);
@@ -646,8 +662,6 @@ int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* /*diag_pos*/, 
     int h_flag[4] = {0, 0, 0, 0};
     // per-launch timing of the SpMV or the update needs plain launches; otherwise the iterations
     // replay from the captured while-loop graph, and only a remainder below the budget runs plainly
-    const int pk = profile_kernel();
-    const bool timed = pk == PK_PCG_SPMV || pk == PK_PCG_UPDATE;
     const int per_iter = a.mg ? 2 + mg_launches_per_cycle(c->mg_levels) : (a.cs_blocks ? 4 : 2);
     int k0 = 0;
     if (!timed && maxit >= PCG3_BODY && pcg3_graph(c, a)) {
@@ -664,7 +678,7 @@ int pcg_solve(fipc_ctx* c, const unsigned char* fixed, const int* /*diag_pos*/, 
         for (int k = k0; k < k1; ++k) {
             {
                 ProfScope ps(PK_PCG_SPMV, s, spmv_bytes, spmv_flops);
-                k_pcg_spmv<<<nb, PCG_THREADS, 0, s>>>(a);
+                launch_spmv(a, nb, s);
             }
             FIPC_LAUNCHED();
             {
