@@ -397,15 +397,16 @@ __global__ void k_bpcg_iters(int S, const int* __restrict__ sflag, int* __restri
 namespace fipc {
 
 int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s);
-int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, unsigned long long* slot, cudaStream_t s);
-int collision_launch(fipc_ctx* c, const double* x, int* hit, cudaStream_t s);
+int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, unsigned long long* slots,
+             cudaStream_t s);
+int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStream_t s);
 
 constexpr int BPCG_CHUNK = 32;   // iterations per captured graph
 
 static RowLists row_lists(const fipc_ctx* c) {
     RowLists rl;
     for (int t = 0; t < N_TYPES; ++t) {
-        rl.rows[t] = c->rows[t].as<int4>();
+        rl.rows[t] = (const int4*)c->list_rows(t);
         rl.n[t] = c->h_counts[t];
     }
     return rl;
@@ -753,6 +754,11 @@ int fipc_batch_create(fipc_ctx** out, int n_scenes, const int* vert_off, const i
     c->h_kappa = kap;
     c->h_inv_dx = idx;
     if (c->prim_off) cudaFree(c->prim_off);
+    for (int l = 0; l < 3; ++l) {
+        const int* o = poff.data() + l * (S + 1);
+        c->max_prims[l] = 0;
+        for (int q = 0; q < S; ++q) c->max_prims[l] = std::max(c->max_prims[l], o[q + 1] - o[q]);
+    }
     st = upload_vec(&c->v_scene, vs) | upload_vec(&c->voff_d, c->h_voff) | upload_vec(&c->toff_d, c->h_toff) |
          upload_vec(&c->s_kappa, kap) | upload_vec(&c->s_inv_dx, idx) | upload_vec(&c->s_hash_inv_dx, hidx) |
          upload_vec(&c->prim_off, poff);
@@ -802,14 +808,14 @@ int fipc_batch_step_size(fipc_ctx* c, const double* x, const double* sol, double
     cudaStream_t s = (cudaStream_t)stream;
     k_fill_f64<<<nblk(c->n_scenes, 128), 128, 0, s>>>(c->n_scenes, alpha, 1.0);
     FIPC_LAUNCHED();
-    return ccd_launch(c, x, sol, eta, inversion != 0, reinterpret_cast<unsigned long long*>(alpha), s);
+    return ccd_step(c, x, sol, eta, inversion != 0, nullptr, reinterpret_cast<unsigned long long*>(alpha), s);
 }
 
 int fipc_batch_check_collision(fipc_ctx* c, const double* x, int* hit, void* stream) {
     if (!c || c->n_scenes < 2 || !x || !hit) return FIPC_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     FIPC_CUDA(cudaMemsetAsync(hit, 0, sizeof(int) * c->n_scenes, s));
-    return collision_launch(c, x, hit, s);
+    return check_collision(c, x, nullptr, hit, s);
 }
 
 int fipc_batch_apply_sol(fipc_ctx* c, const double* xprev, const double* sol, const double* alpha, double* x, void* stream) {

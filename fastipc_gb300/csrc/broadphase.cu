@@ -1,19 +1,28 @@
-// Sort-based spatial hash and the three queries built on it: constraint finding
+// Spatial hash and the three queries built on it: constraint finding
 // (NEWTON_IPC.py:181-357), the CCD step filter (NEWTON_IPC.py:377-468) and the
 // intersection check (NEWTON_IPC.py:855-886).
 //
 // The grid keeps the reference's box conventions, with the median boundary edge as its cell.
 // The reference uses the mean; enumeration is complete for any cell size, so the lists are the
-// same.  What the reference appends to its sparse grid becomes (cell key, id) pairs,
-// radix-sorted by key; unique keys and run starts give each cell's id range, found through an
-// open-addressing table.  A candidate pair whose two cell ranges overlap in several cells is
+// same.  What the reference appends to its sparse grid goes into an open-addressing table: count the
+// entries of every occupied cell, give each cell a run of ids, fill the runs.  The order of the ids
+// in a run, and of the rows found, depends on timing; nothing that is returned does.  A candidate pair whose two cell ranges overlap in several cells is
 // examined only in the overlap's lowest cell (componentwise max of the two lower corners), so
 // every pair is tested once without a hash set.  The narrow phase applies the reference's exact
 // predicates; constraint rows are then sorted lexicographically and de-duplicated per list
 // exactly like np.unique(axis=0) (NEWTON_IPC.py:348-356).
+//
+// A call is a chain of a few kernels and one copy to the host at its end: table and row capacities are
+// kept from call to call and checked on the device; a call that outgrows them is repeated with larger
+// ones.  Measured on a GB300 against radix-sorted grids, one sort per list and a host round trip per grid:
+// constraint finding of two touching cubes (1,458 vertices) 1.16 -> 0.37 ms a call, of a pile of 180 cubes
+// 5.2 -> 1.4 ms, of the 960k-tet bar 1.37 -> 0.99 ms.
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
 
 #include "ccd.cuh"
 #include "ctx.cuh"
@@ -76,47 +85,6 @@ __device__ __forceinline__ void stored_box(int mode, int i, const int* __restric
 
 constexpr long long MAX_CELLS_PER_PRIM = 1ll << 22;
 
-__global__ void k_cell_count(int mode, int n, const int* __restrict__ prim, const double* __restrict__ x,
-                             const double* __restrict__ p, double dh, SceneGeo g, long long* __restrict__ cnt,
-                             int* __restrict__ overflow) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double inv_dx = g.idx(g.scene(prim_vertex(mode, i, prim)));
-    if (mode != 0 && mode != 2 && g.big_edge && g.big_edge[i]) {   // handled by the big-primitive pass
-        cnt[i] = 0;
-        return;
-    }
-    v3 lo, hi;
-    stored_box(mode, i, prim, x, p, dh, &lo, &hi);
-    const C3 a = cell_of(lo, inv_dx), b = cell_of(hi, inv_dx);
-    long long c = (b.x - a.x + 1) * (b.y - a.y + 1) * (b.z - a.z + 1);
-    if (!(c > 0 && c <= MAX_CELLS_PER_PRIM)) {
-        atomicOr(overflow, 1);
-        c = 0;
-    }
-    cnt[i] = c;
-}
-
-__global__ void k_cell_emit(int mode, int n, const int* __restrict__ prim, const double* __restrict__ x,
-                            const double* __restrict__ p, double dh, SceneGeo g, const long long* __restrict__ off,
-                            const long long* __restrict__ cnt, unsigned long long* __restrict__ keys, int* __restrict__ ids) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || cnt[i] == 0) return;
-    const int sc = g.scene(prim_vertex(mode, i, prim));
-    const double inv_dx = g.idx(sc);
-    v3 lo, hi;
-    stored_box(mode, i, prim, x, p, dh, &lo, &hi);
-    const C3 a = cell_of(lo, inv_dx), b = cell_of(hi, inv_dx);
-    long long o = off[i];
-    for (long long cx = a.x; cx <= b.x; ++cx)
-        for (long long cy = a.y; cy <= b.y; ++cy)
-            for (long long cz = a.z; cz <= b.z; ++cz) {
-                keys[o] = gkey(g, sc, cx, cy, cz);
-                ids[o] = i;
-                ++o;
-            }
-}
-
 // Candidate records of the stored primitives, built with the grid, so that the query kernels
 // reject most candidates without FP64 work (GB300 issues FP64 at a small fraction of its FP32
 // rate):
@@ -141,15 +109,9 @@ __device__ __forceinline__ int clamp_cell(long long c) {
     return (int)(c < -(1ll << 30) ? -(1ll << 30) : (c > (1ll << 30) ? (1ll << 30) : c));
 }
 
-__global__ void k_cand_records(int mode, int n, const int* __restrict__ prim, const double* __restrict__ x,
-                               const double* __restrict__ p, double dh, SceneGeo g, int4* __restrict__ cell,
-                               float4* __restrict__ box) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double inv_dx = g.idx(g.scene(prim_vertex(mode, i, prim)));
-    v3 lo, hi;
-    stored_box(mode, i, prim, x, p, dh, &lo, &hi);
-    const C3 c = cell_of(lo, inv_dx);
+__device__ __forceinline__ void cand_record(int mode, int i, const int* __restrict__ prim, const double* __restrict__ x,
+                                            const double* __restrict__ p, double dh, v3 lo, v3 hi, C3 c, int4* __restrict__ cell,
+                                            float4* __restrict__ box) {
     cell[i] = make_int4(clamp_cell(c.x), clamp_cell(c.y), clamp_cell(c.z), 0);
     const v3 d = mk(dh, dh, dh);
     v3 blo = lo, bhi = hi;
@@ -173,10 +135,8 @@ struct CandView {
     const float4* box;
 };
 
-// Cell lookup of a built grid: an open-addressing table (linear probing, load factor <= 1/2)
-// maps each occupied cell key to its run of ids, so a query cell costs one or two probes instead
-// of a binary search over all keys.  The table holds exactly the sorted grid's runs; which slot a
-// key lands in depends on insertion order, the run it maps to does not.
+// Cell table of a grid: open addressing with linear probing, load factor at most 1/2, so a query cell
+// costs one or two probes.  run[slot] = (first id, ids) of the slot's cell.
 constexpr unsigned long long HASH_EMPTY = ~0ull;
 __device__ __forceinline__ unsigned long long mix64(unsigned long long k) {
     k ^= k >> 33;
@@ -188,39 +148,21 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long k) {
 }
 struct GridView {
     const unsigned long long* hk;   // table keys
-    const int* hv;                  // table values: run index
+    const int2* run;
     unsigned long long mask;        // table size - 1
-    const int* us;                  // run starts
     const int* ids;                 // primitive ids by run
-    // run index of key, or -1 (at most mask + 1 probes)
-    __device__ __forceinline__ int find(unsigned long long key) const {
+    // the run of key's cell (empty when there is none; at most mask + 1 probes)
+    __device__ __forceinline__ int2 find(unsigned long long key) const {
         unsigned long long h = mix64(key) & mask;
         for (unsigned long long n = 0; n <= mask; ++n) {
             const unsigned long long k = __ldg(hk + h);
-            if (k == key) return __ldg(hv + h);
-            if (k == HASH_EMPTY) return -1;
+            if (k == key) return __ldg(run + h);
+            if (k == HASH_EMPTY) break;
             h = (h + 1) & mask;
         }
-        return -1;
+        return make_int2(0, 0);
     }
 };
-
-// insert the nu unique keys (nu read on the device); a full table is impossible at load <= 1/2
-__global__ void k_hash_insert(const unsigned long long* __restrict__ ukeys, const int* __restrict__ nu_p, unsigned long long* __restrict__ hk,
-                              int* __restrict__ hv, unsigned long long mask) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= *nu_p) return;
-    const unsigned long long key = ukeys[u];
-    unsigned long long h = mix64(key) & mask;
-    for (unsigned long long n = 0; n <= mask; ++n) {
-        const unsigned long long prev = atomicCAS(hk + h, HASH_EMPTY, key);
-        if (prev == HASH_EMPTY || prev == key) {
-            hv[h] = u;
-            return;
-        }
-        h = (h + 1) & mask;
-    }
-}
 
 // lanes per edge-edge constraint, edge-edge CCD and intersection query: a few lanes share each
 // cell's candidates.  One thread per query leaves most lanes idle in the FP64 narrow phase; a
@@ -229,24 +171,47 @@ __global__ void k_hash_insert(const unsigned long long* __restrict__ ukeys, cons
 constexpr int QG = 8;
 
 // ---------------------------------------------------------------- constraint rows
+// A row as a sort key: list (3 bits) and vertex ids (21 bits each, n_verts < 2^21), so that the order of
+// the keys is the lists' order and the lexicographic order within each.
+struct RowKey {
+    unsigned long long hi, lo;   // list, a, b;  c, d
+};
+__host__ __device__ __forceinline__ bool operator<(const RowKey& p, const RowKey& q) { return p.hi < q.hi || (p.hi == q.hi && p.lo < q.lo); }
+__host__ __device__ __forceinline__ bool operator==(const RowKey& p, const RowKey& q) { return p.hi == q.hi && p.lo == q.lo; }
+struct RowLess {
+    __device__ bool operator()(const RowKey& p, const RowKey& q) const { return p < q; }
+};
+// device counters of a call (zeroed at its start, copied to the host at its end)
+struct BroadCounters {
+    int rows[N_TYPES];          // rows of each list, sorted and unique
+    int flags;                  // FLAG_*
+    int emitted;                // rows emitted (also past the capacity)
+    int sorted;                 // rows[] holds the final counts
+    int big[2];                 // big triangles, edges
+    int work[2];                // step filter: pairs left to the exact test
+    int cursor[2];              // ids handed out to runs (points, edges)
+    unsigned long long total[2];   // grid entries (points, edges)
+    unsigned long long alpha;   // one scene's step (bits of a double)
+    int hit;                    // one scene's intersection flag
+    int pad;
+};
+enum { FLAG_ROWS = 1, FLAG_CELLS = 2, FLAG_TABLE = 4 };
 struct RowSink {
-    int4* rows[N_TYPES];
-    int* counts;   // [N_TYPES + 1]; the last entry is the overflow flag
+    RowKey* rows;
+    BroadCounters* n;
     int cap;
 };
-// Warp-aggregated emission: the lanes that reach this call together are partitioned by target
-// list; one lane of each partition reserves the partition's rows with a single atomicAdd and
-// every lane writes its row at base + its rank.  The lists are sorted and de-duplicated
-// afterwards, so the order of the rows within a list does not matter.
+// Warp-aggregated emission: the lanes that reach this call together reserve their rows with one
+// atomicAdd.  The rows are sorted and de-duplicated afterwards, so their order does not matter.
 __device__ __forceinline__ void emit(const RowSink& s, int t, int a, int b, int c, int d) {
     const cg::coalesced_group active = cg::coalesced_threads();
-    const cg::coalesced_group same = cg::labeled_partition(active, t);
     int base = 0;
-    if (same.thread_rank() == 0) base = atomicAdd(&s.counts[t], (int)same.size());
-    base = same.shfl(base, 0);
-    const int k = base + (int)same.thread_rank();
-    if (k < s.cap) s.rows[t][k] = make_int4(a, b, c, d);
-    else atomicOr(&s.counts[N_TYPES], 1);
+    if (active.thread_rank() == 0) base = atomicAdd(&s.n->emitted, (int)active.size());
+    base = active.shfl(base, 0);
+    const int k = base + (int)active.thread_rank();
+    if (k < s.cap) s.rows[k] = RowKey{((unsigned long long)t << 42) | ((unsigned long long)a << 21) | (unsigned long long)b,
+                                      ((unsigned long long)c << 21) | (unsigned long long)d};
+    else atomicOr(&s.n->flags, FLAG_ROWS);
 }
 
 // attempt_PT, NEWTON_IPC.py:181-212
@@ -302,10 +267,10 @@ __device__ void attempt_ee(const double* __restrict__ x, const double* __restric
 }
 
 // one thread per boundary triangle; points hashed with mode 0
-__global__ void __launch_bounds__(128) k_find_pt(int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
+__device__ __forceinline__ void find_pt(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
                                                  const double* __restrict__ x, double dh, double dh2, SceneGeo g,
                                                  GridView gv, CandView cv, RowSink sink) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = block * 128 + threadIdx.x;
     if (i >= nbt) return;
     if (g.big_tri && g.big_tri[i]) return;
     const int t0 = bt[3 * i], t1 = bt[3 * i + 1], t2 = bt[3 * i + 2];
@@ -319,9 +284,8 @@ __global__ void __launch_bounds__(128) k_find_pt(int nbt, const int* __restrict_
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
             for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int c = gv.find(gkey(g, sc, cx, cy, cz));
-                if (c < 0) continue;
-                for (int k = gv.us[c]; k < gv.us[c + 1]; ++k) {
+                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
+                for (int k = run.x; k < run.x + run.y; ++k) {
                     const int j = gv.ids[k];
                     const int4 pc = __ldg(cv.cell + j);
                     const C3 first = cmax(lo, C3{pc.x, pc.y, pc.z});
@@ -334,11 +298,11 @@ __global__ void __launch_bounds__(128) k_find_pt(int nbt, const int* __restrict_
 }
 
 // one thread per boundary edge (query, box +- dh); stored edges hashed with mode 1
-__global__ void __launch_bounds__(128) k_find_ee(int nbe, const int* __restrict__ be, const double* __restrict__ x,
+__device__ __forceinline__ void find_ee(int block, int nbe, const int* __restrict__ be, const double* __restrict__ x,
                                                  const double* __restrict__ x0, double dh, double dh2, SceneGeo g,
                                                  GridView gv, CandView cv, RowSink sink) {
     // QG lanes per query edge share the candidates of each cell
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / QG, lane = threadIdx.x % QG;
+    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= nbe) return;
     if (g.big_edge && g.big_edge[i]) return;
     const int a0 = be[2 * i], a1 = be[2 * i + 1];
@@ -351,9 +315,8 @@ __global__ void __launch_bounds__(128) k_find_ee(int nbe, const int* __restrict_
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
             for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int c = gv.find(gkey(g, sc, cx, cy, cz));
-                if (c < 0) continue;
-                for (int k = gv.us[c] + lane; k < gv.us[c + 1]; k += QG) {
+                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
+                for (int k = run.x + lane; k < run.x + run.y; k += QG) {
                     const int j = gv.ids[k];
                     if (!(i < j)) continue;
                     const int4 sc4 = __ldg(cv.cell + j);
@@ -407,10 +370,10 @@ __device__ __forceinline__ void atomic_min_pos(unsigned long long* slot, double 
 }
 
 // compute_filter_3D_PT (NEWTON_IPC.py:377-406): triangles query their moving bbox
-__global__ void __launch_bounds__(128) k_ccd_pt(int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
+__device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
                                                 const double* __restrict__ x, const double* __restrict__ p, double dh, SceneGeo g,
                                                 double eta, GridView gv, CandView cv, CcdList L, unsigned long long* __restrict__ alpha) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = block * 128 + threadIdx.x;
     if (i >= nbt) return;
     if (g.big_tri && g.big_tri[i]) return;
     const int t0 = bt[3 * i], t1 = bt[3 * i + 1], t2 = bt[3 * i + 2];
@@ -426,9 +389,8 @@ __global__ void __launch_bounds__(128) k_ccd_pt(int nbt, const int* __restrict__
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
             for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int c = gv.find(gkey(g, sc, cx, cy, cz));
-                if (c < 0) continue;
-                for (int k = gv.us[c]; k < gv.us[c + 1]; ++k) {
+                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
+                for (int k = run.x; k < run.x + run.y; ++k) {
                     const int j = gv.ids[k];
                     const int4 pc = __ldg(cv.cell + j);
                     const C3 first = cmax(lo, C3{pc.x, pc.y, pc.z});
@@ -449,11 +411,11 @@ __global__ void __launch_bounds__(128) k_ccd_pt(int nbt, const int* __restrict__
 }
 
 // compute_filter_3D_EE (NEWTON_IPC.py:409-440): edges query moving bbox +- dh
-__global__ void __launch_bounds__(128) k_ccd_ee(int nbe, const int* __restrict__ be, const double* __restrict__ x,
+__device__ __forceinline__ void ccd_ee(int block, int nbe, const int* __restrict__ be, const double* __restrict__ x,
                                                 const double* __restrict__ p, double dh, SceneGeo g, double eta,
                                                 GridView gv, CandView cv, CcdList L, unsigned long long* __restrict__ alpha) {
     // QG lanes per query edge share the candidates of each cell
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / QG, lane = threadIdx.x % QG;
+    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= nbe) return;
     if (g.big_edge && g.big_edge[i]) return;
     const int a0 = be[2 * i], a1 = be[2 * i + 1];
@@ -467,9 +429,8 @@ __global__ void __launch_bounds__(128) k_ccd_ee(int nbe, const int* __restrict__
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
             for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int c = gv.find(gkey(g, sc, cx, cy, cz));
-                if (c < 0) continue;
-                for (int k = gv.us[c] + lane; k < gv.us[c + 1]; k += QG) {
+                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
+                for (int k = run.x + lane; k < run.x + run.y; k += QG) {
                     const int j = gv.ids[k];
                     if (!(i < j)) continue;
                     const int4 sc4 = __ldg(cv.cell + j);
@@ -490,30 +451,30 @@ __global__ void __launch_bounds__(128) k_ccd_ee(int nbe, const int* __restrict__
             }
 }
 
-// the exact tests of the listed pairs, one thread per pair
-__global__ void __launch_bounds__(128) k_ccd_pt_exact(const int* __restrict__ bt, const double* __restrict__ x,
-                                                      const double* __restrict__ p, double eta, CcdList L,
-                                                      unsigned long long* __restrict__ alpha) {
-    const int n = min(L.count[0], L.cap);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const CcdWork e = L.w[k];
-        const int t0 = bt[3 * e.b], t1 = bt[3 * e.b + 1], t2 = bt[3 * e.b + 2];
-        const v3 P = ld3(x, e.a), dP = ld3(p, e.a);
-        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2), dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
-        atomic_min_pos(alpha + e.slot, pt_ccd_exact(P, A, B, C, dP, dA, dB, dC, eta, e.d2, e.lb));
-    }
-}
-__global__ void __launch_bounds__(128) k_ccd_ee_exact(const int* __restrict__ be, const double* __restrict__ x,
-                                                      const double* __restrict__ p, double eta, CcdList L,
-                                                      unsigned long long* __restrict__ alpha) {
-    const int n = min(L.count[1], L.cap);
-    const CcdWork* w = L.w + L.cap;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+// the exact tests of the listed pairs, one thread per pair: the lower half of the grid takes the
+// point-triangle pairs, the upper the edge-edge pairs.  A pair's toc is at least its additive bound, so
+// one whose bound is not below the minimum so far cannot lower it and is left out.
+__global__ void __launch_bounds__(128) k_ccd_exact(const int* __restrict__ bt, const int* __restrict__ be, const double* __restrict__ x,
+                                                   const double* __restrict__ p, double eta, CcdList L,
+                                                   unsigned long long* __restrict__ alpha) {
+    const int half = gridDim.x / 2;
+    const bool pt = (int)blockIdx.x < half;
+    const int n = min(L.count[pt ? 0 : 1], L.cap);
+    const CcdWork* w = pt ? L.w : L.w + L.cap;
+    for (int k = (pt ? blockIdx.x : blockIdx.x - half) * blockDim.x + threadIdx.x; k < n; k += half * blockDim.x) {
         const CcdWork e = w[k];
-        const int a0 = be[2 * e.a], a1 = be[2 * e.a + 1], b0 = be[2 * e.b], b1 = be[2 * e.b + 1];
-        const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), B0 = ld3(x, b0), B1 = ld3(x, b1);
-        const v3 dA0 = ld3(p, a0), dA1 = ld3(p, a1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
-        atomic_min_pos(alpha + e.slot, ee_ccd_exact(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, e.d2, e.lb));
+        if (!(e.lb < __longlong_as_double((long long)*(volatile unsigned long long*)(alpha + e.slot)))) continue;
+        if (pt) {
+            const int t0 = bt[3 * e.b], t1 = bt[3 * e.b + 1], t2 = bt[3 * e.b + 2];
+            const v3 P = ld3(x, e.a), dP = ld3(p, e.a);
+            const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2), dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
+            atomic_min_pos(alpha + e.slot, pt_ccd_exact(P, A, B, C, dP, dA, dB, dC, eta, e.d2, e.lb));
+        } else {
+            const int a0 = be[2 * e.a], a1 = be[2 * e.a + 1], b0 = be[2 * e.b], b1 = be[2 * e.b + 1];
+            const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), B0 = ld3(x, b0), B1 = ld3(x, b1);
+            const v3 dA0 = ld3(p, a0), dA1 = ld3(p, a1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
+            atomic_min_pos(alpha + e.slot, ee_ccd_exact(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, e.d2, e.lb));
+        }
     }
 }
 
@@ -531,11 +492,11 @@ __global__ void __launch_bounds__(128) k_ccd_inversion(int nT, const int4* __res
 }
 
 // check_collision_3d (NEWTON_IPC.py:855-880): triangles query bbox cells, edges hashed +- dh
-__global__ void __launch_bounds__(128) k_collision(int nbt, const int* __restrict__ bt, const int* __restrict__ be,
+__device__ __forceinline__ void collision_grid(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ be,
                                                    const double* __restrict__ x, double dh, SceneGeo g,
                                                    GridView gv, CandView cv, int* __restrict__ hit) {
     // QG lanes per query triangle share the candidates of each cell
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / QG, lane = threadIdx.x % QG;
+    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= nbt) return;
     if (g.big_tri && g.big_tri[i]) return;
     const int t0 = bt[3 * i], t1 = bt[3 * i + 1], t2 = bt[3 * i + 2];
@@ -550,9 +511,8 @@ __global__ void __launch_bounds__(128) k_collision(int nbt, const int* __restric
         for (long long cy = lo.y; cy <= hi.y; ++cy)
             for (long long cz = lo.z; cz <= hi.z; ++cz) {
                 if (*(volatile int*)hit) return;
-                const int c = gv.find(gkey(g, sc, cx, cy, cz));
-                if (c < 0) continue;
-                for (int k = gv.us[c] + lane; k < gv.us[c + 1]; k += QG) {
+                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
+                for (int k = run.x + lane; k < run.x + run.y; k += QG) {
                     const int j = gv.ids[k];
                     const int4 sc4 = __ldg(cv.cell + j);
                     const C3 first = cmax(lo, C3{sc4.x, sc4.y, sc4.z});
@@ -578,13 +538,157 @@ __device__ __forceinline__ long long box_cells(v3 lo, v3 hi, double inv_dx) {
     return (b.x - a.x + 1) * (b.y - a.y + 1) * (b.z - a.z + 1);
 }
 
-// flags and compacted lists; triangle boxes as queried (static or moving bbox), edge boxes as
-// queried (static or moving bbox +- dh).  lists: [0, nbt) triangles, [nbt, nbt + nbe) edges;
-// counts[0..1] (zeroed by the caller)
-__global__ void k_big_flags(int nbt, int nbe, const int* __restrict__ bt, const int* __restrict__ be, const double* __restrict__ x,
-                            const double* __restrict__ p, double dh, SceneGeo g, unsigned char* __restrict__ tri_big,
-                            unsigned char* __restrict__ edge_big, int* __restrict__ list, int* __restrict__ counts) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// the partners of big primitive q of scene s are lists [off[s], off[s+1]) of its kind, in chunks of
+// BIG_CHUNK: CTA (chunk, y) takes that chunk of the big primitives y, y + ny, ...  (One CTA per big
+// primitive walked all its partners: on a pile of 180 cubes over a 12-triangle ground box 2 to 4 ms per
+// query; the whole queries now take 0.9 to 2.2 ms.)  A partner's FP32 box (CandView; rounded outward, so equality counts as a
+// touch) spares most of the FP64 tests.
+struct BigArgs {
+    const int *bp, *be, *bt;
+    const int* off;        // [3][S+1]: points, edges, triangles
+    int S;
+    const unsigned char *tri_big, *edge_big;
+    const int* list;       // [nbt + nbe]: triangles, then edges
+    const int* counts;     // [2]
+    int nbt, ny;
+};
+constexpr int BIG_CHUNK = 512;
+__device__ __forceinline__ bool f32_touch(float4 alo, float4 ahi, float4 blo, float4 bhi) {
+    return alo.x <= bhi.x && alo.y <= bhi.y && alo.z <= bhi.z && blo.x <= ahi.x && blo.y <= ahi.y && blo.z <= ahi.z;
+}
+// f(i, k, scene) for big primitive i (kind 0: triangle, 1: edge) and its partners k in this CTA's chunk,
+// of list `partners` (0 points, 1 edges, 2 triangles)
+template <class F>
+__device__ __forceinline__ void big_pairs(const BigArgs& b, const SceneGeo& g, int block, int kind, int partners, F f) {
+    const int chunk = block / b.ny;
+    for (int q = block % b.ny; q < b.counts[kind]; q += b.ny) {
+        const int i = b.list[(kind ? b.nbt : 0) + q];
+        const int sc = g.scene(kind ? b.be[2 * i] : b.bt[3 * i]);
+        const int* off = b.off + partners * (b.S + 1);
+        const int k0 = off[sc] + chunk * BIG_CHUNK, k1 = min(off[sc + 1], k0 + BIG_CHUNK);
+        for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) f(i, k, sc);
+    }
+}
+
+// find_constraints: big triangles against the points, big edges against the edges of their scene (a pair
+// of two big edges once, from its lower index; rows formed with the lower list index first as in the
+// grid pass)
+__device__ __forceinline__ void find_pt_big(int block, const BigArgs& b, const double* __restrict__ x, double dh, double dh2,
+                                            const SceneGeo& g, CandView cv, const RowSink& sink) {
+    const v3 d = mk(dh, dh, dh);
+    big_pairs(b, g, block, 0, 0, [&](int i, int k, int) {
+        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2];
+        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
+        if (!f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), f32_lo(vmin(vmin(A, B), C) - d), f32_hi(vmax(vmax(A, B), C) + d)))
+            return;
+        attempt_pt(x, dh, dh2, b.bp[k], t0, t1, t2, sink);
+    });
+}
+__device__ __forceinline__ void find_ee_big(int block, const BigArgs& b, const double* __restrict__ x, const double* __restrict__ x0,
+                                            double dh, double dh2, const SceneGeo& g, CandView cv, const RowSink& sink) {
+    big_pairs(b, g, block, 1, 1, [&](int i, int j, int) {
+        if (j == i || (b.edge_big[j] && j < i)) return;
+        const v3 A0 = ld3(x, b.be[2 * i]), A1 = ld3(x, b.be[2 * i + 1]);
+        if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(vmin(A0, A1)), f32_hi(vmax(A0, A1)))) return;
+        const int lo = i < j ? i : j, hi = i < j ? j : i;
+        attempt_ee(x, x0, dh, dh2, b.be[2 * lo], b.be[2 * lo + 1], b.be[2 * hi], b.be[2 * hi + 1], sink);
+    });
+}
+
+// CCD filter: big moving triangles against the points, big moving edges against the edges of their scene
+__device__ __forceinline__ void ccd_pt_big(int block, const BigArgs& b, const double* __restrict__ x, const double* __restrict__ p, double dh,
+                                           double eta, const SceneGeo& g, CandView cv, const CcdList& L, unsigned long long* __restrict__ alpha) {
+    const v3 d = mk(dh, dh, dh);
+    big_pairs(b, g, block, 0, 0, [&](int i, int k, int sc) {
+        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2], pp = b.bp[k];
+        if (pp == t0 || pp == t1 || pp == t2) return;
+        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2), dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
+        const v3 mn = vmin(vmin(vmin(A, A + dA), vmin(B, B + dB)), vmin(C, C + dC));
+        const v3 mx = vmax(vmax(vmax(A, A + dA), vmax(B, B + dB)), vmax(C, C + dC));
+        if (!f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), f32_lo(mn - d), f32_hi(mx + d))) return;
+        const v3 P = ld3(x, pp), dP = ld3(p, pp);
+        if (!pt_aabb_moving(P, A, B, C, dP, dA, dB, dC, dh)) return;
+        const double d2 = pt_dist2(P, A, B, C);
+        double lb;
+        if (!pt_needs_exact(dP, dA, dB, dC, eta, d2, &lb)) return;
+        const int slot = g.vscene ? sc : 0;
+        if (!ccd_push(L.w, L.count, L.cap, CcdWork{pp, i, slot, 0, d2, lb}))
+            atomic_min_pos(alpha + slot, pt_exact_call(P, A, B, C, dP, dA, dB, dC, eta, d2, lb));
+    });
+}
+__device__ __forceinline__ void ccd_ee_big(int block, const BigArgs& b, const double* __restrict__ x, const double* __restrict__ p, double dh,
+                                           double eta, const SceneGeo& g, CandView cv, const CcdList& L, unsigned long long* __restrict__ alpha) {
+    big_pairs(b, g, block, 1, 1, [&](int i, int j, int sc) {
+        if (j == i || (b.edge_big[j] && j < i)) return;
+        const v3 I0 = ld3(x, b.be[2 * i]), I1 = ld3(x, b.be[2 * i + 1]), dI0 = ld3(p, b.be[2 * i]), dI1 = ld3(p, b.be[2 * i + 1]);
+        const v3 mn = vmin(vmin(I0, I0 + dI0), vmin(I1, I1 + dI1)), mx = vmax(vmax(I0, I0 + dI0), vmax(I1, I1 + dI1));
+        if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(mn), f32_hi(mx))) return;
+        const int lo = i < j ? i : j, hi = i < j ? j : i;
+        const int a0 = b.be[2 * lo], a1 = b.be[2 * lo + 1], b0 = b.be[2 * hi], b1 = b.be[2 * hi + 1];
+        if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) return;
+        const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), B0 = ld3(x, b0), B1 = ld3(x, b1);
+        const v3 dA0 = ld3(p, a0), dA1 = ld3(p, a1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
+        if (!ee_aabb_moving(A0, A1, B0, B1, dA0, dA1, dB0, dB1, dh)) return;
+        const double d2 = ee_dist2(A0, A1, B0, B1);
+        double lb;
+        if (!ee_needs_exact(dA0, dA1, dB0, dB1, eta, d2, &lb)) return;
+        const int slot = g.vscene ? sc : 0;
+        if (!ccd_push(L.w + L.cap, L.count + 1, L.cap, CcdWork{lo, hi, slot, 0, d2, lb}))
+            atomic_min_pos(alpha + slot, ee_exact_call(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, d2, lb));
+    });
+}
+
+// intersection check: big triangles against the edges of their scene, big edges against the triangles of
+// their scene that are not big (kind: which)
+__device__ __forceinline__ void collision_big(int block, int kind, const BigArgs& b, const double* __restrict__ x, const SceneGeo& g, CandView cv,
+                                              int* __restrict__ hit) {
+    big_pairs(b, g, block, kind, kind ? 2 : 1, [&](int i, int k, int sc) {
+        int* h = hit + (g.vscene ? sc : 0);
+        const int e = kind ? i : k, t = kind ? k : i;
+        if (kind && b.tri_big[t]) return;
+        const int t0 = b.bt[3 * t], t1 = b.bt[3 * t + 1], t2 = b.bt[3 * t + 2], a0 = b.be[2 * e], a1 = b.be[2 * e + 1];
+        if (a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2) return;
+        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
+        if (!f32_touch(__ldg(cv.box + 2 * (size_t)e), __ldg(cv.box + 2 * (size_t)e + 1), f32_lo(vmin(vmin(A, B), C)), f32_hi(vmax(vmax(A, B), C)))) return;
+        if (*(volatile int*)h) return;
+        if (seg_tri(ld3(x, a0), ld3(x, a1), A, B, C)) atomicOr(h, 1);
+    });
+}
+
+// ---------------------------------------------------------------- building the grids
+// one grid: n stored primitives of a box mode
+struct GridBuild {
+    const int* prim;
+    int n, mode;
+    int4* cell;
+    float4* box;
+    unsigned long long* hk;
+    int* cnt;
+    int2* run;
+    int* ids;
+    unsigned long long mask;   // table size - 1; the ids hold half the table size
+};
+
+// flags and lists of the big primitives (triangle boxes as queried: static or moving; edge boxes as
+// queried: static or moving, +- dh), candidate records and entry counts of both grids' primitives, and
+// the tables cleared
+__global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict__ bt, int nbe, const int* __restrict__ be, GridBuild gp,
+                                                 GridBuild ge, const double* __restrict__ x, const double* __restrict__ p, double dh,
+                                                 SceneGeo g, unsigned char* __restrict__ tri_big, unsigned char* __restrict__ edge_big,
+                                                 int* __restrict__ list, BroadCounters* __restrict__ n) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+    if (k == 0) n->alpha = (unsigned long long)__double_as_longlong(1.0);
+    for (unsigned long long h = k; h <= gp.mask; h += nthr) {
+        gp.hk[h] = HASH_EMPTY;
+        gp.cnt[h] = 0;
+    }
+    for (unsigned long long h = k; h <= ge.mask; h += nthr) {
+        ge.hk[h] = HASH_EMPTY;
+        ge.cnt[h] = 0;
+    }
+    const v3 d = mk(dh, dh, dh);
+    long long cells = 0;   // entries of this thread's primitive
+    int which = 0;
     if (k < nbt) {
         const int t0 = bt[3 * k], t1 = bt[3 * k + 1], t2 = bt[3 * k + 2];
         v3 lo = vmin(vmin(ld3(x, t0), ld3(x, t1)), ld3(x, t2)), hi = vmax(vmax(ld3(x, t0), ld3(x, t1)), ld3(x, t2));
@@ -595,155 +699,241 @@ __global__ void k_big_flags(int nbt, int nbe, const int* __restrict__ bt, const 
         }
         const bool big = box_cells(lo, hi, g.idx(g.scene(t0))) > BIG_CELLS;
         tri_big[k] = big;
-        if (big) list[atomicAdd(&counts[0], 1)] = k;
-    } else if (k < nbt + nbe) {
-        const int e = k - nbt, a0 = be[2 * e], a1 = be[2 * e + 1];
-        v3 lo = vmin(ld3(x, a0), ld3(x, a1)), hi = vmax(ld3(x, a0), ld3(x, a1));
-        if (p) {
-            const v3 A = ld3(x, a0) + ld3(p, a0), B = ld3(x, a1) + ld3(p, a1);
-            lo = vmin(lo, vmin(A, B));
-            hi = vmax(hi, vmax(A, B));
+        if (big) list[atomicAdd(&n->big[0], 1)] = k;
+    } else if (k < nbt + nbe + gp.n) {
+        const bool edge = k < nbt + nbe;
+        const GridBuild& b = edge ? ge : gp;
+        const int i = edge ? k - nbt : k - nbt - nbe;
+        const int sv = edge ? be[2 * i] : b.prim[i];
+        const double inv_dx = g.idx(g.scene(sv));
+        bool big = false;
+        if (edge) {
+            const int a1 = be[2 * i + 1];
+            v3 lo = vmin(ld3(x, sv), ld3(x, a1)), hi = vmax(ld3(x, sv), ld3(x, a1));
+            if (p) {
+                const v3 A = ld3(x, sv) + ld3(p, sv), B = ld3(x, a1) + ld3(p, a1);
+                lo = vmin(lo, vmin(A, B));
+                hi = vmax(hi, vmax(A, B));
+            }
+            big = box_cells(lo - d, hi + d, inv_dx) > BIG_CELLS;
+            edge_big[i] = big;
+            if (big) list[nbt + atomicAdd(&n->big[1], 1)] = i;
         }
-        const v3 d = mk(dh, dh, dh);
-        const bool big = box_cells(lo - d, hi + d, g.idx(g.scene(a0))) > BIG_CELLS;
-        edge_big[e] = big;
-        if (big) list[nbt + atomicAdd(&counts[1], 1)] = e;
+        v3 lo, hi;
+        stored_box(b.mode, i, b.prim, x, p, dh, &lo, &hi);
+        const C3 a = cell_of(lo, inv_dx), e = cell_of(hi, inv_dx);
+        cand_record(b.mode, i, b.prim, x, p, dh, lo, hi, a, b.cell, b.box);
+        if (!big) {
+            cells = (e.x - a.x + 1) * (e.y - a.y + 1) * (e.z - a.z + 1);
+            if (!(cells > 0 && cells <= MAX_CELLS_PER_PRIM)) {
+                atomicOr(&n->flags, FLAG_CELLS);
+                cells = 0;
+            }
+        }
+        which = edge ? 1 : 0;
+    }
+    // totals: one add per warp and grid
+    for (int w = 0; w < 2; ++w) {
+        long long c = which == w ? cells : 0;
+        if (!__any_sync(0xffffffffu, c != 0)) continue;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&n->total[w], (unsigned long long)c);
     }
 }
 
-// partners of big primitive q of scene s: lists [off[s], off[s+1]) of its kind
-struct BigArgs {
-    const int *bp, *be, *bt;
-    const int* off;        // [3][S+1]: points, edges, triangles
-    int S;
-    const unsigned char *tri_big, *edge_big;
-    const int* list;       // [nbt + nbe]
-    const int* counts;     // [2]
-    int nbt;
+// f(key, i) for every (cell, primitive) entry of both grids; four lanes share a primitive's cells.
+// Nothing happens when a table is too small for its entries (the call is then repeated).
+constexpr int CELL_LANES = 4;
+template <class F>
+__device__ __forceinline__ void each_entry(const GridBuild& gp, const GridBuild& ge, const double* __restrict__ x, const double* __restrict__ p,
+                                           double dh, const SceneGeo& g, BroadCounters* n, F f) {
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) / CELL_LANES, lane = threadIdx.x % CELL_LANES;
+    if (2 * n->total[0] > gp.mask + 1 || 2 * n->total[1] > ge.mask + 1) {
+        if (k == 0 && lane == 0) atomicOr(&n->flags, FLAG_TABLE);
+        return;
+    }
+    if (k >= gp.n + ge.n) return;
+    const bool edge = k >= gp.n;
+    const GridBuild& b = edge ? ge : gp;
+    const int i = edge ? k - gp.n : k;
+    if (edge && g.big_edge[i]) return;   // left to the big-primitive pass
+    const int sc = g.scene(edge ? b.prim[2 * i] : b.prim[i]);
+    const double inv_dx = g.idx(sc);
+    v3 lo, hi;
+    stored_box(b.mode, i, b.prim, x, p, dh, &lo, &hi);
+    const C3 a = cell_of(lo, inv_dx), e = cell_of(hi, inv_dx);
+    const long long ny = e.y - a.y + 1, nz = e.z - a.z + 1, c = (e.x - a.x + 1) * ny * nz;
+    if (!(c > 0 && c <= MAX_CELLS_PER_PRIM)) return;
+    const int nyi = (int)ny, nzi = (int)nz;
+    for (int q = lane; q < (int)c; q += CELL_LANES) {
+        const int qz = q % nzi, qy = q / nzi % nyi, qx = q / nzi / nyi;
+        f(b, edge, gkey(g, sc, a.x + qx, a.y + qy, a.z + qz), i);
+    }
+}
+
+// the occupied cells and their entry counts (a full table is impossible at load <= 1/2)
+__global__ void __launch_bounds__(256) k_grid_insert(GridBuild gp, GridBuild ge, const double* __restrict__ x, const double* __restrict__ p,
+                                                     double dh, SceneGeo g, BroadCounters* __restrict__ n) {
+    each_entry(gp, ge, x, p, dh, g, n, [&](const GridBuild& b, bool, unsigned long long key, int) {
+        unsigned long long h = mix64(key) & b.mask;
+        for (unsigned long long q = 0; q <= b.mask; ++q) {
+            const unsigned long long prev = atomicCAS(b.hk + h, HASH_EMPTY, key);
+            if (prev == HASH_EMPTY || prev == key) {
+                atomicAdd(b.cnt + h, 1);
+                return;
+            }
+            h = (h + 1) & b.mask;
+        }
+    });
+}
+
+// a run of ids for every occupied cell: one atomicAdd per warp on the cursor
+__global__ void __launch_bounds__(256) k_grid_runs(GridBuild gp, GridBuild ge, BroadCounters* __restrict__ n) {
+    const unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const bool second = k > gp.mask;   // tables are multiples of 32 slots
+    const GridBuild& b = second ? ge : gp;
+    const unsigned long long h = second ? k - (gp.mask + 1) : k;
+    const int c = h <= b.mask ? b.cnt[h] : 0;
+    int sum = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, sum, 31);
+    if (total == 0) return;
+    int base = 0;
+    if (lane == 31) base = atomicAdd(&n->cursor[second ? 1 : 0], total);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (c) b.run[h] = make_int2(base + sum - c, 0);
+}
+
+// the ids into their cells' runs; run.y counts up to the run's length
+__global__ void __launch_bounds__(256) k_grid_fill(GridBuild gp, GridBuild ge, const double* __restrict__ x, const double* __restrict__ p,
+                                                   double dh, SceneGeo g, BroadCounters* __restrict__ n) {
+    each_entry(gp, ge, x, p, dh, g, n, [&](const GridBuild& b, bool, unsigned long long key, int i) {
+        unsigned long long h = mix64(key) & b.mask;
+        for (unsigned long long q = 0; q <= b.mask; ++q) {
+            if (b.hk[h] == key) {
+                const int k = b.run[h].x + atomicAdd(&b.run[h].y, 1);
+                b.ids[k] = i;
+                return;
+            }
+            h = (h + 1) & b.mask;
+        }
+    });
+}
+
+// ---------------------------------------------------------------- the queries' kernels
+// Each query is one launch: block ranges for its grid passes and its big-primitive passes, which so run
+// side by side.
+struct QueryBlocks {
+    int pt, ee, pt_big, ee_big;   // blocks of each pass, in this order
 };
-
-// find_constraints, big triangles against every point of their scene
-__global__ void k_find_pt_big(BigArgs b, const double* __restrict__ x, double dh, double dh2, SceneGeo g, RowSink sink) {
-    for (int q = blockIdx.x; q < b.counts[0]; q += gridDim.x) {
-        const int i = b.list[q];
-        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2];
-        const int sc = g.scene(t0);
-        for (int k = b.off[sc] + threadIdx.x; k < b.off[sc + 1]; k += blockDim.x) attempt_pt(x, dh, dh2, b.bp[k], t0, t1, t2, sink);
-    }
+__global__ void __launch_bounds__(128) k_find(QueryBlocks nb, int nbt, const int* __restrict__ bt, const int* __restrict__ bp, int nbe,
+                                              const int* __restrict__ be, const double* __restrict__ x, const double* __restrict__ x0,
+                                              double dh, double dh2, SceneGeo g, GridView gp, CandView cp, GridView ge, CandView ce, BigArgs big,
+                                              RowSink sink) {
+    int b = blockIdx.x;
+    if (b < nb.ee) return find_ee(b, nbe, be, x, x0, dh, dh2, g, ge, ce, sink);
+    if ((b -= nb.ee) < nb.pt) return find_pt(b, nbt, bt, bp, x, dh, dh2, g, gp, cp, sink);
+    if ((b -= nb.pt) < nb.pt_big) return find_pt_big(b, big, x, dh, dh2, g, cp, sink);
+    find_ee_big(b - nb.pt_big, big, x, x0, dh, dh2, g, ce, sink);
 }
-
-// find_constraints, big edges against every edge of their scene (a pair of two big edges once,
-// from its lower index); rows formed with the lower list index first as in the grid pass
-__global__ void k_find_ee_big(BigArgs b, const double* __restrict__ x, const double* __restrict__ x0, double dh, double dh2,
-                              SceneGeo g, RowSink sink) {
-    for (int q = blockIdx.x; q < b.counts[1]; q += gridDim.x) {
-        const int i = b.list[b.nbt + q];
-        const int sc = g.scene(b.be[2 * i]);
-        const int* off = b.off + (b.S + 1);
-        for (int j = off[sc] + threadIdx.x; j < off[sc + 1]; j += blockDim.x) {
-            if (j == i || (b.edge_big[j] && j < i)) continue;
-            const int lo = i < j ? i : j, hi = i < j ? j : i;
-            attempt_ee(x, x0, dh, dh2, b.be[2 * lo], b.be[2 * lo + 1], b.be[2 * hi], b.be[2 * hi + 1], sink);
-        }
-    }
+__global__ void __launch_bounds__(128) k_ccd(QueryBlocks nb, int nbt, const int* __restrict__ bt, const int* __restrict__ bp, int nbe,
+                                             const int* __restrict__ be, const double* __restrict__ x, const double* __restrict__ p, double dh,
+                                             double eta, SceneGeo g, GridView gp, CandView cp, GridView ge, CandView ce, BigArgs big, CcdList L,
+                                             unsigned long long* __restrict__ alpha) {
+    int b = blockIdx.x;
+    if (b < nb.ee) return ccd_ee(b, nbe, be, x, p, dh, g, eta, ge, ce, L, alpha);
+    if ((b -= nb.ee) < nb.pt) return ccd_pt(b, nbt, bt, bp, x, p, dh, g, eta, gp, cp, L, alpha);
+    if ((b -= nb.pt) < nb.pt_big) return ccd_pt_big(b, big, x, p, dh, eta, g, cp, L, alpha);
+    ccd_ee_big(b - nb.pt_big, big, x, p, dh, eta, g, ce, L, alpha);
 }
-
-// CCD filter, big moving triangles against every point of their scene
-__global__ void k_ccd_pt_big(BigArgs b, const double* __restrict__ x, const double* __restrict__ p, double dh, double eta, SceneGeo g,
-                             unsigned long long* __restrict__ alpha) {
-    for (int q = blockIdx.x; q < b.counts[0]; q += gridDim.x) {
-        const int i = b.list[q];
-        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2];
-        const int sc = g.scene(t0);
-        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2), dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
-        for (int k = b.off[sc] + threadIdx.x; k < b.off[sc + 1]; k += blockDim.x) {
-            const int pp = b.bp[k];
-            if (pp == t0 || pp == t1 || pp == t2) continue;
-            const v3 P = ld3(x, pp), dP = ld3(p, pp);
-            if (!pt_aabb_moving(P, A, B, C, dP, dA, dB, dC, dh)) continue;
-            const double d2 = pt_dist2(P, A, B, C);
-            atomic_min_pos(alpha + (g.vscene ? sc : 0), pt_ccd(P, A, B, C, dP, dA, dB, dC, eta, d2));
-        }
-    }
-}
-
-// CCD filter, big moving edges against every edge of their scene
-__global__ void k_ccd_ee_big(BigArgs b, const double* __restrict__ x, const double* __restrict__ p, double dh, double eta, SceneGeo g,
-                             unsigned long long* __restrict__ alpha) {
-    for (int q = blockIdx.x; q < b.counts[1]; q += gridDim.x) {
-        const int i = b.list[b.nbt + q];
-        const int sc = g.scene(b.be[2 * i]);
-        const int* off = b.off + (b.S + 1);
-        for (int j = off[sc] + threadIdx.x; j < off[sc + 1]; j += blockDim.x) {
-            if (j == i || (b.edge_big[j] && j < i)) continue;
-            const int lo = i < j ? i : j, hi = i < j ? j : i;
-            const int a0 = b.be[2 * lo], a1 = b.be[2 * lo + 1], b0 = b.be[2 * hi], b1 = b.be[2 * hi + 1];
-            if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) continue;
-            const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), B0 = ld3(x, b0), B1 = ld3(x, b1);
-            const v3 dA0 = ld3(p, a0), dA1 = ld3(p, a1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
-            if (!ee_aabb_moving(A0, A1, B0, B1, dA0, dA1, dB0, dB1, dh)) continue;
-            const double d2 = ee_dist2(A0, A1, B0, B1);
-            atomic_min_pos(alpha + (g.vscene ? sc : 0), ee_ccd(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, d2));
-        }
-    }
-}
-
-// intersection check: big triangles against every edge of their scene, big edges against every
-// triangle of their scene that is not big
-__global__ void k_collision_big(BigArgs b, const double* __restrict__ x, SceneGeo g, int* __restrict__ hit) {
-    const int nt = b.counts[0], ne = b.counts[1];
-    for (int q = blockIdx.x; q < nt + ne; q += gridDim.x) {
-        const bool tri = q < nt;
-        const int i = tri ? b.list[q] : b.list[b.nbt + q - nt];
-        const int sc = g.scene(tri ? b.bt[3 * i] : b.be[2 * i]);
-        int* h = hit + (g.vscene ? sc : 0);
-        const int* off = b.off + (tri ? 1 : 2) * (b.S + 1);
-        for (int k = off[sc] + threadIdx.x; k < off[sc + 1]; k += blockDim.x) {
-            if (*(volatile int*)h) break;
-            const int e = tri ? k : i, t = tri ? i : k;
-            if (!tri && b.tri_big[t]) continue;
-            const int t0 = b.bt[3 * t], t1 = b.bt[3 * t + 1], t2 = b.bt[3 * t + 2], a0 = b.be[2 * e], a1 = b.be[2 * e + 1];
-            if (a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2) continue;
-            if (seg_tri(ld3(x, a0), ld3(x, a1), ld3(x, t0), ld3(x, t1), ld3(x, t2))) atomicOr(h, 1);
-        }
-    }
+__global__ void __launch_bounds__(128) k_collision(QueryBlocks nb, int nbt, const int* __restrict__ bt, const int* __restrict__ be,
+                                                   const double* __restrict__ x, double dh, SceneGeo g, GridView ge, CandView ce, BigArgs big,
+                                                   int* __restrict__ hit) {
+    int b = blockIdx.x;
+    if (b < nb.pt) return collision_grid(b, nbt, bt, be, x, dh, g, ge, ce, hit);
+    if ((b -= nb.pt) < nb.pt_big) return collision_big(b, 0, big, x, g, ce, hit);
+    collision_big(b - nb.pt_big, 1, big, x, g, ce, hit);
 }
 
 // ---------------------------------------------------------------- row canonicalisation
-// width-2 / width-3 rows: one 63-bit key; width-4 rows: LSD two-pass (last index, then the
-// first three) with the stable radix sort.  21 bits per vertex index (< 2^21 vertices).
-__global__ void k_row_keys(int n, int width, int pass, const int4* __restrict__ rows, const int* __restrict__ perm,
-                           unsigned long long* __restrict__ keys, int* __restrict__ idx) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int src = perm ? perm[i] : i;
-    const int4 r = rows[src];
-    unsigned long long k;
-    if (width == 2) k = ((unsigned long long)r.x << 21) | (unsigned long long)r.y;
-    else if (width == 3 || pass == 1) k = ((unsigned long long)r.x << 42) | ((unsigned long long)r.y << 21) | (unsigned long long)r.z;
-    else k = (unsigned long long)r.w;
-    keys[i] = k;
-    idx[i] = src;
+__device__ __forceinline__ int4 row_of(RowKey k) {
+    const unsigned long long m = (1ull << 21) - 1;
+    return make_int4((int)((k.hi >> 21) & m), (int)(k.hi & m), (int)(k.lo >> 21), (int)(k.lo & m));
 }
-__global__ void k_row_gather_flag(int n, const int4* __restrict__ rows, const int* __restrict__ perm, int4* __restrict__ out,
-                                  int* __restrict__ flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int4 r = rows[perm[i]];
-    out[i] = r;
-    int f = 1;
-    if (i > 0) {
-        const int4 q = rows[perm[i - 1]];
-        f = !(q.x == r.x && q.y == r.y && q.z == r.z && q.w == r.w);
+__device__ __forceinline__ int list_of(RowKey k) { return (int)(k.hi >> 42); }
+
+// Up to SORT_SMALL rows: sorted, made unique and written out by one CTA (bitonic in shared memory)
+// right behind the queries, so that a call of a small scene needs one round trip to the host.  More
+// rows go through a merge sort after that round trip (k_rows_write).
+constexpr int SORT_SMALL = 2048, SORT_THREADS = 1024;
+__global__ void __launch_bounds__(SORT_THREADS) k_rows_small(const RowKey* __restrict__ in, BroadCounters* __restrict__ n, int4* __restrict__ out) {
+    __shared__ RowKey k[SORT_SMALL];
+    __shared__ int warp_sum[SORT_THREADS / 32], list_n[N_TYPES];
+    const int total = n->emitted, t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (n->flags || total > SORT_SMALL) return;
+    int size = 64;
+    while (size < total) size <<= 1;
+    for (int i = t; i < size; i += SORT_THREADS) k[i] = i < total ? in[i] : RowKey{~0ull, ~0ull};
+    if (t < N_TYPES) list_n[t] = 0;
+    __syncthreads();
+    for (int len = 2; len <= size; len <<= 1)
+        for (int step = len >> 1; step > 0; step >>= 1) {
+            if (t < size / 2) {
+                const int i = 2 * step * (t / step) + t % step, j = i + step;
+                const RowKey a = k[i], b = k[j];
+                if ((b < a) == ((i & len) == 0)) {
+                    k[i] = b;
+                    k[j] = a;
+                }
+            }
+            __syncthreads();
+        }
+    // thread t: elements 2t and 2t + 1
+    bool f[2] = {false, false};
+    for (int q = 0; q < 2; ++q) {
+        const int i = 2 * t + q;
+        f[q] = i < total && (i == 0 || !(k[i] == k[i - 1]));
     }
-    flag[i] = f;
+    int sum = (int)f[0] + (int)f[1];
+    const int mine = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    if (lane == 31) warp_sum[w] = sum;
+    __syncthreads();
+    int pos = sum - mine;
+    for (int q = 0; q < w; ++q) pos += warp_sum[q];
+    for (int q = 0; q < 2; ++q)
+        if (f[q]) {
+            const RowKey r = k[2 * t + q];
+            out[pos++] = row_of(r);
+            atomicAdd(&list_n[list_of(r)], 1);
+        }
+    __syncthreads();
+    if (t < N_TYPES) n->rows[t] = list_n[t];
+    if (t == 0) n->sorted = 1;
 }
-__global__ void k_row_compact(int n, const int4* __restrict__ in, const int* __restrict__ flag, const int* __restrict__ pos,
-                              int4* __restrict__ out, int* __restrict__ count) {
+// the sorted, unique keys (their number in *nu) as rows, and the lists' counts
+__global__ void __launch_bounds__(256) k_rows_write(const int* __restrict__ nu, const RowKey* __restrict__ in, BroadCounters* __restrict__ n,
+                                                    int4* __restrict__ out) {
+    __shared__ int list_n[N_TYPES];
+    if (threadIdx.x < N_TYPES) list_n[threadIdx.x] = 0;
+    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (flag[i]) out[pos[i]] = in[i];
-    if (i == n - 1) *count = pos[i] + flag[i];
+    if (i < *nu) {
+        out[i] = row_of(in[i]);
+        atomicAdd(&list_n[list_of(in[i])], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < N_TYPES && list_n[threadIdx.x]) atomicAdd(&n->rows[threadIdx.x], list_n[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------- host side
@@ -767,318 +957,243 @@ static SceneGeo geo(const fipc_ctx* c) {
     return g;
 }
 
-// flag the big triangles and edges for positions x (+ direction p when moving) and return the
-// scene lookup that carries the flags; *b gets the lists for the big-primitive kernels
-static int big_prepare(fipc_ctx* c, const double* x, const double* p, SceneGeo* g, BigArgs* b, cudaStream_t s) {
-    *g = geo(c);
-    const int n = c->nBT + c->nBE;
-    if (c->big_flags.ensure((size_t)n + 16) || c->big_list.ensure(4ll * (n + 2) + 16)) return FIPC_ERR_CUDA;
+constexpr int EXACT_BLOCKS = 8 * 304;
+
+static unsigned long long table_size(long long entries) {
+    unsigned long long size = 1024;
+    while (size < 2ull * (unsigned long long)entries) size <<= 1;
+    return size;
+}
+static int ensure_table(Grid& g, unsigned long long size) {
+    if (size <= g.size) return FIPC_OK;
+    if (g.hkeys.ensure(8 * size) || g.counts.ensure(4 * size) || g.runs.ensure(8 * size) || g.ids.ensure(2 * size)) return FIPC_ERR_CUDA;
+    g.size = size;
+    return FIPC_OK;
+}
+
+// one call's view of the scene: grids, big primitives and counters
+struct Broad {
+    SceneGeo g;
+    BigArgs big;
+    GridBuild gp, ge;
+    BroadCounters* n;
+};
+
+static GridView view(const GridBuild& b) { return GridView{b.hk, b.run, b.mask, b.ids}; }
+static CandView cands(const GridBuild& b) { return CandView{b.cell, b.box}; }
+static int big_blocks(const fipc_ctx* c, int partners, int ny) { return nblk(c->max_prims[partners], BIG_CHUNK) * ny; }
+
+// The grids over the boundary points (mode_p < 0: none) and edges at positions x (+ direction p when
+// moving), and the big primitives.  Tables start at two slots per primitive, twice over, and grow when a
+// call reports that its entries need more.
+static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode_p, int mode_e, Broad* b, cudaStream_t s) {
+    const int n = c->nBT + c->nBE, np = mode_p < 0 ? 0 : c->nBP;
+    if (c->big_flags.ensure((size_t)n + 16) || c->big_list.ensure(4ll * n + 16) || c->broad.ensure(sizeof(BroadCounters))) return FIPC_ERR_CUDA;
+    if (ensure_table(c->gp, table_size(2ll * np)) || ensure_table(c->ge, table_size(2ll * c->nBE))) return FIPC_ERR_CUDA;
+    if (c->gp.cell4.ensure(16ll * np + 16) || c->gp.box4.ensure(32ll * np + 32) || c->ge.cell4.ensure(16ll * c->nBE + 16) ||
+        c->ge.box4.ensure(32ll * c->nBE + 32))
+        return FIPC_ERR_CUDA;
     unsigned char* tri_big = c->big_flags.as<unsigned char>();
-    int* list = c->big_list.as<int>();
-    int* counts = list + n;
-    FIPC_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(int), s));
-    if (n > 0) {
-        k_big_flags<<<nblk(n, 256), 256, 0, s>>>(c->nBT, c->nBE, c->bt, c->be, x, p, c->dhat, *g, tri_big, tri_big + c->nBT, list,
-                                                 counts);
+    b->n = c->broad.as<BroadCounters>();
+    SceneGeo g = geo(c);
+    auto build = [](Grid& gr, const int* prim, int np_, int mode) {
+        return GridBuild{prim, np_, mode, gr.cell4.as<int4>(), gr.box4.as<float4>(), gr.hkeys.as<unsigned long long>(), gr.counts.as<int>(),
+                         gr.runs.as<int2>(), gr.ids.as<int>(), gr.size - 1};
+    };
+    b->gp = build(c->gp, c->bp, np, mode_p);
+    b->ge = build(c->ge, c->be, c->nBE, mode_e);
+    FIPC_CUDA(cudaMemsetAsync(b->n, 0, sizeof(BroadCounters), s));
+    const long long work = (long long)n + np, slots = (long long)(c->gp.size + c->ge.size);
+    const int grid = (int)std::max<long long>(nblk(work, 256), std::min<long long>(nblk(slots, 256), 1216));
+    k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, tri_big, tri_big + c->nBT,
+                                   c->big_list.as<int>(), b->n);
+    FIPC_LAUNCHED();
+    g.big_tri = tri_big;
+    g.big_edge = tri_big + c->nBT;
+    b->g = g;
+    const int entries = nblk((long long)CELL_LANES * (np + c->nBE), 256);
+    if (entries > 0) {
+        k_grid_insert<<<entries, 256, 0, s>>>(b->gp, b->ge, x, p, c->dhat, g, b->n);
+        FIPC_LAUNCHED();
+        k_grid_runs<<<nblk(slots, 256), 256, 0, s>>>(b->gp, b->ge, b->n);
+        FIPC_LAUNCHED();
+        k_grid_fill<<<entries, 256, 0, s>>>(b->gp, b->ge, x, p, c->dhat, g, b->n);
         FIPC_LAUNCHED();
     }
-    g->big_tri = tri_big;
-    g->big_edge = tri_big + c->nBT;
-    b->bp = c->bp;
-    b->be = c->be;
-    b->bt = c->bt;
-    b->off = c->prim_off;
-    b->S = c->n_scenes;
-    b->tri_big = g->big_tri;
-    b->edge_big = g->big_edge;
-    b->list = list;
-    b->counts = counts;
-    b->nbt = c->nBT;
-    return FIPC_OK;
-}
-constexpr int BIG_GRID = 304, BIG_THREADS = 128;
-
-// build grid g over n stored primitives; scal: device int scratch (overflow flag at [0])
-int build_grid(fipc_ctx* c, Grid& g, int mode, int n, const int* prim, const double* x, const double* p, const SceneGeo& sg,
-               cudaStream_t s) {
-    g.n_entries = 0;
-    g.n_unique = 0;
-    if (g.counts.ensure(sizeof(long long) * (n + 1)) || g.offsets.ensure(sizeof(long long) * (n + 1)) ||
-        g.ncells.ensure(sizeof(int) * 2))
-        return FIPC_ERR_CUDA;
-    FIPC_CUDA(cudaMemsetAsync(g.ncells.p, 0, sizeof(int) * 2, s));
-    if (n == 0) return FIPC_OK;
-    int* ovf = g.ncells.as<int>() + 1;
-    k_cell_count<<<nblk(n, 256), 256, 0, s>>>(mode, n, prim, x, p, c->dhat, sg, g.counts.as<long long>(), ovf);
-    FIPC_LAUNCHED();
-    if (g.cell4.ensure(16ll * n) || g.box4.ensure(32ll * n)) return FIPC_ERR_CUDA;
-    k_cand_records<<<nblk(n, 256), 256, 0, s>>>(mode, n, prim, x, p, c->dhat, sg, g.cell4.as<int4>(), g.box4.as<float4>());
-    FIPC_LAUNCHED();
-    long long* cnt = g.counts.as<long long>();
-    long long* off = g.offsets.as<long long>();
-    int st = cub_call(c, [&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveSum(t, b, cnt, off, n, s); });
-    if (st) return st;
-    long long last_off = 0, last_cnt = 0;
-    int h_ovf = 0;
-    FIPC_CUDA(cudaMemcpyAsync(&last_off, off + n - 1, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    FIPC_CUDA(cudaMemcpyAsync(&last_cnt, cnt + n - 1, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    FIPC_CUDA(cudaMemcpyAsync(&h_ovf, ovf, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FIPC_CUDA(cudaStreamSynchronize(s));
-    if (h_ovf) return FIPC_ERR_CAPACITY;
-    const long long total = last_off + last_cnt;
-    if (total > (1ll << 30)) return FIPC_ERR_CAPACITY;
-    g.n_entries = (int)total;
-    if (total == 0) return FIPC_OK;
-    if (g.keys.ensure(8 * total) || g.keys_alt.ensure(8 * total) || g.ids.ensure(4 * total) || g.ids_alt.ensure(4 * total) ||
-        g.ukeys.ensure(8 * total) || g.ustart.ensure(4 * (total + 1)) || g.tmp.ensure(4 * (total + 1)))
-        return FIPC_ERR_CUDA;
-    k_cell_emit<<<nblk(n, 256), 256, 0, s>>>(mode, n, prim, x, p, c->dhat, sg, off, cnt, g.keys.as<unsigned long long>(),
-                                             g.ids.as<int>());
-    FIPC_LAUNCHED();
-    cub::DoubleBuffer<unsigned long long> kb(g.keys.as<unsigned long long>(), g.keys_alt.as<unsigned long long>());
-    cub::DoubleBuffer<int> vb(g.ids.as<int>(), g.ids_alt.as<int>());
-    const int N = (int)total;
-    st = cub_call(c, [&](void* t, size_t& b) { return cub::DeviceRadixSort::SortPairs(t, b, kb, vb, N, 0, 63, s); });
-    if (st) return st;
-    if (kb.Current() != g.keys.as<unsigned long long>()) {
-        FIPC_CUDA(cudaMemcpyAsync(g.keys.p, kb.Current(), 8 * total, cudaMemcpyDeviceToDevice, s));
-        FIPC_CUDA(cudaMemcpyAsync(g.ids.p, vb.Current(), 4 * total, cudaMemcpyDeviceToDevice, s));
-    }
-    int* runs = g.tmp.as<int>();   // run lengths
-    int* nu = g.ncells.as<int>();
-    st = cub_call(c, [&](void* t, size_t& b) {
-        return cub::DeviceRunLengthEncode::Encode(t, b, g.keys.as<unsigned long long>(), g.ukeys.as<unsigned long long>(), runs, nu,
-                                                  N, s);
-    });
-    if (st) return st;
-    st = cub_call(c, [&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveSum(t, b, runs, g.ustart.as<int>(), N + 1, s); });
-    if (st) return st;
-    // cell table
-    unsigned long long size = 1;
-    while (size < 2ull * (unsigned long long)N) size <<= 1;
-    if (g.hkeys.ensure(8 * size) || g.hvals.ensure(4 * size)) return FIPC_ERR_CUDA;
-    FIPC_CUDA(cudaMemsetAsync(g.hkeys.p, 0xff, 8 * size, s));
-    g.hmask = size - 1;
-    k_hash_insert<<<nblk(N, 256), 256, 0, s>>>(g.ukeys.as<unsigned long long>(), nu, g.hkeys.as<unsigned long long>(), g.hvals.as<int>(),
-                                               g.hmask);
-    FIPC_LAUNCHED();
+    b->big = BigArgs{c->bp, c->be, c->bt, c->prim_off, c->n_scenes, g.big_tri, g.big_edge, c->big_list.as<int>(), b->n->big, c->nBT,
+                     c->n_scenes > 1 ? 128 : 32};
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
 }
 
-static CandView cands(const Grid& g) { return CandView{g.cell4.as<int4>(), g.box4.as<float4>()}; }
-
-static GridView view(const Grid& g) {
-    GridView v;
-    v.hk = g.hkeys.as<unsigned long long>();
-    v.hv = g.hvals.as<int>();
-    v.mask = g.hmask;
-    v.us = g.ustart.as<int>();
-    v.ids = g.ids.as<int>();
-    return v;
-}
-
-// sort + unique each list in place (rows_tmp as staging); returns counts in c->h_counts
-static int canonicalize_rows(fipc_ctx* c, cudaStream_t s) {
-    int h[N_TYPES + 1];
-    FIPC_CUDA(cudaMemcpyAsync(h, c->d_counts, sizeof(int) * (N_TYPES + 1), cudaMemcpyDeviceToHost, s));
-    FIPC_CUDA(cudaStreamSynchronize(s));
-    if (h[N_TYPES]) return FIPC_ERR_CAPACITY;
-    static const int width[N_TYPES] = {2, 3, 4, 4, 4, 4, 4};
-    for (int t = 0; t < N_TYPES; ++t) {
-        const int n = h[t];
-        c->h_counts[t] = n;
-        if (n <= 1) continue;
-        if (c->rows_tmp.ensure(16ll * n) || c->sort_keys.ensure(8ll * n) || c->sort_keys_alt.ensure(8ll * n) ||
-            c->sort_vals.ensure(4ll * n) || c->sort_vals_alt.ensure(4ll * n) || c->flags.ensure(4ll * n) || c->scan.ensure(4ll * n))
+// after the counters of a call have reached the host: FIPC_OK, an error, or RETRY with larger tables
+constexpr int RETRY = -1;
+static int broad_status(fipc_ctx* c, const BroadCounters& h) {
+    if (h.flags & FLAG_CELLS) return FIPC_ERR_CAPACITY;
+    if (h.flags & FLAG_TABLE) {
+        if (h.total[0] > (1ull << 30) || h.total[1] > (1ull << 30)) return FIPC_ERR_CAPACITY;
+        // half as much again, so that a slowly growing contact does not repeat every call
+        if (ensure_table(c->gp, table_size((long long)(h.total[0] + h.total[0] / 2))) ||
+            ensure_table(c->ge, table_size((long long)(h.total[1] + h.total[1] / 2))))
             return FIPC_ERR_CUDA;
-        int4* rows = c->rows[t].as<int4>();
-        const int* perm = nullptr;
-        const int passes = width[t] == 4 ? 2 : 1;
-        for (int pass = 0; pass < passes; ++pass) {
-            const int kpass = width[t] == 4 ? pass : 1;
-            k_row_keys<<<nblk(n, 256), 256, 0, s>>>(n, width[t], kpass, rows, perm, c->sort_keys.as<unsigned long long>(),
-                                                   c->sort_vals.as<int>());
-            FIPC_LAUNCHED();
-            cub::DoubleBuffer<unsigned long long> kb(c->sort_keys.as<unsigned long long>(), c->sort_keys_alt.as<unsigned long long>());
-            cub::DoubleBuffer<int> vb(c->sort_vals.as<int>(), c->sort_vals_alt.as<int>());
-            const int end_bit = (width[t] == 2) ? 42 : ((kpass == 1) ? 63 : 32);
-            int st = cub_call(c, [&](void* tm, size_t& b) { return cub::DeviceRadixSort::SortPairs(tm, b, kb, vb, n, 0, end_bit, s); });
-            if (st) return st;
-            if (vb.Current() != c->sort_vals.as<int>())
-                FIPC_CUDA(cudaMemcpyAsync(c->sort_vals.p, vb.Current(), 4ll * n, cudaMemcpyDeviceToDevice, s));
-            // the permutation for the next pass lives in sort_vals_alt
-            FIPC_CUDA(cudaMemcpyAsync(c->sort_vals_alt.p, c->sort_vals.p, 4ll * n, cudaMemcpyDeviceToDevice, s));
-            perm = c->sort_vals_alt.as<int>();
-        }
-        k_row_gather_flag<<<nblk(n, 256), 256, 0, s>>>(n, rows, perm, c->rows_tmp.as<int4>(), c->flags.as<int>());
-        FIPC_LAUNCHED();
-        int* flg = c->flags.as<int>();
-        int* pos = c->scan.as<int>();
-        int st = cub_call(c, [&](void* tm, size_t& b) { return cub::DeviceScan::ExclusiveSum(tm, b, flg, pos, n, s); });
-        if (st) return st;
-        k_row_compact<<<nblk(n, 256), 256, 0, s>>>(n, c->rows_tmp.as<int4>(), flg, pos, rows, c->d_counts + t);
-        FIPC_LAUNCHED();
+        return RETRY;
     }
-    FIPC_CUDA(cudaMemcpyAsync(h, c->d_counts, sizeof(int) * N_TYPES, cudaMemcpyDeviceToHost, s));
+    return FIPC_OK;
+}
+static int broad_read(const Broad& b, BroadCounters* h, cudaStream_t s) {
+    FIPC_CUDA(cudaMemcpyAsync(h, b.n, sizeof(BroadCounters), cudaMemcpyDeviceToHost, s));
     FIPC_CUDA(cudaStreamSynchronize(s));
-    for (int t = 0; t < N_TYPES; ++t) c->h_counts[t] = h[t];
-    FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
 }
 
 int ensure_row_capacity(fipc_ctx* c, int cap) {
     if (cap <= c->cap) return FIPC_OK;
-    for (int t = 0; t < N_TYPES; ++t)
-        if (c->rows[t].ensure(16ll * cap)) return FIPC_ERR_CUDA;
+    if (c->row_keys.ensure(16ll * cap) || c->row_keys_alt.ensure(16ll * cap) || c->rows_all.ensure(16ll * cap)) return FIPC_ERR_CUDA;
     c->cap = cap;
     return FIPC_OK;
 }
 
-// find_constraints (NEWTON_IPC.py:337-357) into c->rows / c->h_counts
+// sort and unique of the n emitted rows when they are too many for one CTA
+static int rows_large(fipc_ctx* c, const Broad& b, int n, BroadCounters* h, cudaStream_t s) {
+    RowKey* k = c->row_keys.as<RowKey>();
+    RowKey* u = c->row_keys_alt.as<RowKey>();
+    int* nu = &b.n->sorted;
+    int st = cub_call(c, [&](void* t, size_t& bytes) { return cub::DeviceMergeSort::SortKeys(t, bytes, k, n, RowLess(), s); });
+    if (st) return st;
+    st = cub_call(c, [&](void* t, size_t& bytes) { return cub::DeviceSelect::Unique(t, bytes, k, u, nu, n, s); });
+    if (st) return st;
+    k_rows_write<<<nblk(n, 256), 256, 0, s>>>(nu, u, b.n, c->rows_all.as<int4>());
+    FIPC_LAUNCHED();
+    return broad_read(b, h, s);
+}
+
+// find_constraints (NEWTON_IPC.py:337-357) into c->rows_all / c->h_counts
 int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
-    for (int attempt = 0; attempt < 8; ++attempt) {
-        FIPC_CUDA(cudaMemsetAsync(c->d_counts, 0, sizeof(int) * (N_TYPES + 1), s));
-        RowSink sink;
-        for (int t = 0; t < N_TYPES; ++t) sink.rows[t] = c->rows[t].as<int4>();
-        sink.counts = c->d_counts;
-        sink.cap = c->cap;
-        SceneGeo sg;
-        BigArgs bg;
-        int st = big_prepare(c, x, nullptr, &sg, &bg, s);
+    for (int attempt = 0; attempt < 12; ++attempt) {
+        Broad b;
+        int st = broad_prepare(c, x, nullptr, 0, 1, &b, s);
         if (st) return st;
-        st = build_grid(c, c->gp, 0, c->nBP, c->bp, x, nullptr, sg, s);
+        const RowSink sink{c->row_keys.as<RowKey>(), b.n, c->cap};
+        QueryBlocks nb{c->nBP > 0 ? nblk(c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
+        nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b.big.ny) : 0;
+        nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b.big.ny) : 0;
+        const int blocks = nb.pt + nb.ee + nb.pt_big + nb.ee_big;
+        if (blocks > 0) {
+            k_find<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bt, c->bp, c->nBE, c->be, x, c->x0, c->dhat, c->dhat2, b.g, view(b.gp), cands(b.gp),
+                                          view(b.ge), cands(b.ge), b.big, sink);
+            FIPC_LAUNCHED();
+        }
+        k_rows_small<<<1, SORT_THREADS, 0, s>>>(sink.rows, b.n, c->rows_all.as<int4>());
+        FIPC_LAUNCHED();
+        BroadCounters h;
+        st = broad_read(b, &h, s);
         if (st) return st;
-        if (c->gp.n_entries > 0 && c->nBT > 0) {
-            k_find_pt<<<nblk(c->nBT, 128), 128, 0, s>>>(c->nBT, c->bt, c->bp, x, c->dhat, c->dhat2, sg,
-                                                         view(c->gp), cands(c->gp), sink);
-            FIPC_LAUNCHED();
-        }
-        if (c->nBT > 0 && c->nBP > 0) {
-            k_find_pt_big<<<BIG_GRID, BIG_THREADS, 0, s>>>(bg, x, c->dhat, c->dhat2, sg, sink);
-            FIPC_LAUNCHED();
-        }
-        st = build_grid(c, c->ge, 1, c->nBE, c->be, x, nullptr, sg, s);
+        st = broad_status(c, h);
+        if (st == RETRY) continue;
         if (st) return st;
-        if (c->ge.n_entries > 0) {
-            k_find_ee<<<nblk((long long)QG * c->nBE, 128), 128, 0, s>>>(c->nBE, c->be, x, c->x0, c->dhat, c->dhat2, sg,
-                                                         view(c->ge), cands(c->ge), sink);
-            FIPC_LAUNCHED();
-        }
-        if (c->nBE > 1) {
-            k_find_ee_big<<<BIG_GRID, BIG_THREADS, 0, s>>>(bg, x, c->x0, c->dhat, c->dhat2, sg, sink);
-            FIPC_LAUNCHED();
-        }
-        FIPC_CUDA(cudaGetLastError());
-        st = canonicalize_rows(c, s);
-        if (st == FIPC_ERR_CAPACITY) {
-            int h[N_TYPES];
-            FIPC_CUDA(cudaMemcpy(h, c->d_counts, sizeof(int) * N_TYPES, cudaMemcpyDeviceToHost));
-            int need = c->cap;
-            for (int t = 0; t < N_TYPES; ++t) need = h[t] > need ? h[t] : need;
-            if (ensure_row_capacity(c, 2 * need)) return FIPC_ERR_CUDA;
+        if (h.flags & FLAG_ROWS) {
+            if (h.emitted > (1 << 29)) return FIPC_ERR_CAPACITY;
+            if (ensure_row_capacity(c, 2 * h.emitted)) return FIPC_ERR_CUDA;
             continue;
         }
-        return st;
+        if (!h.sorted) {
+            st = rows_large(c, b, h.emitted, &h, s);
+            if (st) return st;
+        }
+        int off = 0;
+        for (int t = 0; t < N_TYPES; ++t) {
+            c->h_counts[t] = h.rows[t];
+            c->h_row0[t] = off;
+            off += h.rows[t];
+        }
+        return FIPC_OK;
     }
     return FIPC_ERR_CAPACITY;
 }
 
-// compute_intersection_free_step_size (NEWTON_IPC.py:456-468): the launches, min'd into
-// slots (one double per scene, preset to 1.0 by the caller)
-int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, unsigned long long* slot, cudaStream_t s) {
-    SceneGeo sg;
-    BigArgs bg;
-    int st = big_prepare(c, x, p, &sg, &bg, s);
+// compute_intersection_free_step_size (NEWTON_IPC.py:456-468): the launches, min'd into slots (one
+// double per scene, preset to 1.0 by the caller; null: the call's own)
+static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, unsigned long long* slot, Broad* b,
+                      cudaStream_t s) {
+    int st = broad_prepare(c, x, p, 2, 3, b, s);
     if (st) return st;
+    if (!slot) slot = &b->n->alpha;
     CcdList L;
     {
         long long cap = 65536ll + c->nBE + c->nBT;
         if (cap > (1ll << 21)) cap = 1ll << 21;
-        if (c->ccd_work.ensure(256 + 2 * cap * sizeof(CcdWork))) return FIPC_ERR_CUDA;
-        L.count = c->ccd_work.as<int>();
-        L.w = reinterpret_cast<CcdWork*>(c->ccd_work.as<char>() + 256);
+        if (c->ccd_work.ensure(2 * cap * sizeof(CcdWork))) return FIPC_ERR_CUDA;
+        L.count = b->n->work;
+        L.w = c->ccd_work.as<CcdWork>();
         L.cap = (int)cap;
-        FIPC_CUDA(cudaMemsetAsync(L.count, 0, 2 * sizeof(int), s));
     }
-    st = build_grid(c, c->gp, 2, c->nBP, c->bp, x, p, sg, s);
-    if (st) return st;
-    if (c->gp.n_entries > 0 && c->nBT > 0) {
-        k_ccd_pt<<<nblk(c->nBT, 128), 128, 0, s>>>(c->nBT, c->bt, c->bp, x, p, c->dhat, sg, eta,
-                                                    view(c->gp), cands(c->gp), L, slot);
-        FIPC_LAUNCHED();
-        k_ccd_pt_exact<<<4 * BIG_GRID, 128, 0, s>>>(c->bt, x, p, eta, L, slot);
-        FIPC_LAUNCHED();
-    }
-    if (c->nBT > 0 && c->nBP > 0) {
-        k_ccd_pt_big<<<BIG_GRID, BIG_THREADS, 0, s>>>(bg, x, p, c->dhat, eta, sg, slot);
-        FIPC_LAUNCHED();
-    }
-    st = build_grid(c, c->ge, 3, c->nBE, c->be, x, p, sg, s);
-    if (st) return st;
-    if (c->ge.n_entries > 0) {
-        k_ccd_ee<<<nblk((long long)QG * c->nBE, 128), 128, 0, s>>>(c->nBE, c->be, x, p, c->dhat, sg, eta, view(c->ge), cands(c->ge),
-                                                                   L, slot);
-        FIPC_LAUNCHED();
-        k_ccd_ee_exact<<<4 * BIG_GRID, 128, 0, s>>>(c->be, x, p, eta, L, slot);
-        FIPC_LAUNCHED();
-    }
-    if (c->nBE > 1) {
-        k_ccd_ee_big<<<BIG_GRID, BIG_THREADS, 0, s>>>(bg, x, p, c->dhat, eta, sg, slot);
-        FIPC_LAUNCHED();
-    }
+    QueryBlocks nb{c->nBP > 0 ? nblk(c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
+    nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b->big.ny) : 0;
+    nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b->big.ny) : 0;
     if (inversion && c->nT > 0) {
-        k_ccd_inversion<<<nblk(c->nT, 128), 128, 0, s>>>(c->nT, (const int4*)c->tets, x, p, eta, sg, slot);
+        k_ccd_inversion<<<nblk(c->nT, 128), 128, 0, s>>>(c->nT, (const int4*)c->tets, x, p, eta, b->g, slot);
+        FIPC_LAUNCHED();
+    }
+    const int blocks = nb.pt + nb.ee + nb.pt_big + nb.ee_big;
+    if (blocks > 0) {
+        k_ccd<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bt, c->bp, c->nBE, c->be, x, p, c->dhat, eta, b->g, view(b->gp), cands(b->gp), view(b->ge),
+                                     cands(b->ge), b->big, L, slot);
+        FIPC_LAUNCHED();
+        k_ccd_exact<<<EXACT_BLOCKS, 128, 0, s>>>(c->bt, c->be, x, p, eta, L, slot);
         FIPC_LAUNCHED();
     }
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
 }
 
-// one scene: result in *alpha_h
-int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, cudaStream_t s) {
-    if (c->scal.ensure(64)) return FIPC_ERR_CUDA;
-    unsigned long long* slot = c->scal.as<unsigned long long>();
-    const double one = 1.0;
-    FIPC_CUDA(cudaMemcpyAsync(slot, &one, 8, cudaMemcpyHostToDevice, s));
-    int st = ccd_launch(c, x, p, eta, inversion, slot, s);
-    if (st) return st;
-    FIPC_CUDA(cudaMemcpyAsync(alpha_h, slot, 8, cudaMemcpyDeviceToHost, s));
-    FIPC_CUDA(cudaStreamSynchronize(s));
-    return FIPC_OK;
+// one scene (slots null): the step in *alpha_h; a batch: the steps in slots
+int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, unsigned long long* slots,
+             cudaStream_t s) {
+    for (int attempt = 0; attempt < 4; ++attempt) {
+        Broad b;
+        int st = ccd_launch(c, x, p, eta, inversion, slots, &b, s);
+        if (st) return st;
+        BroadCounters h;
+        st = broad_read(b, &h, s);
+        if (st) return st;
+        st = broad_status(c, h);
+        if (st == RETRY) continue;   // the minimum so far stays valid
+        if (st) return st;
+        if (alpha_h) memcpy(alpha_h, &h.alpha, 8);
+        return FIPC_OK;
+    }
+    return FIPC_ERR_CAPACITY;
 }
 
-// check_collision_3d (NEWTON_IPC.py:881-886): the launches, or'd into hit (one int per scene,
-// zeroed by the caller)
-int collision_launch(fipc_ctx* c, const double* x, int* hit, cudaStream_t s) {
-    SceneGeo sg;
-    BigArgs bg;
-    int st = big_prepare(c, x, nullptr, &sg, &bg, s);
-    if (st) return st;
-    st = build_grid(c, c->ge, 4, c->nBE, c->be, x, nullptr, sg, s);
-    if (st) return st;
-    if (c->ge.n_entries > 0 && c->nBT > 0) {
-        k_collision<<<nblk((long long)QG * c->nBT, 128), 128, 0, s>>>(c->nBT, c->bt, c->be, x, c->dhat, sg, view(c->ge),
-                                                                       cands(c->ge), hit);
-        FIPC_LAUNCHED();
+// check_collision_3d (NEWTON_IPC.py:881-886): one scene (hits null): the flag in *hit_h; a batch: or'd
+// into hits (one int per scene, zeroed by the caller)
+int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStream_t s) {
+    for (int attempt = 0; attempt < 4; ++attempt) {
+        Broad b;
+        int st = broad_prepare(c, x, nullptr, -1, 4, &b, s);
+        if (st) return st;
+        int* hit = hits ? hits : &b.n->hit;
+        QueryBlocks nb{c->nBE > 0 ? nblk((long long)QG * c->nBT, 128) : 0, 0, 0, 0};
+        if (c->nBT > 0 && c->nBE > 0) {
+            nb.pt_big = big_blocks(c, 1, b.big.ny);
+            nb.ee_big = big_blocks(c, 2, b.big.ny);
+        }
+        const int blocks = nb.pt + nb.pt_big + nb.ee_big;
+        if (blocks > 0) {
+            k_collision<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bt, c->be, x, c->dhat, b.g, view(b.ge), cands(b.ge), b.big, hit);
+            FIPC_LAUNCHED();
+        }
+        FIPC_CUDA(cudaGetLastError());
+        BroadCounters h;
+        st = broad_read(b, &h, s);
+        if (st) return st;
+        st = broad_status(c, h);
+        if (st == RETRY) continue;
+        if (st) return st;
+        if (hit_h) *hit_h = h.hit;
+        return FIPC_OK;
     }
-    if (c->nBT > 0 && c->nBE > 0) {
-        k_collision_big<<<BIG_GRID, BIG_THREADS, 0, s>>>(bg, x, sg, hit);
-        FIPC_LAUNCHED();
-    }
-    FIPC_CUDA(cudaGetLastError());
-    return FIPC_OK;
-}
-
-int check_collision(fipc_ctx* c, const double* x, int* hit_h, cudaStream_t s) {
-    if (c->scal.ensure(64)) return FIPC_ERR_CUDA;
-    int* hit = (int*)(c->scal.as<char>() + 16);
-    FIPC_CUDA(cudaMemsetAsync(hit, 0, sizeof(int), s));
-    int st = collision_launch(c, x, hit, s);
-    if (st) return st;
-    FIPC_CUDA(cudaMemcpyAsync(hit_h, hit, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FIPC_CUDA(cudaStreamSynchronize(s));
-    return FIPC_OK;
+    return FIPC_ERR_CAPACITY;
 }
 
 }  // namespace fipc

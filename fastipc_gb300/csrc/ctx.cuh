@@ -50,13 +50,12 @@ struct DBuf {
     T* as() const { return (T*)p; }
 };
 
-// sorted spatial-hash grid over primitives: (cell key, primitive id) pairs sorted by key,
-// unique keys and the start of each key's run
+// spatial-hash grid over primitives: an open-addressing table of occupied cells with their entry counts
+// and id runs, and the ids; kept from call to call and grown on demand
 struct Grid {
-    DBuf keys, ids, keys_alt, ids_alt, ukeys, ustart, counts, offsets, ncells, tmp, hkeys, hvals;
+    DBuf hkeys, counts, runs, ids;
     DBuf cell4, box4;   // per stored primitive: first cell of its pair de-duplication, FP32 box
-    int n_entries = 0, n_unique = 0;
-    unsigned long long hmask = 0;   // cell table size - 1 (a power of two >= 2 x entries)
+    unsigned long long size = 0;   // table slots (a power of two, at least twice the entries)
 };
 
 struct fipc_ctx_impl {
@@ -86,11 +85,12 @@ struct fipc_ctx_impl {
     double* sell_val = nullptr;
     // per-iteration element data and the system
     double *elem_g = nullptr, *elem_H = nullptr, *bsr_val = nullptr, *rhs = nullptr;
-    // constraint lists (capacity rows of 4 ints each) and counts
-    DBuf rows[N_TYPES], rows_tmp, sort_keys, sort_keys_alt, sort_vals, sort_vals_alt, flags, scan, cub_tmp;
-    int *d_counts = nullptr;     // [N_TYPES + 1] device (last: overflow flag)
-    int h_counts[N_TYPES] = {0};
+    // constraint lists: emitted rows as sort keys (capacity cap), the sorted unique rows of all lists one
+    // behind the other ([n][4] int), counts and offsets of the lists
+    DBuf row_keys, row_keys_alt, rows_all, cub_tmp;
+    int h_counts[N_TYPES] = {0}, h_row0[N_TYPES] = {0};
     int cap = 0;
+    int* list_rows(int t) const { return rows_all.as<int>() + 4ll * h_row0[t]; }
     // contact system
     DBuf c_g, c_H, c_keys, c_keys_alt, c_vals, c_vals_alt, c_ukeys, c_ucount, c_ustart, c_val, c_rowptr, c_col;
     int c_rows = 0, c_nnzb = 0;
@@ -116,8 +116,9 @@ struct fipc_ctx_impl {
     // boundary lists of scene s: points [prim_off[0][s], prim_off[0][s+1]), edges [1], triangles
     // [2] (device, 3 x (n_scenes + 1)); big-primitive flags and lists of the spatial hash
     int* prim_off = nullptr;
-    DBuf big_flags, big_list;
-    DBuf ccd_work;                        // step filter: pairs left to the exact test, and their counts
+    int max_prims[3] = {0, 0, 0};         // the largest of a scene's points, edges, triangles
+    DBuf big_flags, big_list, broad;      // broad: the counters of a broad-phase call
+    DBuf ccd_work;                        // step filter: pairs left to the exact test
     std::vector<double> h_kappa, h_inv_dx;
     // batched PCG: tiles of consecutive rows inside one scene
     int n_tiles = 0, tile_rows = 0, pcg_grid = 0;

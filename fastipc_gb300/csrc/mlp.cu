@@ -640,7 +640,7 @@ extern "C" int fipc_mlp_features(fipc_ctx* c, const double* x, const double* v, 
     FIPC_LAUNCHED();
     for (int t = 0; t < N_TYPES; ++t) {
         if (c->h_counts[t] <= 0) continue;
-        k_row_dist<<<nblk(c->h_counts[t], 128), 128, 0, s>>>(t, c->h_counts[t], c->rows[t].as<int4>(), x, dmin);
+        k_row_dist<<<nblk(c->h_counts[t], 128), 128, 0, s>>>(t, c->h_counts[t], (const int4*)c->list_rows(t), x, dmin);
         FIPC_LAUNCHED();
     }
     k_features<<<nblk(c->nV, 128), 128, 0, s>>>(c->nV, c->row_ptr, c->col_idx, x, rest_relative ? c->x0 : nullptr, v, dx_prev, c->dt,

@@ -427,7 +427,7 @@ int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t
     for (int t = 0; t < N_TYPES; ++t) {
         if (!c->h_counts[t]) continue;
         const int off = tt.row0[t];
-        st = launch_barrier_rows(t, c->h_counts[t], c->rows[t].as<int>(), x, c->x0, c->dhat2, c->kappa,
+        st = launch_barrier_rows(t, c->h_counts[t], c->list_rows(t), x, c->x0, c->dhat2, c->kappa,
                                  c->n_scenes > 1 ? c->s_kappa : nullptr, c->v_scene, nullptr,
                                  c->c_g.as<double>() + 12ll * off, c->c_H.as<double>() + 144ll * off, nullptr, s);
         if (st) return st;
@@ -435,8 +435,7 @@ int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t
     return contact_reduce(c, tt, nrows, nent, s);
 }
 
-// The contact rows of the current lists, concatenated in list order into rows_tmp: the type
-// table, the row and block-entry counts, and buffers for the per-row gradients c_g [rows][12]
+// The contact rows of the current lists (rows_all, in list order): the type table, the row and block-entry counts, and buffers for the per-row gradients c_g [rows][12]
 // and 3x3 blocks c_H [rows][16][9] that the caller fills.  With no rows the contact matrix is
 // left empty.
 int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_out, cudaStream_t s) {
@@ -458,15 +457,13 @@ int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_
     }
     if (c->c_g.ensure(96ll * nrows) || c->c_H.ensure(1152ll * nrows) || c->c_keys.ensure(8 * nent) || c->c_keys_alt.ensure(8 * nent) ||
         c->c_vals.ensure(4 * nent) || c->c_vals_alt.ensure(4 * nent) || c->c_ukeys.ensure(8 * nent) || c->c_ucount.ensure(4 * (nent + 1)) ||
-        c->c_ustart.ensure(4 * (nent + 1)) || c->c_val.ensure(72 * nent) || c->c_col.ensure(4 * nent) || c->rows_tmp.ensure(16ll * nrows))
+        c->c_ustart.ensure(4 * (nent + 1)) || c->c_val.ensure(72 * nent) || c->c_col.ensure(4 * nent))
         return FIPC_ERR_CUDA;
-    int4* all = c->rows_tmp.as<int4>();
     int off = 0;
     long long eoff = 0;
     for (int t = 0; t < N_TYPES; ++t) {
         tt->row0[t] = off;
         tt->ent0[t] = eoff;
-        if (c->h_counts[t]) FIPC_CUDA(cudaMemcpyAsync(all + off, c->rows[t].p, 16ll * c->h_counts[t], cudaMemcpyDeviceToDevice, s));
         off += c->h_counts[t];
         eoff += (long long)c->h_counts[t] * type_nverts(t) * type_nverts(t);
     }
@@ -478,7 +475,7 @@ int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_
 // The contact matrix (block CSR, fixed-order sums of every (row, column) block of the rows) and
 // the rows' gradients folded into rhs, from c_g / c_H filled for the rows contact_prepare set up
 int contact_reduce(fipc_ctx* c, const TypeTable& tt, int nrows, long long nent, cudaStream_t s) {
-    const int4* all = c->rows_tmp.as<int4>();
+    const int4* all = c->rows_all.as<int4>();
     k_contact_keys<<<nblk(nrows, 128), 128, 0, s>>>(nrows, all, tt, c->c_keys.as<unsigned long long>(), c->c_vals.as<int>());
     FIPC_LAUNCHED();
     const int N = (int)nent;
