@@ -106,9 +106,7 @@ __global__ void __launch_bounds__(SE_THREADS) k_scene_energy(int S, const int* _
                 X[k] = ld3(x, id[k]);
                 X0[k] = type >= T_EEM ? ld3(x0, id[k]) : mk(0, 0, 0);
             }
-            double e;
-            barrier_row(type, X, X0, dh2, kappa, 0, &e, nullptr, nullptr);
-            acc += e;
+            acc += barrier_energy(type, X, X0, dh2, kappa);
         }
         total += block_sum_t<SE_THREADS>(acc, sh);
     }

@@ -21,8 +21,7 @@ int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStr
 int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t s);
 int pcg_solve(fipc_ctx* c, const unsigned char* fixed, int guess, double rtol, int maxit, double* sol, int* iters, cudaStream_t s);
 int sell_to_bsr(fipc_ctx* c, double* out, cudaStream_t s);
-int launch_energy(const fipc_ctx* c, const double* x, const double* xt, const int* const* rows, const int* counts, double* part,
-                  double* out, cudaStream_t s);
+int launch_energy(const fipc_ctx* c, const double* x, const double* xt, double* part, double* out, cudaStream_t s);
 int launch_absmax(int n, const double* p, double* part, double* out, cudaStream_t s);
 void free_batch(fipc_ctx* c);
 int cs_setup(fipc_ctx* c, int agg_rows, const int* row_ptr_h, const int* col_idx_h);
@@ -439,9 +438,9 @@ int fipc_solve_system(fipc_ctx* c, const unsigned char* fixed, double rtol, int 
 int fipc_output_residual(fipc_ctx* c, const double* sol, double* res_h, void* stream) {
     if (!c || !sol || !res_h) return FIPC_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    if (c->red.ensure(8ull * (RED_BLOCKS * (2 + N_TYPES) + 8))) return FIPC_ERR_CUDA;
+    if (c->red.ensure(8ull * (RED_BLOCKS + 8))) return FIPC_ERR_CUDA;
     double* part = c->red.as<double>();
-    double* outv = part + RED_BLOCKS * (2 + N_TYPES);
+    double* outv = part + RED_BLOCKS;
     const int st = launch_absmax(3 * c->nV, sol, part, outv, s);
     if (st) return st;
     FIPC_CUDA(cudaMemcpyAsync(res_h, outv, 8, cudaMemcpyDeviceToHost, s));
@@ -452,12 +451,10 @@ int fipc_output_residual(fipc_ctx* c, const double* sol, double* res_h, void* st
 int fipc_compute_energy(fipc_ctx* c, const double* x, const double* xtilde, double* e_h, void* stream) {
     if (!c || !x || !xtilde || !e_h) return FIPC_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    if (c->red.ensure(8ull * (RED_BLOCKS * (2 + N_TYPES) + 8))) return FIPC_ERR_CUDA;
+    if (c->red.ensure(8ull * (RED_BLOCKS + 8))) return FIPC_ERR_CUDA;
     double* part = c->red.as<double>();
-    double* outv = part + RED_BLOCKS * (2 + N_TYPES);
-    const int* rows[N_TYPES];
-    for (int t = 0; t < N_TYPES; ++t) rows[t] = c->list_rows(t);
-    const int st = launch_energy(c, x, xtilde, rows, c->h_counts, part, outv, s);
+    double* outv = part + RED_BLOCKS;
+    const int st = launch_energy(c, x, xtilde, part, outv, s);
     if (st) return st;
     FIPC_CUDA(cudaMemcpyAsync(e_h, outv, 8, cudaMemcpyDeviceToHost, s));
     FIPC_CUDA(cudaStreamSynchronize(s));

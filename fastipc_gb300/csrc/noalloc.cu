@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(NOALLOC_THREADS) k_na_barrier(int type, int n,
             X[k] = ld3(x, id[k]);
             X0[k] = type >= T_EEM ? ld3(x0, id[k]) : mk(0, 0, 0);
         }
-        barrier_row(type, X, X0, dh2, kappa, 0, &e, nullptr, nullptr);
+        e = barrier_energy(type, X, X0, dh2, kappa);
     }
     na_block_store(e, part);
 }
