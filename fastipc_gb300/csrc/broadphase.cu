@@ -15,8 +15,8 @@
 // A call is a chain of a few kernels and one copy to the host at its end: table and row capacities are
 // kept from call to call and checked on the device; a call that outgrows them is repeated with larger
 // ones.  Measured on a GB300 against radix-sorted grids, one sort per list and a host round trip per grid:
-// constraint finding of two touching cubes (1,458 vertices) 1.16 -> 0.37 ms a call, of a pile of 180 cubes
-// 5.2 -> 1.4 ms, of the 960k-tet bar 1.37 -> 0.99 ms.
+// constraint finding of two touching cubes (1,458 vertices) 1.16 -> 0.22 ms a call, of a pile of 180 cubes
+// 5.2 -> 1.0 ms; the step filter of the cubes 2.2 -> 0.64 ms.
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
@@ -188,7 +188,8 @@ struct BroadCounters {
     int emitted;                // rows emitted (also past the capacity)
     int sorted;                 // rows[] holds the final counts
     int big[2];                 // big triangles, edges
-    int work[2];                // step filter: pairs left to the exact test
+    int pairs[2];               // candidate pairs of the two kinds of a query
+    int work[2], doubt[2];      // step filter: pairs that pass the additive bound, the sign filter
     int cursor[2];              // ids handed out to runs (points, edges)
     unsigned long long total[2];   // grid entries (points, edges)
     unsigned long long alpha;   // one scene's step (bits of a double)
@@ -266,10 +267,63 @@ __device__ void attempt_ee(const double* __restrict__ x, const double* __restric
     }
 }
 
+// ---------------------------------------------------------------- candidate pairs
+// The grid walks and the big-primitive passes only test FP32 boxes; the pairs that pass go to a list, one
+// per kind, and the FP64 narrow phase runs over the lists with every lane on a pair.  In the walk itself one
+// or two lanes of a warp would run it while the others wait, and an FP64 instruction takes a warp's 18
+// clocks of the SM whatever its active lanes.  A list that is full leaves its pair to the walking lane;
+// the next call's is larger.
+struct PairList {
+    int2* w;               // [2 cap]: pairs of the first kind, then of the second
+    int* count;            // [2] (may exceed cap)
+    int cap;
+};
+// one atomic per coalesced group; false when the list is full
+__device__ __forceinline__ bool pair_push(const PairList& L, int kind, int a, int b) {
+    if (*(volatile int*)(L.count + kind) >= L.cap) return false;
+    const cg::coalesced_group g = cg::coalesced_threads();
+    int base = 0;
+    if (g.thread_rank() == 0) base = atomicAdd(L.count + kind, (int)g.size());
+    base = g.shfl(base, 0);
+    const int k = base + (int)g.thread_rank();
+    if (k >= L.cap) return false;
+    L.w[(size_t)kind * L.cap + k] = make_int2(a, b);
+    return true;
+}
+constexpr int PAIR_THREADS = 64, PAIR_BLOCKS = 16 * 152;
+// f(kind, pair) for every listed pair; a warp's pairs are of one kind
+template <class F>
+__device__ __forceinline__ void each_pair(const PairList& L, F f) {
+    const int n0 = min(L.count[0], L.cap), n1 = min(L.count[1], L.cap), m0 = (n0 + 31) & ~31;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m0 + n1; k += gridDim.x * blockDim.x) {
+        if (k < m0) {
+            if (k < n0) f(0, L.w[k]);
+        } else {
+            f(1, L.w[(size_t)L.cap + (k - m0)]);
+        }
+    }
+}
+
+// the rows of point-triangle (kind 0: vertex, triangle) and edge-edge (kind 1) pairs
+struct FindArgs {
+    const int *bt, *be;
+    const double *x, *x0;
+    double dh, dh2;
+};
+__device__ __forceinline__ void find_pair(const FindArgs& a, int kind, int i, int j, const RowSink& s) {
+    if (kind == 0) attempt_pt(a.x, a.dh, a.dh2, i, a.bt[3 * j], a.bt[3 * j + 1], a.bt[3 * j + 2], s);
+    else attempt_ee(a.x, a.x0, a.dh, a.dh2, a.be[2 * i], a.be[2 * i + 1], a.be[2 * j], a.be[2 * j + 1], s);
+}
+__device__ __noinline__ void find_pair_call(const FindArgs& a, int kind, int i, int j, const RowSink& s) { find_pair(a, kind, i, j, s); }
+__global__ void __launch_bounds__(PAIR_THREADS) k_find_pairs(FindArgs a, PairList L, RowSink s) {
+    each_pair(L, [&](int kind, int2 q) { find_pair(a, kind, q.x, q.y, s); });
+}
+
 // one thread per boundary triangle; points hashed with mode 0
 __device__ __forceinline__ void find_pt(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
-                                                 const double* __restrict__ x, double dh, double dh2, SceneGeo g,
-                                                 GridView gv, CandView cv, RowSink sink) {
+                                                 const FindArgs& fa, const SceneGeo& g, const GridView& gv, const CandView& cv,
+                                                 const PairList& L, const RowSink& sink) {
+    const double* x = fa.x;
     const int i = block * 128 + threadIdx.x;
     if (i >= nbt) return;
     if (g.big_tri && g.big_tri[i]) return;
@@ -279,7 +333,7 @@ __device__ __forceinline__ void find_pt(int block, int nbt, const int* __restric
     const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
     const v3 tmn = vmin(vmin(A, B), C), tmx = vmax(vmax(A, B), C);
     const C3 lo = cell_of(tmn, inv_dx), hi = cell_of(tmx, inv_dx);
-    const v3 d = mk(dh, dh, dh);
+    const v3 d = mk(fa.dh, fa.dh, fa.dh);
     const float4 qlo = f32_lo(tmn - d), qhi = f32_hi(tmx + d);   // pt_aabb's triangle box
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
@@ -292,15 +346,16 @@ __device__ __forceinline__ void find_pt(int block, int nbt, const int* __restric
                     if (first.x != cx || first.y != cy || first.z != cz) continue;
                     if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
                     const int p = bp[j];
-                    attempt_pt(x, dh, dh2, p, t0, t1, t2, sink);
+                    if (p == t0 || p == t1 || p == t2) continue;
+                    if (!pair_push(L, 0, p, i)) find_pair_call(fa, 0, p, i, sink);
                 }
             }
 }
 
 // one thread per boundary edge (query, box +- dh); stored edges hashed with mode 1
-__device__ __forceinline__ void find_ee(int block, int nbe, const int* __restrict__ be, const double* __restrict__ x,
-                                                 const double* __restrict__ x0, double dh, double dh2, SceneGeo g,
-                                                 GridView gv, CandView cv, RowSink sink) {
+__device__ __forceinline__ void find_ee(int block, int nbe, const int* __restrict__ be, const FindArgs& fa, const SceneGeo& g,
+                                        const GridView& gv, const CandView& cv, const PairList& L, const RowSink& sink) {
+    const double* x = fa.x;
     // QG lanes per query edge share the candidates of each cell
     const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= nbe) return;
@@ -309,7 +364,7 @@ __device__ __forceinline__ void find_ee(int block, int nbe, const int* __restric
     const int sc = g.scene(a0);
     const double inv_dx = g.idx(sc);
     const v3 A0 = ld3(x, a0), A1 = ld3(x, a1);
-    const v3 d = mk(dh, dh, dh);
+    const v3 d = mk(fa.dh, fa.dh, fa.dh);
     const C3 lo = cell_of(vmin(A0, A1) - d, inv_dx), hi = cell_of(vmax(A0, A1) + d, inv_dx);
     const float4 qlo = f32_lo(vmin(A0, A1)), qhi = f32_hi(vmax(A0, A1));   // ee_aabb's query edge box
     for (long long cx = lo.x; cx <= hi.x; ++cx)
@@ -324,34 +379,26 @@ __device__ __forceinline__ void find_ee(int block, int nbe, const int* __restric
                     if (first.x != cx || first.y != cy || first.z != cz) continue;
                     if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
                     const int b0 = be[2 * j], b1 = be[2 * j + 1];
-                    attempt_ee(x, x0, dh, dh2, a0, a1, b0, b1, sink);
+                    if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) continue;
+                    if (!pair_push(L, 1, i, j)) find_pair_call(fa, 1, i, j, sink);
                 }
             }
 }
 
 // ---------------------------------------------------------------- CCD step filter
-// Pairs that pass the additive bound go to the exact interval test through a compacted list
-// instead of running it in the candidate loop, where one lane's exact test would hold its whole
-// warp (the candidate loops are divergent: lanes run different cells and candidates).  The
-// minimum over pairs does not depend on where a pair's toc is computed.
+// A query's candidate pairs are tested in three steps of falling width, each over the list the one before
+// leaves: moving boxes and the additive bound (k_ccd_pairs), the signs of the interval test's
+// polynomials (k_ccd_signs), the interval test with its root finding (k_ccd_exact).  The minimum over
+// pairs does not depend on where a pair's toc is computed.
 struct CcdWork {
     int a, b, slot, pad;   // point-triangle: vertex, triangle; edge-edge: edge, edge; filter slot
     double d2, lb;         // current squared distance, additive lower bound
 };
 struct CcdList {
     CcdWork* w;            // [2 cap]: point-triangle pairs, then edge-edge pairs
-    int* count;            // [2] pushes (may exceed cap: the lanes past it test inline)
+    int* count;            // [2] pushes (may exceed cap: the lanes past it run the exact test themselves)
     int cap;
 };
-
-// the exact tests out of line, for the candidate loops' overflow path (keeps their registers low)
-__device__ __noinline__ double pt_exact_call(v3 P, v3 A, v3 B, v3 C, v3 dP, v3 dA, v3 dB, v3 dC, double eta, double d2, double lb) {
-    return pt_ccd_exact(P, A, B, C, dP, dA, dB, dC, eta, d2, lb);
-}
-__device__ __noinline__ double ee_exact_call(v3 A0, v3 A1, v3 B0, v3 B1, v3 dA0, v3 dA1, v3 dB0, v3 dB1, double eta, double d2,
-                                             double lb) {
-    return ee_ccd_exact(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, d2, lb);
-}
 
 // appends e for every calling lane (one atomic per coalesced group); false when the list is full
 __device__ __forceinline__ bool ccd_push(CcdWork* w, int* count, int cap, const CcdWork& e) {
@@ -369,14 +416,188 @@ __device__ __forceinline__ void atomic_min_pos(unsigned long long* slot, double 
     if (v >= 0.0) atomicMin(slot, (unsigned long long)__double_as_longlong(v));
 }
 
+struct CcdArgs {
+    const int *bt, *be;
+    const double *x, *p;
+    double dh, eta;
+    const int* vscene;
+    unsigned long long* alpha;
+};
+struct Quad {
+    v3 X[4], D[4];
+    int v0;
+};
+// a pair's vertices and directions: point, triangle (kind 0) or the two edges (kind 1)
+__device__ __forceinline__ Quad quad_of(const CcdArgs& a, int kind, int i, int j) {
+    int v[4];
+    if (kind == 0) {
+        v[0] = i;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[1 + k] = a.bt[3 * j + k];
+    } else {
+        v[0] = a.be[2 * i];
+        v[1] = a.be[2 * i + 1];
+        v[2] = a.be[2 * j];
+        v[3] = a.be[2 * j + 1];
+    }
+    Quad q;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        q.X[k] = ld3(a.x, v[k]);
+        q.D[k] = ld3(a.p, v[k]);
+    }
+    q.v0 = v[0];
+    return q;
+}
+__device__ __forceinline__ double exact_toc(const Quad& q, int kind, double eta, double d2, double lb) {
+    return kind == 0 ? pt_ccd_exact(q.X[0], q.X[1], q.X[2], q.X[3], q.D[0], q.D[1], q.D[2], q.D[3], eta, d2, lb)
+                     : ee_ccd_exact(q.X[0], q.X[1], q.X[2], q.X[3], q.D[0], q.D[1], q.D[2], q.D[3], eta, d2, lb);
+}
+// moving boxes and the additive bound; a full work list leaves the exact test to the calling lane
+__device__ __forceinline__ void ccd_pair(const CcdArgs& a, int kind, int i, int j, const CcdList& L) {
+    const Quad q = quad_of(a, kind, i, j);
+    double d2, lb;
+    if (kind == 0) {
+        if (!pt_aabb_moving(q.X[0], q.X[1], q.X[2], q.X[3], q.D[0], q.D[1], q.D[2], q.D[3], a.dh)) return;
+        d2 = pt_dist2(q.X[0], q.X[1], q.X[2], q.X[3]);
+        if (!pt_needs_exact(q.D[0], q.D[1], q.D[2], q.D[3], a.eta, d2, &lb)) return;
+    } else {
+        if (!ee_aabb_moving(q.X[0], q.X[1], q.X[2], q.X[3], q.D[0], q.D[1], q.D[2], q.D[3], a.dh)) return;
+        d2 = ee_dist2(q.X[0], q.X[1], q.X[2], q.X[3]);
+        if (!ee_needs_exact(q.D[0], q.D[1], q.D[2], q.D[3], a.eta, d2, &lb)) return;
+    }
+    const int slot = a.vscene ? a.vscene[q.v0] : 0;
+    if (!ccd_push(L.w + (size_t)kind * L.cap, L.count + kind, L.cap, CcdWork{i, j, slot, 0, d2, lb}))
+        atomic_min_pos(a.alpha + slot, exact_toc(q, kind, a.eta, d2, lb));
+}
+__device__ __noinline__ void ccd_pair_call(const CcdArgs& a, int kind, int i, int j, const CcdList& L) { ccd_pair(a, kind, i, j, L); }
+__global__ void __launch_bounds__(PAIR_THREADS) k_ccd_pairs(CcdArgs a, PairList P, CcdList L) {
+    each_pair(P, [&](int kind, int2 q) { ccd_pair(a, kind, q.x, q.y, L); });
+}
+
+// a pair's toc is at least its additive bound: one whose bound is not below the minimum so far cannot
+// lower it
+__device__ __forceinline__ bool may_lower(const CcdArgs& a, const CcdWork& e) {
+    return e.lb < __longlong_as_double((long long)*(volatile unsigned long long*)(a.alpha + e.slot));
+}
+// pairs that the signs of the polynomials do not decide (most never come close), from L to M (as large)
+__global__ void __launch_bounds__(PAIR_THREADS) k_ccd_signs(CcdArgs a, CcdList L, CcdList M) {
+    const int half = gridDim.x / 2, kind = (int)blockIdx.x < half ? 0 : 1;
+    const int n = min(L.count[kind], L.cap);
+    for (int k = (blockIdx.x - (kind ? half : 0)) * blockDim.x + threadIdx.x; k < n; k += half * blockDim.x) {
+        const CcdWork e = L.w[(size_t)kind * L.cap + k];
+        if (!may_lower(a, e)) continue;
+        const Quad q = quad_of(a, kind, e.a, e.b);
+        const double eta = a.eta * sqrt(e.d2);
+        const v3 Y[4] = {q.X[0] + q.D[0], q.X[1] + q.D[1], q.X[2] + q.D[2], q.X[3] + q.D[3]};
+        if (kind == 0 ? vertex_face_apart(q.X[0], q.X[1], q.X[2], q.X[3], Y[0], Y[1], Y[2], Y[3], eta)
+                      : edge_edge_apart(q.X[0], q.X[1], q.X[2], q.X[3], Y[0], Y[1], Y[2], Y[3], eta))
+            continue;
+        ccd_push(M.w + (size_t)kind * M.cap, M.count + kind, M.cap, e);
+    }
+}
+
+// The exact test of the pairs left, eight lanes per pair: each finds the intervals of one of its four
+// (point-triangle: distance, three sides) or five (edge-edge: distance, four barycentric) polynomials, all in
+// the same code, and the first lane intersects them.  One thread per pair runs the root finding of its
+// polynomials one after the other, a chain of dependent FP64 operations of hundreds of microseconds
+// for the few hundred pairs that come this far.
+constexpr int EXACT_LANES = 8;
+__global__ void __launch_bounds__(PAIR_THREADS) k_ccd_exact(CcdArgs a, CcdList M) {
+    __shared__ Ivl sh[PAIR_THREADS][8];
+    __shared__ int sn[PAIR_THREADS];
+    const int half = gridDim.x / 2, kind = (int)blockIdx.x < half ? 0 : 1;
+    const int n = min(M.count[kind], M.cap);
+    const int l = threadIdx.x % EXACT_LANES, t0 = threadIdx.x - l;
+    constexpr int PER = PAIR_THREADS / EXACT_LANES;   // pairs per CTA and pass
+    for (int k0 = (blockIdx.x - (kind ? half : 0)) * PER; k0 < n; k0 += half * PER) {
+        const int k = k0 + threadIdx.x / EXACT_LANES;
+        bool act = k < n;
+        CcdWork e{};
+        if (act) {
+            e = M.w[(size_t)kind * M.cap + k];
+            // one answer for the group: the minimum may move between its lanes' reads
+            const int first = (int)(threadIdx.x & 31) - l;
+            act = __shfl_sync(0xffu << first, (int)may_lower(a, e), first) != 0;
+        }
+        sn[threadIdx.x] = 0;
+        Quad q{};
+        double minD = 0.0;
+        if (act) {
+            q = quad_of(a, kind, e.a, e.b);
+            minD = a.eta * sqrt(e.d2);
+            minD *= minD;
+            v3 V[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) V[v] = (q.X[v] + q.D[v]) - q.X[v];
+            double op[7];
+            int deg = 0;
+            if (kind == 0) {
+                if (l == 3) {
+                    distance_coefficients(q.X[0] - q.X[1], q.X[2] - q.X[1], q.X[3] - q.X[1], V[0] - V[1], V[2] - V[1], V[3] - V[1], minD, op);
+                    deg = 6;
+                } else if (l < 3) {
+                    // side l: from its first vertex the next but one and the next
+                    const v3 o = l == 0 ? q.X[1] : (l == 1 ? q.X[2] : q.X[3]), u = l == 0 ? q.X[3] : (l == 1 ? q.X[1] : q.X[2]),
+                             w = l == 0 ? q.X[2] : (l == 1 ? q.X[3] : q.X[1]);
+                    const v3 vo = l == 0 ? V[1] : (l == 1 ? V[2] : V[3]), vu = l == 0 ? V[3] : (l == 1 ? V[1] : V[2]),
+                             vw = l == 0 ? V[2] : (l == 1 ? V[3] : V[1]);
+                    plane_coefficients(q.X[0] - o, cross(u - o, w - o), u - o, V[0] - vo, cross(vu - vo, vw - vo), vu - vo, op);
+                    deg = 3;
+                }
+            } else {
+                // q0, p0, q1, p1 = X[0..3]
+                if (l == 4) {
+                    distance_coefficients(q.X[1] - q.X[3], q.X[1] - q.X[0], q.X[3] - q.X[2], V[1] - V[3], V[1] - V[0], V[3] - V[2], minD, op);
+                    deg = 6;
+                } else if (l < 4) {
+                    const bool second = l >= 2, flip = l & 1;   // whose parameter; from which end
+                    const v3 q0 = second ? q.X[2] : q.X[0], p0 = second ? q.X[3] : q.X[1], q1 = second ? q.X[0] : q.X[2],
+                             p1 = second ? q.X[1] : q.X[3];
+                    const v3 vq0 = second ? V[2] : V[0], vp0 = second ? V[3] : V[1], vq1 = second ? V[0] : V[2], vp1 = second ? V[1] : V[3];
+                    const v3 s = flip ? q0 : p0, f = flip ? p0 : q0, vs = flip ? vq0 : vp0, vf = flip ? vp0 : vq0;
+                    bary_coefficients(p1 - q1, s - f, f - q1, vp1 - vq1, vs - vf, vf - vq1, op);
+                    deg = 4;
+                }
+            }
+            if (deg) {
+                int ni;
+                find_intervals(op, deg, sh[threadIdx.x], &ni, deg != 6);
+                sn[threadIdx.x] = ni;
+            }
+        }
+        __syncwarp();
+        if (act && l == 0) {
+            double toc = 1.0;
+            bool col = true;
+            for (int v = 0; v < 4 + kind; ++v) col = col && sn[t0 + v] > 0;
+            if (col && kind == 0) {
+                col = vertex_face_meet(sh[t0 + 3], sn[t0 + 3], sh[t0], sn[t0], sh[t0 + 1], sn[t0 + 1], sh[t0 + 2], sn[t0 + 2], &toc);
+            } else if (col) {
+                v3 V[4];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) V[v] = (q.X[v] + q.D[v]) - q.X[v];
+                Ivl cp[8], par[8];
+                int ncp, npar;
+                split_parallel(sh[t0 + 4], sn[t0 + 4], q.X[0] - q.X[1], V[0] - V[1], q.X[2] - q.X[3], V[2] - V[3], cp, &ncp, par, &npar);
+                col = edge_edge_meet(cp, ncp, par, npar, sh[t0], sn[t0], sh[t0 + 1], sn[t0 + 1], sh[t0 + 2], sn[t0 + 2], sh[t0 + 3],
+                                     sn[t0 + 3], &toc);
+            }
+            if (col && toc < e.lb) toc = e.lb;
+            if (toc < 1.0) atomic_min_pos(a.alpha + e.slot, toc);
+        }
+        __syncwarp();
+    }
+}
+
 // compute_filter_3D_PT (NEWTON_IPC.py:377-406): triangles query their moving bbox
-__device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
-                                                const double* __restrict__ x, const double* __restrict__ p, double dh, SceneGeo g,
-                                                double eta, GridView gv, CandView cv, CcdList L, unsigned long long* __restrict__ alpha) {
+__device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict__ bp, const CcdArgs& a, const SceneGeo& g,
+                                       const GridView& gv, const CandView& cv, const PairList& P, const CcdList& L) {
     const int i = block * 128 + threadIdx.x;
     if (i >= nbt) return;
     if (g.big_tri && g.big_tri[i]) return;
-    const int t0 = bt[3 * i], t1 = bt[3 * i + 1], t2 = bt[3 * i + 2];
+    const double *x = a.x, *p = a.p;
+    const int t0 = a.bt[3 * i], t1 = a.bt[3 * i + 1], t2 = a.bt[3 * i + 2];
     const int sc = g.scene(t0);
     const double inv_dx = g.idx(sc);
     const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
@@ -384,7 +605,7 @@ __device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict
     const v3 mn = vmin(vmin(vmin(A, A + dA), vmin(B, B + dB)), vmin(C, C + dC));
     const v3 mx = vmax(vmax(vmax(A, A + dA), vmax(B, B + dB)), vmax(C, C + dC));
     const C3 lo = cell_of(mn, inv_dx), hi = cell_of(mx, inv_dx);
-    const v3 d = mk(dh, dh, dh);
+    const v3 d = mk(a.dh, a.dh, a.dh);
     const float4 qlo = f32_lo(mn - d), qhi = f32_hi(mx + d);   // pt_aabb_moving's triangle box
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
@@ -398,31 +619,25 @@ __device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict
                     if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
                     const int pp = bp[j];
                     if (pp == t0 || pp == t1 || pp == t2) continue;
-                    const v3 P = ld3(x, pp), dP = ld3(p, pp);
-                    if (!pt_aabb_moving(P, A, B, C, dP, dA, dB, dC, dh)) continue;
-                    const double d2 = pt_dist2(P, A, B, C);
-                    double lb;
-                    if (!pt_needs_exact(dP, dA, dB, dC, eta, d2, &lb)) continue;
-                    const int slot = g.vscene ? sc : 0;
-                    if (!ccd_push(L.w, L.count, L.cap, CcdWork{pp, i, slot, 0, d2, lb}))
-                        atomic_min_pos(alpha + slot, pt_exact_call(P, A, B, C, dP, dA, dB, dC, eta, d2, lb));
+                    if (!pair_push(P, 0, pp, i)) ccd_pair_call(a, 0, pp, i, L);
                 }
             }
 }
 
 // compute_filter_3D_EE (NEWTON_IPC.py:409-440): edges query moving bbox +- dh
-__device__ __forceinline__ void ccd_ee(int block, int nbe, const int* __restrict__ be, const double* __restrict__ x,
-                                                const double* __restrict__ p, double dh, SceneGeo g, double eta,
-                                                GridView gv, CandView cv, CcdList L, unsigned long long* __restrict__ alpha) {
+__device__ __forceinline__ void ccd_ee(int block, int nbe, const CcdArgs& a, const SceneGeo& g, const GridView& gv, const CandView& cv,
+                                       const PairList& P, const CcdList& L) {
     // QG lanes per query edge share the candidates of each cell
     const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= nbe) return;
     if (g.big_edge && g.big_edge[i]) return;
+    const int* be = a.be;
+    const double *x = a.x, *p = a.p;
     const int a0 = be[2 * i], a1 = be[2 * i + 1];
     const int sc = g.scene(a0);
     const double inv_dx = g.idx(sc);
     const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), dA0 = ld3(p, a0), dA1 = ld3(p, a1);
-    const v3 d = mk(dh, dh, dh);
+    const v3 d = mk(a.dh, a.dh, a.dh);
     const v3 mn = vmin(vmin(A0, A0 + dA0), vmin(A1, A1 + dA1)), mx = vmax(vmax(A0, A0 + dA0), vmax(A1, A1 + dA1));
     const C3 lo = cell_of(mn - d, inv_dx), hi = cell_of(mx + d, inv_dx);
     const float4 qlo = f32_lo(mn), qhi = f32_hi(mx);   // ee_aabb_moving's query edge box
@@ -439,43 +654,9 @@ __device__ __forceinline__ void ccd_ee(int block, int nbe, const int* __restrict
                     if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
                     const int b0 = be[2 * j], b1 = be[2 * j + 1];
                     if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) continue;
-                    const v3 B0 = ld3(x, b0), B1 = ld3(x, b1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
-                    if (!ee_aabb_moving(A0, A1, B0, B1, dA0, dA1, dB0, dB1, dh)) continue;
-                    const double d2 = ee_dist2(A0, A1, B0, B1);
-                    double lb;
-                    if (!ee_needs_exact(dA0, dA1, dB0, dB1, eta, d2, &lb)) continue;
-                    const int slot = g.vscene ? sc : 0;
-                    if (!ccd_push(L.w + L.cap, L.count + 1, L.cap, CcdWork{i, j, slot, 0, d2, lb}))
-                        atomic_min_pos(alpha + slot, ee_exact_call(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, d2, lb));
+                    if (!pair_push(P, 1, i, j)) ccd_pair_call(a, 1, i, j, L);
                 }
             }
-}
-
-// the exact tests of the listed pairs, one thread per pair: the lower half of the grid takes the
-// point-triangle pairs, the upper the edge-edge pairs.  A pair's toc is at least its additive bound, so
-// one whose bound is not below the minimum so far cannot lower it and is left out.
-__global__ void __launch_bounds__(128) k_ccd_exact(const int* __restrict__ bt, const int* __restrict__ be, const double* __restrict__ x,
-                                                   const double* __restrict__ p, double eta, CcdList L,
-                                                   unsigned long long* __restrict__ alpha) {
-    const int half = gridDim.x / 2;
-    const bool pt = (int)blockIdx.x < half;
-    const int n = min(L.count[pt ? 0 : 1], L.cap);
-    const CcdWork* w = pt ? L.w : L.w + L.cap;
-    for (int k = (pt ? blockIdx.x : blockIdx.x - half) * blockDim.x + threadIdx.x; k < n; k += half * blockDim.x) {
-        const CcdWork e = w[k];
-        if (!(e.lb < __longlong_as_double((long long)*(volatile unsigned long long*)(alpha + e.slot)))) continue;
-        if (pt) {
-            const int t0 = bt[3 * e.b], t1 = bt[3 * e.b + 1], t2 = bt[3 * e.b + 2];
-            const v3 P = ld3(x, e.a), dP = ld3(p, e.a);
-            const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2), dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
-            atomic_min_pos(alpha + e.slot, pt_ccd_exact(P, A, B, C, dP, dA, dB, dC, eta, e.d2, e.lb));
-        } else {
-            const int a0 = be[2 * e.a], a1 = be[2 * e.a + 1], b0 = be[2 * e.b], b1 = be[2 * e.b + 1];
-            const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), B0 = ld3(x, b0), B1 = ld3(x, b1);
-            const v3 dA0 = ld3(p, a0), dA1 = ld3(p, a1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
-            atomic_min_pos(alpha + e.slot, ee_ccd_exact(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, e.d2, e.lb));
-        }
-    }
 }
 
 // compute_filter_3D_inversion_free (NEWTON_IPC.py:443-453)
@@ -491,26 +672,41 @@ __global__ void __launch_bounds__(128) k_ccd_inversion(int nT, const int4* __res
     atomic_min_pos(alpha + (g.vscene ? g.scene(t.x) : 0), inversion_free_step(X, P, eta));
 }
 
-// check_collision_3d (NEWTON_IPC.py:855-880): triangles query bbox cells, edges hashed +- dh
-__device__ __forceinline__ void collision_grid(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ be,
-                                                   const double* __restrict__ x, double dh, SceneGeo g,
-                                                   GridView gv, CandView cv, int* __restrict__ hit) {
+// check_collision_3d (NEWTON_IPC.py:855-880): an edge against a triangle
+struct HitArgs {
+    const int *bt, *be;
+    const double* x;
+    const int* vscene;
+    int* hit;
+};
+__device__ __forceinline__ void hit_pair(const HitArgs& a, int e, int t) {
+    const int t0 = a.bt[3 * t], t1 = a.bt[3 * t + 1], t2 = a.bt[3 * t + 2];
+    int* h = a.hit + (a.vscene ? a.vscene[t0] : 0);
+    if (*(volatile int*)h) return;
+    if (seg_tri(ld3(a.x, a.be[2 * e]), ld3(a.x, a.be[2 * e + 1]), ld3(a.x, t0), ld3(a.x, t1), ld3(a.x, t2))) atomicOr(h, 1);
+}
+__device__ __noinline__ void hit_pair_call(const HitArgs& a, int e, int t) { hit_pair(a, e, t); }
+__global__ void __launch_bounds__(PAIR_THREADS) k_collision_pairs(HitArgs a, PairList P) {
+    each_pair(P, [&](int, int2 q) { hit_pair(a, q.x, q.y); });
+}
+
+// triangles query bbox cells, edges hashed +- dh
+__device__ __forceinline__ void collision_grid(int block, int nbt, const HitArgs& a, const SceneGeo& g, const GridView& gv,
+                                               const CandView& cv, const PairList& P) {
     // QG lanes per query triangle share the candidates of each cell
     const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= nbt) return;
     if (g.big_tri && g.big_tri[i]) return;
-    const int t0 = bt[3 * i], t1 = bt[3 * i + 1], t2 = bt[3 * i + 2];
+    const int t0 = a.bt[3 * i], t1 = a.bt[3 * i + 1], t2 = a.bt[3 * i + 2];
     const int sc = g.scene(t0);
     const double inv_dx = g.idx(sc);
-    const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
+    const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2);
     const v3 tmn = vmin(vmin(A, B), C), tmx = vmax(vmax(A, B), C);
     const C3 lo = cell_of(tmn, inv_dx), hi = cell_of(tmx, inv_dx);
     const float4 qlo = f32_lo(tmn), qhi = f32_hi(tmx);   // the triangle's box; edges carry +- dh
-    hit += g.vscene ? sc : 0;
     for (long long cx = lo.x; cx <= hi.x; ++cx)
         for (long long cy = lo.y; cy <= hi.y; ++cy)
             for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                if (*(volatile int*)hit) return;
                 const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
                 for (int k = run.x + lane; k < run.x + run.y; k += QG) {
                     const int j = gv.ids[k];
@@ -518,10 +714,9 @@ __device__ __forceinline__ void collision_grid(int block, int nbt, const int* __
                     const C3 first = cmax(lo, C3{sc4.x, sc4.y, sc4.z});
                     if (first.x != cx || first.y != cy || first.z != cz) continue;
                     if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
-                    const int a0 = be[2 * j], a1 = be[2 * j + 1];
+                    const int a0 = a.be[2 * j], a1 = a.be[2 * j + 1];
                     if (a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2) continue;
-                    const v3 P = ld3(x, a0), Q = ld3(x, a1);
-                    if (seg_tri(P, Q, A, B, C)) atomicOr(hit, 1);
+                    if (!pair_push(P, 0, j, i)) hit_pair_call(a, j, i);
                 }
             }
 }
@@ -573,85 +768,68 @@ __device__ __forceinline__ void big_pairs(const BigArgs& b, const SceneGeo& g, i
 // find_constraints: big triangles against the points, big edges against the edges of their scene (a pair
 // of two big edges once, from its lower index; rows formed with the lower list index first as in the
 // grid pass)
-__device__ __forceinline__ void find_pt_big(int block, const BigArgs& b, const double* __restrict__ x, double dh, double dh2,
-                                            const SceneGeo& g, CandView cv, const RowSink& sink) {
-    const v3 d = mk(dh, dh, dh);
+__device__ __forceinline__ void find_pt_big(int block, const BigArgs& b, const FindArgs& a, const SceneGeo& g, CandView cv, const PairList& P,
+                                            const RowSink& sink) {
+    const v3 d = mk(a.dh, a.dh, a.dh);
     big_pairs(b, g, block, 0, 0, [&](int i, int k, int) {
         const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2];
-        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
+        const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2);
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), f32_lo(vmin(vmin(A, B), C) - d), f32_hi(vmax(vmax(A, B), C) + d)))
             return;
-        attempt_pt(x, dh, dh2, b.bp[k], t0, t1, t2, sink);
+        if (!pair_push(P, 0, b.bp[k], i)) find_pair_call(a, 0, b.bp[k], i, sink);
     });
 }
-__device__ __forceinline__ void find_ee_big(int block, const BigArgs& b, const double* __restrict__ x, const double* __restrict__ x0,
-                                            double dh, double dh2, const SceneGeo& g, CandView cv, const RowSink& sink) {
+__device__ __forceinline__ void find_ee_big(int block, const BigArgs& b, const FindArgs& a, const SceneGeo& g, CandView cv, const PairList& P,
+                                            const RowSink& sink) {
     big_pairs(b, g, block, 1, 1, [&](int i, int j, int) {
         if (j == i || (b.edge_big[j] && j < i)) return;
-        const v3 A0 = ld3(x, b.be[2 * i]), A1 = ld3(x, b.be[2 * i + 1]);
+        const v3 A0 = ld3(a.x, b.be[2 * i]), A1 = ld3(a.x, b.be[2 * i + 1]);
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(vmin(A0, A1)), f32_hi(vmax(A0, A1)))) return;
         const int lo = i < j ? i : j, hi = i < j ? j : i;
-        attempt_ee(x, x0, dh, dh2, b.be[2 * lo], b.be[2 * lo + 1], b.be[2 * hi], b.be[2 * hi + 1], sink);
+        if (!pair_push(P, 1, lo, hi)) find_pair_call(a, 1, lo, hi, sink);
     });
 }
 
 // CCD filter: big moving triangles against the points, big moving edges against the edges of their scene
-__device__ __forceinline__ void ccd_pt_big(int block, const BigArgs& b, const double* __restrict__ x, const double* __restrict__ p, double dh,
-                                           double eta, const SceneGeo& g, CandView cv, const CcdList& L, unsigned long long* __restrict__ alpha) {
-    const v3 d = mk(dh, dh, dh);
-    big_pairs(b, g, block, 0, 0, [&](int i, int k, int sc) {
+__device__ __forceinline__ void ccd_pt_big(int block, const BigArgs& b, const CcdArgs& a, const SceneGeo& g, CandView cv, const PairList& Q,
+                                           const CcdList& L) {
+    const v3 d = mk(a.dh, a.dh, a.dh);
+    big_pairs(b, g, block, 0, 0, [&](int i, int k, int) {
         const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2], pp = b.bp[k];
         if (pp == t0 || pp == t1 || pp == t2) return;
-        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2), dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
+        const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2), dA = ld3(a.p, t0), dB = ld3(a.p, t1), dC = ld3(a.p, t2);
         const v3 mn = vmin(vmin(vmin(A, A + dA), vmin(B, B + dB)), vmin(C, C + dC));
         const v3 mx = vmax(vmax(vmax(A, A + dA), vmax(B, B + dB)), vmax(C, C + dC));
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), f32_lo(mn - d), f32_hi(mx + d))) return;
-        const v3 P = ld3(x, pp), dP = ld3(p, pp);
-        if (!pt_aabb_moving(P, A, B, C, dP, dA, dB, dC, dh)) return;
-        const double d2 = pt_dist2(P, A, B, C);
-        double lb;
-        if (!pt_needs_exact(dP, dA, dB, dC, eta, d2, &lb)) return;
-        const int slot = g.vscene ? sc : 0;
-        if (!ccd_push(L.w, L.count, L.cap, CcdWork{pp, i, slot, 0, d2, lb}))
-            atomic_min_pos(alpha + slot, pt_exact_call(P, A, B, C, dP, dA, dB, dC, eta, d2, lb));
+        if (!pair_push(Q, 0, pp, i)) ccd_pair_call(a, 0, pp, i, L);
     });
 }
-__device__ __forceinline__ void ccd_ee_big(int block, const BigArgs& b, const double* __restrict__ x, const double* __restrict__ p, double dh,
-                                           double eta, const SceneGeo& g, CandView cv, const CcdList& L, unsigned long long* __restrict__ alpha) {
-    big_pairs(b, g, block, 1, 1, [&](int i, int j, int sc) {
+__device__ __forceinline__ void ccd_ee_big(int block, const BigArgs& b, const CcdArgs& a, const SceneGeo& g, CandView cv, const PairList& Q,
+                                           const CcdList& L) {
+    big_pairs(b, g, block, 1, 1, [&](int i, int j, int) {
         if (j == i || (b.edge_big[j] && j < i)) return;
-        const v3 I0 = ld3(x, b.be[2 * i]), I1 = ld3(x, b.be[2 * i + 1]), dI0 = ld3(p, b.be[2 * i]), dI1 = ld3(p, b.be[2 * i + 1]);
+        const v3 I0 = ld3(a.x, b.be[2 * i]), I1 = ld3(a.x, b.be[2 * i + 1]), dI0 = ld3(a.p, b.be[2 * i]), dI1 = ld3(a.p, b.be[2 * i + 1]);
         const v3 mn = vmin(vmin(I0, I0 + dI0), vmin(I1, I1 + dI1)), mx = vmax(vmax(I0, I0 + dI0), vmax(I1, I1 + dI1));
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(mn), f32_hi(mx))) return;
         const int lo = i < j ? i : j, hi = i < j ? j : i;
         const int a0 = b.be[2 * lo], a1 = b.be[2 * lo + 1], b0 = b.be[2 * hi], b1 = b.be[2 * hi + 1];
         if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) return;
-        const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), B0 = ld3(x, b0), B1 = ld3(x, b1);
-        const v3 dA0 = ld3(p, a0), dA1 = ld3(p, a1), dB0 = ld3(p, b0), dB1 = ld3(p, b1);
-        if (!ee_aabb_moving(A0, A1, B0, B1, dA0, dA1, dB0, dB1, dh)) return;
-        const double d2 = ee_dist2(A0, A1, B0, B1);
-        double lb;
-        if (!ee_needs_exact(dA0, dA1, dB0, dB1, eta, d2, &lb)) return;
-        const int slot = g.vscene ? sc : 0;
-        if (!ccd_push(L.w + L.cap, L.count + 1, L.cap, CcdWork{lo, hi, slot, 0, d2, lb}))
-            atomic_min_pos(alpha + slot, ee_exact_call(A0, A1, B0, B1, dA0, dA1, dB0, dB1, eta, d2, lb));
+        if (!pair_push(Q, 1, lo, hi)) ccd_pair_call(a, 1, lo, hi, L);
     });
 }
 
 // intersection check: big triangles against the edges of their scene, big edges against the triangles of
 // their scene that are not big (kind: which)
-__device__ __forceinline__ void collision_big(int block, int kind, const BigArgs& b, const double* __restrict__ x, const SceneGeo& g, CandView cv,
-                                              int* __restrict__ hit) {
-    big_pairs(b, g, block, kind, kind ? 2 : 1, [&](int i, int k, int sc) {
-        int* h = hit + (g.vscene ? sc : 0);
+__device__ __forceinline__ void collision_big(int block, int kind, const BigArgs& b, const HitArgs& a, const SceneGeo& g, CandView cv,
+                                              const PairList& P) {
+    big_pairs(b, g, block, kind, kind ? 2 : 1, [&](int i, int k, int) {
         const int e = kind ? i : k, t = kind ? k : i;
         if (kind && b.tri_big[t]) return;
         const int t0 = b.bt[3 * t], t1 = b.bt[3 * t + 1], t2 = b.bt[3 * t + 2], a0 = b.be[2 * e], a1 = b.be[2 * e + 1];
         if (a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2) return;
-        const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
+        const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2);
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)e), __ldg(cv.box + 2 * (size_t)e + 1), f32_lo(vmin(vmin(A, B), C)), f32_hi(vmax(vmax(A, B), C)))) return;
-        if (*(volatile int*)h) return;
-        if (seg_tri(ld3(x, a0), ld3(x, a1), A, B, C)) atomicOr(h, 1);
+        if (!pair_push(P, 0, e, t)) hit_pair_call(a, e, t);
     });
 }
 
@@ -832,33 +1010,27 @@ __global__ void __launch_bounds__(256) k_grid_fill(GridBuild gp, GridBuild ge, c
 struct QueryBlocks {
     int pt, ee, pt_big, ee_big;   // blocks of each pass, in this order
 };
-__global__ void __launch_bounds__(128) k_find(QueryBlocks nb, int nbt, const int* __restrict__ bt, const int* __restrict__ bp, int nbe,
-                                              const int* __restrict__ be, const double* __restrict__ x, const double* __restrict__ x0,
-                                              double dh, double dh2, SceneGeo g, GridView gp, CandView cp, GridView ge, CandView ce, BigArgs big,
-                                              RowSink sink) {
+__global__ void __launch_bounds__(128) k_find(QueryBlocks nb, int nbt, const int* __restrict__ bp, int nbe, FindArgs a, SceneGeo g, GridView gp,
+                                              CandView cp, GridView ge, CandView ce, BigArgs big, PairList P, RowSink sink) {
     int b = blockIdx.x;
-    if (b < nb.ee) return find_ee(b, nbe, be, x, x0, dh, dh2, g, ge, ce, sink);
-    if ((b -= nb.ee) < nb.pt) return find_pt(b, nbt, bt, bp, x, dh, dh2, g, gp, cp, sink);
-    if ((b -= nb.pt) < nb.pt_big) return find_pt_big(b, big, x, dh, dh2, g, cp, sink);
-    find_ee_big(b - nb.pt_big, big, x, x0, dh, dh2, g, ce, sink);
+    if (b < nb.ee) return find_ee(b, nbe, a.be, a, g, ge, ce, P, sink);
+    if ((b -= nb.ee) < nb.pt) return find_pt(b, nbt, a.bt, bp, a, g, gp, cp, P, sink);
+    if ((b -= nb.pt) < nb.pt_big) return find_pt_big(b, big, a, g, cp, P, sink);
+    find_ee_big(b - nb.pt_big, big, a, g, ce, P, sink);
 }
-__global__ void __launch_bounds__(128) k_ccd(QueryBlocks nb, int nbt, const int* __restrict__ bt, const int* __restrict__ bp, int nbe,
-                                             const int* __restrict__ be, const double* __restrict__ x, const double* __restrict__ p, double dh,
-                                             double eta, SceneGeo g, GridView gp, CandView cp, GridView ge, CandView ce, BigArgs big, CcdList L,
-                                             unsigned long long* __restrict__ alpha) {
+__global__ void __launch_bounds__(128) k_ccd(QueryBlocks nb, int nbt, const int* __restrict__ bp, int nbe, CcdArgs a, SceneGeo g, GridView gp,
+                                             CandView cp, GridView ge, CandView ce, BigArgs big, PairList P, CcdList L) {
     int b = blockIdx.x;
-    if (b < nb.ee) return ccd_ee(b, nbe, be, x, p, dh, g, eta, ge, ce, L, alpha);
-    if ((b -= nb.ee) < nb.pt) return ccd_pt(b, nbt, bt, bp, x, p, dh, g, eta, gp, cp, L, alpha);
-    if ((b -= nb.pt) < nb.pt_big) return ccd_pt_big(b, big, x, p, dh, eta, g, cp, L, alpha);
-    ccd_ee_big(b - nb.pt_big, big, x, p, dh, eta, g, ce, L, alpha);
+    if (b < nb.ee) return ccd_ee(b, nbe, a, g, ge, ce, P, L);
+    if ((b -= nb.ee) < nb.pt) return ccd_pt(b, nbt, bp, a, g, gp, cp, P, L);
+    if ((b -= nb.pt) < nb.pt_big) return ccd_pt_big(b, big, a, g, cp, P, L);
+    ccd_ee_big(b - nb.pt_big, big, a, g, ce, P, L);
 }
-__global__ void __launch_bounds__(128) k_collision(QueryBlocks nb, int nbt, const int* __restrict__ bt, const int* __restrict__ be,
-                                                   const double* __restrict__ x, double dh, SceneGeo g, GridView ge, CandView ce, BigArgs big,
-                                                   int* __restrict__ hit) {
+__global__ void __launch_bounds__(128) k_collision(QueryBlocks nb, int nbt, HitArgs a, SceneGeo g, GridView ge, CandView ce, BigArgs big, PairList P) {
     int b = blockIdx.x;
-    if (b < nb.pt) return collision_grid(b, nbt, bt, be, x, dh, g, ge, ce, hit);
-    if ((b -= nb.pt) < nb.pt_big) return collision_big(b, 0, big, x, g, ce, hit);
-    collision_big(b - nb.pt_big, 1, big, x, g, ce, hit);
+    if (b < nb.pt) return collision_grid(b, nbt, a, g, ge, ce, P);
+    if ((b -= nb.pt) < nb.pt_big) return collision_big(b, 0, big, a, g, ce, P);
+    collision_big(b - nb.pt_big, 1, big, a, g, ce, P);
 }
 
 // ---------------------------------------------------------------- row canonicalisation
@@ -957,8 +1129,6 @@ static SceneGeo geo(const fipc_ctx* c) {
     return g;
 }
 
-constexpr int EXACT_BLOCKS = 8 * 304;
-
 static unsigned long long table_size(long long entries) {
     unsigned long long size = 1024;
     while (size < 2ull * (unsigned long long)entries) size <<= 1;
@@ -976,6 +1146,7 @@ struct Broad {
     SceneGeo g;
     BigArgs big;
     GridBuild gp, ge;
+    PairList pairs;
     BroadCounters* n;
 };
 
@@ -986,6 +1157,7 @@ static int big_blocks(const fipc_ctx* c, int partners, int ny) { return nblk(c->
 // The grids over the boundary points (mode_p < 0: none) and edges at positions x (+ direction p when
 // moving), and the big primitives.  Tables start at two slots per primitive, twice over, and grow when a
 // call reports that its entries need more.
+constexpr long long PAIRS_MAX = 1ll << 24;
 static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode_p, int mode_e, Broad* b, cudaStream_t s) {
     const int n = c->nBT + c->nBE, np = mode_p < 0 ? 0 : c->nBP;
     if (c->big_flags.ensure((size_t)n + 16) || c->big_list.ensure(4ll * n + 16) || c->broad.ensure(sizeof(BroadCounters))) return FIPC_ERR_CUDA;
@@ -1011,6 +1183,10 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
     g.big_tri = tri_big;
     g.big_edge = tri_big + c->nBT;
     b->g = g;
+    // the pair lists, as long as the last calls needed
+    const long long want = std::min<long long>(std::max<long long>(65536ll + 2ll * n, c->pair_hint), PAIRS_MAX);
+    if (c->pair_list.ensure(16 * want)) return FIPC_ERR_CUDA;
+    b->pairs = PairList{c->pair_list.as<int2>(), b->n->pairs, (int)want};
     const int entries = nblk((long long)CELL_LANES * (np + c->nBE), 256);
     if (entries > 0) {
         k_grid_insert<<<entries, 256, 0, s>>>(b->gp, b->ge, x, p, c->dhat, g, b->n);
@@ -1029,6 +1205,7 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
 // after the counters of a call have reached the host: FIPC_OK, an error, or RETRY with larger tables
 constexpr int RETRY = -1;
 static int broad_status(fipc_ctx* c, const BroadCounters& h) {
+    c->pair_hint = std::max<long long>(c->pair_hint, std::min<long long>(2ll * std::max(h.pairs[0], h.pairs[1]), PAIRS_MAX));
     if (h.flags & FLAG_CELLS) return FIPC_ERR_CAPACITY;
     if (h.flags & FLAG_TABLE) {
         if (h.total[0] > (1ull << 30) || h.total[1] > (1ull << 30)) return FIPC_ERR_CAPACITY;
@@ -1079,8 +1256,11 @@ int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
         nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b.big.ny) : 0;
         const int blocks = nb.pt + nb.ee + nb.pt_big + nb.ee_big;
         if (blocks > 0) {
-            k_find<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bt, c->bp, c->nBE, c->be, x, c->x0, c->dhat, c->dhat2, b.g, view(b.gp), cands(b.gp),
-                                          view(b.ge), cands(b.ge), b.big, sink);
+            const FindArgs a{c->bt, c->be, x, c->x0, c->dhat, c->dhat2};
+            k_find<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bp, c->nBE, a, b.g, view(b.gp), cands(b.gp), view(b.ge), cands(b.ge), b.big, b.pairs,
+                                          sink);
+            FIPC_LAUNCHED();
+            k_find_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b.pairs, sink);
             FIPC_LAUNCHED();
         }
         k_rows_small<<<1, SORT_THREADS, 0, s>>>(sink.rows, b.n, c->rows_all.as<int4>());
@@ -1118,15 +1298,9 @@ static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta,
     int st = broad_prepare(c, x, p, 2, 3, b, s);
     if (st) return st;
     if (!slot) slot = &b->n->alpha;
-    CcdList L;
-    {
-        long long cap = 65536ll + c->nBE + c->nBT;
-        if (cap > (1ll << 21)) cap = 1ll << 21;
-        if (c->ccd_work.ensure(2 * cap * sizeof(CcdWork))) return FIPC_ERR_CUDA;
-        L.count = b->n->work;
-        L.w = c->ccd_work.as<CcdWork>();
-        L.cap = (int)cap;
-    }
+    const long long cap = std::min<long long>(65536ll + c->nBE + c->nBT, 1ll << 21);
+    if (c->ccd_work.ensure(4 * cap * sizeof(CcdWork))) return FIPC_ERR_CUDA;
+    const CcdList L{c->ccd_work.as<CcdWork>(), b->n->work, (int)cap}, M{L.w + 2 * cap, b->n->doubt, (int)cap};
     QueryBlocks nb{c->nBP > 0 ? nblk(c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
     nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b->big.ny) : 0;
     nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b->big.ny) : 0;
@@ -1136,10 +1310,14 @@ static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta,
     }
     const int blocks = nb.pt + nb.ee + nb.pt_big + nb.ee_big;
     if (blocks > 0) {
-        k_ccd<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bt, c->bp, c->nBE, c->be, x, p, c->dhat, eta, b->g, view(b->gp), cands(b->gp), view(b->ge),
-                                     cands(b->ge), b->big, L, slot);
+        const CcdArgs a{c->bt, c->be, x, p, c->dhat, eta, b->g.vscene, slot};
+        k_ccd<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bp, c->nBE, a, b->g, view(b->gp), cands(b->gp), view(b->ge), cands(b->ge), b->big, b->pairs, L);
         FIPC_LAUNCHED();
-        k_ccd_exact<<<EXACT_BLOCKS, 128, 0, s>>>(c->bt, c->be, x, p, eta, L, slot);
+        k_ccd_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b->pairs, L);
+        FIPC_LAUNCHED();
+        k_ccd_signs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, L, M);
+        FIPC_LAUNCHED();
+        k_ccd_exact<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, M);
         FIPC_LAUNCHED();
     }
     FIPC_CUDA(cudaGetLastError());
@@ -1180,7 +1358,10 @@ int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStr
         }
         const int blocks = nb.pt + nb.pt_big + nb.ee_big;
         if (blocks > 0) {
-            k_collision<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bt, c->be, x, c->dhat, b.g, view(b.ge), cands(b.ge), b.big, hit);
+            const HitArgs a{c->bt, c->be, x, b.g.vscene, hit};
+            k_collision<<<blocks, 128, 0, s>>>(nb, c->nBT, a, b.g, view(b.ge), cands(b.ge), b.big, b.pairs);
+            FIPC_LAUNCHED();
+            k_collision_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b.pairs);
             FIPC_LAUNCHED();
         }
         FIPC_CUDA(cudaGetLastError());

@@ -65,27 +65,88 @@ FIPC_HD double bracketed_root(const double* p, int k, double a, double b, double
     return t;
 }
 
-// Sign changes of the Bernstein coefficients of op (degree n <= 6, coefficients at most 1 in magnitude)
-// on [0, 1]: by Descartes' rule in that basis 0 means no root in [0, 1] and 1 exactly one, in (0, 1).
-// -1 when a coefficient is too close to zero for its sign to be certain (their rounding errors stay
-// below 1e-14).  Most polynomials of a pair have 0 or 1, and a pair's time on the GPU is the length of
-// its dependent chain (step filter of a
-// 134k-tet bar: 1.59 -> 1.04 ms with the other changes of its queries).
-FIPC_HD int bernstein_changes(const double* op, int n) {
-    double c[7];
-    double binom = 1.0;   // C(n, j)
-    for (int j = 0; j <= n; ++j) {
-        c[j] = op[n - j] / binom;
-        binom = binom * (double)(n - j) / (double)(j + 1);
-    }
-    for (int r = 1; r <= n; ++r)
-        for (int i = n; i >= r; --i) c[i] += c[i - 1];
+// Root isolation on [0, 1] in the Bernstein basis, for polynomials of degree n <= 6 with coefficients of
+// at most 1 in magnitude, written as degree 6: by Descartes' rule in that basis no sign change among the
+// coefficients means no root in the segment and one exactly one.  Segments with more are halved
+// (de Casteljau).  A coefficient within BERNSTEIN_EPS of zero (their rounding errors stay below 1e-14) leaves
+// the answer open.  Most polynomials of a pair have 0 or 1 change, those of a pair that approaches and
+// leaves 2; bracketing by the roots of all derivatives instead (roots01) is a chain of up to twenty
+// Newton iterations, which one thread of the step filter runs for tens of microseconds each.
+constexpr double BERNSTEIN_EPS = 1e-11;
+FIPC_HD void bernstein6(const double* op, int n, double (&p)[7], double (&c)[7]) {
+#pragma unroll
+    for (int i = 0; i < 7; ++i) p[i] = i < 6 - n ? 0.0 : op[i - (6 - n)];
+    c[0] = p[6];
+    c[1] = p[5] * (1.0 / 6.0);
+    c[2] = p[4] * (1.0 / 15.0);
+    c[3] = p[3] * (1.0 / 20.0);
+    c[4] = p[2] * (1.0 / 15.0);
+    c[5] = p[1] * (1.0 / 6.0);
+    c[6] = p[0];
+#pragma unroll
+    for (int r = 1; r <= 6; ++r)
+#pragma unroll
+        for (int i = 6; i >= r; --i) c[i] += c[i - 1];
+}
+// sign changes; -1 when a sign is uncertain
+FIPC_HD int bernstein_changes(const double (&c)[7]) {
     int changes = 0;
-    for (int i = 0; i <= n; ++i) {
-        if (!(fabs(c[i]) > 1e-11)) return -1;
+    bool sure = true;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        sure = sure && fabs(c[i]) > BERNSTEIN_EPS;
         if (i > 0 && (c[i] < 0.0) != (c[i - 1] < 0.0)) ++changes;
     }
-    return changes;
+    return sure ? changes : -1;
+}
+// op (as given to find_intervals) certainly has the wrong sign, or no sign, all over [0, 1]
+FIPC_HD bool surely_empty(const double* op, int n, bool pos) {
+    double maxval = 0;
+    for (int i = 0; i <= n; ++i) maxval = fmax(maxval, fabs(op[i]));
+    if (!(maxval > 0)) return false;
+    const double inv = 1.0 / maxval;
+    double q[7], p[7], c[7];
+    for (int i = 0; i <= n; ++i) q[i] = op[i] * inv;
+    bernstein6(q, n, p, c);
+    return bernstein_changes(c) == 0 && (c[0] < 0.0) == pos;
+}
+// the roots in [0, 1], ascending; -1 when a sign is uncertain or DEPTH halvings do not separate them
+FIPC_HD int bernstein_roots(const double* op, int n, double* out) {
+    constexpr int DEPTH = 10;
+    double p[7], c[7], stack[DEPTH][7], ends[DEPTH];
+    int level[DEPTH];
+    bernstein6(op, n, p, c);
+    double a = 0.0, b = 1.0;
+    int depth = 0, top = 0, roots = 0;
+    for (;;) {
+        const int changes = bernstein_changes(c);
+        if (changes < 0) return -1;
+        if (changes > 1) {
+            if (depth == DEPTH) return -1;
+            ++depth;
+            // left half into c, right half onto the stack (its coefficients are the last of each round)
+#pragma unroll
+            for (int r = 1; r <= 6; ++r) {
+                stack[top][7 - r] = c[6];
+#pragma unroll
+                for (int i = 6; i >= r; --i) c[i] = 0.5 * (c[i] + c[i - 1]);
+            }
+            stack[top][0] = c[6];
+            ends[top] = b;
+            level[top] = depth;
+            ++top;
+            b = 0.5 * (a + b);
+            continue;
+        }
+        if (changes == 1) out[roots++] = bracketed_root(p, 6, a, b, c[0]);
+        if (top == 0) return roots;
+        --top;
+        a = b;
+        b = ends[top];
+        depth = level[top];
+#pragma unroll
+        for (int i = 0; i < 7; ++i) c[i] = stack[top][i];
+    }
 }
 
 // real roots in [0,1] of op (degree n <= 6, op[0] != 0), ascending; returns the count
@@ -183,13 +244,8 @@ FIPC_HD void find_intervals(double* op, int n, Ivl* iv, int* niv, bool pos) {
     int roots = 0;
     if (rd > 2) {
         if (!could_have_roots(op, rd, pos)) return;
-        const int changes = bernstein_changes(op, rd);
-        if (changes == 1) {
-            tm[0] = bracketed_root(op, rd, 0.0, 1.0, op[rd]);
-            roots = 1;
-        } else if (changes != 0) {
-            roots = roots01(op, rd, tm);
-        }
+        roots = bernstein_roots(op, rd, tm);
+        if (roots < 0) roots = roots01(op, rd, tm);
     } else if (rd == 2) {
         roots = quad_roots(op[0], op[1], op[2], &tm[0], &tm[1]);
     } else if (rd == 1) {
@@ -217,36 +273,32 @@ FIPC_HD void find_intervals(double* op, int n, Ivl* iv, int* niv, bool pos) {
 
 FIPC_HD double triple3(v3 a, v3 b, v3 c) { return dot(a, cross(b, c)); }
 
-FIPC_HD void bary_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, Ivl* iv, int* niv) {
+// the coefficients of the three kinds of polynomials (degrees 4, 3, 6; the sign looked for: +, +, -)
+FIPC_HD void bary_coefficients(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, double* op) {
     const double A = dot(x10, x10), B = 2 * dot(x10, v10), C = dot(v10, v10);
     const double D = dot(x20, x10), E = dot(x20, v10) + dot(v20, x10), F = dot(v20, v10);
     const double G = dot(x30, x20), H = dot(x30, v20) + dot(v30, x20), I = dot(v30, v20);
     const double J = dot(x30, x10), K = dot(x30, v10) + dot(v30, x10), L = dot(v30, v10);
-    double op[5];
     op[0] = F * L - C * I;
     op[1] = F * K + E * L - C * H - B * I;
     op[2] = F * J + D * L + E * K - C * G - A * I - B * H;
     op[3] = D * K + E * J - A * H - B * G;
     op[4] = D * J - A * G;
-    find_intervals(op, 4, iv, niv, true);
 }
 
-FIPC_HD void plane_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, Ivl* iv, int* niv) {
-    double op[4];
+FIPC_HD void plane_coefficients(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, double* op) {
     op[0] = triple3(v10, v20, v30);
     op[1] = triple3(x10, v20, v30) + triple3(v10, x20, v30) + triple3(v10, v20, x30);
     op[2] = triple3(x10, x20, v30) + triple3(x10, v20, x30) + triple3(v10, x20, x30);
     op[3] = triple3(x10, x20, x30);
-    find_intervals(op, 3, iv, niv, true);
 }
 
-FIPC_HD void distance_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, double minD2, Ivl* iv, int* niv) {
+FIPC_HD void distance_coefficients(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, double minD2, double* op) {
     const double A = triple3(v10, v20, v30);
     const double B = triple3(x10, v20, v30) + triple3(v10, x20, v30) + triple3(v10, v20, x30);
     const double C = triple3(x10, x20, v30) + triple3(x10, v20, x30) + triple3(v10, x20, x30);
     const double D = triple3(x10, x20, x30);
     const v3 E = cross(x20, x30), F = cross(x20, v30) + cross(v20, x30), G = cross(v20, v30);
-    double op[7];
     op[0] = A * A;
     op[1] = 2 * A * B;
     op[2] = B * B + 2 * A * C - dot(G, G) * minD2;
@@ -254,6 +306,20 @@ FIPC_HD void distance_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, doubl
     op[4] = 2 * B * D + C * C - (2 * dot(G, E) + dot(F, F)) * minD2;
     op[5] = 2 * C * D - 2 * dot(F, E) * minD2;
     op[6] = D * D - dot(E, E) * minD2;
+}
+FIPC_HD void bary_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, Ivl* iv, int* niv) {
+    double op[5];
+    bary_coefficients(x10, x20, x30, v10, v20, v30, op);
+    find_intervals(op, 4, iv, niv, true);
+}
+FIPC_HD void plane_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, Ivl* iv, int* niv) {
+    double op[4];
+    plane_coefficients(x10, x20, x30, v10, v20, v30, op);
+    find_intervals(op, 3, iv, niv, true);
+}
+FIPC_HD void distance_poly(v3 x10, v3 x20, v3 x30, v3 v10, v3 v20, v3 v30, double minD2, Ivl* iv, int* niv) {
+    double op[7];
+    distance_coefficients(x10, x20, x30, v10, v20, v30, minD2, op);
     find_intervals(op, 6, iv, niv, false);
 }
 
@@ -272,20 +338,8 @@ FIPC_HD Ivl intersect_all(const Ivl* v, int n) {
     return r;
 }
 
-// CTCD.cpp:383-472
-FIPC_HD bool vertex_face_ctcd(v3 q0s, v3 q1s, v3 q2s, v3 q3s, v3 q0e, v3 q1e, v3 q2e, v3 q3e, double eta, double* t) {
-    const double minD = eta * eta;
-    const v3 v0 = q0e - q0s, v1 = q1e - q1s, v2 = q2e - q2s, v3_ = q3e - q3s;
-    Ivl cp[8], e1[8], e2[8], e3[8];
-    int ncp, ne1, ne2, ne3;
-    plane_poly(q0s - q1s, cross(q3s - q1s, q2s - q1s), q3s - q1s, v0 - v1, cross(v3_ - v1, v2 - v1), v3_ - v1, e1, &ne1);
-    if (!ne1) return false;
-    plane_poly(q0s - q2s, cross(q1s - q2s, q3s - q2s), q1s - q2s, v0 - v2, cross(v1 - v2, v3_ - v2), v1 - v2, e2, &ne2);
-    if (!ne2) return false;
-    plane_poly(q0s - q3s, cross(q2s - q3s, q1s - q3s), q2s - q3s, v0 - v3_, cross(v2 - v3_, v1 - v3_), v2 - v3_, e3, &ne3);
-    if (!ne3) return false;
-    distance_poly(q0s - q1s, q2s - q1s, q3s - q1s, v0 - v1, v2 - v1, v3_ - v1, minD, cp, &ncp);
-    if (!ncp) return false;
+// the earliest common start of the coplanarity and side intervals; false when they never meet
+FIPC_HD bool vertex_face_meet(const Ivl* cp, int ncp, const Ivl* e1, int ne1, const Ivl* e2, int ne2, const Ivl* e3, int ne3, double* t) {
     bool col = false;
     double mint = 1.0;
     for (int i = 0; i < ncp; ++i)
@@ -302,31 +356,36 @@ FIPC_HD bool vertex_face_ctcd(v3 q0s, v3 q1s, v3 q2s, v3 q3s, v3 q0e, v3 q1e, v3
     return col;
 }
 
-// CTCD.cpp:245-381
-FIPC_HD bool edge_edge_ctcd(v3 q0s, v3 p0s, v3 q1s, v3 p1s, v3 q0e, v3 p0e, v3 q1e, v3 p1e, double eta, double* t) {
+// CTCD.cpp:383-472
+FIPC_HD bool vertex_face_ctcd(v3 q0s, v3 q1s, v3 q2s, v3 q3s, v3 q0e, v3 q1e, v3 q2e, v3 q3e, double eta, double* t) {
     const double minD = eta * eta;
-    Ivl raw[8], cp[8], par[8], a0[8], a1[8], b0[8], b1[8];
-    int nraw, ncp = 0, npar = 0, na0, na1, nb0, nb1;
-    const v3 vp0 = p0e - p0s, vp1 = p1e - p1s, vq0 = q0e - q0s, vq1 = q1e - q1s;
-    distance_poly(p0s - p1s, p0s - q0s, p1s - q1s, vp0 - vp1, vp0 - vq0, vp1 - vq1, minD, raw, &nraw);
+    const v3 v0 = q0e - q0s, v1 = q1e - q1s, v2 = q2e - q2s, v3_ = q3e - q3s;
+    Ivl cp[8], e1[8], e2[8], e3[8];
+    int ncp, ne1, ne2, ne3;
+    plane_poly(q0s - q1s, cross(q3s - q1s, q2s - q1s), q3s - q1s, v0 - v1, cross(v3_ - v1, v2 - v1), v3_ - v1, e1, &ne1);
+    if (!ne1) return false;
+    plane_poly(q0s - q2s, cross(q1s - q2s, q3s - q2s), q1s - q2s, v0 - v2, cross(v1 - v2, v3_ - v2), v1 - v2, e2, &ne2);
+    if (!ne2) return false;
+    plane_poly(q0s - q3s, cross(q2s - q3s, q1s - q3s), q2s - q3s, v0 - v3_, cross(v2 - v3_, v1 - v3_), v2 - v3_, e3, &ne3);
+    if (!ne3) return false;
+    distance_poly(q0s - q1s, q2s - q1s, q3s - q1s, v0 - v1, v2 - v1, v3_ - v1, minD, cp, &ncp);
+    if (!ncp) return false;
+    return vertex_face_meet(cp, ncp, e1, ne1, e2, ne2, e3, ne3, t);
+}
+
+// the time intervals on which two edges are within the distance but parallel go to par, the others to cp
+FIPC_HD void split_parallel(const Ivl* raw, int nraw, v3 x0, v3 v0, v3 x1, v3 v1, Ivl* cp, int* ncp, Ivl* par, int* npar) {
+    *ncp = *npar = 0;
     for (int i = 0; i < nraw; ++i) {
         const double midt = (raw[i].u + raw[i].l) / 2;
-        const v3 x10 = (q0s - p0s) + midt * (vq0 - vp0), x20 = (q1s - p1s) + midt * (vq1 - vp1);
-        if (sqrt(sq(cross(x10, x20))) < 1e-8) par[npar++] = raw[i];
-        else cp[ncp++] = raw[i];
+        const v3 x10 = x0 + midt * v0, x20 = x1 + midt * v1;
+        if (sqrt(sq(cross(x10, x20))) < 1e-8) par[(*npar)++] = raw[i];
+        else cp[(*ncp)++] = raw[i];
     }
-    if (!ncp) return false;
-    v3 x10 = p1s - q1s, v10 = vp1 - vq1;
-    bary_poly(x10, p0s - q0s, q0s - q1s, v10, vp0 - vq0, vq0 - vq1, a0, &na0);
-    if (!na0) return false;
-    bary_poly(x10, q0s - p0s, p0s - q1s, v10, vq0 - vp0, vp0 - vq1, a1, &na1);
-    if (!na1) return false;
-    x10 = p0s - q0s;
-    v10 = vp0 - vq0;
-    bary_poly(x10, p1s - q1s, q1s - q0s, v10, vp1 - vq1, vq1 - vq0, b0, &nb0);
-    if (!nb0) return false;
-    bary_poly(x10, q1s - p1s, p1s - q0s, v10, vq1 - vp1, vp1 - vq0, b1, &nb1);
-    if (!nb1) return false;
+}
+// the earliest common start of the distance and barycentric intervals outside the parallel ones
+FIPC_HD bool edge_edge_meet(const Ivl* cp, int ncp, const Ivl* par, int npar, const Ivl* a0, int na0, const Ivl* a1, int na1, const Ivl* b0,
+                            int nb0, const Ivl* b1, int nb1, double* t) {
     bool col = false;
     double mint = 1.0;
     for (int i = 0; i < ncp; ++i)
@@ -349,6 +408,58 @@ FIPC_HD bool edge_edge_ctcd(v3 q0s, v3 p0s, v3 q1s, v3 p1s, v3 q0e, v3 p0e, v3 q
                     }
     if (col) *t = mint;
     return col;
+}
+
+// CTCD.cpp:245-381
+FIPC_HD bool edge_edge_ctcd(v3 q0s, v3 p0s, v3 q1s, v3 p1s, v3 q0e, v3 p0e, v3 q1e, v3 p1e, double eta, double* t) {
+    const double minD = eta * eta;
+    Ivl raw[8], cp[8], par[8], a0[8], a1[8], b0[8], b1[8];
+    int nraw, ncp, npar, na0, na1, nb0, nb1;
+    const v3 vp0 = p0e - p0s, vp1 = p1e - p1s, vq0 = q0e - q0s, vq1 = q1e - q1s;
+    distance_poly(p0s - p1s, p0s - q0s, p1s - q1s, vp0 - vp1, vp0 - vq0, vp1 - vq1, minD, raw, &nraw);
+    split_parallel(raw, nraw, q0s - p0s, vq0 - vp0, q1s - p1s, vq1 - vp1, cp, &ncp, par, &npar);
+    if (!ncp) return false;
+    v3 x10 = p1s - q1s, v10 = vp1 - vq1;
+    bary_poly(x10, p0s - q0s, q0s - q1s, v10, vp0 - vq0, vq0 - vq1, a0, &na0);
+    if (!na0) return false;
+    bary_poly(x10, q0s - p0s, p0s - q1s, v10, vq0 - vp0, vp0 - vq1, a1, &na1);
+    if (!na1) return false;
+    x10 = p0s - q0s;
+    v10 = vp0 - vq0;
+    bary_poly(x10, p1s - q1s, q1s - q0s, v10, vp1 - vq1, vq1 - vq0, b0, &nb0);
+    if (!nb0) return false;
+    bary_poly(x10, q1s - p1s, p1s - q0s, v10, vq1 - vp1, vp1 - vq0, b1, &nb1);
+    if (!nb1) return false;
+    return edge_edge_meet(cp, ncp, par, npar, a0, na0, a1, na1, b0, nb0, b1, nb1, t);
+}
+
+// Certainly no collision over the step, by the signs of one of the polynomials' Bernstein coefficients
+// (q*s: start, q*e: end positions as in the exact tests)
+FIPC_HD bool vertex_face_apart(v3 q0s, v3 q1s, v3 q2s, v3 q3s, v3 q0e, v3 q1e, v3 q2e, v3 q3e, double eta) {
+    const v3 v0 = q0e - q0s, v1 = q1e - q1s, v2 = q2e - q2s, v3_ = q3e - q3s;
+    double op[7];
+    distance_coefficients(q0s - q1s, q2s - q1s, q3s - q1s, v0 - v1, v2 - v1, v3_ - v1, eta * eta, op);
+    if (surely_empty(op, 6, false)) return true;
+    plane_coefficients(q0s - q1s, cross(q3s - q1s, q2s - q1s), q3s - q1s, v0 - v1, cross(v3_ - v1, v2 - v1), v3_ - v1, op);
+    if (surely_empty(op, 3, true)) return true;
+    plane_coefficients(q0s - q2s, cross(q1s - q2s, q3s - q2s), q1s - q2s, v0 - v2, cross(v1 - v2, v3_ - v2), v1 - v2, op);
+    if (surely_empty(op, 3, true)) return true;
+    plane_coefficients(q0s - q3s, cross(q2s - q3s, q1s - q3s), q2s - q3s, v0 - v3_, cross(v2 - v3_, v1 - v3_), v2 - v3_, op);
+    return surely_empty(op, 3, true);
+}
+FIPC_HD bool edge_edge_apart(v3 q0s, v3 p0s, v3 q1s, v3 p1s, v3 q0e, v3 p0e, v3 q1e, v3 p1e, double eta) {
+    const v3 vp0 = p0e - p0s, vp1 = p1e - p1s, vq0 = q0e - q0s, vq1 = q1e - q1s;
+    double op[7];
+    distance_coefficients(p0s - p1s, p0s - q0s, p1s - q1s, vp0 - vp1, vp0 - vq0, vp1 - vq1, eta * eta, op);
+    if (surely_empty(op, 6, false)) return true;
+    bary_coefficients(p1s - q1s, p0s - q0s, q0s - q1s, vp1 - vq1, vp0 - vq0, vq0 - vq1, op);
+    if (surely_empty(op, 4, true)) return true;
+    bary_coefficients(p1s - q1s, q0s - p0s, p0s - q1s, vp1 - vq1, vq0 - vp0, vp0 - vq1, op);
+    if (surely_empty(op, 4, true)) return true;
+    bary_coefficients(p0s - q0s, p1s - q1s, q1s - q0s, vp0 - vq0, vp1 - vq1, vq1 - vq0, op);
+    if (surely_empty(op, 4, true)) return true;
+    bary_coefficients(p0s - q0s, q1s - p1s, p1s - q0s, vp0 - vq0, vq1 - vp1, vp1 - vq0, op);
+    return surely_empty(op, 4, true);
 }
 
 // The additive lower bound of wrapper.cpp:254-328: lb = (1 - eta) sqrt(dist2) / maxDisp is the

@@ -118,7 +118,9 @@ struct fipc_ctx_impl {
     int* prim_off = nullptr;
     int max_prims[3] = {0, 0, 0};         // the largest of a scene's points, edges, triangles
     DBuf big_flags, big_list, broad;      // broad: the counters of a broad-phase call
-    DBuf ccd_work;                        // step filter: pairs left to the exact test
+    DBuf ccd_work;                        // step filter: pairs that pass its first two tests
+    DBuf pair_list;                       // candidate pairs of a query
+    long long pair_hint = 0;              // list length for the next query, from what the last ones needed
     std::vector<double> h_kappa, h_inv_dx;
     // batched PCG: tiles of consecutive rows inside one scene
     int n_tiles = 0, tile_rows = 0, pcg_grid = 0;
