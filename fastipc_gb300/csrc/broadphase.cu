@@ -15,8 +15,8 @@
 // A call is a chain of a few kernels and one copy to the host at its end: table and row capacities are
 // kept from call to call and checked on the device; a call that outgrows them is repeated with larger
 // ones.  Measured on a GB300 against radix-sorted grids, one sort per list and a host round trip per grid:
-// constraint finding of two touching cubes (1,458 vertices) 1.16 -> 0.22 ms a call, of a pile of 180 cubes
-// 5.2 -> 1.0 ms; the step filter of the cubes 2.2 -> 0.64 ms.
+// constraint finding of two touching cubes (1,458 vertices) 1.16 -> 0.16 ms a call, of a pile of 180 cubes
+// 5.2 -> 0.81 ms; the step filter of the cubes 2.2 -> 0.55 ms.
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
@@ -43,11 +43,6 @@ __device__ __forceinline__ C3 cmax(C3 a, C3 b) { return C3{a.x > b.x ? a.x : b.x
 __device__ __forceinline__ unsigned long long gkey(const SceneGeo& g, int s, long long cx, long long cy, long long cz) {
     return g.vscene ? cell_key_scene(s, cx, cy, cz) : cell_key(cx, cy, cz);
 }
-// first vertex of stored primitive i (its scene)
-__device__ __forceinline__ int prim_vertex(int mode, int i, const int* __restrict__ prim) {
-    return (mode == 0 || mode == 2) ? prim[i] : prim[2 * i];
-}
-
 // Box modes of stored primitives:
 //  0 point [p - dh, p + dh]               (find constraints, point-triangle)
 //  1 edge  [min, max]                      (find constraints, edge-edge)
@@ -89,7 +84,8 @@ constexpr long long MAX_CELLS_PER_PRIM = 1ll << 22;
 // reject most candidates without FP64 work (GB300 issues FP64 at a small fraction of its FP32
 // rate):
 //  * cell: cell_of(stored lower corner), the first-cell test of the queries' pair
-//    de-duplication, computed with the same FP64 expression;
+//    de-duplication, computed with the same FP64 expression; ext: the number of cells per axis
+//    (0: not stored) and the scene, so that filling the table needs no FP64 work either;
 //  * box: an FP32 box rounded outward around the FP64 box that the query's own FP64 test
 //    compares against: mode 0 the point; 1 and 3 the (moving) edge box +- dh (ee_aabb,
 //    ee_aabb_moving); 2 the moving point's box (pt_aabb_moving); 4 the edge box +- dh (the
@@ -134,6 +130,22 @@ struct CandView {
     const int4* cell;
     const float4* box;
 };
+// the queries' records: the lowest cell of the query box and its cells per axis (10 bits each; 0 for a big
+// primitive), the FP32 box that candidates are tested against and the scene (in box[2 i].w)
+struct QueryView {
+    int4* cell;
+    float4* box;
+};
+__device__ __forceinline__ void query_record(const QueryView& q, int i, int sc, bool big, C3 lo, C3 hi, v3 blo, v3 bhi) {
+    const long long nx = hi.x - lo.x + 1, ny = hi.y - lo.y + 1, nz = hi.z - lo.z + 1;
+    // at most BIG_CELLS cells unless a position is not finite
+    const bool any = !big && nx > 0 && ny > 0 && nz > 0 && nx < 1024 && ny < 1024 && nz < 1024;
+    q.cell[i] = make_int4(clamp_cell(lo.x), clamp_cell(lo.y), clamp_cell(lo.z), any ? (int)(nx | ny << 10 | nz << 20) : 0);
+    float4 l = f32_lo(blo);
+    l.w = __int_as_float(sc);
+    q.box[2 * (size_t)i] = l;
+    q.box[2 * (size_t)i + 1] = f32_hi(bhi);
+}
 
 // Cell table of a grid: open addressing with linear probing, load factor at most 1/2, so a query cell
 // costs one or two probes.  run[slot] = (first id, ids) of the slot's cell.
@@ -164,11 +176,51 @@ struct GridView {
     }
 };
 
-// lanes per edge-edge constraint, edge-edge CCD and intersection query: a few lanes share each
-// cell's candidates.  One thread per query leaves most lanes idle in the FP64 narrow phase; a
-// whole warp repeats the cell walk in every lane while most cells hold a handful of candidates.
-// The point-triangle queries, whose cells hold fewer candidates, keep one thread per query.
+// A grid query: f(i, j) for query i and every stored primitive j of its cells whose FP32 box it overlaps, each
+// once (in the lowest cell of the two ranges' overlap).  QG lanes per query look its cells up side by side,
+// eight at a time, and then share all their candidates: a cell holds a handful of candidates and a box a few
+// to BIG_CELLS cells, and each look-up and each candidate is a chain of dependent loads, so one cell after
+// the other leaves lanes idle and makes a wide box the kernel's tail (a batch of 64 scenes: 1.24 ms with
+// SMs busy 57% of it; 0.66 so).  ORDERED: pairs within one list, only those with i < j.
 constexpr int QG = 8;
+template <bool ORDERED, class F>
+__device__ __forceinline__ void grid_walk(int block, int n, const QueryView& qv, const SceneGeo& g, const GridView& gv, const CandView& cv, F f) {
+    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
+    if (i >= n) return;
+    const int4 qc = __ldg(qv.cell + i);
+    if (qc.w == 0) return;
+    const float4 qlo = __ldg(qv.box + 2 * (size_t)i), qhi = __ldg(qv.box + 2 * (size_t)i + 1);
+    const int sc = __float_as_int(qlo.w);
+    const int nx = qc.w & 1023, ny = qc.w >> 10 & 1023, nz = qc.w >> 20, cells = nx * ny * nz;
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    for (int c0 = 0; c0 < cells; c0 += QG) {
+        const int c = c0 + lane, z = c % nz, y = c / nz % ny, x = c / nz / ny;
+        const int2 run = c < cells ? gv.find(gkey(g, sc, (long long)qc.x + x, (long long)qc.y + y, (long long)qc.z + z)) : make_int2(0, 0);
+        int upto = run.y;   // candidates in the cells up to this lane's
+#pragma unroll
+        for (int o = 1; o < QG; o <<= 1) {
+            const int v = __shfl_up_sync(group, upto, o, QG);
+            if (lane >= o) upto += v;
+        }
+        const int total = __shfl_sync(group, upto, QG - 1, QG), base = run.x - (upto - run.y), packed = x | y << 10 | z << 20;
+        for (int q0 = 0; q0 < total; q0 += QG) {
+            const int q = q0 + lane;
+            int o = 0;   // the cell of candidate q: cells whose count is used up
+#pragma unroll
+            for (int st = QG / 2; st > 0; st >>= 1)
+                if (__shfl_sync(group, upto, o + st - 1, QG) <= q) o += st;
+            const int at = __shfl_sync(group, base, o, QG) + q, cell = __shfl_sync(group, packed, o, QG);
+            if (q >= total) continue;
+            const int j = __ldg(gv.ids + at);
+            if (ORDERED && !(i < j)) continue;
+            const int4 pc = __ldg(cv.cell + j);
+            if (max(qc.x, pc.x) != qc.x + (cell & 1023) || max(qc.y, pc.y) != qc.y + (cell >> 10 & 1023) || max(qc.z, pc.z) != qc.z + (cell >> 20))
+                continue;
+            if (!f32_overlap(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), qlo, qhi)) continue;
+            f(i, j);
+        }
+    }
+}
 
 // ---------------------------------------------------------------- constraint rows
 // A row as a sort key: list (3 bits) and vertex ids (21 bits each, n_verts < 2^21), so that the order of
@@ -319,70 +371,26 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_find_pairs(FindArgs a, PairLis
     each_pair(L, [&](int kind, int2 q) { find_pair(a, kind, q.x, q.y, s); });
 }
 
-// one thread per boundary triangle; points hashed with mode 0
-__device__ __forceinline__ void find_pt(int block, int nbt, const int* __restrict__ bt, const int* __restrict__ bp,
-                                                 const FindArgs& fa, const SceneGeo& g, const GridView& gv, const CandView& cv,
-                                                 const PairList& L, const RowSink& sink) {
-    const double* x = fa.x;
-    const int i = block * 128 + threadIdx.x;
-    if (i >= nbt) return;
-    if (g.big_tri && g.big_tri[i]) return;
-    const int t0 = bt[3 * i], t1 = bt[3 * i + 1], t2 = bt[3 * i + 2];
-    const int sc = g.scene(t0);
-    const double inv_dx = g.idx(sc);
-    const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
-    const v3 tmn = vmin(vmin(A, B), C), tmx = vmax(vmax(A, B), C);
-    const C3 lo = cell_of(tmn, inv_dx), hi = cell_of(tmx, inv_dx);
-    const v3 d = mk(fa.dh, fa.dh, fa.dh);
-    const float4 qlo = f32_lo(tmn - d), qhi = f32_hi(tmx + d);   // pt_aabb's triangle box
-    for (long long cx = lo.x; cx <= hi.x; ++cx)
-        for (long long cy = lo.y; cy <= hi.y; ++cy)
-            for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
-                for (int k = run.x; k < run.x + run.y; ++k) {
-                    const int j = gv.ids[k];
-                    const int4 pc = __ldg(cv.cell + j);
-                    const C3 first = cmax(lo, C3{pc.x, pc.y, pc.z});
-                    if (first.x != cx || first.y != cy || first.z != cz) continue;
-                    if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
-                    const int p = bp[j];
-                    if (p == t0 || p == t1 || p == t2) continue;
-                    if (!pair_push(L, 0, p, i)) find_pair_call(fa, 0, p, i, sink);
-                }
-            }
+// triangles query points hashed with mode 0 (their box against pt_aabb's, the point's +- dh), edges edges
+// hashed with mode 1 (query box +- dh)
+__device__ __forceinline__ void find_pt(int block, int nbt, const int* __restrict__ bp, const FindArgs& a, const QueryView& qv,
+                                        const SceneGeo& g, const GridView& gv, const CandView& cv, const PairList& L, const RowSink& sink) {
+    grid_walk<false>(block, nbt, qv, g, gv, cv, [&](int i, int j) {
+        const int p = bp[j];
+        if (p == a.bt[3 * i] || p == a.bt[3 * i + 1] || p == a.bt[3 * i + 2]) return;
+        if (!pair_push(L, 0, p, i)) find_pair_call(a, 0, p, i, sink);
+    });
 }
-
-// one thread per boundary edge (query, box +- dh); stored edges hashed with mode 1
-__device__ __forceinline__ void find_ee(int block, int nbe, const int* __restrict__ be, const FindArgs& fa, const SceneGeo& g,
-                                        const GridView& gv, const CandView& cv, const PairList& L, const RowSink& sink) {
-    const double* x = fa.x;
-    // QG lanes per query edge share the candidates of each cell
-    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
-    if (i >= nbe) return;
-    if (g.big_edge && g.big_edge[i]) return;
-    const int a0 = be[2 * i], a1 = be[2 * i + 1];
-    const int sc = g.scene(a0);
-    const double inv_dx = g.idx(sc);
-    const v3 A0 = ld3(x, a0), A1 = ld3(x, a1);
-    const v3 d = mk(fa.dh, fa.dh, fa.dh);
-    const C3 lo = cell_of(vmin(A0, A1) - d, inv_dx), hi = cell_of(vmax(A0, A1) + d, inv_dx);
-    const float4 qlo = f32_lo(vmin(A0, A1)), qhi = f32_hi(vmax(A0, A1));   // ee_aabb's query edge box
-    for (long long cx = lo.x; cx <= hi.x; ++cx)
-        for (long long cy = lo.y; cy <= hi.y; ++cy)
-            for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
-                for (int k = run.x + lane; k < run.x + run.y; k += QG) {
-                    const int j = gv.ids[k];
-                    if (!(i < j)) continue;
-                    const int4 sc4 = __ldg(cv.cell + j);
-                    const C3 first = cmax(lo, C3{sc4.x, sc4.y, sc4.z});
-                    if (first.x != cx || first.y != cy || first.z != cz) continue;
-                    if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
-                    const int b0 = be[2 * j], b1 = be[2 * j + 1];
-                    if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) continue;
-                    if (!pair_push(L, 1, i, j)) find_pair_call(fa, 1, i, j, sink);
-                }
-            }
+__device__ __forceinline__ bool edges_touch(const int* __restrict__ be, int i, int j) {
+    const int a0 = be[2 * i], a1 = be[2 * i + 1], b0 = be[2 * j], b1 = be[2 * j + 1];
+    return a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1;
+}
+__device__ __forceinline__ void find_ee(int block, int nbe, const FindArgs& a, const QueryView& qv, const SceneGeo& g, const GridView& gv,
+                                        const CandView& cv, const PairList& L, const RowSink& sink) {
+    grid_walk<true>(block, nbe, qv, g, gv, cv, [&](int i, int j) {
+        if (edges_touch(a.be, i, j)) return;
+        if (!pair_push(L, 1, i, j)) find_pair_call(a, 1, i, j, sink);
+    });
 }
 
 // ---------------------------------------------------------------- CCD step filter
@@ -590,73 +598,22 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_ccd_exact(CcdArgs a, CcdList M
     }
 }
 
-// compute_filter_3D_PT (NEWTON_IPC.py:377-406): triangles query their moving bbox
-__device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict__ bp, const CcdArgs& a, const SceneGeo& g,
+// compute_filter_3D_PT (NEWTON_IPC.py:377-406): triangles query their moving bbox; compute_filter_3D_EE
+// (409-440): edges query moving bbox +- dh
+__device__ __forceinline__ void ccd_pt(int block, int nbt, const int* __restrict__ bp, const CcdArgs& a, const QueryView& qv, const SceneGeo& g,
                                        const GridView& gv, const CandView& cv, const PairList& P, const CcdList& L) {
-    const int i = block * 128 + threadIdx.x;
-    if (i >= nbt) return;
-    if (g.big_tri && g.big_tri[i]) return;
-    const double *x = a.x, *p = a.p;
-    const int t0 = a.bt[3 * i], t1 = a.bt[3 * i + 1], t2 = a.bt[3 * i + 2];
-    const int sc = g.scene(t0);
-    const double inv_dx = g.idx(sc);
-    const v3 A = ld3(x, t0), B = ld3(x, t1), C = ld3(x, t2);
-    const v3 dA = ld3(p, t0), dB = ld3(p, t1), dC = ld3(p, t2);
-    const v3 mn = vmin(vmin(vmin(A, A + dA), vmin(B, B + dB)), vmin(C, C + dC));
-    const v3 mx = vmax(vmax(vmax(A, A + dA), vmax(B, B + dB)), vmax(C, C + dC));
-    const C3 lo = cell_of(mn, inv_dx), hi = cell_of(mx, inv_dx);
-    const v3 d = mk(a.dh, a.dh, a.dh);
-    const float4 qlo = f32_lo(mn - d), qhi = f32_hi(mx + d);   // pt_aabb_moving's triangle box
-    for (long long cx = lo.x; cx <= hi.x; ++cx)
-        for (long long cy = lo.y; cy <= hi.y; ++cy)
-            for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
-                for (int k = run.x; k < run.x + run.y; ++k) {
-                    const int j = gv.ids[k];
-                    const int4 pc = __ldg(cv.cell + j);
-                    const C3 first = cmax(lo, C3{pc.x, pc.y, pc.z});
-                    if (first.x != cx || first.y != cy || first.z != cz) continue;
-                    if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
-                    const int pp = bp[j];
-                    if (pp == t0 || pp == t1 || pp == t2) continue;
-                    if (!pair_push(P, 0, pp, i)) ccd_pair_call(a, 0, pp, i, L);
-                }
-            }
+    grid_walk<false>(block, nbt, qv, g, gv, cv, [&](int i, int j) {
+        const int p = bp[j];
+        if (p == a.bt[3 * i] || p == a.bt[3 * i + 1] || p == a.bt[3 * i + 2]) return;
+        if (!pair_push(P, 0, p, i)) ccd_pair_call(a, 0, p, i, L);
+    });
 }
-
-// compute_filter_3D_EE (NEWTON_IPC.py:409-440): edges query moving bbox +- dh
-__device__ __forceinline__ void ccd_ee(int block, int nbe, const CcdArgs& a, const SceneGeo& g, const GridView& gv, const CandView& cv,
-                                       const PairList& P, const CcdList& L) {
-    // QG lanes per query edge share the candidates of each cell
-    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
-    if (i >= nbe) return;
-    if (g.big_edge && g.big_edge[i]) return;
-    const int* be = a.be;
-    const double *x = a.x, *p = a.p;
-    const int a0 = be[2 * i], a1 = be[2 * i + 1];
-    const int sc = g.scene(a0);
-    const double inv_dx = g.idx(sc);
-    const v3 A0 = ld3(x, a0), A1 = ld3(x, a1), dA0 = ld3(p, a0), dA1 = ld3(p, a1);
-    const v3 d = mk(a.dh, a.dh, a.dh);
-    const v3 mn = vmin(vmin(A0, A0 + dA0), vmin(A1, A1 + dA1)), mx = vmax(vmax(A0, A0 + dA0), vmax(A1, A1 + dA1));
-    const C3 lo = cell_of(mn - d, inv_dx), hi = cell_of(mx + d, inv_dx);
-    const float4 qlo = f32_lo(mn), qhi = f32_hi(mx);   // ee_aabb_moving's query edge box
-    for (long long cx = lo.x; cx <= hi.x; ++cx)
-        for (long long cy = lo.y; cy <= hi.y; ++cy)
-            for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
-                for (int k = run.x + lane; k < run.x + run.y; k += QG) {
-                    const int j = gv.ids[k];
-                    if (!(i < j)) continue;
-                    const int4 sc4 = __ldg(cv.cell + j);
-                    const C3 first = cmax(lo, C3{sc4.x, sc4.y, sc4.z});
-                    if (first.x != cx || first.y != cy || first.z != cz) continue;
-                    if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
-                    const int b0 = be[2 * j], b1 = be[2 * j + 1];
-                    if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) continue;
-                    if (!pair_push(P, 1, i, j)) ccd_pair_call(a, 1, i, j, L);
-                }
-            }
+__device__ __forceinline__ void ccd_ee(int block, int nbe, const CcdArgs& a, const QueryView& qv, const SceneGeo& g, const GridView& gv,
+                                       const CandView& cv, const PairList& P, const CcdList& L) {
+    grid_walk<true>(block, nbe, qv, g, gv, cv, [&](int i, int j) {
+        if (edges_touch(a.be, i, j)) return;
+        if (!pair_push(P, 1, i, j)) ccd_pair_call(a, 1, i, j, L);
+    });
 }
 
 // compute_filter_3D_inversion_free (NEWTON_IPC.py:443-453)
@@ -690,35 +647,18 @@ __global__ void __launch_bounds__(PAIR_THREADS) k_collision_pairs(HitArgs a, Pai
     each_pair(P, [&](int, int2 q) { hit_pair(a, q.x, q.y); });
 }
 
+// an edge and a triangle of which it is no part
+__device__ __forceinline__ bool edge_of_triangle(const int* __restrict__ be, const int* __restrict__ bt, int e, int t) {
+    const int t0 = bt[3 * t], t1 = bt[3 * t + 1], t2 = bt[3 * t + 2], a0 = be[2 * e], a1 = be[2 * e + 1];
+    return a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2;
+}
 // triangles query bbox cells, edges hashed +- dh
-__device__ __forceinline__ void collision_grid(int block, int nbt, const HitArgs& a, const SceneGeo& g, const GridView& gv,
+__device__ __forceinline__ void collision_grid(int block, int nbt, const HitArgs& a, const QueryView& qv, const SceneGeo& g, const GridView& gv,
                                                const CandView& cv, const PairList& P) {
-    // QG lanes per query triangle share the candidates of each cell
-    const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
-    if (i >= nbt) return;
-    if (g.big_tri && g.big_tri[i]) return;
-    const int t0 = a.bt[3 * i], t1 = a.bt[3 * i + 1], t2 = a.bt[3 * i + 2];
-    const int sc = g.scene(t0);
-    const double inv_dx = g.idx(sc);
-    const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2);
-    const v3 tmn = vmin(vmin(A, B), C), tmx = vmax(vmax(A, B), C);
-    const C3 lo = cell_of(tmn, inv_dx), hi = cell_of(tmx, inv_dx);
-    const float4 qlo = f32_lo(tmn), qhi = f32_hi(tmx);   // the triangle's box; edges carry +- dh
-    for (long long cx = lo.x; cx <= hi.x; ++cx)
-        for (long long cy = lo.y; cy <= hi.y; ++cy)
-            for (long long cz = lo.z; cz <= hi.z; ++cz) {
-                const int2 run = gv.find(gkey(g, sc, cx, cy, cz));
-                for (int k = run.x + lane; k < run.x + run.y; k += QG) {
-                    const int j = gv.ids[k];
-                    const int4 sc4 = __ldg(cv.cell + j);
-                    const C3 first = cmax(lo, C3{sc4.x, sc4.y, sc4.z});
-                    if (first.x != cx || first.y != cy || first.z != cz) continue;
-                    if (!f32_overlap(__ldg(cv.box + 2 * j), __ldg(cv.box + 2 * j + 1), qlo, qhi)) continue;
-                    const int a0 = a.be[2 * j], a1 = a.be[2 * j + 1];
-                    if (a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2) continue;
-                    if (!pair_push(P, 0, j, i)) hit_pair_call(a, j, i);
-                }
-            }
+    grid_walk<false>(block, nbt, qv, g, gv, cv, [&](int i, int j) {
+        if (edge_of_triangle(a.be, a.bt, j, i)) return;
+        if (!pair_push(P, 0, j, i)) hit_pair_call(a, j, i);
+    });
 }
 
 // ---------------------------------------------------------------- big primitives
@@ -786,6 +726,7 @@ __device__ __forceinline__ void find_ee_big(int block, const BigArgs& b, const F
         const v3 A0 = ld3(a.x, b.be[2 * i]), A1 = ld3(a.x, b.be[2 * i + 1]);
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(vmin(A0, A1)), f32_hi(vmax(A0, A1)))) return;
         const int lo = i < j ? i : j, hi = i < j ? j : i;
+        if (edges_touch(b.be, lo, hi)) return;
         if (!pair_push(P, 1, lo, hi)) find_pair_call(a, 1, lo, hi, sink);
     });
 }
@@ -812,8 +753,7 @@ __device__ __forceinline__ void ccd_ee_big(int block, const BigArgs& b, const Cc
         const v3 mn = vmin(vmin(I0, I0 + dI0), vmin(I1, I1 + dI1)), mx = vmax(vmax(I0, I0 + dI0), vmax(I1, I1 + dI1));
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(mn), f32_hi(mx))) return;
         const int lo = i < j ? i : j, hi = i < j ? j : i;
-        const int a0 = b.be[2 * lo], a1 = b.be[2 * lo + 1], b0 = b.be[2 * hi], b1 = b.be[2 * hi + 1];
-        if (a0 == b0 || a0 == b1 || a1 == b0 || a1 == b1) return;
+        if (edges_touch(b.be, lo, hi)) return;
         if (!pair_push(Q, 1, lo, hi)) ccd_pair_call(a, 1, lo, hi, L);
     });
 }
@@ -825,9 +765,8 @@ __device__ __forceinline__ void collision_big(int block, int kind, const BigArgs
     big_pairs(b, g, block, kind, kind ? 2 : 1, [&](int i, int k, int) {
         const int e = kind ? i : k, t = kind ? k : i;
         if (kind && b.tri_big[t]) return;
-        const int t0 = b.bt[3 * t], t1 = b.bt[3 * t + 1], t2 = b.bt[3 * t + 2], a0 = b.be[2 * e], a1 = b.be[2 * e + 1];
-        if (a0 == t0 || a0 == t1 || a0 == t2 || a1 == t0 || a1 == t1 || a1 == t2) return;
-        const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2);
+        if (edge_of_triangle(b.be, b.bt, e, t)) return;
+        const v3 A = ld3(a.x, b.bt[3 * t]), B = ld3(a.x, b.bt[3 * t + 1]), C = ld3(a.x, b.bt[3 * t + 2]);
         if (!f32_touch(__ldg(cv.box + 2 * (size_t)e), __ldg(cv.box + 2 * (size_t)e + 1), f32_lo(vmin(vmin(A, B), C)), f32_hi(vmax(vmax(A, B), C)))) return;
         if (!pair_push(P, 0, e, t)) hit_pair_call(a, e, t);
     });
@@ -838,7 +777,7 @@ __device__ __forceinline__ void collision_big(int block, int kind, const BigArgs
 struct GridBuild {
     const int* prim;
     int n, mode;
-    int4* cell;
+    int4 *cell, *ext;
     float4* box;
     unsigned long long* hk;
     int* cnt;
@@ -852,8 +791,8 @@ struct GridBuild {
 // the tables cleared
 __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict__ bt, int nbe, const int* __restrict__ be, GridBuild gp,
                                                  GridBuild ge, const double* __restrict__ x, const double* __restrict__ p, double dh,
-                                                 SceneGeo g, unsigned char* __restrict__ tri_big, unsigned char* __restrict__ edge_big,
-                                                 int* __restrict__ list, BroadCounters* __restrict__ n) {
+                                                 SceneGeo g, QueryView qt, QueryView qe, unsigned char* __restrict__ tri_big,
+                                                 unsigned char* __restrict__ edge_big, int* __restrict__ list, BroadCounters* __restrict__ n) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
     if (k == 0) n->alpha = (unsigned long long)__double_as_longlong(1.0);
     for (unsigned long long h = k; h <= gp.mask; h += nthr) {
@@ -875,7 +814,10 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
             lo = vmin(lo, vmin(vmin(A, B), C));
             hi = vmax(hi, vmax(vmax(A, B), C));
         }
-        const bool big = box_cells(lo, hi, g.idx(g.scene(t0))) > BIG_CELLS;
+        const int sc = g.scene(t0);
+        const double inv_dx = g.idx(sc);
+        const bool big = box_cells(lo, hi, inv_dx) > BIG_CELLS, check = ge.mode == 4;   // the intersection check's boxes carry no dh
+        query_record(qt, k, sc, big, cell_of(lo, inv_dx), cell_of(hi, inv_dx), check ? lo : lo - d, check ? hi : hi + d);
         tri_big[k] = big;
         if (big) list[atomicAdd(&n->big[0], 1)] = k;
     } else if (k < nbt + nbe + gp.n) {
@@ -883,7 +825,8 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
         const GridBuild& b = edge ? ge : gp;
         const int i = edge ? k - nbt : k - nbt - nbe;
         const int sv = edge ? be[2 * i] : b.prim[i];
-        const double inv_dx = g.idx(g.scene(sv));
+        const int sc = g.scene(sv);
+        const double inv_dx = g.idx(sc);
         bool big = false;
         if (edge) {
             const int a1 = be[2 * i + 1];
@@ -894,6 +837,7 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
                 hi = vmax(hi, vmax(A, B));
             }
             big = box_cells(lo - d, hi + d, inv_dx) > BIG_CELLS;
+            if (ge.mode != 4) query_record(qe, i, sc, big, cell_of(lo - d, inv_dx), cell_of(hi + d, inv_dx), lo, hi);
             edge_big[i] = big;
             if (big) list[nbt + atomicAdd(&n->big[1], 1)] = i;
         }
@@ -908,6 +852,7 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
                 cells = 0;
             }
         }
+        b.ext[i] = cells ? make_int4((int)(e.x - a.x + 1), (int)(e.y - a.y + 1), (int)(e.z - a.z + 1), sc) : make_int4(0, 0, 0, sc);
         which = edge ? 1 : 0;
     }
     // totals: one add per warp and grid
@@ -924,8 +869,7 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
 // Nothing happens when a table is too small for its entries (the call is then repeated).
 constexpr int CELL_LANES = 4;
 template <class F>
-__device__ __forceinline__ void each_entry(const GridBuild& gp, const GridBuild& ge, const double* __restrict__ x, const double* __restrict__ p,
-                                           double dh, const SceneGeo& g, BroadCounters* n, F f) {
+__device__ __forceinline__ void each_entry(const GridBuild& gp, const GridBuild& ge, const SceneGeo& g, BroadCounters* n, F f) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) / CELL_LANES, lane = threadIdx.x % CELL_LANES;
     if (2 * n->total[0] > gp.mask + 1 || 2 * n->total[1] > ge.mask + 1) {
         if (k == 0 && lane == 0) atomicOr(&n->flags, FLAG_TABLE);
@@ -935,25 +879,17 @@ __device__ __forceinline__ void each_entry(const GridBuild& gp, const GridBuild&
     const bool edge = k >= gp.n;
     const GridBuild& b = edge ? ge : gp;
     const int i = edge ? k - gp.n : k;
-    if (edge && g.big_edge[i]) return;   // left to the big-primitive pass
-    const int sc = g.scene(edge ? b.prim[2 * i] : b.prim[i]);
-    const double inv_dx = g.idx(sc);
-    v3 lo, hi;
-    stored_box(b.mode, i, b.prim, x, p, dh, &lo, &hi);
-    const C3 a = cell_of(lo, inv_dx), e = cell_of(hi, inv_dx);
-    const long long ny = e.y - a.y + 1, nz = e.z - a.z + 1, c = (e.x - a.x + 1) * ny * nz;
-    if (!(c > 0 && c <= MAX_CELLS_PER_PRIM)) return;
-    const int nyi = (int)ny, nzi = (int)nz;
-    for (int q = lane; q < (int)c; q += CELL_LANES) {
-        const int qz = q % nzi, qy = q / nzi % nyi, qx = q / nzi / nyi;
-        f(b, edge, gkey(g, sc, a.x + qx, a.y + qy, a.z + qz), i);
+    const int4 a = __ldg(b.cell + i), e = __ldg(b.ext + i);   // no cells: left to the big-primitive pass
+    const int ny = e.y, nz = e.z, c = e.x * ny * nz;
+    for (int q = lane; q < c; q += CELL_LANES) {
+        const int qz = q % nz, qy = q / nz % ny, qx = q / nz / ny;
+        f(b, edge, gkey(g, e.w, (long long)a.x + qx, (long long)a.y + qy, (long long)a.z + qz), i);
     }
 }
 
 // the occupied cells and their entry counts (a full table is impossible at load <= 1/2)
-__global__ void __launch_bounds__(256) k_grid_insert(GridBuild gp, GridBuild ge, const double* __restrict__ x, const double* __restrict__ p,
-                                                     double dh, SceneGeo g, BroadCounters* __restrict__ n) {
-    each_entry(gp, ge, x, p, dh, g, n, [&](const GridBuild& b, bool, unsigned long long key, int) {
+__global__ void __launch_bounds__(256) k_grid_insert(GridBuild gp, GridBuild ge, SceneGeo g, BroadCounters* __restrict__ n) {
+    each_entry(gp, ge, g, n, [&](const GridBuild& b, bool, unsigned long long key, int) {
         unsigned long long h = mix64(key) & b.mask;
         for (unsigned long long q = 0; q <= b.mask; ++q) {
             const unsigned long long prev = atomicCAS(b.hk + h, HASH_EMPTY, key);
@@ -989,9 +925,8 @@ __global__ void __launch_bounds__(256) k_grid_runs(GridBuild gp, GridBuild ge, B
 }
 
 // the ids into their cells' runs; run.y counts up to the run's length
-__global__ void __launch_bounds__(256) k_grid_fill(GridBuild gp, GridBuild ge, const double* __restrict__ x, const double* __restrict__ p,
-                                                   double dh, SceneGeo g, BroadCounters* __restrict__ n) {
-    each_entry(gp, ge, x, p, dh, g, n, [&](const GridBuild& b, bool, unsigned long long key, int i) {
+__global__ void __launch_bounds__(256) k_grid_fill(GridBuild gp, GridBuild ge, SceneGeo g, BroadCounters* __restrict__ n) {
+    each_entry(gp, ge, g, n, [&](const GridBuild& b, bool, unsigned long long key, int i) {
         unsigned long long h = mix64(key) & b.mask;
         for (unsigned long long q = 0; q <= b.mask; ++q) {
             if (b.hk[h] == key) {
@@ -1010,25 +945,29 @@ __global__ void __launch_bounds__(256) k_grid_fill(GridBuild gp, GridBuild ge, c
 struct QueryBlocks {
     int pt, ee, pt_big, ee_big;   // blocks of each pass, in this order
 };
-__global__ void __launch_bounds__(128) k_find(QueryBlocks nb, int nbt, const int* __restrict__ bp, int nbe, FindArgs a, SceneGeo g, GridView gp,
-                                              CandView cp, GridView ge, CandView ce, BigArgs big, PairList P, RowSink sink) {
+constexpr int WALK_CTAS = 8;   // per SM, of 128 threads: the walks are chains of dependent loads
+__global__ void __launch_bounds__(128, WALK_CTAS) k_find(QueryBlocks nb, int nbt, const int* __restrict__ bp, int nbe, FindArgs a, QueryView qt,
+                                                         QueryView qe, SceneGeo g, GridView gp, CandView cp, GridView ge, CandView ce,
+                                                         BigArgs big, PairList P, RowSink sink) {
     int b = blockIdx.x;
-    if (b < nb.ee) return find_ee(b, nbe, a.be, a, g, ge, ce, P, sink);
-    if ((b -= nb.ee) < nb.pt) return find_pt(b, nbt, a.bt, bp, a, g, gp, cp, P, sink);
+    if (b < nb.ee) return find_ee(b, nbe, a, qe, g, ge, ce, P, sink);
+    if ((b -= nb.ee) < nb.pt) return find_pt(b, nbt, bp, a, qt, g, gp, cp, P, sink);
     if ((b -= nb.pt) < nb.pt_big) return find_pt_big(b, big, a, g, cp, P, sink);
     find_ee_big(b - nb.pt_big, big, a, g, ce, P, sink);
 }
-__global__ void __launch_bounds__(128) k_ccd(QueryBlocks nb, int nbt, const int* __restrict__ bp, int nbe, CcdArgs a, SceneGeo g, GridView gp,
-                                             CandView cp, GridView ge, CandView ce, BigArgs big, PairList P, CcdList L) {
+__global__ void __launch_bounds__(128, WALK_CTAS) k_ccd(QueryBlocks nb, int nbt, const int* __restrict__ bp, int nbe, CcdArgs a, QueryView qt,
+                                                        QueryView qe, SceneGeo g, GridView gp, CandView cp, GridView ge, CandView ce,
+                                                        BigArgs big, PairList P, CcdList L) {
     int b = blockIdx.x;
-    if (b < nb.ee) return ccd_ee(b, nbe, a, g, ge, ce, P, L);
-    if ((b -= nb.ee) < nb.pt) return ccd_pt(b, nbt, bp, a, g, gp, cp, P, L);
+    if (b < nb.ee) return ccd_ee(b, nbe, a, qe, g, ge, ce, P, L);
+    if ((b -= nb.ee) < nb.pt) return ccd_pt(b, nbt, bp, a, qt, g, gp, cp, P, L);
     if ((b -= nb.pt) < nb.pt_big) return ccd_pt_big(b, big, a, g, cp, P, L);
     ccd_ee_big(b - nb.pt_big, big, a, g, ce, P, L);
 }
-__global__ void __launch_bounds__(128) k_collision(QueryBlocks nb, int nbt, HitArgs a, SceneGeo g, GridView ge, CandView ce, BigArgs big, PairList P) {
+__global__ void __launch_bounds__(128, WALK_CTAS) k_collision(QueryBlocks nb, int nbt, HitArgs a, QueryView qt, SceneGeo g, GridView ge, CandView ce,
+                                                              BigArgs big, PairList P) {
     int b = blockIdx.x;
-    if (b < nb.pt) return collision_grid(b, nbt, a, g, ge, ce, P);
+    if (b < nb.pt) return collision_grid(b, nbt, a, qt, g, ge, ce, P);
     if ((b -= nb.pt) < nb.pt_big) return collision_big(b, 0, big, a, g, ce, P);
     collision_big(b - nb.pt_big, 1, big, a, g, ce, P);
 }
@@ -1147,6 +1086,7 @@ struct Broad {
     BigArgs big;
     GridBuild gp, ge;
     PairList pairs;
+    QueryView qt, qe;
     BroadCounters* n;
 };
 
@@ -1162,26 +1102,27 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
     const int n = c->nBT + c->nBE, np = mode_p < 0 ? 0 : c->nBP;
     if (c->big_flags.ensure((size_t)n + 16) || c->big_list.ensure(4ll * n + 16) || c->broad.ensure(sizeof(BroadCounters))) return FIPC_ERR_CUDA;
     if (ensure_table(c->gp, table_size(2ll * np)) || ensure_table(c->ge, table_size(2ll * c->nBE))) return FIPC_ERR_CUDA;
-    if (c->gp.cell4.ensure(16ll * np + 16) || c->gp.box4.ensure(32ll * np + 32) || c->ge.cell4.ensure(16ll * c->nBE + 16) ||
-        c->ge.box4.ensure(32ll * c->nBE + 32))
+    if (c->gp.cell4.ensure(16ll * np + 16) || c->gp.ext4.ensure(16ll * np + 16) || c->gp.box4.ensure(32ll * np + 32) ||
+        c->ge.cell4.ensure(16ll * c->nBE + 16) || c->ge.ext4.ensure(16ll * c->nBE + 16) || c->ge.box4.ensure(32ll * c->nBE + 32) ||
+        c->query_cell.ensure(16ll * n + 16) || c->query_box.ensure(32ll * n + 32))
         return FIPC_ERR_CUDA;
     unsigned char* tri_big = c->big_flags.as<unsigned char>();
     b->n = c->broad.as<BroadCounters>();
     SceneGeo g = geo(c);
     auto build = [](Grid& gr, const int* prim, int np_, int mode) {
-        return GridBuild{prim, np_, mode, gr.cell4.as<int4>(), gr.box4.as<float4>(), gr.hkeys.as<unsigned long long>(), gr.counts.as<int>(),
+        return GridBuild{prim, np_, mode, gr.cell4.as<int4>(), gr.ext4.as<int4>(), gr.box4.as<float4>(), gr.hkeys.as<unsigned long long>(), gr.counts.as<int>(),
                          gr.runs.as<int2>(), gr.ids.as<int>(), gr.size - 1};
     };
     b->gp = build(c->gp, c->bp, np, mode_p);
     b->ge = build(c->ge, c->be, c->nBE, mode_e);
+    b->qt = QueryView{c->query_cell.as<int4>(), c->query_box.as<float4>()};
+    b->qe = QueryView{b->qt.cell + c->nBT, b->qt.box + 2ll * c->nBT};
     FIPC_CUDA(cudaMemsetAsync(b->n, 0, sizeof(BroadCounters), s));
     const long long work = (long long)n + np, slots = (long long)(c->gp.size + c->ge.size);
     const int grid = (int)std::max<long long>(nblk(work, 256), std::min<long long>(nblk(slots, 256), 1216));
-    k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, tri_big, tri_big + c->nBT,
+    k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, b->qt, b->qe, tri_big, tri_big + c->nBT,
                                    c->big_list.as<int>(), b->n);
     FIPC_LAUNCHED();
-    g.big_tri = tri_big;
-    g.big_edge = tri_big + c->nBT;
     b->g = g;
     // the pair lists, as long as the last calls needed
     const long long want = std::min<long long>(std::max<long long>(65536ll + 2ll * n, c->pair_hint), PAIRS_MAX);
@@ -1189,14 +1130,14 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
     b->pairs = PairList{c->pair_list.as<int2>(), b->n->pairs, (int)want};
     const int entries = nblk((long long)CELL_LANES * (np + c->nBE), 256);
     if (entries > 0) {
-        k_grid_insert<<<entries, 256, 0, s>>>(b->gp, b->ge, x, p, c->dhat, g, b->n);
+        k_grid_insert<<<entries, 256, 0, s>>>(b->gp, b->ge, g, b->n);
         FIPC_LAUNCHED();
         k_grid_runs<<<nblk(slots, 256), 256, 0, s>>>(b->gp, b->ge, b->n);
         FIPC_LAUNCHED();
-        k_grid_fill<<<entries, 256, 0, s>>>(b->gp, b->ge, x, p, c->dhat, g, b->n);
+        k_grid_fill<<<entries, 256, 0, s>>>(b->gp, b->ge, g, b->n);
         FIPC_LAUNCHED();
     }
-    b->big = BigArgs{c->bp, c->be, c->bt, c->prim_off, c->n_scenes, g.big_tri, g.big_edge, c->big_list.as<int>(), b->n->big, c->nBT,
+    b->big = BigArgs{c->bp, c->be, c->bt, c->prim_off, c->n_scenes, tri_big, tri_big + c->nBT, c->big_list.as<int>(), b->n->big, c->nBT,
                      c->n_scenes > 1 ? 128 : 32};
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
@@ -1251,13 +1192,13 @@ int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
         int st = broad_prepare(c, x, nullptr, 0, 1, &b, s);
         if (st) return st;
         const RowSink sink{c->row_keys.as<RowKey>(), b.n, c->cap};
-        QueryBlocks nb{c->nBP > 0 ? nblk(c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
+        QueryBlocks nb{c->nBP > 0 ? nblk((long long)QG * c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
         nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b.big.ny) : 0;
         nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b.big.ny) : 0;
         const int blocks = nb.pt + nb.ee + nb.pt_big + nb.ee_big;
         if (blocks > 0) {
             const FindArgs a{c->bt, c->be, x, c->x0, c->dhat, c->dhat2};
-            k_find<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bp, c->nBE, a, b.g, view(b.gp), cands(b.gp), view(b.ge), cands(b.ge), b.big, b.pairs,
+            k_find<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bp, c->nBE, a, b.qt, b.qe, b.g, view(b.gp), cands(b.gp), view(b.ge), cands(b.ge), b.big, b.pairs,
                                           sink);
             FIPC_LAUNCHED();
             k_find_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b.pairs, sink);
@@ -1301,7 +1242,7 @@ static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta,
     const long long cap = std::min<long long>(65536ll + c->nBE + c->nBT, 1ll << 21);
     if (c->ccd_work.ensure(4 * cap * sizeof(CcdWork))) return FIPC_ERR_CUDA;
     const CcdList L{c->ccd_work.as<CcdWork>(), b->n->work, (int)cap}, M{L.w + 2 * cap, b->n->doubt, (int)cap};
-    QueryBlocks nb{c->nBP > 0 ? nblk(c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
+    QueryBlocks nb{c->nBP > 0 ? nblk((long long)QG * c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
     nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b->big.ny) : 0;
     nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b->big.ny) : 0;
     if (inversion && c->nT > 0) {
@@ -1311,7 +1252,7 @@ static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta,
     const int blocks = nb.pt + nb.ee + nb.pt_big + nb.ee_big;
     if (blocks > 0) {
         const CcdArgs a{c->bt, c->be, x, p, c->dhat, eta, b->g.vscene, slot};
-        k_ccd<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bp, c->nBE, a, b->g, view(b->gp), cands(b->gp), view(b->ge), cands(b->ge), b->big, b->pairs, L);
+        k_ccd<<<blocks, 128, 0, s>>>(nb, c->nBT, c->bp, c->nBE, a, b->qt, b->qe, b->g, view(b->gp), cands(b->gp), view(b->ge), cands(b->ge), b->big, b->pairs, L);
         FIPC_LAUNCHED();
         k_ccd_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b->pairs, L);
         FIPC_LAUNCHED();
@@ -1359,7 +1300,7 @@ int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStr
         const int blocks = nb.pt + nb.pt_big + nb.ee_big;
         if (blocks > 0) {
             const HitArgs a{c->bt, c->be, x, b.g.vscene, hit};
-            k_collision<<<blocks, 128, 0, s>>>(nb, c->nBT, a, b.g, view(b.ge), cands(b.ge), b.big, b.pairs);
+            k_collision<<<blocks, 128, 0, s>>>(nb, c->nBT, a, b.qt, b.g, view(b.ge), cands(b.ge), b.big, b.pairs);
             FIPC_LAUNCHED();
             k_collision_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b.pairs);
             FIPC_LAUNCHED();

@@ -79,12 +79,12 @@ void free_ctx(fipc_ctx* c) {
                     c->up_spos, c->up_tspos, c->diag_spos, c->sell_val, c->prim_off};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    DBuf* bufs[] = {&c->row_keys, &c->row_keys_alt, &c->rows_all, &c->cub_tmp, &c->broad, &c->big_flags, &c->big_list, &c->ccd_work, &c->pair_list, &c->c_g, &c->c_H, &c->c_keys, &c->c_keys_alt, &c->c_vals, &c->c_vals_alt, &c->c_ukeys,
+    DBuf* bufs[] = {&c->row_keys, &c->row_keys_alt, &c->rows_all, &c->cub_tmp, &c->broad, &c->big_flags, &c->big_list, &c->ccd_work, &c->pair_list, &c->query_cell, &c->query_box, &c->c_g, &c->c_H, &c->c_keys, &c->c_keys_alt, &c->c_vals, &c->c_vals_alt, &c->c_ukeys,
                     &c->c_ucount, &c->c_ustart, &c->c_val, &c->c_rowptr, &c->c_col, &c->pcg_vec, &c->pcg_part, &c->scal, &c->red, &c->mlp_dist};
     for (DBuf* b : bufs) b->release();
     Grid* gs[] = {&c->gp, &c->ge};
     for (Grid* g : gs) {
-        DBuf* gb[] = {&g->hkeys, &g->counts, &g->runs, &g->ids, &g->cell4, &g->box4};
+        DBuf* gb[] = {&g->hkeys, &g->counts, &g->runs, &g->ids, &g->cell4, &g->ext4, &g->box4};
         for (DBuf* b : gb) b->release();
     }
     delete c;

@@ -54,7 +54,7 @@ struct DBuf {
 // and id runs, and the ids; kept from call to call and grown on demand
 struct Grid {
     DBuf hkeys, counts, runs, ids;
-    DBuf cell4, box4;   // per stored primitive: first cell of its pair de-duplication, FP32 box
+    DBuf cell4, ext4, box4;   // per stored primitive: lowest cell, cells per axis and scene, FP32 box
     unsigned long long size = 0;   // table slots (a power of two, at least twice the entries)
 };
 
@@ -119,6 +119,7 @@ struct fipc_ctx_impl {
     int max_prims[3] = {0, 0, 0};         // the largest of a scene's points, edges, triangles
     DBuf big_flags, big_list, broad;      // broad: the counters of a broad-phase call
     DBuf ccd_work;                        // step filter: pairs that pass its first two tests
+    DBuf query_cell, query_box;           // per query (triangles, then edges): cell range, FP32 box
     DBuf pair_list;                       // candidate pairs of a query
     long long pair_hint = 0;              // list length for the next query, from what the last ones needed
     std::vector<double> h_kappa, h_inv_dx;
@@ -149,10 +150,6 @@ struct SceneGeo {
     const int* vscene = nullptr;
     const double* inv_dx_s = nullptr;
     double inv_dx = 1.0;
-    // primitives whose query box covers more than BIG_CELLS cells: tested against every
-    // primitive of their scene instead of through the grid (null: none)
-    const unsigned char* big_tri = nullptr;
-    const unsigned char* big_edge = nullptr;
 #if defined(__CUDACC__)
     __device__ __forceinline__ int scene(int v) const { return vscene ? __ldg(vscene + v) : 0; }
     __device__ __forceinline__ double idx(int s) const { return vscene ? __ldg(inv_dx_s + s) : inv_dx; }
