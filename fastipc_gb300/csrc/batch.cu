@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(TR) k_bpcg_start(BPCG a, const double* __restr
             continue;
         }
         double rr = 0.0, bb = 0.0, y0, y1, y2;
-        row_apply<3>(a.m, i, i < a.voff[s + 1], a.m.x, y0, y1, y2);
+        row_apply<3>(a.m, i, i < a.voff[s + 1] && !a.m.fixed[i], a.m.x, y0, y1, y2);
         if (i < a.voff[s + 1]) {
             double Mi[9];
             const bool fx = a.m.fixed[i] != 0;

@@ -141,7 +141,7 @@ __global__ void k_cs_regularize(int n, double* __restrict__ Ac) {
 // needed: the A_KK met are Schur complements of an SPD matrix.  Only the tiles on and below the
 // diagonal are kept, which halves the FP64 work of a full Gauss-Jordan inverse; the upper
 // triangle is filled at the end.  One cooperative launch:
-//   prologue   CTA 0: T = A_00^-1 (Gauss-Jordan on one tile in shared memory)
+//   prologue   CTA 0: T = A_00^-1 (symmetric sweeps of one tile)
 //   per K      A: every CTA: panel P_I = A_IK (tile (K, I) transposed for I < K) and W_I = P_I T
 //              B: CTA 0 writes A_KK = -T, then updates tile (K+1, K+1) and inverts it into T
 //                 (the next block's T, ready by the next barrier); the other CTAs take the other
@@ -150,25 +150,81 @@ __global__ void k_cs_regularize(int n, double* __restrict__ Ac) {
 // buf: T (B^2) + P (n B) + W (n B) doubles.  Every sum runs in a fixed order.
 constexpr int GJ_B = 32, GJ_THREADS = 256;
 
-// in-place Gauss-Jordan inverse of the SPD tile s (shared memory, row stride GJ_B + 1)
-__device__ void gj_tile_inverse(double (*s)[GJ_B + 1], double* prow, double* pcol) {
+// The tile of CTA 0 in registers: eight threads per row i, thread q of them holding the columns j = q + 8 u up
+// to the diagonal, so that a warp's four rows cost 1 to 4 FP64 instructions per step.  A warp's FP64
+// instruction takes 75 clocks of its scheduler (warp % 4): the rows are dealt so that the schedulers'
+// loads are 2, 6, 6 and 6, and warp 0, with the least, keeps the pivots.
+struct GjTile {
+    int i, q;
+    __device__ __forceinline__ GjTile() {
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+        const int rows = w == 0 ? 0 : (w == 4 ? 1 : (w == 1 ? 2 : (w == 5 ? 6 : (w == 2 ? 3 : (w == 6 ? 7 : (w == 3 ? 4 : 5))))));
+        i = 4 * rows + (l >> 3);
+        q = l & 7;
+    }
+    __device__ __forceinline__ bool has(int u) const { return q + 8 * u <= i; }
+};
+// 1 / d to within an ulp from an FP32 reciprocal (two Newton steps: 24, 48, 96 bits)
+__device__ __forceinline__ double gj_reciprocal(double d) {
+    const float f = (float)d;
+    if (!(f > 1e-30f && f < 1e30f)) return 1.0 / d;
+    double r = (double)(1.f / f);
+    r = fma(r, fma(-d, r, 1.0), r);
+    return fma(r, fma(-d, r, 1.0), r);
+}
+// e <- the lower half of -S^-1 for the SPD tile S whose lower half e holds, by 32 symmetric sweeps
+//     s_kk -> -1/p,  s_ik -> c_i / p,  s_ij -> s_ij - c_i c_j / p   (p = s_kk, c_i = s_ik).
+// Bounded by the chain of a sweep: publish column k + 1, barrier, update.  Warp 0 carries all diagonals
+// and forms the next pivot's reciprocal while the others update (with the column, the division and the
+// update one behind the other a tile took 43 us of the 49 of a block step).
+__device__ void gj_tile_sweep(const GjTile& m, double (&e)[4], double (*col)[GJ_B], double* pinv, double* diag) {
     const int t = threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int j = m.q + 8 * u;
+        if (j == 0) col[0][m.i] = e[u];
+        if (j == m.i) diag[j] = e[u];
+    }
+    __syncthreads();
+    double d = 0.0;
+    if (t < GJ_B) {
+        d = diag[t];
+        if (t == 0) pinv[0] = gj_reciprocal(d);
+    }
+    __syncthreads();
     for (int k = 0; k < GJ_B; ++k) {
-        if (t < GJ_B) {
-            const double inv = 1.0 / s[k][k];
-            prow[t] = t == k ? inv : s[k][t] * inv;
-            pcol[t] = s[t][k];
+        const int b = k & 1;
+        const double pin = pinv[b], ci = col[b][m.i];
+        if (t < GJ_B && k + 1 < GJ_B) {
+            const double c = col[b][t];
+            d = fma(-c * pin, c, d);
+            if (t == k + 1) pinv[b ^ 1] = gj_reciprocal(d);
+        }
+        const double r = ci * pin;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (!m.has(u)) continue;
+            const int j = m.q + 8 * u;
+            const bool ik = m.i == k, jk = j == k;
+            const double cj = col[b][j];
+            // one FMA whatever the case
+            const double x = ik || jk ? pin : -r, y = ik ? (jk ? -1.0 : cj) : (jk ? ci : cj), z = ik || jk ? 0.0 : e[u];
+            e[u] = fma(x, y, z);
+            if (j == k + 1) col[b ^ 1][m.i] = e[u];
+            else if (m.i == k + 1) col[b ^ 1][j] = e[u];
         }
         __syncthreads();
-        for (int e = t; e < GJ_B * GJ_B; e += GJ_THREADS) {
-            const int i = e / GJ_B, j = e % GJ_B;
-            double v;
-            if (i == k) v = prow[j];
-            else if (j == k) v = -pcol[i] * prow[k];
-            else v = fma(-pcol[i], prow[j], s[i][j]);
-            s[i][j] = v;
-        }
-        __syncthreads();
+    }
+}
+
+// T = -e, both halves
+__device__ __forceinline__ void gj_store(const GjTile& m, const double (&e)[4], double* __restrict__ T) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int j = m.q + 8 * u;
+        if (!m.has(u)) continue;
+        T[m.i * GJ_B + j] = -e[u];
+        T[j * GJ_B + m.i] = -e[u];
     }
 }
 
@@ -185,7 +241,7 @@ __global__ void __launch_bounds__(GJ_THREADS) k_cs_gauss_jordan(int n, double* _
     cg::grid_group grid = cg::this_grid();
     __shared__ double sa[GJ_B][GJ_B + 1];
     __shared__ double sb[GJ_B][GJ_B + 1];
-    __shared__ double prow[GJ_B], pcol[GJ_B];
+    __shared__ double col[2][GJ_B], pinv[2], diag[GJ_B];
     const int nb = n / GJ_B, t = threadIdx.x;
     const long long gtid = (long long)blockIdx.x * GJ_THREADS + t, gthr = (long long)gridDim.x * GJ_THREADS;
     double* T = buf;
@@ -196,10 +252,12 @@ __global__ void __launch_bounds__(GJ_THREADS) k_cs_gauss_jordan(int n, double* _
     const int worker = solo ? 0 : (int)blockIdx.x - 1, workers = solo ? 1 : (int)gridDim.x - 1;
     const int n_lower = nb * (nb + 1) / 2;
     if (blockIdx.x == 0) {
-        for (int e = t; e < GJ_B * GJ_B; e += GJ_THREADS) sa[e / GJ_B][e % GJ_B] = A[(size_t)(e / GJ_B) * n + e % GJ_B];
-        __syncthreads();
-        gj_tile_inverse(sa, prow, pcol);
-        for (int e = t; e < GJ_B * GJ_B; e += GJ_THREADS) T[e] = sa[e / GJ_B][e % GJ_B];
+        const GjTile m;
+        double e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u] = m.has(u) ? A[(size_t)m.i * n + m.q + 8 * u] : 0.0;
+        gj_tile_sweep(m, e, col, pinv, diag);
+        gj_store(m, e, T);
     }
     grid.sync();
     for (int K = 0; K < nb; ++K) {
@@ -230,21 +288,21 @@ __global__ void __launch_bounds__(GJ_THREADS) k_cs_gauss_jordan(int n, double* _
                     sb[e / GJ_B][e % GJ_B] = P[(size_t)i0 * GJ_B + e];
                 }
                 __syncthreads();
-                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                const GjTile m;
+                double e[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) e[u] = m.has(u) ? A[(size_t)(i0 + m.i) * n + i0 + m.q + 8 * u] : 0.0;
+#pragma unroll 4
                 for (int q = 0; q < GJ_B; ++q) {
-                    const double pj = sb[c][q];
+                    const double wi = sa[m.i][q];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[u] = fma(sa[rb + 8 * u][q], pj, acc[u]);
+                    for (int u = 0; u < 4; ++u)
+                        if (m.has(u)) acc[u] = fma(wi, sb[m.q + 8 * u][q], acc[u]);
                 }
-                double v[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) v[u] = A[(size_t)(i0 + rb + 8 * u) * n + i0 + c] - acc[u];
-                __syncthreads();
-#pragma unroll
-                for (int u = 0; u < 4; ++u) sa[rb + 8 * u][c] = v[u];
-                __syncthreads();
-                gj_tile_inverse(sa, prow, pcol);
-                for (int e = t; e < GJ_B * GJ_B; e += GJ_THREADS) T[e] = sa[e / GJ_B][e % GJ_B];
+                for (int u = 0; u < 4; ++u) e[u] -= acc[u];
+                gj_tile_sweep(m, e, col, pinv, diag);
+                gj_store(m, e, T);
             }
         }
         if (blockIdx.x != 0 || solo) {

@@ -248,7 +248,8 @@ template <bool WIDE>
 __global__ void __launch_bounds__(PCG_THREADS) k_pcg_start(PCGArgs a, const double* __restrict__ rhs, double rtol, int maxit) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double rr = 0.0, bb = 0.0, r3[3] = {0.0, 0.0, 0.0}, y0, y1, y2;
-    row_apply<3, WIDE>(a, i, i < a.nV, a.x, y0, y1, y2);
+    // fixed rows have no residual (and those of a ground plane most of the contact blocks)
+    row_apply<3, WIDE>(a, i, i < a.nV && !a.fixed[i], a.x, y0, y1, y2);
     if (i < a.nV) {
         double Mi[9];
         const bool fx = a.fixed[i] != 0;
