@@ -164,14 +164,6 @@ struct GjTile {
     }
     __device__ __forceinline__ bool has(int u) const { return q + 8 * u <= i; }
 };
-// 1 / d to within an ulp from an FP32 reciprocal (two Newton steps: 24, 48, 96 bits)
-__device__ __forceinline__ double gj_reciprocal(double d) {
-    const float f = (float)d;
-    if (!(f > 1e-30f && f < 1e30f)) return 1.0 / d;
-    double r = (double)(1.f / f);
-    r = fma(r, fma(-d, r, 1.0), r);
-    return fma(r, fma(-d, r, 1.0), r);
-}
 // e <- the lower half of -S^-1 for the SPD tile S whose lower half e holds, by 32 symmetric sweeps
 //     s_kk -> -1/p,  s_ik -> c_i / p,  s_ij -> s_ij - c_i c_j / p   (p = s_kk, c_i = s_ik).
 // Bounded by the chain of a sweep: publish column k + 1, barrier, update.  Warp 0 carries all diagonals
@@ -189,7 +181,7 @@ __device__ void gj_tile_sweep(const GjTile& m, double (&e)[4], double (*col)[GJ_
     double d = 0.0;
     if (t < GJ_B) {
         d = diag[t];
-        if (t == 0) pinv[0] = gj_reciprocal(d);
+        if (t == 0) pinv[0] = reciprocal(d);
     }
     __syncthreads();
     for (int k = 0; k < GJ_B; ++k) {
@@ -198,7 +190,7 @@ __device__ void gj_tile_sweep(const GjTile& m, double (&e)[4], double (*col)[GJ_
         if (t < GJ_B && k + 1 < GJ_B) {
             const double c = col[b][t];
             d = fma(-c * pin, c, d);
-            if (t == k + 1) pinv[b ^ 1] = gj_reciprocal(d);
+            if (t == k + 1) pinv[b ^ 1] = reciprocal(d);
         }
         const double r = ci * pin;
 #pragma unroll

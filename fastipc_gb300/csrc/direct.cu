@@ -10,10 +10,10 @@
 //    as NEWTON_IPC.py:758-772 makes it) scattered into the fronts, elastic then contact;
 //  * per tree height, children's update matrices pulled into their parents (each entry sums its
 //    children in a fixed order), then every front of the height factored panel by panel: the
-//    64 x 64 diagonal tile by one CTA, the rows below it in 64-row chunks, and the trailing
-//    update in 64 x 64 tiles (4 x 4 register blocks, operands staged in shared memory) across
+//    64 x 64 diagonal tile by one CTA, the rows below it 16 per CTA, and the trailing
+//    update in 32 x 32 tiles (register blocks, operands staged in shared memory) across
 //    all fronts of the height at once;
-//  * forward and backward substitution through the tree (one CTA per front).
+//  * forward and backward substitution through the tree by the same panels.
 // Every sum runs in a fixed order, so the solve is deterministic.  FP64 throughout: the
 // trailing update, which holds nearly all the flops, is bound by the FP64 pipe.
 #include <cuda_runtime.h>
@@ -106,128 +106,175 @@ __device__ __forceinline__ void panel_geometry(const MfDev& d, const PanelArgs& 
     *kb = min(MF_TILE, 3 * d.npiv[*f] - *c0);
 }
 
-// Cholesky of the diagonal tile, one CTA per front, right-looking in shared memory
+// Cholesky of the diagonal tile, one CTA per front.  Bounded by the chain of its 64 pivots: the lower half
+// stays in registers (four threads per row, thread q of them the columns q + 4 u), the unscaled column of a
+// pivot goes through shared memory, and warp 0 carries all diagonals, so that the next pivot's
+// reciprocal is formed while the others update: s_ij -= c_i c_j / p.  The columns are scaled to L
+// at the end.  Rows are dealt to the warps so that the four schedulers (warp % 4) have the same FP64
+// work.  Column by column in shared memory, with the square root, the division and the update behind one
+// another, a tile took 94 us.
 __global__ void __launch_bounds__(MF_THREADS) k_mf_potrf(MfDev d, PanelArgs p) {
-    __shared__ double T[MF_TILE * MF_LDS];
+    __shared__ double col[2][MF_TILE], pinv[2], piv[MF_TILE];
     int f, N, c0, kb;
     panel_geometry(d, p, blockIdx.x, &f, &N, &c0, &kb);
     double* F = d.F + d.foff[f] + c0 + (long long)c0 * N;
-    for (int idx = threadIdx.x; idx < kb * kb; idx += MF_THREADS) {
-        const int i = idx % kb, j = idx / kb;
-        if (i >= j) T[i + j * MF_LDS] = F[i + (long long)j * N];
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31, rb = w < 4 ? w : 11 - w;
+    const int i = 8 * rb + (lane >> 2), q = lane & 3;
+    double e[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int j = q + 4 * u;
+        e[u] = j <= i && i < kb ? F[i + (long long)j * N] : 0.0;
+        if (j == 0) col[0][i] = e[u];
+    }
+    // the diagonals: rows lane and lane + 32
+    double d0 = 0.0, d1 = 0.0;
+    auto next_pivot = [&](int k, int b) {   // the calling lane holds diagonal k
+        double v = k < 32 ? d0 : d1;
+        if (!(v > 0.0) || !isfinite(v)) {
+            atomicOr(d.flag, 1);
+            v = 1.0;
+        }
+        piv[k] = v;
+        pinv[b] = reciprocal(v);
+    };
+    if (w == 0) {
+        if (lane < kb) d0 = F[lane + (long long)lane * N];
+        if (lane + 32 < kb) d1 = F[lane + 32 + (long long)(lane + 32) * N];
+        if (lane == 0) next_pivot(0, 0);
     }
     __syncthreads();
-    for (int j = 0; j < kb; ++j) {
-        if (threadIdx.x == 0) {
-            double dj = T[j + j * MF_LDS];
-            if (!(dj > 0.0) || !isfinite(dj)) {
-                atomicOr(d.flag, 1);
-                dj = 1.0;
-            }
-            T[j + j * MF_LDS] = sqrt(dj);
+    for (int k = 0; k < kb; ++k) {
+        const int b = k & 1;
+        const double pin = pinv[b];
+        if (w == 0 && k + 1 < kb) {
+            const double x0 = col[b][lane], x1 = col[b][lane + 32];
+            d0 = fma(-x0 * pin, x0, d0);
+            d1 = fma(-x1 * pin, x1, d1);
+            if (lane == ((k + 1) & 31)) next_pivot(k + 1, b ^ 1);
         }
-        __syncthreads();
-        const double piv = T[j + j * MF_LDS];
-        for (int i = j + 1 + threadIdx.x; i < kb; i += MF_THREADS) T[i + j * MF_LDS] /= piv;
-        __syncthreads();
-        const int r = kb - j - 1;
-        for (int idx = threadIdx.x; idx < r * r; idx += MF_THREADS) {
-            const int i = j + 1 + idx % r, l = j + 1 + idx / r;
-            if (i >= l) T[i + l * MF_LDS] -= T[i + j * MF_LDS] * T[l + j * MF_LDS];
+        if (8 * rb + 7 > k) {
+            const double r = col[b][i] * pin;
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                if (4 * u + 3 <= k || 4 * u > 8 * rb + 7) continue;   // uniform over the warp
+                const int j = q + 4 * u;
+                if (j > k && j <= i) {
+                    e[u] = fma(-r, col[b][j], e[u]);
+                    if (j == k + 1) col[b ^ 1][i] = e[u];
+                }
+            }
         }
         __syncthreads();
     }
-    for (int idx = threadIdx.x; idx < kb * kb; idx += MF_THREADS) {
-        const int i = idx % kb, j = idx / kb;
-        if (i >= j) F[i + (long long)j * N] = T[i + j * MF_LDS];
+    // L_jj = sqrt(p_j), L_ij = c_ij / sqrt(p_j)
+    if (t < kb) col[0][t] = 1.0 / sqrt(piv[t]);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int j = q + 4 * u;
+        if (j <= i && i < kb) F[i + (long long)j * N] = j == i ? sqrt(piv[j]) : e[u] * col[0][j];
     }
 }
 
-// rows below the diagonal tile, 64 per CTA: X L^T = B, right-looking over the panel's columns
+// the panel's diagonal tile into shared memory, scaled so that a substitution step is one FMA: column j
+// divided by L_jj (forward: S[j][l] = L_lj / L_jj, l > j) or row i by L_ii (backward: S[i][j] = L_ij / L_ii,
+// j < i), zero elsewhere; rinv = 1 / diagonal
+template <bool FORWARD>
+__device__ __forceinline__ void load_tile(const double* __restrict__ F, int N, int kb, double* __restrict__ S, double* __restrict__ rinv) {
+    for (int j = threadIdx.x; j < MF_TILE; j += blockDim.x) rinv[j] = j < kb ? 1.0 / F[j + (long long)j * N] : 0.0;
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < MF_TILE * MF_TILE; idx += blockDim.x) {
+        const int l = idx % MF_TILE, j = idx / MF_TILE;   // row, column
+        const double v = l > j && l < kb ? F[l + (long long)j * N] : 0.0;
+        if (FORWARD) S[j * MF_LDS + l] = v * rinv[j];
+        else S[l * MF_LDS + j] = v * rinv[l];
+    }
+    __syncthreads();
+}
+
+// rows below the diagonal tile: X L^T = B, 16 rows per CTA (a quarter of a 64-row chunk), 16 lanes per row
+// with four columns each in registers.  A step is one shuffle and one to four FMAs, without a barrier;
+// 64 rows per CTA and two barriers per column left most SMs idle on 100 us of one CTA's FP64 work.
+constexpr int TRSM_ROWS = 16;
 __global__ void __launch_bounds__(MF_THREADS) k_mf_trsm(MfDev d, PanelArgs p) {
-    extern __shared__ double sm[];
-    double* L = sm;
-    double* B = sm + MF_TILE * MF_LDS;
-    const int e = mf_find(p.chunk0, p.n_fronts + 1, blockIdx.x);
+    __shared__ double S[MF_TILE * MF_LDS], rinv[MF_TILE];
+    const int chunk = blockIdx.x / (MF_TILE / TRSM_ROWS), part = blockIdx.x % (MF_TILE / TRSM_ROWS);
+    const int e = mf_find(p.chunk0, p.n_fronts + 1, chunk);
     int f, N, c0, kb;
     panel_geometry(d, p, e, &f, &N, &c0, &kb);
-    const int r0 = c0 + kb + (int)(blockIdx.x - p.chunk0[e]) * MF_TILE;
-    const int nr = min(MF_TILE, N - r0);
-    const double* Fd = d.F + d.foff[f] + c0 + (long long)c0 * N;
-    double* Fb = d.F + d.foff[f] + r0 + (long long)c0 * N;
-    for (int idx = threadIdx.x; idx < kb * kb; idx += MF_THREADS) {
-        const int i = idx % kb, j = idx / kb;
-        if (i >= j) L[i + j * MF_LDS] = Fd[i + (long long)j * N];
+    const int r0 = c0 + kb + (int)(chunk - p.chunk0[e]) * MF_TILE + part * TRSM_ROWS;
+    if (r0 >= N) return;
+    const int t = threadIdx.x & 15, r = r0 + (threadIdx.x >> 4);
+    double* Fb = d.F + d.foff[f] + r + (long long)c0 * N;
+    double b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int j = t + 16 * u;
+        b[u] = r < N && j < kb ? Fb[(long long)j * N] : 0.0;
     }
-    for (int idx = threadIdx.x; idx < nr * kb; idx += MF_THREADS) {
-        const int r = idx % nr, j = idx / nr;
-        B[r + j * MF_LDS] = Fb[r + (long long)j * N];
-    }
-    __syncthreads();
-    for (int j = 0; j < kb; ++j) {
-        const double piv = L[j + j * MF_LDS];
-        for (int r = threadIdx.x; r < nr; r += MF_THREADS) B[r + j * MF_LDS] /= piv;
-        __syncthreads();
-        const int w = kb - j - 1;
-        for (int idx = threadIdx.x; idx < nr * w; idx += MF_THREADS) {
-            const int r = idx % nr, l = j + 1 + idx / nr;
-            B[r + l * MF_LDS] -= B[r + j * MF_LDS] * L[l + j * MF_LDS];
+    load_tile<true>(d.F + d.foff[f] + c0 + (long long)c0 * N, N, kb, S, rinv);
+#pragma unroll
+    for (int u0 = 0; u0 < 4; ++u0)
+        for (int jj = 0; jj < 16; ++jj) {
+            const double bj = __shfl_sync(0xffffffffu, b[u0], jj, 16);
+            const double* Sj = S + (16 * u0 + jj) * MF_LDS + t;
+#pragma unroll
+            for (int u = u0; u < 4; ++u) b[u] = fma(-bj, Sj[16 * u], b[u]);
         }
-        __syncthreads();
-    }
-    for (int idx = threadIdx.x; idx < nr * kb; idx += MF_THREADS) {
-        const int r = idx % nr, j = idx / nr;
-        Fb[r + (long long)j * N] = B[r + j * MF_LDS];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int j = t + 16 * u;
+        if (r < N && j < kb) Fb[(long long)j * N] = b[u] * rinv[j];
     }
 }
 
-// trailing update of one 64 x 64 lower tile: C -= A_i A_j^T over the panel's kb columns.
-// Thread (tr, tc) owns rows tr + 16 a and columns tc + 16 b (a, b < 4): a warp's loads and
-// stores of C cover 16 consecutive rows of two columns.
-__global__ void __launch_bounds__(MF_THREADS) k_mf_update(MfDev d, PanelArgs p) {
-    extern __shared__ double sm[];
-    double* As = sm;                      // [l][row], 64 x 64
-    double* Bs = sm + MF_TILE * MF_TILE;
-    const int e = mf_find(p.tile0, p.n_fronts + 1, blockIdx.x);
+// trailing update of the lower tiles, C -= A_i A_j^T over the panel's kb columns, a quarter (32 x 32) of a
+// 64 x 64 tile per CTA: bound by the FP64 pipe (19 us a quarter on one SM), and whole tiles left SMs idle
+// in the panels with fewer tiles than SMs, and computed the upper quarter of diagonal tiles.
+// Thread (tr, tc) owns rows tr + 16 a (a < 2) and columns tc + 8 b (b < 4).
+constexpr int UPD_TILE = 32, UPD_THREADS = 128;
+__global__ void __launch_bounds__(UPD_THREADS) k_mf_update(MfDev d, PanelArgs p) {
+    __shared__ double As[MF_TILE * UPD_TILE], Bs[MF_TILE * UPD_TILE];   // [l][row]
+    const int tile = blockIdx.x >> 2, qi = blockIdx.x >> 1 & 1, qj = blockIdx.x & 1;
+    const int e = mf_find(p.tile0, p.n_fronts + 1, tile);
     int f, N, c0, kb;
     panel_geometry(d, p, e, &f, &N, &c0, &kb);
     int ti, tj;
-    mf_tile(blockIdx.x - p.tile0[e], &ti, &tj);
+    mf_tile(tile - p.tile0[e], &ti, &tj);
+    if (ti == tj && qi < qj) return;
     const int s0 = c0 + kb;
-    const int i0 = s0 + ti * MF_TILE, j0 = s0 + tj * MF_TILE;
-    const int ni = min(MF_TILE, N - i0), nj = min(MF_TILE, N - j0);
+    const int i0 = s0 + ti * MF_TILE + qi * UPD_TILE, j0 = s0 + tj * MF_TILE + qj * UPD_TILE;
+    if (i0 >= N || j0 >= N) return;
+    const int ni = min(UPD_TILE, N - i0), nj = min(UPD_TILE, N - j0);
     const double* F = d.F + d.foff[f];
-    for (int idx = threadIdx.x; idx < MF_TILE * kb; idx += MF_THREADS) {
-        const int r = idx % MF_TILE, l = idx / MF_TILE;
-        As[l * MF_TILE + r] = r < ni ? F[(i0 + r) + (long long)(c0 + l) * N] : 0.0;
-        Bs[l * MF_TILE + r] = r < nj ? F[(j0 + r) + (long long)(c0 + l) * N] : 0.0;
+    for (int idx = threadIdx.x; idx < UPD_TILE * kb; idx += UPD_THREADS) {
+        const int r = idx % UPD_TILE, l = idx / UPD_TILE;
+        As[idx] = r < ni ? F[(i0 + r) + (long long)(c0 + l) * N] : 0.0;
+        Bs[idx] = r < nj ? F[(j0 + r) + (long long)(c0 + l) * N] : 0.0;
     }
     __syncthreads();
     const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
-    double acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+    double acc[2][4] = {};
+#pragma unroll 2
     for (int l = 0; l < kb; ++l) {
-        double av[4], bv[4];
+        double av[2], bv[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            av[a] = As[l * MF_TILE + tr + 16 * a];
-            bv[a] = Bs[l * MF_TILE + tc + 16 * a];
-        }
+        for (int a = 0; a < 2; ++a) av[a] = As[l * UPD_TILE + tr + 16 * a];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int b = 0; b < 4; ++b) bv[b] = Bs[l * UPD_TILE + tc + 8 * b];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int b = 0; b < 4; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
     }
     double* C = d.F + d.foff[f];
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-        const int j = tc + 16 * b;
+        const int j = tc + 8 * b;
         if (j >= nj) continue;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int a = 0; a < 2; ++a) {
             const int i = tr + 16 * a;
             if (i < ni) C[(i0 + i) + (long long)(j0 + j) * N] -= acc[a][b];
         }
@@ -235,15 +282,16 @@ __global__ void __launch_bounds__(MF_THREADS) k_mf_update(MfDev d, PanelArgs p) 
 }
 
 // ---------------------------------------------------------------- substitution
-// forward: w = gathered right-hand side + children's updates; pivots solved column by column
-// (pivot results to Y), the rest of w updated; one CTA per front of the height
-__global__ void __launch_bounds__(MF_THREADS) k_mf_forward(MfDev d, int h0, const double* __restrict__ rhs) {
+// By the panels of the factorisation: one CTA per front walking its columns one after the other, each a
+// load from memory and a barrier, took 11.5 (forward) and 13.2 ms (backward) on a pile of 8,000
+// vertices, nine heights and 61 panels.
+//
+// forward, per height: w = gathered right-hand side + children's updates (all rows)
+__global__ void __launch_bounds__(MF_THREADS) k_mf_forward_gather(MfDev d, int h0, const double* __restrict__ rhs) {
     const int f = d.level_nodes[h0 + blockIdx.x];
-    const int N = 3 * d.nvf[f], P = 3 * d.npiv[f];
+    const int N = 3 * d.nvf[f];
     double* w = d.W + d.woff[f];
-    double* y = d.Y + d.woff[f];
-    const double* F = d.F + d.foff[f];
-    for (int i = threadIdx.x; i < N; i += MF_THREADS) {
+    for (int i = blockIdx.y * MF_THREADS + threadIdx.x; i < N; i += gridDim.y * MF_THREADS) {
         const int I = i / 3, ib = i % 3;
         double v = I < d.npiv[f] ? rhs[3ll * d.order[d.piv0[f] + I] + ib] : 0.0;
         for (int t = d.child0[f]; t < d.child0[f + 1]; ++t) {
@@ -253,48 +301,138 @@ __global__ void __launch_bounds__(MF_THREADS) k_mf_forward(MfDev d, int h0, cons
         }
         w[i] = v;
     }
-    __syncthreads();
-    for (int j = 0; j < P; ++j) {
-        const double wj = w[j] / F[j + (long long)j * N];
-        if (threadIdx.x == 0) y[j] = wj;
-        for (int i = j + 1 + threadIdx.x; i < N; i += MF_THREADS) w[i] -= F[i + (long long)j * N] * wj;
-        __syncthreads();
-    }
-    for (int j = threadIdx.x; j < P; j += MF_THREADS) w[j] = y[j];
 }
 
-// backward, one CTA per front of the height (parents first): the structure's values from the
-// solution, w_j -= L_ij x_i over them (a warp per column), then the pivots' triangle by one
-// warp, written to the solution
-__global__ void __launch_bounds__(MF_THREADS) k_mf_backward(MfDev d, int h0, double* __restrict__ sol) {
+// per panel: the tile's triangle (by warp 0, two rows per lane; x to shared memory), in every CTA of the
+// front; the first n_fronts CTAs store it to Y, the others update 64 rows below, w -= L x, with
+// their rows of L loaded before the chain
+__global__ void __launch_bounds__(MF_THREADS) k_mf_forward(MfDev d, PanelArgs p) {
+    __shared__ double S[MF_TILE * MF_LDS], rinv[MF_TILE], x[MF_TILE], sum[3][MF_TILE];
+    const bool diag = (int)blockIdx.x < p.n_fronts;
+    const int chunk = (int)blockIdx.x - p.n_fronts;
+    const int e = diag ? (int)blockIdx.x : mf_find(p.chunk0, p.n_fronts + 1, chunk);
+    int f, N, c0, kb;
+    panel_geometry(d, p, e, &f, &N, &c0, &kb);
+    const double* F = d.F + d.foff[f];
+    double* w = d.W + d.woff[f];
+    const int r0 = diag ? N : c0 + kb + (int)(chunk - p.chunk0[e]) * MF_TILE;
+    const int r = r0 + (threadIdx.x & 63), part = threadIdx.x >> 6;   // 16 columns each
+    double v[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] = r < N && 16 * part + c < kb ? F[r + (long long)(c0 + 16 * part + c) * N] : 0.0;
+    load_tile<true>(F + c0 + (long long)c0 * N, N, kb, S, rinv);
+    if (threadIdx.x < 32) {
+        const int l = threadIdx.x;
+        double w0 = l < kb ? w[c0 + l] : 0.0, w1 = l + 32 < kb ? w[c0 + 32 + l] : 0.0;
+#pragma unroll 4
+        for (int j = 0; j < 32; ++j) {
+            const double wj = __shfl_sync(0xffffffffu, w0, j);
+            w0 = fma(-wj, S[j * MF_LDS + l], w0);
+            w1 = fma(-wj, S[j * MF_LDS + l + 32], w1);
+        }
+#pragma unroll 4
+        for (int j = 0; j < 32; ++j) w1 = fma(-__shfl_sync(0xffffffffu, w1, j), S[(j + 32) * MF_LDS + l + 32], w1);
+        x[l] = w0 * rinv[l];
+        x[l + 32] = w1 * rinv[l + 32];
+    }
+    __syncthreads();
+    if (diag) {
+        if (threadIdx.x < kb) d.Y[d.woff[f] + c0 + threadIdx.x] = x[threadIdx.x];
+        return;
+    }
+    double a = 0.0;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) a = fma(v[c], x[16 * part + c], a);
+    if (part) sum[part - 1][threadIdx.x & 63] = a;
+    __syncthreads();
+    if (part == 0 && r < N) w[r] -= ((a + sum[0][threadIdx.x]) + sum[1][threadIdx.x]) + sum[2][threadIdx.x];
+}
+
+// backward, per height (parents first): y -= L^T x over the structure's rows, whose x the solution holds;
+// 32 columns per CTA, four per warp
+constexpr int BWD_COLS = 32, BWD_ROWS = 512;
+__global__ void __launch_bounds__(MF_THREADS) k_mf_backward_gather(MfDev d, int h0, const double* __restrict__ sol) {
+    __shared__ double x[BWD_ROWS];
     const int f = d.level_nodes[h0 + blockIdx.x];
     const int N = 3 * d.nvf[f], P = 3 * d.npiv[f];
-    double* w = d.W + d.woff[f];
+    double* y = d.Y + d.woff[f];
     const double* F = d.F + d.foff[f];
     const int* fl = d.fidx + d.fidx0[f];
-    for (int i = P + threadIdx.x; i < N; i += MF_THREADS) w[i] = sol[3ll * d.order[fl[i / 3]] + i % 3];
-    __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int j = wid; j < P; j += MF_THREADS / 32) {
-        double s = 0.0;
-        for (int i = P + lane; i < N; i += 32) s += F[i + (long long)j * N] * w[i];
+    for (int j0 = blockIdx.y * BWD_COLS; j0 < P; j0 += gridDim.y * BWD_COLS) {
+        const int j = j0 + 4 * wid;
+        double a[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int i0 = P; i0 < N; i0 += BWD_ROWS) {
+            const int n = min(BWD_ROWS, N - i0);
+            __syncthreads();
+            for (int i = threadIdx.x; i < n; i += MF_THREADS) x[i] = sol[3ll * d.order[fl[(i0 + i) / 3]] + (i0 + i) % 3];
+            __syncthreads();
+#pragma unroll 2
+            for (int i = lane; i < n; i += 32) {
+                const double xi = x[i];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) w[j] -= s;
-    }
-    __syncthreads();
-    if (wid == 0) {
-        for (int j = P - 1; j >= 0; --j) {
-            double s = 0.0;
-            for (int i = j + 1 + lane; i < P; i += 32) s += F[i + (long long)j * N] * w[i];
+                for (int c = 0; c < 4; ++c)
+                    if (j + c < P) a[c] = fma(F[i0 + i + (long long)(j + c) * N], xi, a[c]);
+            }
+        }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-            if (lane == 0) w[j] = (w[j] - s) / F[j + (long long)j * N];
-            __syncwarp();
+        for (int c = 0; c < 4; ++c) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a[c] += __shfl_down_sync(0xffffffffu, a[c], o);
+            if (lane == 0 && j + c < P) y[j + c] -= a[c];
         }
     }
+}
+
+// per panel k, the last first: the tile's transposed triangle in every CTA of the front; CTA k of them
+// stores it to the solution, CTA c < k updates the 64 columns of panel c, y -= L^T x
+__global__ void __launch_bounds__(MF_THREADS) k_mf_backward(MfDev d, PanelArgs p, double* __restrict__ sol) {
+    __shared__ double S[MF_TILE * MF_LDS], rinv[MF_TILE], x[MF_TILE];
+    const int e = blockIdx.x / (p.k + 1), c = blockIdx.x % (p.k + 1);
+    int f, N, c0, kb;
+    panel_geometry(d, p, e, &f, &N, &c0, &kb);
+    const double* F = d.F + d.foff[f];
+    double* y = d.Y + d.woff[f];
+    // rows t + 16 q of the panel, columns 64 c + g + 16 m
+    const int t = threadIdx.x & 15, g = threadIdx.x >> 4;
+    double v[4][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int row = t + 16 * q;
+            v[m][q] = c < p.k && row < kb ? F[c0 + row + (long long)(MF_TILE * c + g + 16 * m) * N] : 0.0;
+        }
+    load_tile<false>(F + c0 + (long long)c0 * N, N, kb, S, rinv);
+    if (threadIdx.x < 32) {
+        const int l = threadIdx.x;
+        double y0 = l < kb ? y[c0 + l] : 0.0, y1 = l + 32 < kb ? y[c0 + 32 + l] : 0.0;
+#pragma unroll 4
+        for (int j = 31; j >= 0; --j) {
+            const double yj = __shfl_sync(0xffffffffu, y1, j);
+            y0 = fma(-yj, S[(j + 32) * MF_LDS + l], y0);
+            y1 = fma(-yj, S[(j + 32) * MF_LDS + l + 32], y1);
+        }
+#pragma unroll 4
+        for (int j = 31; j >= 0; --j) y0 = fma(-__shfl_sync(0xffffffffu, y0, j), S[j * MF_LDS + l], y0);
+        x[l] = y0 * rinv[l];
+        x[l + 32] = y1 * rinv[l + 32];
+    }
     __syncthreads();
-    for (int j = threadIdx.x; j < P; j += MF_THREADS) sol[3ll * d.order[d.piv0[f] + j / 3] + j % 3] = w[j];
+    if (c == p.k) {
+        const int j = threadIdx.x;
+        if (j < kb) sol[3ll * d.order[d.piv0[f] + (c0 + j) / 3] + (c0 + j) % 3] = x[j];
+        return;
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        double a = 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a = fma(v[m][q], x[t + 16 * q], a);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o, 16);
+        if (t == 0) y[MF_TILE * c + g + 16 * m] -= a;
+    }
 }
 
 struct DevMem {
@@ -325,8 +463,6 @@ struct Arena {
         return true;
     }
 };
-
-bool g_attr_set = false;
 
 }  // namespace
 }  // namespace fipc
@@ -428,11 +564,6 @@ int fipc_solve_system_direct(fipc_ctx* c, const unsigned char* fixed, double* so
     d.flag = flag.as<int>();
     FIPC_CUDA(cudaMemsetAsync(d.F, 0, 8ull * P.f_total, s));
     FIPC_CUDA(cudaMemsetAsync(d.flag, 0, 16, s));
-    if (!g_attr_set) {
-        FIPC_CUDA(cudaFuncSetAttribute(k_mf_update, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * MF_TILE * MF_TILE));
-        FIPC_CUDA(cudaFuncSetAttribute(k_mf_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * MF_TILE * MF_LDS));
-        g_attr_set = true;
-    }
     int st = sell_to_bsr(c, ev.as<double>(), s);
     if (st) return st;
     if (e_nnzb) {
@@ -443,6 +574,10 @@ int fipc_solve_system_direct(fipc_ctx* c, const unsigned char* fixed, double* so
         k_mf_scatter<<<nbd(c_nnzb, 256), 256, 0, s>>>(c_nnzb, c->c_val.as<double>(), c_dst, c_ld, d.F, 1);
         FIPC_LAUNCHED();
     }
+    auto panel = [&](size_t k) {
+        const MfPlan::Panel& pl = P.panels[k];
+        return PanelArgs{pl.k, pl.n_fronts, pl.t0, d.task_chunk0 + P.task_off[k], d.task_tile0 + P.task_off[k]};
+    };
     size_t pn = 0;
     for (int h = 0; h <= P.height_max; ++h) {
         const int nf = (int)(ext_at[h + 1] - ext_at[h]);
@@ -453,27 +588,44 @@ int fipc_solve_system_direct(fipc_ctx* c, const unsigned char* fixed, double* so
         }
         for (; pn < P.panels.size() && P.panels[pn].height == h; ++pn) {
             const MfPlan::Panel& pl = P.panels[pn];
-            PanelArgs pa{pl.k, pl.n_fronts, pl.t0, d.task_chunk0 + P.task_off[pn], d.task_tile0 + P.task_off[pn]};
+            const PanelArgs pa = panel(pn);
             k_mf_potrf<<<pl.n_fronts, MF_THREADS, 0, s>>>(d, pa);
             FIPC_LAUNCHED();
             if (pl.n_chunks) {
-                k_mf_trsm<<<(unsigned)pl.n_chunks, MF_THREADS, 16 * MF_TILE * MF_LDS, s>>>(d, pa);
+                k_mf_trsm<<<(unsigned)(pl.n_chunks * (MF_TILE / TRSM_ROWS)), MF_THREADS, 0, s>>>(d, pa);
                 FIPC_LAUNCHED();
             }
             if (pl.n_tiles) {
-                k_mf_update<<<(unsigned)pl.n_tiles, MF_THREADS, 16 * MF_TILE * MF_TILE, s>>>(d, pa);
+                k_mf_update<<<(unsigned)(4 * pl.n_tiles), UPD_THREADS, 0, s>>>(d, pa);
                 FIPC_LAUNCHED();
             }
         }
     }
     // right-hand side with zeros at fixed vertices is implied: only free vertices are gathered
+    std::vector<int> max_n(P.height_max + 1, 0), max_p(P.height_max + 1, 0);   // rows and pivots of a height's largest front
+    for (int h = 0; h <= P.height_max; ++h)
+        for (int q = P.lvl0[h]; q < P.lvl0[h + 1]; ++q) {
+            max_n[h] = std::max(max_n[h], 3 * P.nvf[P.level_nodes[q]]);
+            max_p[h] = std::max(max_p[h], 3 * P.npiv[P.level_nodes[q]]);
+        }
+    pn = 0;
     for (int h = 0; h <= P.height_max; ++h) {
-        k_mf_forward<<<P.lvl0[h + 1] - P.lvl0[h], MF_THREADS, 0, s>>>(d, P.lvl0[h], c->rhs);
+        k_mf_forward_gather<<<dim3(P.lvl0[h + 1] - P.lvl0[h], std::max(1, std::min(16, nbd(max_n[h], MF_THREADS)))), MF_THREADS, 0, s>>>(
+            d, P.lvl0[h], c->rhs);
         FIPC_LAUNCHED();
+        for (; pn < P.panels.size() && P.panels[pn].height == h; ++pn) {
+            k_mf_forward<<<(unsigned)(P.panels[pn].n_fronts + P.panels[pn].n_chunks), MF_THREADS, 0, s>>>(d, panel(pn));
+            FIPC_LAUNCHED();
+        }
     }
     for (int h = P.height_max; h >= 0; --h) {
-        k_mf_backward<<<P.lvl0[h + 1] - P.lvl0[h], MF_THREADS, 0, s>>>(d, P.lvl0[h], sol);
+        k_mf_backward_gather<<<dim3(P.lvl0[h + 1] - P.lvl0[h], std::max(1, std::min(64, nbd(max_p[h], BWD_COLS)))), MF_THREADS, 0, s>>>(
+            d, P.lvl0[h], sol);
         FIPC_LAUNCHED();
+        for (; pn > 0 && P.panels[pn - 1].height == h; --pn) {
+            k_mf_backward<<<(unsigned)(P.panels[pn - 1].n_fronts * (P.panels[pn - 1].k + 1)), MF_THREADS, 0, s>>>(d, panel(pn - 1), sol);
+            FIPC_LAUNCHED();
+        }
     }
     FIPC_CUDA(cudaGetLastError());
     int bad = 0;
