@@ -417,14 +417,17 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_res0(PCGArgs a, const double
 }
 
 // t0 = r - A z0 with FP32 products (values and z0 as FP32, FP32 sums); the residual in FP64
+template <int PARTS>
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_res0_f32(PCGArgs a, const float* __restrict__ v32, const float* __restrict__ c32,
                                                              const float4* __restrict__ z0f, double* __restrict__ t0) {
     if (*(volatile int*)&a.flag[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const RowPart<PARTS> q;
+    const int i = q.i;
     const bool fx = i < a.nV && a.fixed[i];
     float y0, y1, y2;
-    row_apply_f32(a, v32, c32, i, i < a.nV && !fx, z0f, y0, y1, y2);
-    if (i >= a.nV) return;
+    row_apply_f32<PARTS>(a, v32, c32, i, i < a.nV && !fx, z0f, y0, y1, y2, q.part);
+    combine_parts<PARTS>(q.part, y0, y1, y2);
+    if (i >= a.nV || q.part) return;
     t0[3 * (size_t)i] = fx ? 0.0 : a.r[3 * (size_t)i] - (double)y0;
     t0[3 * (size_t)i + 1] = fx ? 0.0 : a.r[3 * (size_t)i + 1] - (double)y1;
     t0[3 * (size_t)i + 2] = fx ? 0.0 : a.r[3 * (size_t)i + 2] - (double)y2;
@@ -576,15 +579,18 @@ __global__ void __launch_bounds__(PCG_THREADS) k_mg_post0(PCGArgs a, const doubl
 }
 
 // the same with FP32 products
+template <int PARTS>
 __global__ void __launch_bounds__(PCG_THREADS) k_mg_post0_f32(PCGArgs a, const float* __restrict__ v32, const float* __restrict__ c32,
                                                               const float4* __restrict__ z0f, const double* __restrict__ z0,
                                                               const double* __restrict__ omega) {
     if (*(volatile int*)&a.flag[0]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const RowPart<PARTS> q;
+    const int i = q.i;
     const bool fx = i < a.nV && a.fixed[i];
     float y0, y1, y2;
-    row_apply_f32(a, v32, c32, i, i < a.nV && !fx, z0f, y0, y1, y2);
-    if (i >= a.nV) return;
+    row_apply_f32<PARTS>(a, v32, c32, i, i < a.nV && !fx, z0f, y0, y1, y2, q.part);
+    combine_parts<PARTS>(q.part, y0, y1, y2);
+    if (i >= a.nV || q.part) return;
     if (fx) {
         a.u[4 * (size_t)i] = a.u[4 * (size_t)i + 1] = a.u[4 * (size_t)i + 2] = 0.0;
         return;
@@ -898,8 +904,10 @@ void mg_vcycle(const fipc_ctx* c, const PCGArgs& a, cudaStream_t s) {
     const MgState* M = reinterpret_cast<const MgState*>(c->mg);
     const MgArgs& m = M->args;
     const int NL = m.levels, nV = c->nV;
-    const int nb0 = nblk_m(nV, PCG_THREADS);
-    if (m.z0f) k_mg_res0_f32<<<nb0, PCG_THREADS, 0, s>>>(a, m.v32, m.c32, reinterpret_cast<const float4*>(m.z0f), m.t0);
+    const int nb0 = nblk_m(nV, PCG_THREADS), parts = row_parts(nV);
+    const float4* z0f = reinterpret_cast<const float4*>(m.z0f);
+    if (m.z0f && parts == 2) k_mg_res0_f32<2><<<nblk_m(nV, PCG_THREADS / 2), PCG_THREADS, 0, s>>>(a, m.v32, m.c32, z0f, m.t0);
+    else if (m.z0f) k_mg_res0_f32<1><<<nb0, PCG_THREADS, 0, s>>>(a, m.v32, m.c32, z0f, m.t0);
     else k_mg_res0<<<nb0, PCG_THREADS, 0, s>>>(a, m.z0, m.t0);
     for (int l = 1; l < NL; ++l) {
         const MgLev& L = m.L[l];
@@ -915,7 +923,8 @@ void mg_vcycle(const fipc_ctx* c, const PCGArgs& a, cudaStream_t s) {
                                                                     l == 1);
         if (l - 1 >= 1) launch_smooth<true>(a, m.L[l - 1], m.omega + (l - 1), s);
     }
-    if (m.z0f) k_mg_post0_f32<<<nb0, PCG_THREADS, 0, s>>>(a, m.v32, m.c32, reinterpret_cast<const float4*>(m.z0f), m.z0, m.omega);
+    if (m.z0f && parts == 2) k_mg_post0_f32<2><<<nblk_m(nV, PCG_THREADS / 2), PCG_THREADS, 0, s>>>(a, m.v32, m.c32, z0f, m.z0, m.omega);
+    else if (m.z0f) k_mg_post0_f32<1><<<nb0, PCG_THREADS, 0, s>>>(a, m.v32, m.c32, z0f, m.z0, m.omega);
     else k_mg_post0<<<nb0, PCG_THREADS, 0, s>>>(a, m.z0, m.omega);
     g_launches.fetch_add(mg_launches_per_cycle(NL), std::memory_order_relaxed);
 }

@@ -101,13 +101,13 @@ __device__ __forceinline__ int nth_bit(unsigned mask, int r) {
 // dependent loads of its row while the lanes of rows without contact idled.)
 template <class T, class LOAD>
 __device__ __forceinline__ void contact_rows(const int* __restrict__ crp, const int* __restrict__ cci, const T* __restrict__ cva, int i,
-                                             bool act, LOAD load, T& y0, T& y1, T& y2) {
+                                             bool act, LOAD load, T& y0, T& y1, T& y2, int part = 0, int parts = 1) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const int b = act ? __ldg(crp + i) : 0, e = act ? __ldg(crp + i + 1) : 0;
     const unsigned mask = __ballot_sync(full, e > b);
     const int n = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u));
-    for (int r0 = 0; r0 < n; r0 += 4) {
+    for (int r0 = 4 * part; r0 < n; r0 += 4 * parts) {
         const int r = r0 + (lane >> 3), row = nth_bit(mask, r < n ? r : 0);
         const int eb = __shfl_sync(full, b, row), ee = __shfl_sync(full, e, row);
         T s[3] = {T(0), T(0), T(0)};
@@ -139,6 +139,42 @@ __device__ __forceinline__ void contact_rows(const int* __restrict__ crp, const 
             y2 += s[2];
         }
     }
+}
+
+// Rows of a CTA of PCG_THREADS when PARTS warps share a slice of 32 rows, each taking every PARTS-th pair of
+// blocks and group of contact rows; the sums of parts 1, .. reach part 0 in combine_parts.  For FP32 products of
+// scenes that leave the SMs with few warps: a row's 14 blocks are then a chain of seven dependent loads
+// with nothing to hide it.  (FP64 products are bound by the FP64 pipe and lose by the second part's adds.)
+// Up to two dozen slices per SM: 61,700 rows (13 per SM) res0 22 -> 16 us, post0 28 -> 17; 182,000 (37 per
+// SM) 23.5 -> 24.5 and 26.8 -> 27.1.
+inline int row_parts(int nV) { return nV <= 24 * 152 * 32 ? 2 : 1; }
+template <int PARTS>
+struct RowPart {
+    int i, part;
+    __device__ __forceinline__ RowPart() {
+        const int w = threadIdx.x >> 5;
+        i = (blockIdx.x * (PCG_THREADS / 32 / PARTS) + w / PARTS) * 32 + (threadIdx.x & 31);
+        part = w % PARTS;
+    }
+};
+template <int PARTS, class T>
+__device__ __forceinline__ void combine_parts(int part, T& y0, T& y1, T& y2) {
+    if (PARTS == 1) return;
+    __shared__ T sh[PCG_THREADS / 32][3][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (part) {
+        sh[w][0][lane] = y0;
+        sh[w][1][lane] = y1;
+        sh[w][2][lane] = y2;
+    }
+    __syncthreads();
+    if (part == 0)
+#pragma unroll
+        for (int q = 1; q < PARTS; ++q) {
+            y0 += sh[w + q][0][lane];
+            y1 += sh[w + q][1][lane];
+            y2 += sh[w + q][2][lane];
+        }
 }
 
 // act: the lane has a row; all lanes of a warp call.  WIDE: contact blocks by groups of lanes, else each
@@ -203,13 +239,14 @@ __device__ __forceinline__ void row_apply(const PCGArgs& a, int i, bool act, con
 
 // y = A v with FP32 copies of the values (v32: the sliced-ELL layout of sval; c32: the contact
 // blocks) and an FP32 vector (stride 4), accumulated in FP32: the multigrid's smoothing products
+template <int PARTS>
 __device__ __forceinline__ void row_apply_f32(const PCGArgs& a, const float* __restrict__ v32, const float* __restrict__ c32, int i,
-                                              bool act, const float4* __restrict__ v, float& y0, float& y1, float& y2) {
+                                              bool act, const float4* __restrict__ v, float& y0, float& y1, float& y2, int part) {
     y0 = y1 = y2 = 0.f;
     const int sl = i >> 5, lane = i & 31;
     const int base = act ? a.soff[sl] : 0, len = act ? a.rlen[i] : 0;
-    int k = 0;
-    for (; k + 1 < len; k += 2) {
+    int k = 2 * part;
+    for (; k + 1 < len; k += 2 * PARTS) {
         const size_t s0 = (size_t)(base + k), s1 = s0 + 1;
         const int j0 = __ldg(a.scol + s0 * 32 + lane), j1 = __ldg(a.scol + s1 * 32 + lane);
         const float* B = v32 + s0 * 288 + lane;
@@ -243,7 +280,7 @@ __device__ __forceinline__ void row_apply_f32(const PCGArgs& a, const float* __r
         v0 = p.x;
         v1 = p.y;
         v2 = p.z;
-    }, y0, y1, y2);
+    }, y0, y1, y2, part, PARTS);
 }
 
 // block sums of NV per-thread values into the shared array out[NV] (valid in every thread on
