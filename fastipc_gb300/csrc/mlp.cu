@@ -22,19 +22,22 @@ constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + MLP_H * MLP_IN, OFF_W2 = OFF_B1 + ML
 
 // ---------------------------------------------------------------- tiles
 // A CTA holds a tile of R rows in shared memory, k-major (Hs[k][row]), and multiplies it with a
-// 128-column weight matrix whose K slices of 32 pass through a double buffer Ws.  Thread (tx, ty)
+// 128-column weight matrix whose K slices of 16 pass through a double buffer Ws.  Thread (tx, ty)
 // of 16 x 16 owns R/16 consecutive rows and the columns 4 tx .. 4 tx + 3 and 64 + 4 tx ..; per k
-// it loads its rows and two float4 of weights for (R/16) x 8 FMAs.  FP32 FMA issue binds: at
-// R = 128 a k step is 64 FMAs per thread against 4 shared-memory loads.  Rows are swizzled by the
+// it loads its rows and two float4 of weights for (R/16) x 8 FMAs, two rows' in one instruction.  The
+// FP32 FMA pipe binds (51% busy; the rest is waits of 4 warps per scheduler on it, on shared memory and on
+// the slices' barriers): at R = 128 a k step is 32 paired FMAs per thread against 4 shared-memory loads.
+// Slices of 32 hold 8 more registers in flight and spill; R = 64 and 256 are slower at 176,841 rows (0.51, 0.53
+// ms against 0.45).  Rows are swizzled by the
 // column group (row ^ 4 ((k / 4) % 8)) so that the transposed store of a layer's output, which
 // strides by columns, meets distinct banks while the row loads stay aligned.  Every output sums
 // its K range in ascending order in one FMA chain.
 // R = 128 needs n >= 2 x 152 such tiles to fill the GPU; below that R = 64, then 32, keep more SMs
 // busy.  Measured on a GB300, forward pass: 176,841 rows 1.19 ms as separate 64 x 64 products with
-// bias and activation passes, 0.50 ms here; a training step of 8,192 rows 5.3 ms, of
+// bias and activation passes, 0.45 ms here; a training step of 8,192 rows 5.3 ms, of
 // which 97% were products (the weight gradients, 128 x 128 outputs over all rows, ran on 2 to 4
 // CTAs), 0.17 ms here.
-constexpr int MLP_THREADS = 256, KS = 32, WLD = MLP_H + 4;
+constexpr int MLP_THREADS = 256, KS = 16, WLD = MLP_H + 4;
 
 // four consecutive floats of global memory: one 16-byte access when every array of the call is
 // 16-byte aligned (al), else four (callers may pass any float address)
@@ -74,18 +77,18 @@ __device__ __forceinline__ void load_rows(float* Hs, const float* __restrict__ s
 // one K slice of the weights, held in registers between its load and its store to shared memory:
 // T (transposed): W [128][K], slice[kk][c] = W[c][k0 + kk];  else W [K][128], slice[kk][c] = W[k0 + kk][c]
 template <bool T>
-__device__ __forceinline__ void fetch_slice(float4 (&w)[4], const float* __restrict__ W, int K, int k0, bool al) {
+__device__ __forceinline__ void fetch_slice(float4 (&w)[2], const float* __restrict__ W, int K, int k0, bool al) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < 2; ++q) {
         const int e = threadIdx.x + q * MLP_THREADS;
         if (T) w[q] = ld4(W + (size_t)(e % MLP_H) * K + k0 + 4 * (e / MLP_H), al);
         else w[q] = ld4(W + (size_t)(k0 + e / 32) * MLP_H + 4 * (e % 32), al);
     }
 }
 template <bool T>
-__device__ __forceinline__ void store_slice(float* Ws, const float4 (&w)[4]) {
+__device__ __forceinline__ void store_slice(float* Ws, const float4 (&w)[2]) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < 2; ++q) {
         const int e = threadIdx.x + q * MLP_THREADS;
         if (T) {
             float* p = Ws + 4 * (e / MLP_H) * WLD + e % MLP_H;
@@ -99,17 +102,33 @@ __device__ __forceinline__ void store_slice(float* Ws, const float4 (&w)[4]) {
     }
 }
 
+// two FP32 FMAs in one instruction (each rounded as fmaf): the FMA pipe takes them in two cycles, so a k
+// step's other instructions issue beside it instead of before it
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 // acc[i][j] = sum_k Hs[k][row i] W(k, col j) for the thread's rows and columns; Hs complete on entry
 template <int R, bool T>
 __device__ __forceinline__ void tile_product(float (&acc)[R / 16][8], const float* Hs, float* Ws, const float* __restrict__ W, int K,
                                              bool al) {
     constexpr int TR = R / 16;
     const int tx = threadIdx.x % 16, row0 = (threadIdx.x / 16) * TR;
+    f32x2 sum[TR / 2][8];   // pairs of rows
 #pragma unroll
-    for (int i = 0; i < TR; ++i)
+    for (int i = 0; i < TR / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    float4 w[4];
+        for (int j = 0; j < 8; ++j) sum[i][j] = 0;
+    float4 w[2];
     fetch_slice<T>(w, W, K, 0, al);
     store_slice<T>(Ws, w);
     __syncthreads();
@@ -139,13 +158,19 @@ __device__ __forceinline__ void tile_product(float (&acc)[R / 16][8], const floa
             const float4 b0 = *reinterpret_cast<const float4*>(Wb + kk * WLD), b1 = *reinterpret_cast<const float4*>(Wb + kk * WLD + 64);
             const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-            for (int i = 0; i < TR; ++i)
+            for (int j = 0; j < 8; ++j) {
+                const f32x2 bb = pack2(b[j], b[j]);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int i = 0; i < TR / 2; ++i) sum[i][j] = fma2(pack2(a[2 * i], a[2 * i + 1]), bb, sum[i][j]);
+            }
         }
         if (more) store_slice<T>(Ws + (buf ^ 1) * KS * WLD, w);
         __syncthreads();
     }
+#pragma unroll
+    for (int i = 0; i < TR / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) unpack2(sum[i][j], acc[2 * i][j], acc[2 * i + 1][j]);
 }
 __device__ __forceinline__ int tile_col(int j) { return 4 * (threadIdx.x % 16) + (j & 3) + 64 * (j >> 2); }
 
