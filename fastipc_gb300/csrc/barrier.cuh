@@ -158,14 +158,14 @@ FIPC_HD RowMap row_map(int type) {
     return m;
 }
 
-// Orthonormal basis of zero-sum combinations of nv vertices (Helmert), Qb[v][a], a < nv-1
-FIPC_HD double helmert(int nv, int v, int a) {
-    // column a: (1, .., 1, -(a+1), 0, ..) / sqrt((a+1)(a+2)) with a+1 ones
-    const double s = 1.0 / sqrt((double)((a + 1) * (a + 2)));
-    if (v <= a) return s;
-    if (v == a + 1) return -(double)(a + 1) * s;
-    (void)nv;
-    return 0.0;
+// Orthonormal basis of zero-sum combinations of nv vertices (Helmert), Qb[v][a], a < nv-1: column a is
+// (1, .., 1, -(a+1), 0, ..) / sqrt((a+1)(a+2)) with a+1 ones, whatever nv
+struct Helmert {
+    double q[4][3];
+};
+FIPC_HD Helmert helmert_basis() {
+    constexpr double r2 = 0.70710678118654752440, r6 = 0.40824829046386301637, r12 = 0.28867513459481288225;
+    return Helmert{{{r2, r6, r12}, {-r2, r6, r12}, {0.0, -2.0 * r6, r12}, {0.0, 0.0, -3.0 * r12}}};
 }
 
 // ---------------------------------------------------------------- unmollified rows in closed form
@@ -428,21 +428,23 @@ FIPC_HD void remove_negative(double (&A)[N][N]) {
 // component a of the Helmert basis (orthonormal, zero-sum) of a pattern over NV vertices
 template <int NV>
 FIPC_HD void helmert_components(const double (&w)[NV], double (&h)[NV - 1]) {
+    const Helmert Q = helmert_basis();
     double sum = 0.0;
 #pragma unroll
     for (int a = 0; a < NV - 1; ++a) {
         sum += w[a];
-        h[a] = (sum - (a + 1) * w[a + 1]) / sqrt((double)((a + 1) * (a + 2)));
+        h[a] = (sum - (a + 1) * w[a + 1]) * Q.q[0][a];
     }
 }
 // the pattern over the vertices of Helmert components h
 template <int NV>
 FIPC_HD void helmert_pattern(const double (&h)[NV - 1], double (&w)[NV]) {
+    const Helmert Q = helmert_basis();
 #pragma unroll
     for (int v = 0; v < NV; ++v) w[v] = 0.0;
 #pragma unroll
     for (int a = 0; a < NV - 1; ++a) {
-        const double s = h[a] / sqrt((double)((a + 1) * (a + 2)));
+        const double s = h[a] * Q.q[0][a];
 #pragma unroll
         for (int v = 0; v <= a; ++v) w[v] += s;
         w[a + 1] -= (a + 1) * s;
@@ -769,38 +771,46 @@ FIPC_HD int barrier_row(int type, const v3* X, const v3* X0, double dh2, double 
         }
     // K = C Q (ny x ny coefficient matrix), M = K^T Hy K (blockwise, 3x3 identity factor)
     const int na = m.nv - 1;   // == ny
+    const Helmert Q = helmert_basis();
     double K[3][3];
     for (int k = 0; k < m.ny; ++k)
         for (int a = 0; a < na; ++a) {
             double s = 0.0;
-            for (int v = 0; v < m.nv; ++v) s += m.C[k][v] * helmert(m.nv, v, a);
+            for (int v = 0; v < m.nv; ++v) s += m.C[k][v] * Q.q[v][a];
             K[k][a] = s;
         }
-    double M[81];
-    for (int a = 0; a < na; ++a)
-        for (int bb = 0; bb < na; ++bb)
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) {
-                    double s = 0.0;
-                    for (int k = 0; k < m.ny; ++k)
-                        for (int l = 0; l < m.ny; ++l) s += K[k][a] * K[l][bb] * Hy[(3 * k + i) * 9 + 3 * l + j];
-                    M[(3 * a + i) * 9 + 3 * bb + j] = s;
-                }
+    double M[81], HK[27];
+    for (int bb = 0; bb < na; ++bb) {
+        for (int r = 0; r < n; ++r)
+            for (int j = 0; j < 3; ++j) {
+                double s = 0.0;
+                for (int l = 0; l < m.ny; ++l) s += K[l][bb] * Hy[r * 9 + 3 * l + j];
+                HK[r * 3 + j] = s;
+            }
+        for (int a = 0; a < na; ++a)
+            for (int ij = 0; ij < 9; ++ij) {
+                double s = 0.0;
+                for (int k = 0; k < m.ny; ++k) s += K[k][a] * HK[9 * k + ij];
+                M[(3 * a + ij / 3) * 9 + 3 * bb + ij % 3] = s;
+            }
+    }
     int st = 0;
     if (want != 2) st = psd_project(n, M);
     // H = Q proj(M) Q^T in 3x3 vertex blocks
-    for (int v = 0; v < m.nv; ++v)
-        for (int w = 0; w < m.nv; ++w)
-            for (int i = 0; i < 3; ++i)
-                for (int j = 0; j < 3; ++j) {
-                    double s = 0.0;
-                    for (int a = 0; a < na; ++a) {
-                        const double qa = helmert(m.nv, v, a);
-                        if (qa == 0.0) continue;
-                        for (int bb = 0; bb < na; ++bb) s += qa * helmert(m.nv, w, bb) * M[(3 * a + i) * 9 + 3 * bb + j];
-                    }
-                    Hb[(v * 4 + w) * 9 + i * 3 + j] = s;
-                }
+    for (int w = 0; w < m.nv; ++w) {
+        for (int r = 0; r < n; ++r)
+            for (int j = 0; j < 3; ++j) {
+                double s = 0.0;
+                for (int bb = 0; bb < na; ++bb) s += Q.q[w][bb] * M[r * 9 + 3 * bb + j];
+                HK[r * 3 + j] = s;
+            }
+        for (int v = 0; v < m.nv; ++v)
+            for (int ij = 0; ij < 9; ++ij) {
+                double s = 0.0;
+                for (int a = 0; a < na; ++a) s += Q.q[v][a] * HK[9 * a + ij];
+                Hb[(v * 4 + w) * 9 + ij] = s;
+            }
+    }
     return st;
 }
 

@@ -30,8 +30,9 @@ FIPC_HD int sym_eig_ld(int n, double* a, double* d) {
             if (scale == 0.0) {
                 e[i] = A_(i, l);
             } else {
+                const double iscale = 1.0 / scale;
                 for (int k = 0; k <= l; ++k) {
-                    A_(i, k) /= scale;
+                    A_(i, k) *= iscale;
                     h += A_(i, k) * A_(i, k);
                 }
                 double f = A_(i, l);
@@ -40,12 +41,13 @@ FIPC_HD int sym_eig_ld(int n, double* a, double* d) {
                 h -= f * g;
                 A_(i, l) = f - g;
                 f = 0.0;
+                const double ih = 1.0 / h;
                 for (int j = 0; j <= l; ++j) {
-                    A_(j, i) = A_(i, j) / h;
+                    A_(j, i) = A_(i, j) * ih;
                     g = 0.0;
                     for (int k = 0; k <= j; ++k) g += A_(j, k) * A_(i, k);
                     for (int k = j + 1; k <= l; ++k) g += A_(k, j) * A_(i, k);
-                    e[j] = g / h;
+                    e[j] = g * ih;
                     f += e[j] * A_(i, j);
                 }
                 const double hh = f / (h + h);
@@ -103,8 +105,9 @@ FIPC_HD int sym_eig_ld(int n, double* a, double* d) {
                         e[m] = 0.0;
                         break;
                     }
-                    s = f / r;
-                    c = g / r;
+                    const double ir = 1.0 / r;
+                    s = f * ir;
+                    c = g * ir;
                     g = d[i + 1] - p;
                     r = (d[i] - g) * s + 2.0 * c * b;
                     p = s * r;

@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(128) k_elasticity(int nT, const int4* __restri
 // for b in [block0[t], block0[t+1])): a type's rows are a few hundred warps, less than the chip holds, and
 // a launch lasts as long as one warp's FP64 instructions, which issue one in 18 clocks of an SM.  The
 // mollified types, the longest, come first.  With the closed forms of barrier.cuh, assembling the system of
-// two cubes in contact (2,000 rows) takes 1.06 ms against 4.08, that of 64 bodies in a pile (32,000 rows)
-// 2.5 against 8.5 (the element and run sums included).
+// two cubes in contact (2,000 rows) takes 0.72 ms against 4.08, that of 180 cubes in a pile (32,000 rows)
+// 1.9 against 8.5 (the element and run sums included).
 constexpr int ROW_THREADS = 64;
 struct RowBlocks {
     int block0[N_TYPES + 1], n[N_TYPES], first[N_TYPES], type[N_TYPES];   // in launch order

@@ -127,7 +127,7 @@ __global__ void k_contact_keys(int n_rows, const int4* __restrict__ rows, TypeTa
 // of up to RUN_LONG blocks (nearly all; the summands are the rows two vertices share) are summed in list
 // order.  The vertices of a large face, a ground plane above all, share a run with every row on it: such
 // a run is left to the whole CTA, 32 interleaved parts summed in list order and then in a fixed order.
-// One thread per run took 1.6 ms on a pile of 64 bodies on a ground plane: the longest run's loads, one after
+// One thread per run took 1.6 ms on a pile of 180 cubes on a ground box: the longest run's loads, one after
 // the other.
 constexpr int RUN_THREADS = 512, RUN_GROUPS = RUN_THREADS / 16, RUN_LONG = 128;
 __device__ __forceinline__ double run_sum(const int* __restrict__ vals, const double* __restrict__ cH, const double* __restrict__ cg,
