@@ -68,49 +68,55 @@ __global__ void k_scene_row_offsets(int S, const int* __restrict__ voff, RowList
     }
 }
 
-// incremental potential per scene (NEWTON_IPC.py:515-542): one block per scene
+// incremental potential per scene (NEWTON_IPC.py:515-542): `parts` CTAs per scene, their sums into
+// part[scene][parts], added in order by k_scene_sum.  One CTA per scene left 64 scenes on 64 SMs (1.12 ms,
+// bound by one SM's FP64 pipe).
 constexpr int SE_THREADS = 256;
-__global__ void __launch_bounds__(SE_THREADS) k_scene_energy(int S, const int* __restrict__ voff, const int* __restrict__ toff,
+__global__ void __launch_bounds__(SE_THREADS) k_scene_energy(int S, int parts, const int* __restrict__ voff, const int* __restrict__ toff,
                                                              const int* __restrict__ roff, RowLists rl, const double* __restrict__ x,
                                                              const double* __restrict__ xt, const double* __restrict__ m,
                                                              const int4* __restrict__ tets, const double* __restrict__ dminv,
                                                              const double* __restrict__ vol, const double* __restrict__ lam,
                                                              const double* __restrict__ mu, double dt2, const double* __restrict__ x0,
-                                                             double dh2, const double* __restrict__ kap_s, double* __restrict__ out) {
+                                                             double dh2, const double* __restrict__ kap_s, double* __restrict__ part) {
     __shared__ double sh[SE_THREADS];
-    const int s = blockIdx.x;
-    double acc = 0.0;
-    for (int i = voff[s] + threadIdx.x; i < voff[s + 1]; i += SE_THREADS) acc += 0.5 * m[i] * sq(ld3(x, i) - ld3(xt, i));
-    double total = block_sum_t<SE_THREADS>(acc, sh);
-    acc = 0.0;
-    for (int e = toff[s] + threadIdx.x; e < toff[s + 1]; e += SE_THREADS) {
+    const int s = blockIdx.x / parts, first = (int)(blockIdx.x % parts) * SE_THREADS + threadIdx.x, step = parts * SE_THREADS;
+    double in = 0.0, el = 0.0, ba = 0.0;
+    for (int i = voff[s] + first; i < voff[s + 1]; i += step) in += 0.5 * m[i] * sq(ld3(x, i) - ld3(xt, i));
+    for (int e = toff[s] + first; e < toff[s + 1]; e += step) {
         const int4 t = tets[e];
         const v3 X[4] = {ld3(x, t.x), ld3(x, t.y), ld3(x, t.z), ld3(x, t.w)};
         double IB[9], F[9];
+#pragma unroll
         for (int i = 0; i < 9; ++i) IB[i] = dminv[9 * (size_t)e + i];
         deformation_gradient(X, IB, F);
-        acc += nh_psi_F(F, lam[e], mu[e]) * dt2 * vol[e];
+        el += nh_psi_F(F, lam[e], mu[e]) * dt2 * vol[e];
     }
-    total += block_sum_t<SE_THREADS>(acc, sh);
     const double kappa = kap_s[s];
     for (int type = 0; type < N_TYPES; ++type) {
         const int r0 = roff[type * (S + 1) + s], r1 = roff[type * (S + 1) + s + 1];
-        if (r0 >= r1) continue;
         const int nv = type_nverts(type);
-        acc = 0.0;
-        for (int r = r0 + threadIdx.x; r < r1; r += SE_THREADS) {
+        for (int r = r0 + first; r < r1; r += step) {
             const int4 q = rl.rows[type][r];
             const int id[4] = {q.x, q.y, nv > 2 ? q.z : q.x, nv > 3 ? q.w : q.x};
             v3 X[4], X0[4];
+#pragma unroll
             for (int k = 0; k < 4; ++k) {
                 X[k] = ld3(x, id[k]);
                 X0[k] = type >= T_EEM ? ld3(x0, id[k]) : mk(0, 0, 0);
             }
-            acc += barrier_energy(type, X, X0, dh2, kappa);
+            ba += barrier_energy(type, X, X0, dh2, kappa);
         }
-        total += block_sum_t<SE_THREADS>(acc, sh);
     }
-    if (threadIdx.x == 0) out[s] = total;
+    const double total = block_sum_t<SE_THREADS>(in + el + ba, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = total;
+}
+__global__ void k_scene_sum(int S, int parts, const double* __restrict__ part, double* __restrict__ out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= S) return;
+    double t = 0.0;
+    for (int k = 0; k < parts; ++k) t += part[(size_t)s * parts + k];
+    out[s] = t;
 }
 
 // max |p| per scene (NEWTON_IPC.py:805-812)
@@ -782,12 +788,16 @@ int fipc_batch_compute_energy(fipc_ctx* c, const double* x, const double* xt, do
     if (!c || c->n_scenes < 2 || !x || !xt || !energy) return FIPC_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     const int S = c->n_scenes;
-    if (c->s_rowoff.ensure(4ll * N_TYPES * (S + 1))) return FIPC_ERR_CUDA;
+    const int parts = std::max(1, std::min(16, 4 * 152 / S));   // CTAs for four per SM
+    if (c->s_rowoff.ensure(4ll * N_TYPES * (S + 1)) || c->s_red.ensure(8ll * S * parts)) return FIPC_ERR_CUDA;
     const RowLists rl = row_lists(c);
     k_scene_row_offsets<<<nblk(S + 1, 128), 128, 0, s>>>(S, c->voff_d, rl, c->s_rowoff.as<int>());
     FIPC_LAUNCHED();
-    k_scene_energy<<<S, SE_THREADS, 0, s>>>(S, c->voff_d, c->toff_d, c->s_rowoff.as<int>(), rl, x, xt, c->mass, (const int4*)c->tets,
-                                            c->dminv, c->vol, c->lam, c->mu, c->dt * c->dt, c->x0, c->dhat2, c->s_kappa, energy);
+    k_scene_energy<<<S * parts, SE_THREADS, 0, s>>>(S, parts, c->voff_d, c->toff_d, c->s_rowoff.as<int>(), rl, x, xt, c->mass, (const int4*)c->tets,
+                                                    c->dminv, c->vol, c->lam, c->mu, c->dt * c->dt, c->x0, c->dhat2, c->s_kappa,
+                                                    c->s_red.as<double>());
+    FIPC_LAUNCHED();
+    k_scene_sum<<<nblk(S, 64), 64, 0, s>>>(S, parts, c->s_red.as<double>(), energy);
     FIPC_LAUNCHED();
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
