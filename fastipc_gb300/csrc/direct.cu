@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(UPD_THREADS) k_mf_update(MfDev d, PanelArgs p)
 
 // ---------------------------------------------------------------- substitution
 // By the panels of the factorisation: one CTA per front walking its columns one after the other, each a
-// load from memory and a barrier, took 11.5 (forward) and 13.2 ms (backward) on a pile of 8,000
-// vertices, nine heights and 61 panels.
+// load from memory and a barrier, took 11.5 (forward) and 13.2 ms (backward) on a pile of 27 cubes (9,300
+// vertices), nine heights and 61 panels.
 //
 // forward, per height: w = gathered right-hand side + children's updates (all rows)
 __global__ void __launch_bounds__(MF_THREADS) k_mf_forward_gather(MfDev d, int h0, const double* __restrict__ rhs) {

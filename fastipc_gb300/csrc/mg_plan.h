@@ -45,7 +45,17 @@ struct MgLevelPlan {
     MgPattern C;                     // contact pattern (rebuilt by mg_contact)
 };
 
+// working arrays of galerkin_pattern, kept with the plan
+struct MgScratch {
+    struct Entry {
+        int src, row, col;
+    };
+    std::vector<Entry> e, by_col;
+    std::vector<int> row0, col0, at;
+};
+
 struct MgPlan {
+    MgScratch scratch;
     int levels = 0;                  // number of levels (>= 2 when the hierarchy is in use)
     std::vector<MgLevelPlan> L;
 };
@@ -53,42 +63,64 @@ struct MgPlan {
 namespace mg_detail {
 
 // pattern of the aggregated level and its contribution lists from a finer pattern (rp, ci)
-// (fixed, may be null: fine rows and columns to leave out)
+// (fixed, may be null: fine rows and columns to leave out), ordered by coarse row, coarse column and
+// source position.  Two stable counting sorts (columns, then rows; the sources ascend as they are met): the
+// contact pattern is rebuilt every Newton iteration on the host while the GPU waits, and a comparison sort
+// of its 280,000 blocks took most of the 16 ms that this set-up costs on a pile of 180 cubes.
 inline void galerkin_pattern(int n_fine, const int* rp, const int* ci, const std::vector<int>& agg_of, int n_coarse, MgPattern& out,
-                             const unsigned char* fixed = nullptr) {
-    struct E {
-        long long key;
-        int src, r, c;
-    };
-    std::vector<E> e;
-    e.reserve(rp ? (size_t)rp[n_fine] : 0);
+                             MgScratch& w, const unsigned char* fixed = nullptr) {
+    std::vector<int>&row0 = w.row0, &col0 = w.col0;   // entries per coarse row, column, then their starts
+    row0.assign(n_coarse + 1, 0);
+    col0.assign(n_coarse + 1, 0);
+    if (rp && w.e.size() < (size_t)rp[n_fine]) {
+        w.e.resize(rp[n_fine]);
+        w.by_col.resize(rp[n_fine]);
+    }
+    size_t n = 0;
     if (rp)
-        for (int i = 0; i < n_fine; ++i)
+        for (int i = 0; i < n_fine; ++i) {
+            if (fixed && fixed[i]) continue;
+            const size_t n0 = n;
             for (int k = rp[i]; k < rp[i + 1]; ++k) {
                 const int j = ci[k];
-                if (fixed && (fixed[i] || fixed[j])) continue;
-                e.push_back({(long long)agg_of[i] * n_coarse + agg_of[j], k, i, j});
+                if (fixed && fixed[j]) continue;
+                w.e[n++] = {k, i, j};
+                ++col0[agg_of[j] + 1];
             }
-    std::sort(e.begin(), e.end(), [](const E& a, const E& b) { return a.key < b.key || (a.key == b.key && a.src < b.src); });
+            row0[agg_of[i] + 1] += (int)(n - n0);
+        }
+    for (int q = 0; q < n_coarse; ++q) {
+        row0[q + 1] += row0[q];
+        col0[q + 1] += col0[q];
+    }
+    w.at.assign(col0.begin(), col0.end() - 1);
+    for (size_t q = 0; q < n; ++q) w.by_col[w.at[agg_of[w.e[q].col]]++] = w.e[q];
+    out.src.resize(n);
+    out.src_row.resize(n);
+    out.src_col.resize(n);
+    w.at.assign(row0.begin(), row0.end() - 1);
+    for (size_t q = 0; q < n; ++q) {
+        const MgScratch::Entry& e = w.by_col[q];
+        const int o = w.at[agg_of[e.row]]++;
+        out.src[o] = e.src;
+        out.src_row[o] = e.row;
+        out.src_col[o] = e.col;
+    }
     out.rp.assign(n_coarse + 1, 0);
     out.ci.clear();
     out.con_ptr.assign(1, 0);
-    out.src.resize(e.size());
-    out.src_row.resize(e.size());
-    out.src_col.resize(e.size());
-    for (size_t q = 0; q < e.size(); ++q) {
-        if (q == 0 || e[q].key != e[q - 1].key) {
-            const int I = (int)(e[q].key / n_coarse), J = (int)(e[q].key % n_coarse);
+    for (int I = 0; I < n_coarse; ++I) {
+        int last = -1;
+        for (int q = row0[I]; q < row0[I + 1]; ++q) {
+            const int J = agg_of[out.src_col[q]];
+            if (J == last) continue;
+            if (q) out.con_ptr.push_back(q);
             out.ci.push_back(J);
-            ++out.rp[I + 1];
-            if (q) out.con_ptr.push_back((int)q);
+            last = J;
         }
-        out.src[q] = e[q].src;
-        out.src_row[q] = e[q].r;
-        out.src_col[q] = e[q].c;
+        out.rp[I + 1] = (int)out.ci.size();
     }
-    if (!e.empty()) out.con_ptr.push_back((int)e.size());
-    for (int I = 0; I < n_coarse; ++I) out.rp[I + 1] += out.rp[I];
+    if (n) out.con_ptr.push_back((int)n);
 }
 
 }  // namespace mg_detail
@@ -163,7 +195,7 @@ inline void mg_build(int nV, const double* x0, const int* rp, const int* ci, dou
             std::vector<int> fill(c.mem_ptr.begin(), c.mem_ptr.end() - 1);
             for (int i = 0; i < n; ++i) c.mem[fill[c.agg_of[i]]++] = i;
         }
-        mg_detail::galerkin_pattern(n, f.S.rp.data(), f.S.ci.data(), c.agg_of, na, c.S);
+        mg_detail::galerkin_pattern(n, f.S.rp.data(), f.S.ci.data(), c.agg_of, na, c.S, P.scratch);
         std::vector<double> cp(3 * (size_t)na, 0.0);
         std::vector<int> cc(na, 0);
         for (int a = 0; a < na; ++a) {
@@ -215,18 +247,18 @@ inline void mg_build(int nV, const double* x0, const int* rp, const int* ci, dou
 // vertices (fixed, may be null) contribute nothing to a coarse matrix and are left out: a ground
 // body's few nodes would otherwise couple, through zero blocks, with every node that rests on it.
 inline void mg_contact(MgPlan& P, int nV, const int* crp, const int* cci, const unsigned char* fixed = nullptr) {
-    MgLevelPlan& l0 = P.L[0];
-    l0.C = MgPattern();
+    MgPattern& c0 = P.L[0].C;
     if (crp && crp[nV] > 0) {
-        l0.C.rp.assign(crp, crp + nV + 1);
-        l0.C.ci.assign(cci, cci + crp[nV]);
+        c0.rp.assign(crp, crp + nV + 1);
+        c0.ci.assign(cci, cci + crp[nV]);
+    } else {
+        c0 = MgPattern();
     }
     for (int l = 1; l < P.levels; ++l) {
         const MgLevelPlan& f = P.L[l - 1];
         MgLevelPlan& c = P.L[l];
-        c.C = MgPattern();
-        if (f.C.nnz() == 0) continue;
-        mg_detail::galerkin_pattern(f.n, f.C.rp.data(), f.C.ci.data(), c.agg_of, c.n, c.C, l == 1 ? fixed : nullptr);
+        if (f.C.nnz() == 0) c.C = MgPattern();
+        else mg_detail::galerkin_pattern(f.n, f.C.rp.data(), f.C.ci.data(), c.agg_of, c.n, c.C, P.scratch, l == 1 ? fixed : nullptr);
     }
 }
 
