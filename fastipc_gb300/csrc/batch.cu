@@ -454,17 +454,14 @@ static void launch_spmv(const BPCG& a, int grid, cudaStream_t s) {
 }
 static void dispatch_start(int tr, const BPCG& a, int grid, const double* rhs, cudaStream_t s) {
     if (tr == 64) launch_start<64>(a, grid, rhs, s);
-    else if (tr == 256) launch_start<256>(a, grid, rhs, s);
     else launch_start<128>(a, grid, rhs, s);
 }
 static void dispatch_iter(int tr, const BPCG& a, int grid, cudaStream_t s) {
     if (tr == 64) launch_iter<64>(a, grid, s);
-    else if (tr == 256) launch_iter<256>(a, grid, s);
     else launch_iter<128>(a, grid, s);
 }
 static void dispatch_spmv(int tr, const BPCG& a, int grid, cudaStream_t s) {
     if (tr == 64) launch_spmv<64>(a, grid, s);
-    else if (tr == 256) launch_spmv<256>(a, grid, s);
     else launch_spmv<128>(a, grid, s);
 }
 
@@ -478,8 +475,11 @@ static void fill_tables(const fipc_ctx* c, BPCG& a) {
 
 // persistent grid of the batched PCG, chosen by timing the SpMV on the live system: every
 // candidate runs its SpMV without reductions, best of three launches.  The tile (rows per tile =
-// threads per block) stays at 128 rows: it sets the order of the per-scene sums, so choosing it by
-// timing would make the directions depend on the timing; the grid does not change any sum.
+// threads per block) is not timed: it sets the order of the per-scene sums, so choosing it by
+// timing would make the directions depend on the timing; the grid does not change any sum.  It has 64
+// rows while the tiles of 128 would all be resident at once (ten per SM): an SM's share of so few is uneven
+// (16 scenes 65.5 -> 61.7 ms a solve, 64 scenes 145.0 -> 141.7), and 128 beyond (256 scenes 419 ms against
+// 426: half as many partial sums).
 static int autotune(fipc_ctx* c, BPCG a, cudaStream_t s) {
     int dev = 0, nsm = 152;
     cudaGetDevice(&dev);
@@ -487,44 +487,41 @@ static int autotune(fipc_ctx* c, BPCG a, cudaStream_t s) {
     cudaEvent_t e0, e1;
     FIPC_CUDA(cudaEventCreate(&e0));
     FIPC_CUDA(cudaEventCreate(&e1));
-    const int trs[1] = {128};
+    int tiles = 0;
+    for (int q = 0; q < c->n_scenes; ++q) tiles += (c->h_voff[q + 1] - c->h_voff[q] + 127) / 128;
+    const int tr = tiles <= 10 * nsm ? 64 : 128;
     const int mult[5] = {2, 4, 8, 16, 0};   // 0: one block per tile
     float best = 1e30f;
-    int best_tr = 128, best_grid = 0;
+    int best_grid = 0;
     a.dry = 1;
-    for (int tr : trs) {
-        int st = build_tiles(c, tr, s);
-        if (st) return st;
-        fill_tables(c, a);
-        for (int m : mult) {
-            int grid = m ? m * nsm : c->n_tiles;
-            if (grid > c->n_tiles) grid = c->n_tiles;
-            if (grid < 1) grid = 1;
-            dispatch_spmv(tr, a, grid, s);   // warm-up
+    int st = build_tiles(c, tr, s);
+    if (st) return st;
+    fill_tables(c, a);
+    for (int m : mult) {
+        int grid = m ? m * nsm : c->n_tiles;
+        if (grid > c->n_tiles) grid = c->n_tiles;
+        if (grid < 1) grid = 1;
+        dispatch_spmv(tr, a, grid, s);   // warm-up
+        FIPC_LAUNCHED();
+        float tmin = 1e30f;
+        for (int rep = 0; rep < 3; ++rep) {
+            FIPC_CUDA(cudaEventRecord(e0, s));
+            dispatch_spmv(tr, a, grid, s);
             FIPC_LAUNCHED();
-            float tmin = 1e30f;
-            for (int rep = 0; rep < 3; ++rep) {
-                FIPC_CUDA(cudaEventRecord(e0, s));
-                dispatch_spmv(tr, a, grid, s);
-                FIPC_LAUNCHED();
-                FIPC_CUDA(cudaEventRecord(e1, s));
-                FIPC_CUDA(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                FIPC_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                tmin = ms < tmin ? ms : tmin;
-            }
-            if (tmin < best) {
-                best = tmin;
-                best_tr = tr;
-                best_grid = m ? m * nsm : 0;
-            }
+            FIPC_CUDA(cudaEventRecord(e1, s));
+            FIPC_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.f;
+            FIPC_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            tmin = ms < tmin ? ms : tmin;
+        }
+        if (tmin < best) {
+            best = tmin;
+            best_grid = m ? m * nsm : 0;
         }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     FIPC_CUDA(cudaGetLastError());
-    int st = build_tiles(c, best_tr, s);
-    if (st) return st;
     c->pcg_grid = best_grid ? (best_grid < c->n_tiles ? best_grid : c->n_tiles) : c->n_tiles;
     c->tune_ms = best;
     return FIPC_OK;
