@@ -706,24 +706,17 @@ FIPC_HD double barrier_energy(int type, const v3* X, const v3* X0, double dh2, d
     return type >= T_EEM ? b * mollifier(D, X0).val : b;
 }
 
-// Energy (E), gradient (g, 12 = 3*nv used) and projected Hessian in 3x3 vertex blocks
-// (Hb[(v*4+w)*9 + i*3+j] for v,w < nv) of one constraint row.  X: the row's vertices
-// (nv used), X0: rest positions of the four EE-type vertices (mollified types only).
-// want: 0 energy only, 1 energy + gradient + projected Hessian, 2 energy + gradient + the
-// Hessian without the projection.  Returns the eigen-solver status.
-FIPC_HD int barrier_row(int type, const v3* X, const v3* X0, double dh2, double kappa, int want,
-                        double* E, double* g, double* Hb) {
-    if (!want) {
-        *E = barrier_energy(type, X, X0, dh2, kappa);
-        return 0;
-    }
-    if (want == 1 && type <= T_EE) {
-        if (type == T_PP) barrier_row_pp(X, dh2, kappa, E, g, Hb);
-        else if (type == T_PE) barrier_row_pe(X, dh2, kappa, E, g, Hb);
-        else if (type == T_PT) barrier_row_plane<false>(X, dh2, kappa, E, g, Hb);
-        else barrier_row_plane<true>(X, dh2, kappa, E, g, Hb);
-        return 0;
-    }
+// Unmollified rows with their projected Hessian, for kappa > 0: the closed forms know the signs of the
+// barrier's derivatives
+FIPC_HD void barrier_row_closed(int type, const v3* X, double dh2, double kappa, double* E, double* g, double* Hb) {
+    if (type == T_PP) barrier_row_pp(X, dh2, kappa, E, g, Hb);
+    else if (type == T_PE) barrier_row_pe(X, dh2, kappa, E, g, Hb);
+    else if (type == T_PT) barrier_row_plane<false>(X, dh2, kappa, E, g, Hb);
+    else barrier_row_plane<true>(X, dh2, kappa, E, g, Hb);
+}
+
+// A row in reduced coordinates: any type and kappa, want = 1 or 2 (see barrier_row)
+FIPC_HD int barrier_row_reduced(int type, const v3* X, const v3* X0, double dh2, double kappa, int want, double* E, double* g, double* Hb) {
     const RowMap m = row_map(type);
     v3 y[3];
     for (int k = 0; k < m.ny; ++k) {
@@ -812,6 +805,35 @@ FIPC_HD int barrier_row(int type, const v3* X, const v3* X0, double dh2, double 
             }
     }
     return st;
+}
+
+// the same out of line, for the rare callers
+#if defined(__CUDACC__)
+__host__ __device__ __noinline__ static
+#else
+static inline
+#endif
+int barrier_row_rare(int type, const v3* X, const v3* X0, double dh2, double kappa, int want, double* E, double* g, double* Hb) {
+    return barrier_row_reduced(type, X, X0, dh2, kappa, want, E, g, Hb);
+}
+
+// Energy (E), gradient (g, 12 = 3*nv used) and projected Hessian in 3x3 vertex blocks
+// (Hb[(v*4+w)*9 + i*3+j] for v,w < nv) of one constraint row.  X: the row's vertices
+// (nv used), X0: rest positions of the four EE-type vertices (mollified types only).
+// want: 0 energy only, 1 energy + gradient + projected Hessian, 2 energy + gradient + the
+// Hessian without the projection.  Returns the eigen-solver status.
+FIPC_HD int barrier_row(int type, const v3* X, const v3* X0, double dh2, double kappa, int want,
+                        double* E, double* g, double* Hb) {
+    if (!want) {
+        *E = barrier_energy(type, X, X0, dh2, kappa);
+        return 0;
+    }
+    if (want == 1 && type <= T_EE) {
+        if (!(kappa > 0.0)) return barrier_row_rare(type, X, X0, dh2, kappa, want, E, g, Hb);
+        barrier_row_closed(type, X, dh2, kappa, E, g, Hb);
+        return 0;
+    }
+    return barrier_row_reduced(type, X, X0, dh2, kappa, want, E, g, Hb);
 }
 
 }  // namespace fipc

@@ -984,7 +984,9 @@ __device__ __forceinline__ int list_of(RowKey k) { return (int)(k.hi >> 42); }
 
 // Up to SORT_SMALL rows: sorted, made unique and written out by one CTA (bitonic in shared memory)
 // right behind the queries, so that a call of a small scene needs one round trip to the host.  More
-// rows go through a merge sort after that round trip (k_rows_write).
+// rows go through a merge sort after that round trip (k_rows_write).  Near the line, two cubes with up to 1,900
+// rows: 162 us a call against 173 through the merge sort; the CTA's stages double in number from 2,048 rows to
+// 4,096, whose keys no longer fit the static shared memory.
 constexpr int SORT_SMALL = 2048, SORT_THREADS = 1024;
 __global__ void __launch_bounds__(SORT_THREADS) k_rows_small(const RowKey* __restrict__ in, BroadCounters* __restrict__ n, int4* __restrict__ out) {
     __shared__ RowKey k[SORT_SMALL];

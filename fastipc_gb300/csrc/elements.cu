@@ -89,7 +89,8 @@ __device__ __forceinline__ void barrier_row_of(const int4 q, const double* __res
         X0[k] = TYPE >= T_EEM ? ld3(x0, id[k]) : mk(0, 0, 0);
     }
     double e;
-    if (g) barrier_row(TYPE, X, X0, dh2, kappa, 1, &e, g, Hb);
+    if (g && TYPE <= T_EE) barrier_row_closed(TYPE, X, dh2, kappa, &e, g, Hb);
+    else if (g) barrier_row_reduced(TYPE, X, X0, dh2, kappa, 1, &e, g, Hb);
     else e = barrier_energy(TYPE, X, X0, dh2, kappa);
     if (E) *E = e;
 }
@@ -116,6 +117,35 @@ __global__ void __launch_bounds__(ROW_THREADS) k_barrier_rows(RowBlocks rb, cons
         case T_PPM: barrier_row_of<T_PPM>(q, x, x0, dh2, kappa, Er, gr, Hr); break;
         default: barrier_row_of<T_PEM>(q, x, x0, dh2, kappa, Er, gr, Hr); break;
     }
+}
+
+// the same for any kappa: every type in reduced coordinates
+__global__ void __launch_bounds__(ROW_THREADS) k_barrier_rows_any(RowBlocks rb, const int4* __restrict__ rows, const double* __restrict__ x,
+                                                              const double* __restrict__ x0, double dh2, double kappa,
+                                                              const double* __restrict__ kap_s, const int* __restrict__ vscene,
+                                                              double* __restrict__ E, double* __restrict__ g, double* __restrict__ Hb) {
+    int k = 0;
+    while (k < N_TYPES - 1 && (int)blockIdx.x >= rb.block0[k + 1]) ++k;
+    const int i = ((int)blockIdx.x - rb.block0[k]) * ROW_THREADS + threadIdx.x;
+    if (i >= rb.n[k]) return;
+    const int r = rb.first[k] + i;
+    const int4 q = rows[r];
+    if (kap_s) kappa = kap_s[vscene[q.x]];   // batched scenes: the row's own scene
+    double* Er = E ? E + r : nullptr;
+    double* gr = g ? g + 12 * (size_t)r : nullptr;
+    double* Hr = g ? Hb + 144 * (size_t)r : nullptr;
+    const int t = rb.type[k], nv = type_nverts(t);
+    const int id[4] = {q.x, q.y, nv > 2 ? q.z : q.x, nv > 3 ? q.w : q.x};
+    v3 X[4], X0[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        X[v] = ld3(x, id[v]);
+        X0[v] = t >= T_EEM ? ld3(x0, id[v]) : mk(0, 0, 0);
+    }
+    double e;
+    if (gr) barrier_row_reduced(t, X, X0, dh2, kappa, 1, &e, gr, Hr);
+    else e = barrier_energy(t, X, X0, dh2, kappa);
+    if (Er) *Er = e;
 }
 
 // ---------------------------------------------------------------- deterministic reductions
@@ -327,9 +357,10 @@ int launch_elasticity(int nT, const int* tets, const double* x, const double* dm
     return FIPC_OK;
 }
 
-// the rows of all types (type t: counts[t] rows from row first[t] of `rows`; outputs by row number)
+// the rows of all types (type t: counts[t] rows from row first[t] of `rows`; outputs by row number);
+// positive: every kappa is, as the closed forms need
 int launch_barrier_rows(const int* counts, const int* first, const int* rows, const double* x, const double* x0, double dh2, double kappa,
-                        const double* kap_s, const int* vscene, double* E, double* g, double* Hb, cudaStream_t s) {
+                        const double* kap_s, const int* vscene, double* E, double* g, double* Hb, bool positive, cudaStream_t s) {
     static const int order[N_TYPES] = {T_EEM, T_PEM, T_PPM, T_EE, T_PT, T_PE, T_PP};
     RowBlocks rb;
     int nb = 0;
@@ -343,7 +374,8 @@ int launch_barrier_rows(const int* counts, const int* first, const int* rows, co
     }
     rb.block0[N_TYPES] = nb;
     if (nb == 0) return FIPC_OK;
-    k_barrier_rows<<<nb, ROW_THREADS, 0, s>>>(rb, (const int4*)rows, x, x0, dh2, kappa, kap_s, vscene, E, g, Hb);
+    auto kernel = positive ? k_barrier_rows : k_barrier_rows_any;
+    kernel<<<nb, ROW_THREADS, 0, s>>>(rb, (const int4*)rows, x, x0, dh2, kappa, kap_s, vscene, E, g, Hb);
     FIPC_LAUNCHED();
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
@@ -396,7 +428,7 @@ int fipc_barrier_rows(int type, int n_rows, const int* rows, const double* x, co
     int counts[N_TYPES] = {0};
     const int first[N_TYPES] = {0};
     counts[type] = n_rows;
-    return launch_barrier_rows(counts, first, rows, x, x0, dhat2, kappa, nullptr, nullptr, E, g, H, (cudaStream_t)stream);
+    return launch_barrier_rows(counts, first, rows, x, x0, dhat2, kappa, nullptr, nullptr, E, g, H, kappa > 0.0, (cudaStream_t)stream);
 }
 
 int fipc_ccd_pairs(int kind, int n, const double* xq, const double* pq, double eta, double* toc, void* stream) {

@@ -406,7 +406,7 @@ static int cub_call(fipc_ctx* c, F&& f) {
 int launch_elasticity(int nT, const int* tets, const double* x, const double* dminv, const double* vol, const double* lam,
                       const double* mu, double dt, double* E, double* g, double* Hu, cudaStream_t s, bool tiled);
 int launch_barrier_rows(const int* counts, const int* first, const int* rows, const double* x, const double* x0, double dh2, double kappa,
-                        const double* kap_s, const int* vscene, double* E, double* g, double* Hb, cudaStream_t s);
+                        const double* kap_s, const int* vscene, double* E, double* g, double* Hb, bool positive, cudaStream_t s);
 
 int cs_offsets(fipc_ctx* c, const double* x, cudaStream_t s);
 int cs_prepare(fipc_ctx* c, const unsigned char* fixed, PCGArgs& a, cudaStream_t s);
@@ -452,8 +452,12 @@ int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t
     st = contact_prepare(c, &tt, &nrows, &nent, s);
     if (st || nrows == 0) return st;
     // the rows' barrier gradients / projected Hessians
+    bool positive = c->n_scenes > 1 || c->kappa > 0.0;
+    if (c->n_scenes > 1)
+        for (double k : c->h_kappa) positive = positive && k > 0.0;
     st = launch_barrier_rows(c->h_counts, tt.row0, c->rows_all.as<int>(), x, c->x0, c->dhat2, c->kappa,
-                             c->n_scenes > 1 ? c->s_kappa : nullptr, c->v_scene, nullptr, c->c_g.as<double>(), c->c_H.as<double>(), s);
+                             c->n_scenes > 1 ? c->s_kappa : nullptr, c->v_scene, nullptr, c->c_g.as<double>(), c->c_H.as<double>(),
+                             positive, s);
     if (st) return st;
     return contact_reduce(c, tt, nrows, nent, s);
 }

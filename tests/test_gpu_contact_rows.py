@@ -65,6 +65,19 @@ def test_graded_rows(t, N, gap):
 
 
 @pytest.mark.parametrize('t', range(4))
+def test_negative_stiffness(t):
+    """The closed forms' signs are a positive kappa's; others take the general projection."""
+    N = 70
+    X = _rows(t, N, 0.1, np.random.default_rng(t))
+    E, g, H = barrier_gpu(t, X, X, 0.04, -1e4)
+    rows = (np.arange(N)[:, None] * 4 + np.arange(O.TYPE_NV[t])[None, :]).astype(np.int32)
+    Eo, go, Ho = O.barrier_rows(t, rows, X.reshape(-1, 3), X.reshape(-1, 3), 0.04, -1e4)
+    np.testing.assert_allclose(E, Eo, rtol=1e-11)
+    assert _rel(g, go) < 1e-11
+    assert _rel(H, Ho) < 1e-11
+
+
+@pytest.mark.parametrize('t', range(4))
 def test_rows_outside_the_barrier_are_zero(t):
     E, g, H = barrier_gpu(t, _rows(t, 5, 0.1, np.random.default_rng(t)), np.zeros((5, 4, 3)), 1e-4, 1e4)
     assert not E.any() and not g.any() and not H.any()
