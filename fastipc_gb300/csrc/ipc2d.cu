@@ -22,6 +22,7 @@
 #include "barrier.cuh"
 #include "ctx.cuh"
 #include "fc2d.cuh"
+#include "slot_order.h"
 
 namespace fipc {
 
@@ -483,8 +484,8 @@ __global__ void __launch_bounds__(T2) k2_pcg_dir(PCG2 a) {
 //  * an exchange is one step, not a grid barrier followed by a read of partial sums: every CTA stores its
 //    partial sums to its slot, and one warp of every CTA polls all slots until they are there and adds
 //    them in CTA order (so all CTAs hold the same scalars and take the same branch).  Slots start as
-//    NO_VALUE and rotate over three buffers: a CTA that has read exchange e knows that every CTA is
-//    past e - 1, and clears its slot of that one for e + 2.  A poll gives up after POLL_LIMIT reads.
+//    NO_VALUE, rotate over four buffers and are cleared for reuse (slot_order.h: the order of stores, polls and
+//    fences).  A poll gives up after POLL_LIMIT reads.
 // 4,600 rows, 145 CTAs: 18 us per iteration with three grid barriers -> 11.  What is left is latency: a
 // dependent FP64 operation takes 50 ns, and the reductions, the two round trips through L2 and the scalars of
 // an iteration are some 100 of them one after the other; 580 rows take 9 us, 9,250 take 14.
@@ -497,7 +498,7 @@ struct Coop2 {
     double rtol;
     int rows;                    // rows per CTA (threads / 2)
     double2* zp;                 // [nV][2]: (z, p) of a row
-    unsigned long long* slot;    // [3][gridDim.x][2]
+    unsigned long long* slot;    // [SLOT_BUFFERS][gridDim.x][2]
 };
 
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
@@ -506,42 +507,27 @@ __device__ __forceinline__ ulonglong2 slot_read(const unsigned long long* p) {
     asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
     return v;
 }
-// f(sums over all CTAs of the rows' v0, and v1 if TWO) in one thread, seen by all.  Returns false in every thread when a poll gave up.  FENCE: stores before the exchange are visible to
-// all CTAs after it.
-template <bool TWO, bool FENCE, class F>
-__device__ __forceinline__ bool exchange(const Coop2& c, int epoch, double v0, double v1, F f) {
-    __shared__ double part[2][16];
-    __shared__ int ok;
-    constexpr int AT_ONCE = 5;   // slots per lane and poll: one round trip for 160 CTAs
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, G = gridDim.x;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-        if (TWO) v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+// the polling warp's side of an exchange (slot_order.h): lanes 0 and 1 post the CTA's two sums and clear its slots;
+// every lane polls the slots lane, lane + 32, ... and adds them in CTA order
+template <bool TWO>
+struct WarpSlots {
+    const Coop2& c;
+    unsigned long long bits;     // lanes 0, 1: the sum to post
+    double a0, a1;               // the lane's share of the totals
+    static constexpr int AT_ONCE = 5;   // slots per lane and poll: one round trip for 160 CTAs
+    __device__ __forceinline__ unsigned long long* at(int buffer, int cta) const { return c.slot + ((size_t)buffer * gridDim.x + cta) * 2; }
+    __device__ __forceinline__ void fence() const { fence_gpu(); }
+    __device__ __forceinline__ void post(int buffer) const {
+        const int lane = threadIdx.x & 31;
+        if (lane < 2) *(volatile unsigned long long*)(at(buffer, blockIdx.x) + lane) = bits;
     }
-    if (lane == 0) {
-        part[0][w] = v0;
-        part[1][w] = v1;
+    __device__ __forceinline__ void clear(int buffer) const {
+        const int lane = threadIdx.x & 31;
+        if (lane < 2) *(volatile unsigned long long*)(at(buffer, blockIdx.x) + lane) = NO_VALUE;
     }
-    __syncthreads();
-    if (w == 0) {
-        unsigned long long* buf = c.slot + (size_t)(epoch % 3) * 2 * G;
-        if (lane < 2) {
-            double t = 0.0;
-            if (TWO || lane == 0) {
-                double h[4] = {0.0, 0.0, 0.0, 0.0};
-                for (int k = 0; k < nw; k += 4)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (k + q < nw) h[q] += part[lane][k + q];
-                t = (h[0] + h[1]) + (h[2] + h[3]);
-            }
-            unsigned long long b = (unsigned long long)__double_as_longlong(t);
-            if (b == NO_VALUE) b = 0x7ff8000000000000ull;
-            if (FENCE) fence_gpu();   // the CTA's rows, stored before the barrier above, come first
-            *(volatile unsigned long long*)(buf + 2 * blockIdx.x + lane) = b;
-        }
-        double a0 = 0.0, a1 = 0.0;
+    __device__ __forceinline__ bool poll(int buffer) {
+        const int lane = threadIdx.x & 31, G = gridDim.x;
+        a0 = a1 = 0.0;
         int n = 0;
         for (int k0 = lane; k0 < G; k0 += 32 * AT_ONCE) {
             ulonglong2 b[AT_ONCE];
@@ -551,7 +537,7 @@ __device__ __forceinline__ bool exchange(const Coop2& c, int epoch, double v0, d
 #pragma unroll
                 for (int u = 0; u < AT_ONCE; ++u) {
                     b[u] = make_ulonglong2(0, 0);
-                    if (k0 + 32 * u < G) b[u] = slot_read(buf + 2 * (k0 + 32 * u));
+                    if (k0 + 32 * u < G) b[u] = slot_read(at(buffer, k0 + 32 * u));
                 }
 #pragma unroll
                 for (int u = 0; u < AT_ONCE; ++u) missing = missing || b[u].x == NO_VALUE || b[u].y == NO_VALUE;
@@ -564,18 +550,53 @@ __device__ __forceinline__ bool exchange(const Coop2& c, int epoch, double v0, d
             a0 += five(b[0].x, b[1].x, b[2].x, b[3].x, b[4].x);
             if (TWO) a1 += five(b[0].y, b[1].y, b[2].y, b[3].y, b[4].y);
         }
-        if (FENCE) fence_gpu();
+        return __all_sync(0xffffffffu, n < POLL_LIMIT);
+    }
+};
+// f(sums over all CTAs of the rows' v0, and v1 if TWO) in one thread, seen by all.  Returns false in every thread
+// when a poll gave up.  FENCE: stores before the exchange are visible to all CTAs after it.
+template <bool TWO, bool FENCE, class F>
+__device__ __forceinline__ bool exchange(const Coop2& c, int epoch, double v0, double v1, F f) {
+    __shared__ double part[2][16];
+    __shared__ int ok;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+        if (TWO) v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    if (lane == 0) {
+        part[0][w] = v0;
+        part[1][w] = v1;
+    }
+    __syncthreads();
+    if (w == 0) {
+        WarpSlots<TWO> s{c, 0ull, 0.0, 0.0};
+        if (lane < 2) {
+            double t = 0.0;
+            if (TWO || lane == 0) {
+                double h[4] = {0.0, 0.0, 0.0, 0.0};
+                for (int k = 0; k < nw; k += 4)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (k + q < nw) h[q] += part[lane][k + q];
+                t = (h[0] + h[1]) + (h[2] + h[3]);
+            }
+            s.bits = (unsigned long long)__double_as_longlong(t);
+            if (s.bits == NO_VALUE) s.bits = 0x7ff8000000000000ull;
+        }
+        __syncwarp();
+        const bool all = slot_exchange<FENCE>(s, epoch);
+        double a0 = s.a0, a1 = s.a1;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             a0 += __shfl_xor_sync(0xffffffffu, a0, o);
             if (TWO) a1 += __shfl_xor_sync(0xffffffffu, a1, o);
         }
-        const bool all = __all_sync(0xffffffffu, n < POLL_LIMIT);
         if (lane == 0) {
             f(a0, a1);
             ok = all;
         }
-        if (lane < 2) *(volatile unsigned long long*)(c.slot + (size_t)((epoch + 2) % 3) * 2 * G + 2 * blockIdx.x + lane) = NO_VALUE;
     }
     __syncthreads();
     return ok != 0;
@@ -1337,8 +1358,9 @@ int fipc2d_solve_system(fipc2d_ctx_impl* h, const unsigned char* fixed, double r
     if (maxit > 0 && per_sm <= COOP_ROWS) {
         const int rows = std::max(16, (per_sm + 15) / 16 * 16), threads = 2 * rows, grid = (c->nV + rows - 1) / rows;
         const size_t smem = (size_t)COOP_SLOTS * threads * (sizeof(double2) + sizeof(int));
-        if (c->pslot.ensure(48ull * grid)) return FIPC_ERR_CUDA;
-        FIPC_CUDA(cudaMemsetAsync(c->pslot.p, 0xff, 48ull * grid, s));
+        const size_t slots = 16ull * SLOT_BUFFERS * grid;
+        if (c->pslot.ensure(slots)) return FIPC_ERR_CUDA;
+        FIPC_CUDA(cudaMemsetAsync(c->pslot.p, 0xff, slots, s));
         Coop2 args{a, c->rhs.as<double>(), rtol, rows, (double2*)v, c->pslot.as<unsigned long long>()};
         void* argp[] = {&args};
         const void* f = (const void*)k2_pcg_coop;
