@@ -30,7 +30,7 @@ EXPORTS = [
     'fipc_admm_dual', 'fipc2d_ctx_create', 'fipc2d_ctx_destroy', 'fipc2d_ctx_params', 'fipc2d_ctx_set_kappa', 'fipc2d_ctx_mass',
     'fipc2d_compute_xn_and_xtilde', 'fipc2d_move_nodes', 'fipc2d_apply_sol', 'fipc2d_compute_v', 'fipc2d_elements',
     'fipc2d_barrier_rows', 'fipc2d_ccd_pairs', 'fipc2d_find_constraints', 'fipc2d_get_constraints',
-    'fipc2d_compute_hessian_and_gradient', 'fipc2d_system_nnzb', 'fipc2d_export_system', 'fipc2d_solve_system',
+    'fipc2d_compute_hessian_and_gradient', 'fipc2d_system_nnzb', 'fipc2d_export_system', 'fipc2d_solve_system', 'fipc2d_ctx_set_poll_limit',
     'fipc2d_output_residual', 'fipc2d_compute_energy', 'fipc2d_compute_intersection_free_step_size', 'fipc2d_check_collision',
 ]
 

@@ -76,6 +76,7 @@ struct Ctx2 {
     DBuf val, col, row_ptr, dpos, rhs;      // assembled 2x2-block CSR and right-hand side
     int nnzb = 0;
     DBuf pvec, ppart, pflag, pslot;         // PCG
+    int poll_limit = 1 << 20;               // reads of a slot poll of the one-launch PCG (about a second)
     DBuf epart, eout;
     // PCG_CHUNK iterations captured as a CUDA graph on a private stream, keyed by the kernels'
     // arguments, and replayed on the caller's stream
@@ -485,11 +486,11 @@ __global__ void __launch_bounds__(T2) k2_pcg_dir(PCG2 a) {
 //    partial sums to its slot, and one warp of every CTA polls all slots until they are there and adds
 //    them in CTA order (so all CTAs hold the same scalars and take the same branch).  Slots start as
 //    NO_VALUE, rotate over four buffers and are cleared for reuse (slot_order.h: the order of stores, polls and
-//    fences).  A poll gives up after POLL_LIMIT reads.
+//    fences).  A poll gives up after `limit` reads, the launch then ends and the three kernels above take the solve.
 // 4,600 rows, 145 CTAs: 18 us per iteration with three grid barriers -> 11.  What is left is latency: a
 // dependent FP64 operation takes 50 ns, and the reductions, the two round trips through L2 and the scalars of
 // an iteration are some 100 of them one after the other; 580 rows take 9 us, 9,250 take 14.
-constexpr int COOP_ROWS = 256, COOP_SLOTS = 16, POLL_LIMIT = 1 << 20;
+constexpr int COOP_ROWS = 256, COOP_SLOTS = 16;
 constexpr unsigned long long NO_VALUE = ~0ull;   // not a NaN that arithmetic produces
 
 struct Coop2 {
@@ -499,6 +500,7 @@ struct Coop2 {
     int rows;                    // rows per CTA (threads / 2)
     double2* zp;                 // [nV][2]: (z, p) of a row
     unsigned long long* slot;    // [SLOT_BUFFERS][gridDim.x][2]
+    int limit;                   // reads of a poll before it gives up
 };
 
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
@@ -541,7 +543,7 @@ struct WarpSlots {
                 }
 #pragma unroll
                 for (int u = 0; u < AT_ONCE; ++u) missing = missing || b[u].x == NO_VALUE || b[u].y == NO_VALUE;
-            } while (missing && ++n < POLL_LIMIT);
+            } while (missing && ++n < c.limit);
             auto five = [](unsigned long long p, unsigned long long q, unsigned long long r, unsigned long long s, unsigned long long t) {
                 const double d[AT_ONCE] = {__longlong_as_double((long long)p), __longlong_as_double((long long)q), __longlong_as_double((long long)r),
                                            __longlong_as_double((long long)s), __longlong_as_double((long long)t)};
@@ -550,7 +552,7 @@ struct WarpSlots {
             a0 += five(b[0].x, b[1].x, b[2].x, b[3].x, b[4].x);
             if (TWO) a1 += five(b[0].y, b[1].y, b[2].y, b[3].y, b[4].y);
         }
-        return __all_sync(0xffffffffu, n < POLL_LIMIT);
+        return __all_sync(0xffffffffu, n < c.limit);
     }
 };
 // f(sums over all CTAs of the rows' v0, and v1 if TWO) in one thread, seen by all.  Returns false in every thread
@@ -1361,7 +1363,7 @@ int fipc2d_solve_system(fipc2d_ctx_impl* h, const unsigned char* fixed, double r
         const size_t slots = 16ull * SLOT_BUFFERS * grid;
         if (c->pslot.ensure(slots)) return FIPC_ERR_CUDA;
         FIPC_CUDA(cudaMemsetAsync(c->pslot.p, 0xff, slots, s));
-        Coop2 args{a, c->rhs.as<double>(), rtol, rows, (double2*)v, c->pslot.as<unsigned long long>()};
+        Coop2 args{a, c->rhs.as<double>(), rtol, rows, (double2*)v, c->pslot.as<unsigned long long>(), c->poll_limit};
         void* argp[] = {&args};
         const void* f = (const void*)k2_pcg_coop;
         if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
@@ -1370,10 +1372,14 @@ int fipc2d_solve_system(fipc2d_ctx_impl* h, const unsigned char* fixed, double r
             FIPC_CUDA(cudaMemcpyAsync(hf, a.flag, 8, cudaMemcpyDeviceToHost, s));
             FIPC_CUDA(cudaStreamSynchronize(s));
             FIPC_CUDA(cudaGetLastError());
-            if (iters_h) *iters_h = hf[1];
-            return hf[0] == 1 ? FIPC_OK : FIPC_ERR_ITERATION;
+            if (hf[0] != 3) {
+                if (iters_h) *iters_h = hf[1];
+                return hf[0] == 1 ? FIPC_OK : FIPC_ERR_ITERATION;
+            }
+            FIPC_CUDA(cudaMemsetAsync(a.flag, 0, 16, s));   // a poll gave up: the multi-kernel path below
+        } else {
+            cudaGetLastError();   // not launchable here: the same
         }
-        cudaGetLastError();   // not launchable here: the multi-kernel path below
     }
     k2_pcg_start<<<nb, T2, 0, s>>>(a, c->rhs.as<double>(), rtol);
     FIPC_LAUNCHED();
@@ -1395,6 +1401,12 @@ int fipc2d_solve_system(fipc2d_ctx_impl* h, const unsigned char* fixed, double r
     FIPC_CUDA(cudaGetLastError());
     if (iters_h) *iters_h = hf[1];
     return hf[0] == 1 ? FIPC_OK : FIPC_ERR_ITERATION;
+}
+
+int fipc2d_ctx_set_poll_limit(fipc2d_ctx_impl* h, int limit) {
+    if (!h || limit < 0) return FIPC_ERR_ARGUMENT;
+    h->c.poll_limit = limit;
+    return FIPC_OK;
 }
 
 int fipc2d_output_residual(fipc2d_ctx_impl* h, const double* sol, double* res_h, void* stream) {

@@ -309,6 +309,9 @@ int fipc2d_export_system(fipc2d_ctx* ctx, int* row_ptr, int* col_idx, double* va
 /* solve_system (NEWTON_IPC.py:750-777) by block-Jacobi PCG to |r| <= rtol |b| */
 int fipc2d_solve_system(fipc2d_ctx* ctx, const unsigned char* fixed, double rtol, int maxit, double* sol, int* iters_h,
                         void* stream);
+/* reads that a wait between the CTAs of the one-launch PCG makes before it gives up (2^20 by default); the solve is
+ * then done again by separate kernels */
+int fipc2d_ctx_set_poll_limit(fipc2d_ctx* ctx, int limit);
 int fipc2d_output_residual(fipc2d_ctx* ctx, const double* sol, double* res_h, void* stream);    /* :805-812 */
 int fipc2d_compute_energy(fipc2d_ctx* ctx, const double* x, const double* xtilde, double* e_h, void* stream);  /* :514-542 */
 /* compute_filter_2D_PE (NEWTON_IPC.py:361-374, 456-468) */
