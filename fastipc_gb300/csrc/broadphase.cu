@@ -130,22 +130,35 @@ struct CandView {
     const int4* cell;
     const float4* box;
 };
+// a primitive's size, by the cells of its query box: SIZE_BIG leaves the grid, SIZE_MID may (big primitives, below)
+enum : unsigned char { SIZE_GRID = 0, SIZE_MID = 1, SIZE_BIG = 2 };
+constexpr int RECORD_MID = 1 << 30;   // in the records' last word
 // the queries' records: the lowest cell of the query box and its cells per axis (10 bits each; 0 for a big
 // primitive), the FP32 box that candidates are tested against and the scene (in box[2 i].w)
 struct QueryView {
     int4* cell;
     float4* box;
+    const unsigned long long* mid_pairs;   // of the queries' kind
 };
-__device__ __forceinline__ void query_record(const QueryView& q, int i, int sc, bool big, C3 lo, C3 hi, v3 blo, v3 bhi) {
+__device__ __forceinline__ void query_record(const QueryView& q, int i, int sc, int size, C3 lo, C3 hi, v3 blo, v3 bhi) {
     const long long nx = hi.x - lo.x + 1, ny = hi.y - lo.y + 1, nz = hi.z - lo.z + 1;
     // at most BIG_CELLS cells unless a position is not finite
-    const bool any = !big && nx > 0 && ny > 0 && nz > 0 && nx < 1024 && ny < 1024 && nz < 1024;
-    q.cell[i] = make_int4(clamp_cell(lo.x), clamp_cell(lo.y), clamp_cell(lo.z), any ? (int)(nx | ny << 10 | nz << 20) : 0);
+    const bool any = size != SIZE_BIG && nx > 0 && ny > 0 && nz > 0 && nx < 1024 && ny < 1024 && nz < 1024;
+    q.cell[i] = make_int4(clamp_cell(lo.x), clamp_cell(lo.y), clamp_cell(lo.z),
+                          any ? (int)(nx | ny << 10 | nz << 20) | (size == SIZE_MID ? RECORD_MID : 0) : 0);
     float4 l = f32_lo(blo);
     l.w = __int_as_float(sc);
     q.box[2 * (size_t)i] = l;
     q.box[2 * (size_t)i + 1] = f32_hi(bhi);
 }
+
+// The line between the grid and the pass over all partners (big primitives, below): more than BIG_CELLS cells leave
+// the grid; between MID_CELLS and BIG_CELLS all of a call's primitives of a kind leave it or none, by the number of tests
+// that they would take outside.
+constexpr long long MID_CELLS = 64, BIG_CELLS = 256;
+constexpr unsigned long long MID_PAIRS = 1ull << 23;
+__device__ __forceinline__ bool mids_leave(const unsigned long long* mid_pairs) { return *mid_pairs <= MID_PAIRS; }
+__device__ __forceinline__ int size_of(long long cells) { return cells > BIG_CELLS ? SIZE_BIG : (cells > MID_CELLS ? SIZE_MID : SIZE_GRID); }
 
 // Cell table of a grid: open addressing with linear probing, load factor at most 1/2, so a query cell
 // costs one or two probes.  run[slot] = (first id, ids) of the slot's cell.
@@ -188,10 +201,10 @@ __device__ __forceinline__ void grid_walk(int block, int n, const QueryView& qv,
     const int i = (block * 128 + threadIdx.x) / QG, lane = threadIdx.x % QG;
     if (i >= n) return;
     const int4 qc = __ldg(qv.cell + i);
-    if (qc.w == 0) return;
+    if (qc.w == 0 || ((qc.w & RECORD_MID) && mids_leave(qv.mid_pairs))) return;
     const float4 qlo = __ldg(qv.box + 2 * (size_t)i), qhi = __ldg(qv.box + 2 * (size_t)i + 1);
     const int sc = __float_as_int(qlo.w);
-    const int nx = qc.w & 1023, ny = qc.w >> 10 & 1023, nz = qc.w >> 20, cells = nx * ny * nz;
+    const int nx = qc.w & 1023, ny = qc.w >> 10 & 1023, nz = qc.w >> 20 & 1023, cells = nx * ny * nz;
     const unsigned group = 0xffu << (threadIdx.x & 24);
     for (int c0 = 0; c0 < cells; c0 += QG) {
         const int c = c0 + lane, z = c % nz, y = c / nz % ny, x = c / nz / ny;
@@ -239,11 +252,13 @@ struct BroadCounters {
     int flags;                  // FLAG_*
     int emitted;                // rows emitted (also past the capacity)
     int sorted;                 // rows[] holds the final counts
-    int big[2];                 // big triangles, edges
+    int big[2], mid[2];         // triangles, edges of the sizes SIZE_BIG, SIZE_MID
     int pairs[2];               // candidate pairs of the two kinds of a query
     int work[2], doubt[2];      // step filter: pairs that pass the additive bound, the sign filter
     int cursor[2];              // ids handed out to runs (points, edges)
-    unsigned long long total[2];   // grid entries (points, edges)
+    unsigned long long total[2];   // grid entries (points, edges), but for those of
+    unsigned long long mid_total;  // edges of SIZE_MID
+    unsigned long long mid_pairs[2];   // tests that the primitives of SIZE_MID would take outside the grid (triangles, edges)
     unsigned long long alpha;   // one scene's step (bits of a double)
     int hit;                    // one scene's intersection flag
     int pad;
@@ -666,10 +681,14 @@ __device__ __forceinline__ void collision_grid(int block, int nbt, const HitArgs
 // with a few large triangles next to finely meshed bodies) would enumerate, or be stored in,
 // thousands of cells.  Such primitives leave the grid: each is tested against every primitive
 // of its own scene with the same narrow phase, so the results are the grid's.
-// The line: at 256 cells the boxes just below it are the tail of every walk and of filling the table (pile of 180
-// cubes: intersection check 0.65 ms, find 0.80; 64 scenes: find 1.47); at 64, 0.52, 0.77 and 1.39; scenes without
-// such boxes do not change.
-constexpr long long BIG_CELLS = 64;
+// Between MID_CELLS and BIG_CELLS both are possible.  A few such boxes are the tail of every walk and of filling the table
+// (us in the grid / outside: pile of 180 cubes at rest, 8 edges, intersection check 636 / 522, find 759 / 726;
+// 64 scenes, find 1365 / 1266; a pile of 8 cubes, the step filter 150 / 126).  But a moving box grows with its step: from
+// some two cells along every axis or 14 along one, all triangles and edges of a body are such boxes, and outside the grid a
+// step filter tests all pairs (180 cubes that fall by 40 cells 85 ms / 310, one of them 1.9 / 2.6).  So the line counts the
+// tests outside, MID_PAIRS = 8.4M a kind.  Both sides near it: 3.8M and 8.2M pairs of edges, find 396 / 315 and 396 / 406;
+// 6.1M and 13.9M pairs of a triangle and an edge, check 514 / 355 and 515 / 569; 10.8M and 29M pairs of edges, step
+// filter 2169 / 1589 and 1331 / 1545.
 
 __device__ __forceinline__ long long box_cells(v3 lo, v3 hi, double inv_dx) {
     const C3 a = cell_of(lo, inv_dx), b = cell_of(hi, inv_dx);
@@ -685,49 +704,64 @@ struct BigArgs {
     const int *bp, *be, *bt;
     const int* off;        // [3][S+1]: points, edges, triangles
     int S;
-    const unsigned char *tri_big, *edge_big;
-    const int* list;       // [nbt + nbe]: triangles, then edges
-    const int* counts;     // [2]
-    int nbt, ny;
+    const unsigned char *tri_size, *edge_size;
+    const int* list;       // [nbt + nbe]: triangles, then edges; of each the big ones from the front, the mid ones from the end
+    const BroadCounters* n;
+    int nbt, nbe, ny;
+    __device__ __forceinline__ bool mids(int kind) const { return mids_leave(n->mid_pairs + kind); }
+    // whether a primitive of this size is out of the grid (mids: mids(kind))
+    __device__ __forceinline__ bool out(unsigned char size, bool mids) const { return size == SIZE_BIG || (size == SIZE_MID && mids); }
 };
 constexpr int BIG_CHUNK = 512;
 __device__ __forceinline__ bool f32_touch(float4 alo, float4 ahi, float4 blo, float4 bhi) {
     return alo.x <= bhi.x && alo.y <= bhi.y && alo.z <= bhi.z && blo.x <= ahi.x && blo.y <= ahi.y && blo.z <= ahi.z;
 }
-// f(i, k, scene) for big primitive i (kind 0: triangle, 1: edge) and its partners k in this CTA's chunk,
-// of list `partners` (0 points, 1 edges, 2 triangles)
-template <class F>
-__device__ __forceinline__ void big_pairs(const BigArgs& b, const SceneGeo& g, int block, int kind, int partners, F f) {
-    const int chunk = block / b.ny;
-    for (int q = block % b.ny; q < b.counts[kind]; q += b.ny) {
-        const int i = b.list[(kind ? b.nbt : 0) + q];
+struct BoxF {
+    float4 lo, hi;
+};
+__device__ __forceinline__ bool touches(const CandView& cv, int k, const BoxF& b) {
+    return f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), b.lo, b.hi);
+}
+// f(i, k, box(i)) for primitive i out of the grid (kind 0: triangle, 1: edge) and its partners k in this CTA's chunk, of
+// list `partners` (0 points, 1 edges, 2 triangles)
+template <class BOX, class F>
+__device__ __forceinline__ void big_pairs(const BigArgs& b, const SceneGeo& g, int block, int kind, int partners, BOX box, F f) {
+    const int chunk = block / b.ny, big = b.n->big[kind], count = big + (b.mids(kind) ? b.n->mid[kind] : 0);
+    const int first = kind ? b.nbt : 0, last = (kind ? b.nbt + b.nbe : b.nbt) - 1;
+    const int* off = b.off + partners * (b.S + 1);
+    for (int q = block % b.ny; q < count; q += b.ny) {
+        const int i = q < big ? b.list[first + q] : b.list[last - (q - big)];
         const int sc = g.scene(kind ? b.be[2 * i] : b.bt[3 * i]);
-        const int* off = b.off + partners * (b.S + 1);
         const int k0 = off[sc] + chunk * BIG_CHUNK, k1 = min(off[sc + 1], k0 + BIG_CHUNK);
-        for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) f(i, k, sc);
+        if (k0 >= k1) continue;
+        const BoxF bx = box(i);
+        for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) f(i, k, bx);
     }
 }
 
 // find_constraints: big triangles against the points, big edges against the edges of their scene (a pair
 // of two big edges once, from its lower index; rows formed with the lower list index first as in the
 // grid pass)
+__device__ __forceinline__ BoxF triangle_box(const int* __restrict__ bt, int i, const double* __restrict__ x, double dh) {
+    const v3 A = ld3(x, bt[3 * i]), B = ld3(x, bt[3 * i + 1]), C = ld3(x, bt[3 * i + 2]), d = mk(dh, dh, dh);
+    return BoxF{f32_lo(vmin(vmin(A, B), C) - d), f32_hi(vmax(vmax(A, B), C) + d)};
+}
 __device__ __forceinline__ void find_pt_big(int block, const BigArgs& b, const FindArgs& a, const SceneGeo& g, CandView cv, const PairList& P,
                                             const RowSink& sink) {
-    const v3 d = mk(a.dh, a.dh, a.dh);
-    big_pairs(b, g, block, 0, 0, [&](int i, int k, int) {
-        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2];
-        const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2);
-        if (!f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), f32_lo(vmin(vmin(A, B), C) - d), f32_hi(vmax(vmax(A, B), C) + d)))
-            return;
+    big_pairs(b, g, block, 0, 0, [&](int i) { return triangle_box(b.bt, i, a.x, a.dh); }, [&](int i, int k, const BoxF& bx) {
+        if (!touches(cv, k, bx)) return;
         if (!pair_push(P, 0, b.bp[k], i)) find_pair_call(a, 0, b.bp[k], i, sink);
     });
 }
 __device__ __forceinline__ void find_ee_big(int block, const BigArgs& b, const FindArgs& a, const SceneGeo& g, CandView cv, const PairList& P,
                                             const RowSink& sink) {
-    big_pairs(b, g, block, 1, 1, [&](int i, int j, int) {
-        if (j == i || (b.edge_big[j] && j < i)) return;
+    const bool mids = b.mids(1);
+    big_pairs(b, g, block, 1, 1, [&](int i) {
         const v3 A0 = ld3(a.x, b.be[2 * i]), A1 = ld3(a.x, b.be[2 * i + 1]);
-        if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(vmin(A0, A1)), f32_hi(vmax(A0, A1)))) return;
+        return BoxF{f32_lo(vmin(A0, A1)), f32_hi(vmax(A0, A1))};
+    }, [&](int i, int j, const BoxF& bx) {
+        if (j == i || (j < i && b.out(b.edge_size[j], mids))) return;
+        if (!touches(cv, j, bx)) return;
         const int lo = i < j ? i : j, hi = i < j ? j : i;
         if (edges_touch(b.be, lo, hi)) return;
         if (!pair_push(P, 1, lo, hi)) find_pair_call(a, 1, lo, hi, sink);
@@ -737,24 +771,28 @@ __device__ __forceinline__ void find_ee_big(int block, const BigArgs& b, const F
 // CCD filter: big moving triangles against the points, big moving edges against the edges of their scene
 __device__ __forceinline__ void ccd_pt_big(int block, const BigArgs& b, const CcdArgs& a, const SceneGeo& g, CandView cv, const PairList& Q,
                                            const CcdList& L) {
-    const v3 d = mk(a.dh, a.dh, a.dh);
-    big_pairs(b, g, block, 0, 0, [&](int i, int k, int) {
-        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2], pp = b.bp[k];
-        if (pp == t0 || pp == t1 || pp == t2) return;
+    big_pairs(b, g, block, 0, 0, [&](int i) {
+        const int t0 = b.bt[3 * i], t1 = b.bt[3 * i + 1], t2 = b.bt[3 * i + 2];
         const v3 A = ld3(a.x, t0), B = ld3(a.x, t1), C = ld3(a.x, t2), dA = ld3(a.p, t0), dB = ld3(a.p, t1), dC = ld3(a.p, t2);
         const v3 mn = vmin(vmin(vmin(A, A + dA), vmin(B, B + dB)), vmin(C, C + dC));
-        const v3 mx = vmax(vmax(vmax(A, A + dA), vmax(B, B + dB)), vmax(C, C + dC));
-        if (!f32_touch(__ldg(cv.box + 2 * (size_t)k), __ldg(cv.box + 2 * (size_t)k + 1), f32_lo(mn - d), f32_hi(mx + d))) return;
+        const v3 mx = vmax(vmax(vmax(A, A + dA), vmax(B, B + dB)), vmax(C, C + dC)), d = mk(a.dh, a.dh, a.dh);
+        return BoxF{f32_lo(mn - d), f32_hi(mx + d)};
+    }, [&](int i, int k, const BoxF& bx) {
+        if (!touches(cv, k, bx)) return;
+        const int pp = b.bp[k];
+        if (pp == b.bt[3 * i] || pp == b.bt[3 * i + 1] || pp == b.bt[3 * i + 2]) return;
         if (!pair_push(Q, 0, pp, i)) ccd_pair_call(a, 0, pp, i, L);
     });
 }
 __device__ __forceinline__ void ccd_ee_big(int block, const BigArgs& b, const CcdArgs& a, const SceneGeo& g, CandView cv, const PairList& Q,
                                            const CcdList& L) {
-    big_pairs(b, g, block, 1, 1, [&](int i, int j, int) {
-        if (j == i || (b.edge_big[j] && j < i)) return;
+    const bool mids = b.mids(1);
+    big_pairs(b, g, block, 1, 1, [&](int i) {
         const v3 I0 = ld3(a.x, b.be[2 * i]), I1 = ld3(a.x, b.be[2 * i + 1]), dI0 = ld3(a.p, b.be[2 * i]), dI1 = ld3(a.p, b.be[2 * i + 1]);
-        const v3 mn = vmin(vmin(I0, I0 + dI0), vmin(I1, I1 + dI1)), mx = vmax(vmax(I0, I0 + dI0), vmax(I1, I1 + dI1));
-        if (!f32_touch(__ldg(cv.box + 2 * (size_t)j), __ldg(cv.box + 2 * (size_t)j + 1), f32_lo(mn), f32_hi(mx))) return;
+        return BoxF{f32_lo(vmin(vmin(I0, I0 + dI0), vmin(I1, I1 + dI1))), f32_hi(vmax(vmax(I0, I0 + dI0), vmax(I1, I1 + dI1)))};
+    }, [&](int i, int j, const BoxF& bx) {
+        if (j == i || (j < i && b.out(b.edge_size[j], mids))) return;
+        if (!touches(cv, j, bx)) return;
         const int lo = i < j ? i : j, hi = i < j ? j : i;
         if (edges_touch(b.be, lo, hi)) return;
         if (!pair_push(Q, 1, lo, hi)) ccd_pair_call(a, 1, lo, hi, L);
@@ -762,15 +800,22 @@ __device__ __forceinline__ void ccd_ee_big(int block, const BigArgs& b, const Cc
 }
 
 // intersection check: big triangles against the edges of their scene, big edges against the triangles of
-// their scene that are not big (kind: which)
+// their scene that are in the grid (kind: which)
 __device__ __forceinline__ void collision_big(int block, int kind, const BigArgs& b, const HitArgs& a, const SceneGeo& g, CandView cv,
                                               const PairList& P) {
-    big_pairs(b, g, block, kind, kind ? 2 : 1, [&](int i, int k, int) {
+    const bool mids = b.mids(0);
+    big_pairs(b, g, block, kind, kind ? 2 : 1, [&](int i) {
+        return kind ? BoxF{__ldg(cv.box + 2 * (size_t)i), __ldg(cv.box + 2 * (size_t)i + 1)} : triangle_box(b.bt, i, a.x, 0.0);
+    }, [&](int i, int k, const BoxF& bx) {
         const int e = kind ? i : k, t = kind ? k : i;
-        if (kind && b.tri_big[t]) return;
+        if (kind && b.out(b.tri_size[t], mids)) return;
         if (edge_of_triangle(b.be, b.bt, e, t)) return;
-        const v3 A = ld3(a.x, b.bt[3 * t]), B = ld3(a.x, b.bt[3 * t + 1]), C = ld3(a.x, b.bt[3 * t + 2]);
-        if (!f32_touch(__ldg(cv.box + 2 * (size_t)e), __ldg(cv.box + 2 * (size_t)e + 1), f32_lo(vmin(vmin(A, B), C)), f32_hi(vmax(vmax(A, B), C)))) return;
+        if (kind) {
+            const BoxF tb = triangle_box(b.bt, t, a.x, 0.0);
+            if (!f32_touch(bx.lo, bx.hi, tb.lo, tb.hi)) return;
+        } else if (!touches(cv, e, bx)) {
+            return;
+        }
         if (!pair_push(P, 0, e, t)) hit_pair_call(a, e, t);
     });
 }
@@ -789,13 +834,14 @@ struct GridBuild {
     unsigned long long mask;   // table size - 1; the ids hold half the table size
 };
 
-// flags and lists of the big primitives (triangle boxes as queried: static or moving; edge boxes as
+// sizes and lists of the big and mid primitives (triangle boxes as queried: static or moving; edge boxes as
 // queried: static or moving, +- dh), candidate records and entry counts of both grids' primitives, and
-// the tables cleared
+// the tables cleared.  off, S: the scenes' boundary lists (BigArgs)
 __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict__ bt, int nbe, const int* __restrict__ be, GridBuild gp,
                                                  GridBuild ge, const double* __restrict__ x, const double* __restrict__ p, double dh,
-                                                 SceneGeo g, QueryView qt, QueryView qe, unsigned char* __restrict__ tri_big,
-                                                 unsigned char* __restrict__ edge_big, int* __restrict__ list, BroadCounters* __restrict__ n) {
+                                                 SceneGeo g, QueryView qt, QueryView qe, const int* __restrict__ off, int S,
+                                                 unsigned char* __restrict__ tri_size, unsigned char* __restrict__ edge_size,
+                                                 int* __restrict__ list, BroadCounters* __restrict__ n) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
     if (k == 0) n->alpha = (unsigned long long)__double_as_longlong(1.0);
     for (unsigned long long h = k; h <= gp.mask; h += nthr) {
@@ -807,8 +853,10 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
         ge.cnt[h] = 0;
     }
     const v3 d = mk(dh, dh, dh);
-    long long cells = 0;   // entries of this thread's primitive
-    int which = 0;
+    const bool check = ge.mode == 4;   // the intersection check: triangles against edges, boxes without dh
+    auto partners = [&](int l, int sc) { return (long long)(off[l * (S + 1) + sc + 1] - off[l * (S + 1) + sc]); };
+    // entries of this thread's primitive (a point, an edge, one of SIZE_MID) and its tests outside the grid
+    long long point_cells = 0, edge_cells = 0, mid_cells = 0, tri_pairs = 0, edge_pairs = 0;
     if (k < nbt) {
         const int t0 = bt[3 * k], t1 = bt[3 * k + 1], t2 = bt[3 * k + 2];
         v3 lo = vmin(vmin(ld3(x, t0), ld3(x, t1)), ld3(x, t2)), hi = vmax(vmax(ld3(x, t0), ld3(x, t1)), ld3(x, t2));
@@ -819,10 +867,14 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
         }
         const int sc = g.scene(t0);
         const double inv_dx = g.idx(sc);
-        const bool big = box_cells(lo, hi, inv_dx) > BIG_CELLS, check = ge.mode == 4;   // the intersection check's boxes carry no dh
-        query_record(qt, k, sc, big, cell_of(lo, inv_dx), cell_of(hi, inv_dx), check ? lo : lo - d, check ? hi : hi + d);
-        tri_big[k] = big;
-        if (big) list[atomicAdd(&n->big[0], 1)] = k;
+        const int size = size_of(box_cells(lo, hi, inv_dx));
+        query_record(qt, k, sc, size, cell_of(lo, inv_dx), cell_of(hi, inv_dx), check ? lo : lo - d, check ? hi : hi + d);
+        tri_size[k] = size;
+        if (size == SIZE_BIG) list[atomicAdd(&n->big[0], 1)] = k;
+        if (size == SIZE_MID) {
+            list[nbt - 1 - atomicAdd(&n->mid[0], 1)] = k;
+            tri_pairs = partners(check ? 1 : 0, sc);
+        }
     } else if (k < nbt + nbe + gp.n) {
         const bool edge = k < nbt + nbe;
         const GridBuild& b = edge ? ge : gp;
@@ -830,7 +882,7 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
         const int sv = edge ? be[2 * i] : b.prim[i];
         const int sc = g.scene(sv);
         const double inv_dx = g.idx(sc);
-        bool big = false;
+        int size = SIZE_GRID;
         if (edge) {
             const int a1 = be[2 * i + 1];
             v3 lo = vmin(ld3(x, sv), ld3(x, a1)), hi = vmax(ld3(x, sv), ld3(x, a1));
@@ -839,33 +891,45 @@ __global__ void __launch_bounds__(256) k_prepare(int nbt, const int* __restrict_
                 lo = vmin(lo, vmin(A, B));
                 hi = vmax(hi, vmax(A, B));
             }
-            big = box_cells(lo - d, hi + d, inv_dx) > BIG_CELLS;
-            if (ge.mode != 4) query_record(qe, i, sc, big, cell_of(lo - d, inv_dx), cell_of(hi + d, inv_dx), lo, hi);
-            edge_big[i] = big;
-            if (big) list[nbt + atomicAdd(&n->big[1], 1)] = i;
+            size = size_of(box_cells(lo - d, hi + d, inv_dx));
+            if (!check) query_record(qe, i, sc, size, cell_of(lo - d, inv_dx), cell_of(hi + d, inv_dx), lo, hi);
+            edge_size[i] = size;
+            if (size == SIZE_BIG) list[nbt + atomicAdd(&n->big[1], 1)] = i;
+            if (size == SIZE_MID) {
+                list[nbt + nbe - 1 - atomicAdd(&n->mid[1], 1)] = i;
+                edge_pairs = partners(check ? 2 : 1, sc);
+            }
         }
         v3 lo, hi;
         stored_box(b.mode, i, b.prim, x, p, dh, &lo, &hi);
         const C3 a = cell_of(lo, inv_dx), e = cell_of(hi, inv_dx);
         cand_record(b.mode, i, b.prim, x, p, dh, lo, hi, a, b.cell, b.box);
-        if (!big) {
-            cells = (e.x - a.x + 1) * (e.y - a.y + 1) * (e.z - a.z + 1);
-            if (!(cells > 0 && cells <= MAX_CELLS_PER_PRIM)) {
+        long long c = 0;
+        if (size != SIZE_BIG) {
+            c = (e.x - a.x + 1) * (e.y - a.y + 1) * (e.z - a.z + 1);
+            if (!(c > 0 && c <= MAX_CELLS_PER_PRIM)) {
                 atomicOr(&n->flags, FLAG_CELLS);
-                cells = 0;
+                c = 0;
             }
         }
-        b.ext[i] = cells ? make_int4((int)(e.x - a.x + 1), (int)(e.y - a.y + 1), (int)(e.z - a.z + 1), sc) : make_int4(0, 0, 0, sc);
-        which = edge ? 1 : 0;
+        b.ext[i] = c ? make_int4((int)(e.x - a.x + 1), (int)(e.y - a.y + 1), (int)(e.z - a.z + 1), sc | (size == SIZE_MID ? RECORD_MID : 0))
+                     : make_int4(0, 0, 0, sc);
+        if (size == SIZE_MID) mid_cells = c;
+        else if (edge) edge_cells = c;
+        else point_cells = c;
     }
-    // totals: one add per warp and grid
-    for (int w = 0; w < 2; ++w) {
-        long long c = which == w ? cells : 0;
-        if (!__any_sync(0xffffffffu, c != 0)) continue;
+    // totals: one add per warp
+    auto add = [](long long c, unsigned long long* to) {
+        if (!__any_sync(0xffffffffu, c != 0)) return;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&n->total[w], (unsigned long long)c);
-    }
+        if ((threadIdx.x & 31) == 0) atomicAdd(to, (unsigned long long)c);
+    };
+    add(point_cells, n->total);
+    add(edge_cells, n->total + 1);
+    add(mid_cells, &n->mid_total);
+    add(tri_pairs, n->mid_pairs);
+    add(edge_pairs, n->mid_pairs + 1);
 }
 
 // f(key, i) for every (cell, primitive) entry of both grids; four lanes share a primitive's cells.
@@ -874,7 +938,8 @@ constexpr int CELL_LANES = 4;
 template <class F>
 __device__ __forceinline__ void each_entry(const GridBuild& gp, const GridBuild& ge, const SceneGeo& g, BroadCounters* n, F f) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) / CELL_LANES, lane = threadIdx.x % CELL_LANES;
-    if (2 * n->total[0] > gp.mask + 1 || 2 * n->total[1] > ge.mask + 1) {
+    const bool mids = mids_leave(n->mid_pairs + 1);
+    if (2 * n->total[0] > gp.mask + 1 || 2 * (n->total[1] + (mids ? 0 : n->mid_total)) > ge.mask + 1) {
         if (k == 0 && lane == 0) atomicOr(&n->flags, FLAG_TABLE);
         return;
     }
@@ -883,10 +948,10 @@ __device__ __forceinline__ void each_entry(const GridBuild& gp, const GridBuild&
     const GridBuild& b = edge ? ge : gp;
     const int i = edge ? k - gp.n : k;
     const int4 a = __ldg(b.cell + i), e = __ldg(b.ext + i);   // no cells: left to the big-primitive pass
-    const int ny = e.y, nz = e.z, c = e.x * ny * nz;
+    const int ny = e.y, nz = e.z, c = (e.w & RECORD_MID) && mids ? 0 : e.x * ny * nz, sc = e.w & ~RECORD_MID;
     for (int q = lane; q < c; q += CELL_LANES) {
         const int qz = q % nz, qy = q / nz % ny, qx = q / nz / ny;
-        f(b, edge, gkey(g, e.w, (long long)a.x + qx, (long long)a.y + qy, (long long)a.z + qz), i);
+        f(b, edge, gkey(g, sc, (long long)a.x + qx, (long long)a.y + qy, (long long)a.z + qz), i);
     }
 }
 
@@ -1111,7 +1176,7 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
         c->ge.cell4.ensure(16ll * c->nBE + 16) || c->ge.ext4.ensure(16ll * c->nBE + 16) || c->ge.box4.ensure(32ll * c->nBE + 32) ||
         c->query_cell.ensure(16ll * n + 16) || c->query_box.ensure(32ll * n + 32))
         return FIPC_ERR_CUDA;
-    unsigned char* tri_big = c->big_flags.as<unsigned char>();
+    unsigned char* tri_size = c->big_flags.as<unsigned char>();
     b->n = c->broad.as<BroadCounters>();
     SceneGeo g = geo(c);
     auto build = [](Grid& gr, const int* prim, int np_, int mode) {
@@ -1120,13 +1185,13 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
     };
     b->gp = build(c->gp, c->bp, np, mode_p);
     b->ge = build(c->ge, c->be, c->nBE, mode_e);
-    b->qt = QueryView{c->query_cell.as<int4>(), c->query_box.as<float4>()};
-    b->qe = QueryView{b->qt.cell + c->nBT, b->qt.box + 2ll * c->nBT};
+    b->qt = QueryView{c->query_cell.as<int4>(), c->query_box.as<float4>(), b->n->mid_pairs};
+    b->qe = QueryView{b->qt.cell + c->nBT, b->qt.box + 2ll * c->nBT, b->n->mid_pairs + 1};
     FIPC_CUDA(cudaMemsetAsync(b->n, 0, sizeof(BroadCounters), s));
     const long long work = (long long)n + np, slots = (long long)(c->gp.size + c->ge.size);
     const int grid = (int)std::max<long long>(nblk(work, 256), std::min<long long>(nblk(slots, 256), 1216));
-    k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, b->qt, b->qe, tri_big, tri_big + c->nBT,
-                                   c->big_list.as<int>(), b->n);
+    k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, b->qt, b->qe, c->prim_off,
+                                   c->n_scenes, tri_size, tri_size + c->nBT, c->big_list.as<int>(), b->n);
     FIPC_LAUNCHED();
     b->g = g;
     // the pair lists, as long as the last calls needed
@@ -1142,7 +1207,7 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
         k_grid_fill<<<entries, 256, 0, s>>>(b->gp, b->ge, g, b->n);
         FIPC_LAUNCHED();
     }
-    b->big = BigArgs{c->bp, c->be, c->bt, c->prim_off, c->n_scenes, tri_big, tri_big + c->nBT, c->big_list.as<int>(), b->n->big, c->nBT,
+    b->big = BigArgs{c->bp, c->be, c->bt, c->prim_off, c->n_scenes, tri_size, tri_size + c->nBT, c->big_list.as<int>(), b->n, c->nBT, c->nBE,
                      c->n_scenes > 1 ? 128 : 32};
     FIPC_CUDA(cudaGetLastError());
     return FIPC_OK;
@@ -1151,13 +1216,20 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
 // after the counters of a call have reached the host: FIPC_OK, an error, or RETRY with larger tables
 constexpr int RETRY = -1;
 static int broad_status(fipc_ctx* c, const BroadCounters& h) {
+    for (int k = 0; k < 2; ++k) {
+        const bool out = h.mid_pairs[k] <= MID_PAIRS;
+        c->broad_stats[k] = h.pairs[k];
+        c->broad_stats[2 + k] = h.work[k];
+        c->broad_stats[4 + k] = h.big[k] + (out ? h.mid[k] : 0);
+        c->broad_stats[6 + k] = out ? 0 : h.mid[k];
+    }
     c->pair_hint = std::max<long long>(c->pair_hint, std::min<long long>(2ll * std::max(h.pairs[0], h.pairs[1]), PAIRS_MAX));
     if (h.flags & FLAG_CELLS) return FIPC_ERR_CAPACITY;
     if (h.flags & FLAG_TABLE) {
-        if (h.total[0] > (1ull << 30) || h.total[1] > (1ull << 30)) return FIPC_ERR_CAPACITY;
+        const unsigned long long np = h.total[0], ne = h.total[1] + (h.mid_pairs[1] <= MID_PAIRS ? 0 : h.mid_total);
+        if (np > (1ull << 30) || ne > (1ull << 30)) return FIPC_ERR_CAPACITY;
         // half as much again, so that a slowly growing contact does not repeat every call
-        if (ensure_table(c->gp, table_size((long long)(h.total[0] + h.total[0] / 2))) ||
-            ensure_table(c->ge, table_size((long long)(h.total[1] + h.total[1] / 2))))
+        if (ensure_table(c->gp, table_size((long long)(np + np / 2))) || ensure_table(c->ge, table_size((long long)(ne + ne / 2))))
             return FIPC_ERR_CUDA;
         return RETRY;
     }

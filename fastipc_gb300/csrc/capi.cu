@@ -389,6 +389,12 @@ int fipc_find_constraints(fipc_ctx* c, const double* x, int* counts_h, void* str
     return FIPC_OK;
 }
 
+int fipc_broadphase_stats(const fipc_ctx* c, long long* out) {
+    if (!c || !out) return FIPC_ERR_ARGUMENT;
+    for (int k = 0; k < 8; ++k) out[k] = c->broad_stats[k];
+    return FIPC_OK;
+}
+
 int fipc_get_constraints(fipc_ctx* c, int type, int* rows, void* stream) {
     if (!c || type < 0 || type >= N_TYPES || !rows) return FIPC_ERR_ARGUMENT;
     if (c->h_counts[type] == 0) return FIPC_OK;

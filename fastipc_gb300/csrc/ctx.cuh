@@ -122,6 +122,7 @@ struct fipc_ctx_impl {
     DBuf query_cell, query_box;           // per query (triangles, then edges): cell range, FP32 box
     DBuf pair_list;                       // candidate pairs of a query
     long long pair_hint = 0;              // list length for the next query, from what the last ones needed
+    long long broad_stats[8] = {0};       // fipc_broadphase_stats
     std::vector<double> h_kappa, h_inv_dx;
     // batched PCG: tiles of consecutive rows inside one scene
     int n_tiles = 0, tile_rows = 0, pcg_grid = 0;
