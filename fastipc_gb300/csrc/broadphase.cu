@@ -12,9 +12,9 @@
 // predicates; constraint rows are then sorted lexicographically and de-duplicated per list
 // exactly like np.unique(axis=0) (NEWTON_IPC.py:348-356).
 //
-// A call is a chain of a few kernels and one copy to the host at its end: table and row capacities are
-// kept from call to call and checked on the device; a call that outgrows them is repeated with larger
-// ones.  Measured on a GB300 against radix-sorted grids, one sort per list and a host round trip per grid:
+// A call is a chain of a few kernels and one copy to the host at its end: table sizes (of each query by itself) and row
+// capacities are kept from call to call and checked on the device; a call that outgrows them is repeated with larger
+// ones, and a table much larger than its query's last call needed shrinks.  Measured on a GB300 against radix-sorted grids, one sort per list and a host round trip per grid:
 // constraint finding of two touching cubes (1,458 vertices) 1.16 -> 0.16 ms a call, of a pile of 180 cubes
 // 5.2 -> 0.81 ms; the step filter of the cubes 2.2 -> 0.55 ms.
 #include <cooperative_groups.h>
@@ -1138,11 +1138,15 @@ static SceneGeo geo(const fipc_ctx* c) {
     return g;
 }
 
-static unsigned long long table_size(long long entries) {
+// the queries that build grids
+enum { Q_FIND = 0, Q_STEP = 1, Q_CHECK = 2 };
+static unsigned long long table_size(unsigned long long entries) {
     unsigned long long size = 1024;
-    while (size < 2ull * (unsigned long long)entries) size <<= 1;
+    while (size < 2ull * entries) size <<= 1;
     return size;
 }
+// for a call with this many entries: half as much again, so that a slowly growing contact does not repeat every call
+static unsigned long long table_for(unsigned long long entries) { return table_size(entries < (1ull << 26) ? entries + entries / 2 : entries); }
 static int ensure_table(Grid& g, unsigned long long size) {
     if (size <= g.size) return FIPC_OK;
     if (g.hkeys.ensure(8 * size) || g.counts.ensure(4 * size) || g.runs.ensure(8 * size) || g.ids.ensure(2 * size)) return FIPC_ERR_CUDA;
@@ -1158,6 +1162,7 @@ struct Broad {
     PairList pairs;
     QueryView qt, qe;
     BroadCounters* n;
+    int query;
 };
 
 static GridView view(const GridBuild& b) { return GridView{b.hk, b.run, b.mask, b.ids}; }
@@ -1166,12 +1171,19 @@ static int big_blocks(const fipc_ctx* c, int partners, int ny) { return nblk(c->
 
 // The grids over the boundary points (mode_p < 0: none) and edges at positions x (+ direction p when
 // moving), and the big primitives.  Tables start at two slots per primitive, twice over, and grow when a
-// call reports that its entries need more.
+// call reports that its entries need more.  Each query has a size of its own in the tables' memory: its moving boxes
+// make a fast step's filter need up to hundreds of times the entries of the other queries, and clearing and scanning
+// that many slots would cost every later call (find_constraints of 180 cubes 0.73 ms, 1.37 after such a filter).
 constexpr long long PAIRS_MAX = 1ll << 24;
-static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode_p, int mode_e, Broad* b, cudaStream_t s) {
-    const int n = c->nBT + c->nBE, np = mode_p < 0 ? 0 : c->nBP;
+static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int query, Broad* b, cudaStream_t s) {
+    static const int modes_p[3] = {0, 2, -1}, modes_e[3] = {1, 3, 4};
+    const int n = c->nBT + c->nBE, mode_p = modes_p[query], mode_e = modes_e[query], np = mode_p < 0 ? 0 : c->nBP;
+    b->query = query;
     if (c->big_flags.ensure((size_t)n + 16) || c->big_list.ensure(4ll * n + 16) || c->broad.ensure(sizeof(BroadCounters))) return FIPC_ERR_CUDA;
-    if (ensure_table(c->gp, table_size(2ll * np)) || ensure_table(c->ge, table_size(2ll * c->nBE))) return FIPC_ERR_CUDA;
+    const unsigned long long slots_p = std::max(c->gp.use[query], table_size(2ull * np)), slots_e = std::max(c->ge.use[query], table_size(2ull * c->nBE));
+    if (ensure_table(c->gp, slots_p) || ensure_table(c->ge, slots_e)) return FIPC_ERR_CUDA;
+    c->gp.use[query] = slots_p;
+    c->ge.use[query] = slots_e;
     if (c->gp.cell4.ensure(16ll * np + 16) || c->gp.ext4.ensure(16ll * np + 16) || c->gp.box4.ensure(32ll * np + 32) ||
         c->ge.cell4.ensure(16ll * c->nBE + 16) || c->ge.ext4.ensure(16ll * c->nBE + 16) || c->ge.box4.ensure(32ll * c->nBE + 32) ||
         c->query_cell.ensure(16ll * n + 16) || c->query_box.ensure(32ll * n + 32))
@@ -1179,16 +1191,16 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
     unsigned char* tri_size = c->big_flags.as<unsigned char>();
     b->n = c->broad.as<BroadCounters>();
     SceneGeo g = geo(c);
-    auto build = [](Grid& gr, const int* prim, int np_, int mode) {
+    auto build = [](Grid& gr, const int* prim, int np_, int mode, unsigned long long slots) {
         return GridBuild{prim, np_, mode, gr.cell4.as<int4>(), gr.ext4.as<int4>(), gr.box4.as<float4>(), gr.hkeys.as<unsigned long long>(), gr.counts.as<int>(),
-                         gr.runs.as<int2>(), gr.ids.as<int>(), gr.size - 1};
+                         gr.runs.as<int2>(), gr.ids.as<int>(), slots - 1};
     };
-    b->gp = build(c->gp, c->bp, np, mode_p);
-    b->ge = build(c->ge, c->be, c->nBE, mode_e);
+    b->gp = build(c->gp, c->bp, np, mode_p, slots_p);
+    b->ge = build(c->ge, c->be, c->nBE, mode_e, slots_e);
     b->qt = QueryView{c->query_cell.as<int4>(), c->query_box.as<float4>(), b->n->mid_pairs};
     b->qe = QueryView{b->qt.cell + c->nBT, b->qt.box + 2ll * c->nBT, b->n->mid_pairs + 1};
     FIPC_CUDA(cudaMemsetAsync(b->n, 0, sizeof(BroadCounters), s));
-    const long long work = (long long)n + np, slots = (long long)(c->gp.size + c->ge.size);
+    const long long work = (long long)n + np, slots = (long long)(slots_p + slots_e);
     const int grid = (int)std::max<long long>(nblk(work, 256), std::min<long long>(nblk(slots, 256), 1216));
     k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, b->qt, b->qe, c->prim_off,
                                    c->n_scenes, tri_size, tri_size + c->nBT, c->big_list.as<int>(), b->n);
@@ -1215,24 +1227,28 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int mode
 
 // after the counters of a call have reached the host: FIPC_OK, an error, or RETRY with larger tables
 constexpr int RETRY = -1;
-static int broad_status(fipc_ctx* c, const BroadCounters& h) {
+static int broad_status(fipc_ctx* c, const Broad& b, const BroadCounters& h) {
     for (int k = 0; k < 2; ++k) {
         const bool out = h.mid_pairs[k] <= MID_PAIRS;
         c->broad_stats[k] = h.pairs[k];
         c->broad_stats[2 + k] = h.work[k];
         c->broad_stats[4 + k] = h.big[k] + (out ? h.mid[k] : 0);
         c->broad_stats[6 + k] = out ? 0 : h.mid[k];
+        c->broad_stats[8 + k] = (k ? b.ge : b.gp).mask + 1;
     }
     c->pair_hint = std::max<long long>(c->pair_hint, std::min<long long>(2ll * std::max(h.pairs[0], h.pairs[1]), PAIRS_MAX));
     if (h.flags & FLAG_CELLS) return FIPC_ERR_CAPACITY;
+    const unsigned long long entries[2] = {h.total[0], h.total[1] + (h.mid_pairs[1] <= MID_PAIRS ? 0 : h.mid_total)};
+    Grid* grid[2] = {&c->gp, &c->ge};
     if (h.flags & FLAG_TABLE) {
-        const unsigned long long np = h.total[0], ne = h.total[1] + (h.mid_pairs[1] <= MID_PAIRS ? 0 : h.mid_total);
-        if (np > (1ull << 30) || ne > (1ull << 30)) return FIPC_ERR_CAPACITY;
-        // half as much again, so that a slowly growing contact does not repeat every call
-        if (ensure_table(c->gp, table_size((long long)(np + np / 2))) || ensure_table(c->ge, table_size((long long)(ne + ne / 2))))
-            return FIPC_ERR_CUDA;
+        if (entries[0] > (1ull << 30) || entries[1] > (1ull << 30)) return FIPC_ERR_CAPACITY;
+        for (int k = 0; k < 2; ++k)
+            if (2 * entries[k] > grid[k]->use[b.query]) grid[k]->use[b.query] = table_for(entries[k]);
         return RETRY;
     }
+    // by halves: a fast step is often followed by another
+    for (int k = 0; k < 2; ++k)
+        if (grid[k]->use[b.query] >= 4 * table_for(entries[k])) grid[k]->use[b.query] /= 2;
     return FIPC_OK;
 }
 static int broad_read(const Broad& b, BroadCounters* h, cudaStream_t s) {
@@ -1266,7 +1282,7 @@ static int rows_large(fipc_ctx* c, const Broad& b, int n, BroadCounters* h, cuda
 int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
     for (int attempt = 0; attempt < 12; ++attempt) {
         Broad b;
-        int st = broad_prepare(c, x, nullptr, 0, 1, &b, s);
+        int st = broad_prepare(c, x, nullptr, Q_FIND, &b, s);
         if (st) return st;
         const RowSink sink{c->row_keys.as<RowKey>(), b.n, c->cap};
         QueryBlocks nb{c->nBP > 0 ? nblk((long long)QG * c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
@@ -1286,7 +1302,7 @@ int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
         BroadCounters h;
         st = broad_read(b, &h, s);
         if (st) return st;
-        st = broad_status(c, h);
+        st = broad_status(c, b, h);
         if (st == RETRY) continue;
         if (st) return st;
         if (h.flags & FLAG_ROWS) {
@@ -1313,7 +1329,7 @@ int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
 // double per scene, preset to 1.0 by the caller; null: the call's own)
 static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, unsigned long long* slot, Broad* b,
                       cudaStream_t s) {
-    int st = broad_prepare(c, x, p, 2, 3, b, s);
+    int st = broad_prepare(c, x, p, Q_STEP, b, s);
     if (st) return st;
     if (!slot) slot = &b->n->alpha;
     const long long cap = std::min<long long>(65536ll + c->nBE + c->nBT, 1ll << 21);
@@ -1352,7 +1368,7 @@ int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inv
         BroadCounters h;
         st = broad_read(b, &h, s);
         if (st) return st;
-        st = broad_status(c, h);
+        st = broad_status(c, b, h);
         if (st == RETRY) continue;   // the minimum so far stays valid
         if (st) return st;
         if (alpha_h) memcpy(alpha_h, &h.alpha, 8);
@@ -1366,7 +1382,7 @@ int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inv
 int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStream_t s) {
     for (int attempt = 0; attempt < 4; ++attempt) {
         Broad b;
-        int st = broad_prepare(c, x, nullptr, -1, 4, &b, s);
+        int st = broad_prepare(c, x, nullptr, Q_CHECK, &b, s);
         if (st) return st;
         int* hit = hits ? hits : &b.n->hit;
         QueryBlocks nb{c->nBE > 0 ? nblk((long long)QG * c->nBT, 128) : 0, 0, 0, 0};
@@ -1386,7 +1402,7 @@ int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStr
         BroadCounters h;
         st = broad_read(b, &h, s);
         if (st) return st;
-        st = broad_status(c, h);
+        st = broad_status(c, b, h);
         if (st == RETRY) continue;
         if (st) return st;
         if (hit_h) *hit_h = h.hit;

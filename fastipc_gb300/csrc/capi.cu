@@ -391,7 +391,7 @@ int fipc_find_constraints(fipc_ctx* c, const double* x, int* counts_h, void* str
 
 int fipc_broadphase_stats(const fipc_ctx* c, long long* out) {
     if (!c || !out) return FIPC_ERR_ARGUMENT;
-    for (int k = 0; k < 8; ++k) out[k] = c->broad_stats[k];
+    for (int k = 0; k < 10; ++k) out[k] = c->broad_stats[k];
     return FIPC_OK;
 }
 

@@ -55,7 +55,8 @@ struct DBuf {
 struct Grid {
     DBuf hkeys, counts, runs, ids;
     DBuf cell4, ext4, box4;   // per stored primitive: lowest cell, cells per axis and scene, FP32 box
-    unsigned long long size = 0;   // table slots (a power of two, at least twice the entries)
+    unsigned long long size = 0;   // slots that the buffers hold
+    unsigned long long use[3] = {0, 0, 0};   // slots of each query's calls (powers of two, at least twice the entries)
 };
 
 struct fipc_ctx_impl {
@@ -122,7 +123,7 @@ struct fipc_ctx_impl {
     DBuf query_cell, query_box;           // per query (triangles, then edges): cell range, FP32 box
     DBuf pair_list;                       // candidate pairs of a query
     long long pair_hint = 0;              // list length for the next query, from what the last ones needed
-    long long broad_stats[8] = {0};       // fipc_broadphase_stats
+    long long broad_stats[10] = {0};       // fipc_broadphase_stats
     std::vector<double> h_kappa, h_inv_dx;
     // batched PCG: tiles of consecutive rows inside one scene
     int n_tiles = 0, tile_rows = 0, pcg_grid = 0;

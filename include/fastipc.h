@@ -113,10 +113,10 @@ int fipc_dense_spd_inverse(int n, double* a, double* work, void* stream);
  * lists, sorted lexicographically and de-duplicated; counts_h [7] receives their sizes. */
 int fipc_find_constraints(fipc_ctx* ctx, const double* x, int* counts_h, void* stream);
 int fipc_get_constraints(fipc_ctx* ctx, int type, int* rows, void* stream);
-/* counts of the context's last constraint, step-size or intersection query, out[8]: [0..1] candidate pairs (point or edge
+/* counts of the context's last constraint, step-size or intersection query, out[10]: [0..1] candidate pairs (point or edge
  * against triangle; edge against edge), [2..3] those that pass the step filter's additive bound, [4..5] triangles and
  * edges tested against all primitives of their scene instead of through the grid, [6..7] those of more than 64 cells in
- * the grid */
+ * the grid, [8..9] slots of the point and the edge table */
 int fipc_broadphase_stats(const fipc_ctx* ctx, long long* out);
 
 /* compute_hessian_and_gradient, NEWTON_IPC.py:736-747 (inertia :558-567, elasticity

@@ -19,9 +19,9 @@ pytestmark = pytest.mark.gpu
 
 
 def stats(s):
-    out = (ctypes.c_longlong * 8)()
+    out = (ctypes.c_longlong * 10)()
     assert N.lib().fipc_broadphase_stats(s.ctx, out) == 0
-    return list(out)
+    return list(out)[:8]
 
 
 def cell_of(sc):
