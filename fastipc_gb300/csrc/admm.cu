@@ -481,7 +481,7 @@ __global__ void k_admm_dual_rows(int n, const int4* __restrict__ rows, TypeTable
 
 static inline int nblk_a(long long n, int b) { return (int)((n + b - 1) / b); }
 
-// the current lists concatenated (rows_all) with their type table
+// the current lists concatenated (rows.all) with their type table
 static int current_rows(fipc_ctx* c, TypeTable* tt, int* n, cudaStream_t s) {
     long long nent = 0;
     return contact_prepare(c, tt, n, &nent, s);
@@ -544,7 +544,7 @@ int fipc_admm_reuse(fipc_ctx* c, double alpha, const double* x, const double* xt
     const double dhat = sqrt(c->dhat2);
     const double minQ = sqrt(pp_hessian_norm(9e-1 * dhat, c->dhat2, c->kappa)) / 10;
     const double maxQ = sqrt(pp_hessian_norm(1e-4 * dhat, c->dhat2, c->kappa)) * 10;
-    k_admm_reuse<<<nblk_a(n, 128), 128, 0, s>>>(n, c->rows_all.as<int4>(), tt, x, xtilde, c->x0, alpha, c->dhat2, c->kappa, minQ, maxQ,
+    k_admm_reuse<<<nblk_a(n, 128), 128, 0, s>>>(n, c->rows.all.as<int4>(), tt, x, xtilde, c->x0, alpha, c->dhat2, c->kappa, minQ, maxQ,
                                                 (const int4*)old_rows, ot, old_y, old_r, old_Q, y, r, Q);
     FIPC_LAUNCHED();
     FIPC_CUDA(cudaGetLastError());
@@ -600,7 +600,7 @@ int fipc_admm_local(fipc_ctx* c, const double* x, const double* W, double* z, co
     if (st) return st;
     if (n > 0) {
         if (!y || !r || !Q) return FIPC_ERR_ARGUMENT;
-        k_admm_local_rows<<<nblk_a(32ll * n, 64), 64, 0, s>>>(n, c->rows_all.as<int4>(), tt, x, c->x0, c->dhat2, c->kappa, Q, r, y, status);
+        k_admm_local_rows<<<nblk_a(32ll * n, 64), 64, 0, s>>>(n, c->rows.all.as<int4>(), tt, x, c->x0, c->dhat2, c->kappa, Q, r, y, status);
         FIPC_LAUNCHED();
     }
     int h = 0;
@@ -623,7 +623,7 @@ int fipc_admm_dual(fipc_ctx* c, const double* x, const double* z, double* u, con
     if (st) return st;
     if (n > 0) {
         if (!y || !r) return FIPC_ERR_ARGUMENT;
-        k_admm_dual_rows<<<nblk_a(n, 128), 128, 0, s>>>(n, c->rows_all.as<int4>(), tt, x, y, r);
+        k_admm_dual_rows<<<nblk_a(n, 128), 128, 0, s>>>(n, c->rows.all.as<int4>(), tt, x, y, r);
         FIPC_LAUNCHED();
     }
     FIPC_CUDA(cudaGetLastError());

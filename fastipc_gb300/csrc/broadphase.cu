@@ -1147,12 +1147,6 @@ static unsigned long long table_size(unsigned long long entries) {
 }
 // for a call with this many entries: half as much again, so that a slowly growing contact does not repeat every call
 static unsigned long long table_for(unsigned long long entries) { return table_size(entries < (1ull << 26) ? entries + entries / 2 : entries); }
-static int ensure_table(Grid& g, unsigned long long size) {
-    if (size <= g.size) return FIPC_OK;
-    if (g.hkeys.ensure(8 * size) || g.counts.ensure(4 * size) || g.runs.ensure(8 * size) || g.ids.ensure(2 * size)) return FIPC_ERR_CUDA;
-    g.size = size;
-    return FIPC_OK;
-}
 
 // one call's view of the scene: grids, big primitives and counters
 struct Broad {
@@ -1181,9 +1175,7 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int quer
     b->query = query;
     if (c->big_flags.ensure((size_t)n + 16) || c->big_list.ensure(4ll * n + 16) || c->broad.ensure(sizeof(BroadCounters))) return FIPC_ERR_CUDA;
     const unsigned long long slots_p = std::max(c->gp.use[query], table_size(2ull * np)), slots_e = std::max(c->ge.use[query], table_size(2ull * c->nBE));
-    if (ensure_table(c->gp, slots_p) || ensure_table(c->ge, slots_e)) return FIPC_ERR_CUDA;
-    c->gp.use[query] = slots_p;
-    c->ge.use[query] = slots_e;
+    if (c->gp.ensure(slots_p, query) || c->ge.ensure(slots_e, query)) return FIPC_ERR_CUDA;
     if (c->gp.cell4.ensure(16ll * np + 16) || c->gp.ext4.ensure(16ll * np + 16) || c->gp.box4.ensure(32ll * np + 32) ||
         c->ge.cell4.ensure(16ll * c->nBE + 16) || c->ge.ext4.ensure(16ll * c->nBE + 16) || c->ge.box4.ensure(32ll * c->nBE + 32) ||
         c->query_cell.ensure(16ll * n + 16) || c->query_box.ensure(32ll * n + 32))
@@ -1257,34 +1249,27 @@ static int broad_read(const Broad& b, BroadCounters* h, cudaStream_t s) {
     return FIPC_OK;
 }
 
-int ensure_row_capacity(fipc_ctx* c, int cap) {
-    if (cap <= c->cap) return FIPC_OK;
-    if (c->row_keys.ensure(16ll * cap) || c->row_keys_alt.ensure(16ll * cap) || c->rows_all.ensure(16ll * cap)) return FIPC_ERR_CUDA;
-    c->cap = cap;
-    return FIPC_OK;
-}
-
 // sort and unique of the n emitted rows when they are too many for one CTA
 static int rows_large(fipc_ctx* c, const Broad& b, int n, BroadCounters* h, cudaStream_t s) {
-    RowKey* k = c->row_keys.as<RowKey>();
-    RowKey* u = c->row_keys_alt.as<RowKey>();
+    RowKey* k = c->rows.keys.as<RowKey>();
+    RowKey* u = c->rows.keys_alt.as<RowKey>();
     int* nu = &b.n->sorted;
     int st = cub_call(c, [&](void* t, size_t& bytes) { return cub::DeviceMergeSort::SortKeys(t, bytes, k, n, RowLess(), s); });
     if (st) return st;
     st = cub_call(c, [&](void* t, size_t& bytes) { return cub::DeviceSelect::Unique(t, bytes, k, u, nu, n, s); });
     if (st) return st;
-    k_rows_write<<<nblk(n, 256), 256, 0, s>>>(nu, u, b.n, c->rows_all.as<int4>());
+    k_rows_write<<<nblk(n, 256), 256, 0, s>>>(nu, u, b.n, c->rows.all.as<int4>());
     FIPC_LAUNCHED();
     return broad_read(b, h, s);
 }
 
-// find_constraints (NEWTON_IPC.py:337-357) into c->rows_all / c->h_counts
+// find_constraints (NEWTON_IPC.py:337-357) into c->rows.all / c->h_counts
 int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
     for (int attempt = 0; attempt < 12; ++attempt) {
         Broad b;
         int st = broad_prepare(c, x, nullptr, Q_FIND, &b, s);
         if (st) return st;
-        const RowSink sink{c->row_keys.as<RowKey>(), b.n, c->cap};
+        const RowSink sink{c->rows.keys.as<RowKey>(), b.n, c->rows.cap};
         QueryBlocks nb{c->nBP > 0 ? nblk((long long)QG * c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
         nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b.big.ny) : 0;
         nb.ee_big = c->nBE > 1 ? big_blocks(c, 1, b.big.ny) : 0;
@@ -1297,7 +1282,7 @@ int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
             k_find_pairs<<<PAIR_BLOCKS, PAIR_THREADS, 0, s>>>(a, b.pairs, sink);
             FIPC_LAUNCHED();
         }
-        k_rows_small<<<1, SORT_THREADS, 0, s>>>(sink.rows, b.n, c->rows_all.as<int4>());
+        k_rows_small<<<1, SORT_THREADS, 0, s>>>(sink.rows, b.n, c->rows.all.as<int4>());
         FIPC_LAUNCHED();
         BroadCounters h;
         st = broad_read(b, &h, s);
@@ -1307,7 +1292,8 @@ int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s) {
         if (st) return st;
         if (h.flags & FLAG_ROWS) {
             if (h.emitted > (1 << 29)) return FIPC_ERR_CAPACITY;
-            if (ensure_row_capacity(c, 2 * h.emitted)) return FIPC_ERR_CUDA;
+            for (int t = 0; t < N_TYPES; ++t) c->h_counts[t] = 0;   // the former lists' rows go with their buffer
+            if (c->rows.ensure(2 * h.emitted)) return FIPC_ERR_CUDA;
             continue;
         }
         if (!h.sorted) {

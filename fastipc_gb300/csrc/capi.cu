@@ -14,7 +14,6 @@
 
 namespace fipc {
 int find_constraints(fipc_ctx* c, const double* x, cudaStream_t s);
-int ensure_row_capacity(fipc_ctx* c, int cap);
 int ccd_step(fipc_ctx* c, const double* x, const double* p, double eta, bool inversion, double* alpha_h, unsigned long long* slots,
              cudaStream_t s);
 int check_collision(fipc_ctx* c, const double* x, int* hit_h, int* hits, cudaStream_t s);
@@ -79,7 +78,7 @@ void free_ctx(fipc_ctx* c) {
                     c->up_spos, c->up_tspos, c->diag_spos, c->sell_val, c->prim_off};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    DBuf* bufs[] = {&c->row_keys, &c->row_keys_alt, &c->rows_all, &c->cub_tmp, &c->broad, &c->big_flags, &c->big_list, &c->ccd_work, &c->pair_list, &c->query_cell, &c->query_box, &c->c_g, &c->c_H, &c->c_keys, &c->c_keys_alt, &c->c_vals, &c->c_vals_alt, &c->c_ukeys,
+    DBuf* bufs[] = {&c->rows.keys, &c->rows.keys_alt, &c->rows.all, &c->cub_tmp, &c->broad, &c->big_flags, &c->big_list, &c->ccd_work, &c->pair_list, &c->query_cell, &c->query_box, &c->c_g, &c->c_H, &c->c_keys, &c->c_keys_alt, &c->c_vals, &c->c_vals_alt, &c->c_ukeys,
                     &c->c_ucount, &c->c_ustart, &c->c_val, &c->c_rowptr, &c->c_col, &c->pcg_vec, &c->pcg_part, &c->scal, &c->red, &c->mlp_dist};
     for (DBuf* b : bufs) b->release();
     Grid* gs[] = {&c->gp, &c->ge};
@@ -309,7 +308,7 @@ int fipc_ctx_create(fipc_ctx** out, int n_verts, int n_tets, const int* tets, co
     c->max_prims[0] = n_bp;
     c->max_prims[1] = n_be;
     c->max_prims[2] = n_bt;
-    if (st == FIPC_OK) st = ensure_row_capacity(c, 8192);
+    if (st == FIPC_OK) st = c->rows.ensure(8192);
     if (st == FIPC_OK) st = cs_setup(c, default_agg_rows(n_verts), row_ptr.data(), col_idx.data());
     if (st == FIPC_OK) st = mg_setup(c, 0.0);
     if (st != FIPC_OK) {

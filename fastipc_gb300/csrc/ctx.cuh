@@ -57,6 +57,32 @@ struct Grid {
     DBuf cell4, ext4, box4;   // per stored primitive: lowest cell, cells per axis and scene, FP32 box
     unsigned long long size = 0;   // slots that the buffers hold
     unsigned long long use[3] = {0, 0, 0};   // slots of each query's calls (powers of two, at least twice the entries)
+    // room for a table of this many slots.  A buffer whose allocation fails is gone, so the size counts only once all
+    // have it; a query that asked for too much starts over from its smallest table.
+    int ensure(unsigned long long slots, int query) {
+        if (slots > size) {
+            size = 0;
+            use[query] = 0;
+            if (hkeys.ensure(8 * slots) || counts.ensure(4 * slots) || runs.ensure(8 * slots) || ids.ensure(2 * slots)) return FIPC_ERR_CUDA;
+            size = slots;
+        }
+        use[query] = slots;
+        return FIPC_OK;
+    }
+};
+
+// constraint rows: as sort keys where they are emitted, the keys sorted and unique, and the rows of all lists one
+// behind the other ([n][4] int)
+struct RowStore {
+    DBuf keys, keys_alt, all;
+    int cap = 0;   // rows that all three hold (none after a failed allocation)
+    int ensure(int rows) {
+        if (rows <= cap) return FIPC_OK;
+        cap = 0;
+        if (keys.ensure(16ll * rows) || keys_alt.ensure(16ll * rows) || all.ensure(16ll * rows)) return FIPC_ERR_CUDA;
+        cap = rows;
+        return FIPC_OK;
+    }
 };
 
 struct fipc_ctx_impl {
@@ -86,12 +112,11 @@ struct fipc_ctx_impl {
     double* sell_val = nullptr;
     // per-iteration element data and the system
     double *elem_g = nullptr, *elem_H = nullptr, *bsr_val = nullptr, *rhs = nullptr;
-    // constraint lists: emitted rows as sort keys (capacity cap), the sorted unique rows of all lists one
-    // behind the other ([n][4] int), counts and offsets of the lists
-    DBuf row_keys, row_keys_alt, rows_all, cub_tmp;
+    // constraint lists, counts and offsets of the lists
+    RowStore rows;
+    DBuf cub_tmp;
     int h_counts[N_TYPES] = {0}, h_row0[N_TYPES] = {0};
-    int cap = 0;
-    int* list_rows(int t) const { return rows_all.as<int>() + 4ll * h_row0[t]; }
+    int* list_rows(int t) const { return rows.all.as<int>() + 4ll * h_row0[t]; }
     // contact system
     DBuf c_g, c_H, c_keys, c_keys_alt, c_vals, c_vals_alt, c_ukeys, c_ucount, c_ustart, c_val, c_rowptr, c_col;
     int c_rows = 0, c_nnzb = 0;

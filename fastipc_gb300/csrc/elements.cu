@@ -391,7 +391,7 @@ int launch_energy(const fipc_ctx* c, const double* x, const double* xt, double* 
     }
     tt.row0[N_TYPES] = n;
     k_energy<<<RED_BLOCKS, RED_THREADS, 0, s>>>(c->nV, c->nT, n, x, xt, c->mass, (const int4*)c->tets, c->dminv, c->vol, c->lam, c->mu,
-                                                c->dt * c->dt, c->rows_all.as<int4>(), tt, c->x0, c->dhat2, c->kappa,
+                                                c->dt * c->dt, c->rows.all.as<int4>(), tt, c->x0, c->dhat2, c->kappa,
                                                 c->n_scenes > 1 ? c->s_kappa : nullptr, c->v_scene, part);
     FIPC_LAUNCHED();
     k_sum_parts<<<1, RED_THREADS, 0, s>>>(part, out);

@@ -455,14 +455,14 @@ int assemble_system(fipc_ctx* c, const double* x, const double* xt, cudaStream_t
     bool positive = c->n_scenes > 1 || c->kappa > 0.0;
     if (c->n_scenes > 1)
         for (double k : c->h_kappa) positive = positive && k > 0.0;
-    st = launch_barrier_rows(c->h_counts, tt.row0, c->rows_all.as<int>(), x, c->x0, c->dhat2, c->kappa,
+    st = launch_barrier_rows(c->h_counts, tt.row0, c->rows.all.as<int>(), x, c->x0, c->dhat2, c->kappa,
                              c->n_scenes > 1 ? c->s_kappa : nullptr, c->v_scene, nullptr, c->c_g.as<double>(), c->c_H.as<double>(),
                              positive, s);
     if (st) return st;
     return contact_reduce(c, tt, nrows, nent, s);
 }
 
-// The contact rows of the current lists (rows_all, in list order): the type table, the row and block-entry counts, and buffers for the per-row gradients c_g [rows][12]
+// The contact rows of the current lists (rows.all, in list order): the type table, the row and block-entry counts, and buffers for the per-row gradients c_g [rows][12]
 // and 3x3 blocks c_H [rows][16][9] that the caller fills.  With no rows the contact matrix is
 // left empty.
 int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_out, cudaStream_t s) {
@@ -502,7 +502,7 @@ int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_
 // The contact matrix (block CSR, fixed-order sums of every (row, column) block of the rows) and
 // the rows' gradients folded into rhs, from c_g / c_H filled for the rows contact_prepare set up
 int contact_reduce(fipc_ctx* c, const TypeTable& tt, int nrows, long long nent, cudaStream_t s) {
-    const int4* all = c->rows_all.as<int4>();
+    const int4* all = c->rows.all.as<int4>();
     k_contact_keys<<<nblk(nrows, 128), 128, 0, s>>>(nrows, all, tt, c->c_keys.as<unsigned long long>(), c->c_vals.as<int>());
     FIPC_LAUNCHED();
     const int N = (int)nent;
