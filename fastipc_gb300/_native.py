@@ -18,7 +18,7 @@ STATUS = {0: 'ok', 1: 'capacity exceeded', 2: 'iteration limit reached', 3: 'non
 EXPORTS = [
     'fipc_elasticity', 'fipc_barrier_rows', 'fipc_ccd_pairs', 'fipc_inversion_free_pairs', 'fipc_compute_xn_and_xtilde',
     'fipc_move_nodes', 'fipc_dirichlet_script', 'fipc_apply_sol', 'fipc_compute_v', 'fipc_ctx_create', 'fipc_ctx_destroy', 'fipc_ctx_params',
-    'fipc_ctx_set_params', 'fipc_ctx_mass', 'fipc_ctx_set_x0', 'fipc_find_constraints', 'fipc_get_constraints', 'fipc_broadphase_stats',
+    'fipc_ctx_set_params', 'fipc_ctx_mass', 'fipc_ctx_set_x0', 'fipc_find_constraints', 'fipc_get_constraints', 'fipc_broadphase_stats', 'fipc_ctx_set_list_limit',
     'fipc_compute_hessian_and_gradient', 'fipc_system_sizes', 'fipc_export_system', 'fipc_solve_system',
     'fipc_output_residual', 'fipc_compute_energy', 'fipc_compute_intersection_free_step_size', 'fipc_check_collision',
     'fipc_launch_count', 'fipc_status_string', 'fipc_profile_enable', 'fipc_profile_read', 'fipc_fp64_fma_probe',

@@ -1199,8 +1199,9 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int quer
     FIPC_LAUNCHED();
     b->g = g;
     // the pair lists, as long as the last calls needed
-    const long long want = std::min<long long>(std::max<long long>(65536ll + 2ll * n, c->pair_hint), PAIRS_MAX);
-    if (c->pair_list.ensure(16 * want)) return FIPC_ERR_CUDA;
+    long long want = std::min<long long>(std::max<long long>(65536ll + 2ll * n, c->pair_hint), PAIRS_MAX);
+    if (c->list_limit >= 0) want = std::min<long long>(want, c->list_limit);
+    if (c->pair_list.ensure(16 * want + 16)) return FIPC_ERR_CUDA;
     b->pairs = PairList{c->pair_list.as<int2>(), b->n->pairs, (int)want};
     const int entries = nblk((long long)CELL_LANES * (np + c->nBE), 256);
     if (entries > 0) {
@@ -1318,8 +1319,9 @@ static int ccd_launch(fipc_ctx* c, const double* x, const double* p, double eta,
     int st = broad_prepare(c, x, p, Q_STEP, b, s);
     if (st) return st;
     if (!slot) slot = &b->n->alpha;
-    const long long cap = std::min<long long>(65536ll + c->nBE + c->nBT, 1ll << 21);
-    if (c->ccd_work.ensure(4 * cap * sizeof(CcdWork))) return FIPC_ERR_CUDA;
+    long long cap = std::min<long long>(65536ll + c->nBE + c->nBT, 1ll << 21);
+    if (c->list_limit >= 0) cap = std::min<long long>(cap, c->list_limit);
+    if (c->ccd_work.ensure(4 * cap * sizeof(CcdWork) + sizeof(CcdWork))) return FIPC_ERR_CUDA;
     const CcdList L{c->ccd_work.as<CcdWork>(), b->n->work, (int)cap}, M{L.w + 2 * cap, b->n->doubt, (int)cap};
     QueryBlocks nb{c->nBP > 0 ? nblk((long long)QG * c->nBT, 128) : 0, nblk((long long)QG * c->nBE, 128), 0, 0};
     nb.pt_big = c->nBT > 0 && c->nBP > 0 ? big_blocks(c, 0, b->big.ny) : 0;

@@ -388,6 +388,12 @@ int fipc_find_constraints(fipc_ctx* c, const double* x, int* counts_h, void* str
     return FIPC_OK;
 }
 
+int fipc_ctx_set_list_limit(fipc_ctx* c, int limit) {
+    if (!c || limit < -1) return FIPC_ERR_ARGUMENT;
+    c->list_limit = limit;
+    return FIPC_OK;
+}
+
 int fipc_broadphase_stats(const fipc_ctx* c, long long* out) {
     if (!c || !out) return FIPC_ERR_ARGUMENT;
     for (int k = 0; k < 10; ++k) out[k] = c->broad_stats[k];

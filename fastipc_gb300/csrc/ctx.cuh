@@ -148,6 +148,7 @@ struct fipc_ctx_impl {
     DBuf query_cell, query_box;           // per query (triangles, then edges): cell range, FP32 box
     DBuf pair_list;                       // candidate pairs of a query
     long long pair_hint = 0;              // list length for the next query, from what the last ones needed
+    int list_limit = -1;                  // most entries of a pair or filter list (-1: by their own rules)
     long long broad_stats[10] = {0};       // fipc_broadphase_stats
     std::vector<double> h_kappa, h_inv_dx;
     // batched PCG: tiles of consecutive rows inside one scene

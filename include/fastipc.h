@@ -113,6 +113,9 @@ int fipc_dense_spd_inverse(int n, double* a, double* work, void* stream);
  * lists, sorted lexicographically and de-duplicated; counts_h [7] receives their sizes. */
 int fipc_find_constraints(fipc_ctx* ctx, const double* x, int* counts_h, void* stream);
 int fipc_get_constraints(fipc_ctx* ctx, int type, int* rows, void* stream);
+/* at most this many entries in each candidate list of the broad phase (-1, the default: as many as the scene's size and the
+ * last calls suggest).  Pairs past a list's end are tested where they are found: slower, the results are the same */
+int fipc_ctx_set_list_limit(fipc_ctx* ctx, int limit);
 /* counts of the context's last constraint, step-size or intersection query, out[10]: [0..1] candidate pairs (point or edge
  * against triangle; edge against edge), [2..3] those that pass the step filter's additive bound, [4..5] triangles and
  * edges tested against all primitives of their scene instead of through the grid, [6..7] those of more than 64 cells in
