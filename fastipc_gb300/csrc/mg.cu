@@ -479,7 +479,11 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(PCGArgs a, MgLev L, 
 
 // level >= 1: POST = false: t = g - A z;  POST = true: z2 = z + w D^-1 (g - A z).  One node per warp,
 // or (FIVE) five: lane = 6 n + p takes output p of node n's whole row, a third fewer FP64
-// instructions per node; taken for levels with enough nodes to fill the GPU with such warps.
+// instructions per node.  Taken for levels that fill the GPU with such warps and whose rows are alike: a warp of
+// five lasts as long as its longest row, and a node in contact has a longer one.  us per PCG iteration, five nodes a
+// warp / one, by the nodes of level 1: without contact 2,597 119.8 / 120.1, 3,234 140.1 / 138.8, 3,675 151.6 / 151.6,
+// 4,165 162.6 / 168.8, 4,802 179.9 / 188.3, 6,419 216.8 / 225.3; with contact 3,431 140.8 / 130.8, 5,039 165.8 / 163.5,
+// 8,018 211.1 / 212.1, 14,264 342.0 / 334.2, 19,871 430.6 / 432.2.
 template <bool POST, bool FIVE>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_smooth(PCGArgs a, MgLev L, const double* __restrict__ omega) {
     if (*(volatile int*)&a.flag[0]) return;
@@ -504,11 +508,11 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_smooth(PCGArgs a, MgLev L, co
     const double z = node_minv(L.minv + 36 * (size_t)J, r, omega[0], FIVE ? 6 * (n < 5 ? n : 0) : 0, p);
     if (live) L.z2[6 * (size_t)I + p] = L.z[6 * (size_t)I + p] + z;
 }
-constexpr int MG_FIVE_MIN = 2432;   // nodes from which five share a warp
+constexpr int MG_FIVE_MIN = 4096;
 
 template <bool POST>
 static void launch_smooth(const PCGArgs& a, const MgLev& L, const double* omega, cudaStream_t s) {
-    if (L.n >= MG_FIVE_MIN) k_mg_smooth<POST, true><<<nblk_m(32ll * ((L.n + 4) / 5), MG_THREADS), MG_THREADS, 0, s>>>(a, L, omega);
+    if (L.n >= MG_FIVE_MIN && !L.c_rp) k_mg_smooth<POST, true><<<nblk_m(32ll * ((L.n + 4) / 5), MG_THREADS), MG_THREADS, 0, s>>>(a, L, omega);
     else k_mg_smooth<POST, false><<<nblk_m(32ll * L.n, MG_THREADS), MG_THREADS, 0, s>>>(a, L, omega);
 }
 

@@ -11,7 +11,7 @@ namespace fipc {
 //   * one node per warp: lane = 6 kk + p (kk < 5; lanes 30, 31 idle) takes output p of the row's
 //     blocks kk, kk + 5, ...; the five partial sums of an output are added in a fixed order;
 //   * five nodes per warp (lane = 6 n + p takes output p of node n's whole row): a third fewer FP64
-//     instructions per node, for levels with more nodes than the GPU has warps.
+//     instructions per node (mg.cu has the rule).
 // NB: blocks in flight.  Warps that hold five whole rows are few (8 per SM for 6,419 nodes), so each
 // keeps four blocks in flight: a PCG iteration of the 960k-tet bar takes 218 us so, 226 us with two
 // and 227 us with one node per warp.
