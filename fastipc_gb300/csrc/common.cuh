@@ -29,6 +29,17 @@ FIPC_HD double comp(v3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }
 FIPC_HD v3 vmin(v3 a, v3 b) { return v3{fmin(a.x, b.x), fmin(a.y, b.y), fmin(a.z, b.z)}; }
 FIPC_HD v3 vmax(v3 a, v3 b) { return v3{fmax(a.x, b.x), fmax(a.y, b.y), fmax(a.z, b.z)}; }
 
+// 1 / d to within an ulp from an FP32 reciprocal: a shorter chain than the division's where one thread's pivot holds up
+// a tile.  The FP32 one is off by 2^-23 at most (its operand's and its own rounding), and each Newton step squares that:
+// 2^-46, 2^-92, so what remains is the last step's rounding.
+FIPC_HD double reciprocal(double d) {
+    const float f = (float)d;
+    if (!(f > 1e-30f && f < 1e30f)) return 1.0 / d;
+    double r = (double)(1.f / f);
+    r = fma(r, fma(-d, r, 1.0), r);
+    return fma(r, fma(-d, r, 1.0), r);
+}
+
 FIPC_HD v3 load3(const double* p, int i) { return v3{p[3 * i], p[3 * i + 1], p[3 * i + 2]}; }
 
 // status codes shared with the C ABI (include/fastipc.h)

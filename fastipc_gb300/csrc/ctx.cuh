@@ -189,15 +189,6 @@ struct SceneGeo {
 __device__ __forceinline__ v3 ld3(const double* __restrict__ x, int i) {
     return v3{__ldg(x + 3 * i), __ldg(x + 3 * i + 1), __ldg(x + 3 * i + 2)};
 }
-// 1 / d to within an ulp from an FP32 reciprocal (two Newton steps: 24, 48, 96 bits): a shorter chain than the
-// division's where one thread's pivot holds up a tile
-__device__ __forceinline__ double reciprocal(double d) {
-    const float f = (float)d;
-    if (!(f > 1e-30f && f < 1e30f)) return 1.0 / d;
-    double r = (double)(1.f / f);
-    r = fma(r, fma(-d, r, 1.0), r);
-    return fma(r, fma(-d, r, 1.0), r);
-}
 #endif
 
 // row ranges of the concatenated lists: rows [row0[t], row0[t+1]) are of type t and their
