@@ -163,6 +163,7 @@ __device__ __forceinline__ int size_of(long long cells) { return cells > BIG_CEL
 // Cell table of a grid: open addressing with linear probing, load factor at most 1/2, so a query cell
 // costs one or two probes.  run[slot] = (first id, ids) of the slot's cell.
 constexpr unsigned long long HASH_EMPTY = ~0ull;
+// the 64-bit finaliser of MurmurHash3
 __device__ __forceinline__ unsigned long long mix64(unsigned long long k) {
     k ^= k >> 33;
     k *= 0xff51afd7ed558ccdull;
@@ -193,8 +194,7 @@ struct GridView {
 // once (in the lowest cell of the two ranges' overlap).  QG lanes per query look its cells up side by side,
 // eight at a time, and then share all their candidates: a cell holds a handful of candidates and a box a few
 // to BIG_CELLS cells, and each look-up and each candidate is a chain of dependent loads, so one cell after
-// the other leaves lanes idle and makes a wide box the kernel's tail (a batch of 64 scenes: 1.24 ms with
-// SMs busy 57% of it; 0.66 so).  ORDERED: pairs within one list, only those with i < j.
+// the other leaves lanes idle and makes a wide box the kernel's tail (a batch of 64 scenes: 1.24 ms; 0.66 so).  ORDERED: pairs within one list, only those with i < j.
 constexpr int QG = 8;
 template <bool ORDERED, class F>
 __device__ __forceinline__ void grid_walk(int block, int n, const QueryView& qv, const SceneGeo& g, const GridView& gv, const CandView& cv, F f) {
@@ -337,7 +337,7 @@ __device__ void attempt_ee(const double* __restrict__ x, const double* __restric
 // ---------------------------------------------------------------- candidate pairs
 // The grid walks and the big-primitive passes only test FP32 boxes; the pairs that pass go to a list, one
 // per kind, and the FP64 narrow phase runs over the lists with every lane on a pair.  In the walk itself one
-// or two lanes of a warp would run it while the others wait, and an FP64 instruction takes a warp's 18
+// or two lanes of a warp would run it while the others wait, and a warp's FP64 instruction takes 19
 // clocks of the SM whatever its active lanes.  A list that is full leaves its pair to the walking lane;
 // the next call's is larger.
 struct PairList {

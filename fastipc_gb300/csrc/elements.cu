@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(128) k_elasticity(int nT, const int4* __restri
 // (v*4+w, nv x nv used) of the projected barrier Hessian (common/math/ipc.py *_g_and_H); E, or g and Hb,
 // may be null.  One launch for the rows of all types, each block working on one type (block b on type t
 // for b in [block0[t], block0[t+1])): a type's rows are a few hundred warps, less than the chip holds, and
-// a launch lasts as long as one warp's FP64 instructions, which issue one in 18 clocks of an SM.  The
+// a launch lasts as long as one warp's FP64 instructions, which issue one in 19 clocks of an SM.  The
 // mollified types, the longest, come first.  With the closed forms of barrier.cuh, assembling the system of
 // two cubes in contact (2,000 rows) takes 0.72 ms against 4.08, that of 180 cubes in a pile (32,000 rows)
 // 1.9 against 8.5 (the element and run sums included).

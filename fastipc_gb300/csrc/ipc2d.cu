@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(T2) k2_pcg_dir(PCG2 a) {
 //    them in CTA order (so all CTAs hold the same scalars and take the same branch).  Slots start as
 //    NO_VALUE, rotate over four buffers and are cleared for reuse (slot_order.h: the order of stores, polls and
 //    fences).  A poll gives up after `limit` reads, the launch then ends and the three kernels above take the solve.
-// 4,600 rows, 145 CTAs: 18 us per iteration with three grid barriers -> 11.  What is left is latency: a
+// 4,600 rows, 145 CTAs: 18 us per iteration with three grid barriers, 11 so.  What is left is latency: a
 // dependent FP64 operation takes 50 ns, and the reductions, the two round trips through L2 and the scalars of
 // an iteration are some 100 of them one after the other; 580 rows take 9 us, 9,250 take 14.
 constexpr int COOP_ROWS = 256, COOP_SLOTS = 16;

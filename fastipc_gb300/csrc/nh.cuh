@@ -114,7 +114,7 @@ FIPC_HD void svd3_start(const double* F, double* V) {
 // F = U diag(s) V^T, det U = det V = +1, s descending in magnitude, s[2] < 0 iff det F < 0.
 // The rotations are FP64, on F V with V from svd3_start: one sweep of small angles and one that finds nothing
 // left, where starting from F takes four to six sweeps.  Element Hessians issue FP64 instructions
-// back to back (89% of the pipe), so their count is the time: assembling the 960k-tet bar 4.5 -> 3.2 ms with
+// back to back (88% of the pipe), so their count is the time: assembling the 960k-tet bar 4.5 -> 3.2 ms with
 // the element Hessian's other savings below.
 FIPC_HD void svd3(const double* F, double* U, double* s, double* V) {
     double B[9];

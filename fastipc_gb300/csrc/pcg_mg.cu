@@ -13,9 +13,9 @@
 //   * the post-smoothing of a level also prolongates its result into the next finer level.
 // Per iteration: 3 L barriers for L levels.  Every sum runs in a fixed order for a given GPU and
 // scene, so a solve is reproducible bit for bit.
-// Measured per PCG iteration on a GB300, kernel chain before -> one launch: 1,458 vertices 46 -> 29 us,
-// 1,736 with 608 contact rows 79 -> 49, 6,152 with 1,935 82 -> 53, 13,832 with 4,932 96 -> 57, 24,584
-// with 9,531 148 -> 86, 25,704 without contact 74 -> 63.  What is left of the small scenes' time is the
+// Per PCG iteration on a GB300, kernel chain against one launch: 1,458 vertices 40 us against 28, 1,736 with 608
+// contact rows 65 / 50, 6,182 with 2,048 67 / 53, 10,376 with 5,133 70 / 55, 24,584 with 9,531 91 / 83 (system.cu has the
+// line between them).  What is left of the small scenes' time is the
 // barriers (1.1 us each) and, per phase, one or two dependent L2 accesses and a chain of FP64
 // instructions at some 50 ns each.
 #include <cooperative_groups.h>

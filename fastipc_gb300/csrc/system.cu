@@ -416,11 +416,10 @@ int mg_start(fipc_ctx* c, const PCGArgs& a, cudaStream_t s);
 void mg_vcycle(const fipc_ctx* c, const PCGArgs& a, cudaStream_t s);
 int mg_launches_per_cycle(int levels);
 int pcg_mg_run(fipc_ctx* c, const PCGArgs& a, double rtol, int maxit, int guess, int* iters, cudaStream_t s);
-// Up to this many vertices a multigrid-preconditioned solve is one cooperative launch (pcg_mg.cu);
-// above, the kernel chain below, whose level-0 kernels fill the GPU, is faster.  Per PCG iteration,
-// chain against one launch: 46 us
-// against 29 us on 1,458 vertices, 79 / 49 us on 1,736 with 608 contact rows, 74 / 57 us on 13,832 with
-// 4,932, 69 / 63 us on 25,704 without, but 113 / 133 us on 58,089.
+// Up to this many vertices a multigrid-preconditioned solve is one cooperative launch (pcg_mg.cu); above, the
+// kernel chain below, whose level-0 kernels fill the GPU, is as fast or faster.  us per PCG iteration, chain / one launch:
+//   bars without contact   16,473 57.2 / 52.0, 26,010 64.3 / 60.7, 32,946 82.0 / 76.1, 39,015 83.4 / 90.7, 58,089 108.8 / 117.1
+//   piles in contact       1,736 64.6 / 49.5, 10,376 69.6 / 54.9, 24,584 90.7 / 83.4, 42,883 130.2 / 128.1, 51,208 131.3 / 135.8
 constexpr int PCG_RUN_MAX_VERTICES = 32768;
 
 int contact_prepare(fipc_ctx* c, TypeTable* tt, int* nrows_out, long long* nent_out, cudaStream_t s);
