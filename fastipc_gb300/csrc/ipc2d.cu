@@ -1173,11 +1173,15 @@ int fipc2d_find_constraints(fipc2d_ctx_impl* h, const double* x, int* counts_h, 
     cudaStream_t s = (cudaStream_t)stream;
     if (c->cnt_d.ensure(16) || c->scal.ensure(64)) return FIPC_ERR_CUDA;
     int* cnt = c->cnt_d.as<int>();
+    // room for a list's rows: its capacity counts once the buffer has it, and its former rows go with the buffer
+    auto room = [c](int t, int rows) {
+        c->cap[t] = c->h_counts[t] = 0;
+        if (c->rows[t].ensure(16ull * rows)) return false;
+        c->cap[t] = rows;
+        return true;
+    };
     for (int t = 0; t < 2; ++t)
-        if (c->cap[t] == 0) {
-            c->cap[t] = 1024;
-            if (c->rows[t].ensure(16ull * c->cap[t])) return FIPC_ERR_CUDA;
-        }
+        if (c->cap[t] == 0 && !room(t, 1024)) return FIPC_ERR_CUDA;
     int hc[3] = {0, 0, 0};
     for (int attempt = 0; attempt < 8; ++attempt) {
         FIPC_CUDA(cudaMemsetAsync(cnt, 0, 16, s));
@@ -1190,10 +1194,7 @@ int fipc2d_find_constraints(fipc2d_ctx_impl* h, const double* x, int* counts_h, 
         FIPC_CUDA(cudaStreamSynchronize(s));
         if (!hc[2]) break;
         for (int t = 0; t < 2; ++t)
-            if (hc[t] > c->cap[t]) {
-                c->cap[t] = hc[t] + hc[t] / 2 + 1024;
-                if (c->rows[t].ensure(16ull * c->cap[t])) return FIPC_ERR_CUDA;
-            }
+            if (hc[t] > c->cap[t] && !room(t, hc[t] + hc[t] / 2 + 1024)) return FIPC_ERR_CUDA;
     }
     if (hc[2]) return FIPC_ERR_CAPACITY;
     // np.unique(rows, axis=0) (NEWTON_IPC.py:348-356): sort the packed keys, drop repeats
