@@ -30,7 +30,12 @@ FIPC_HD int sym_eig_ld(int n, double* a, double* d) {
             if (scale == 0.0) {
                 e[i] = A_(i, l);
             } else {
-                const double iscale = 1.0 / scale;
+                double up = 1.0;
+                if (scale < 2.2250738585072014e-308) {   // subnormal: its reciprocal may be infinite
+                    up = 0x1p600;
+                    for (int k = 0; k <= l; ++k) A_(i, k) *= up;
+                }
+                const double iscale = 1.0 / (scale * up);
                 for (int k = 0; k <= l; ++k) {
                     A_(i, k) *= iscale;
                     h += A_(i, k) * A_(i, k);
