@@ -49,8 +49,9 @@ struct PpShared {
     double row[3 * PP_THREADS];  // per-warp row sums
     double con[3 * PP_THREADS];  // contact sums
     double tot[8];
-    double alpha, beta, inv_gamma, inv_alpha, tol2;   // scalars of the recurrences
+    double alpha, beta, gamma, inv_gamma, inv_alpha, tol2;   // scalars of the recurrences
     int done;
+    int tiny;                    // gamma is subnormal (tolerance 0, a residual of some 1e-154) and its reciprocal may be infinite
     unsigned mask[PP_WARPS];     // rows of a slice with contact blocks
     int next;                    // next contact task of the pass
 };
@@ -422,6 +423,7 @@ __device__ __forceinline__ bool phase_tolerance(const PcgLoop& P, PpShared& sh) 
         const double rr = sh.tot[0];
         sh.tol2 = P.rtol * P.rtol * sh.tot[1];
         sh.inv_gamma = sh.inv_alpha = 1.0;
+        sh.tiny = 0;
         sh.done = rr == 0.0 || rr <= sh.tol2;
         if (blockIdx.x == 0 && sh.done) P.a.flag[0] = 1;
     }
@@ -548,7 +550,14 @@ __device__ __forceinline__ bool phase_update(const PcgLoop& P, PpShared& sh, int
                       const double G = sh.tot[0];
                       sh.done = sh.tot[2] <= sh.tol2;
                       sh.beta = k == 0 ? 0.0 : G * sh.inv_gamma;
-                      sh.alpha = G / (sh.tot[1] - sh.beta * G * sh.inv_alpha);
+                      if (sh.tiny) {
+                          sh.beta = G / sh.gamma;
+                          sh.alpha = G / (sh.tot[1] - sh.beta * G / sh.alpha);
+                          // subnormal sums hold few digits, or none: a step that they do not give is left out
+                          if (!isfinite(sh.alpha) || !isfinite(sh.beta)) sh.alpha = sh.beta = 0.0;
+                      } else {
+                          sh.alpha = G / (sh.tot[1] - sh.beta * G * sh.inv_alpha);
+                      }
                       if (blockIdx.x == 0) {
                           a.flag[3] = sh.done ? k : k + 1;
                           if (sh.done) {
@@ -561,6 +570,8 @@ __device__ __forceinline__ bool phase_update(const PcgLoop& P, PpShared& sh, int
                   alpha = sh.alpha;
                   beta = sh.beta;
                   if (threadIdx.x == 0) {   // for the next iteration, off the critical path
+                      sh.gamma = sh.tot[0];
+                      sh.tiny = sh.gamma < 2.2250738585072014e-308;
                       sh.inv_gamma = 1.0 / sh.tot[0];
                       sh.inv_alpha = 1.0 / alpha;
                   }
