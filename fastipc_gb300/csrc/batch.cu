@@ -481,7 +481,7 @@ static void fill_tables(const fipc_ctx* c, BPCG& a) {
 // (16 scenes 65.5 -> 61.7 ms a solve, 64 scenes 145.0 -> 141.7), and 128 beyond (256 scenes 419 ms against
 // 426: half as many partial sums).
 static int autotune(fipc_ctx* c, BPCG a, cudaStream_t s) {
-    int dev = 0, nsm = 152;
+    int dev = 0, nsm = SMS;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     cudaEvent_t e0, e1;
@@ -785,7 +785,7 @@ int fipc_batch_compute_energy(fipc_ctx* c, const double* x, const double* xt, do
     if (!c || c->n_scenes < 2 || !x || !xt || !energy) return FIPC_ERR_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
     const int S = c->n_scenes;
-    const int parts = std::max(1, std::min(16, 4 * 152 / S));   // CTAs for four per SM
+    const int parts = std::max(1, std::min(16, 4 * SMS / S));   // CTAs for four per SM
     if (c->s_rowoff.ensure(4ll * N_TYPES * (S + 1)) || c->s_red.ensure(8ll * S * parts)) return FIPC_ERR_CUDA;
     const RowLists rl = row_lists(c);
     k_scene_row_offsets<<<nblk(S + 1, 128), 128, 0, s>>>(S, c->voff_d, rl, c->s_rowoff.as<int>());

@@ -357,7 +357,7 @@ __device__ __forceinline__ bool pair_push(const PairList& L, int kind, int a, in
     L.w[(size_t)kind * L.cap + k] = make_int2(a, b);
     return true;
 }
-constexpr int PAIR_THREADS = 64, PAIR_BLOCKS = 16 * 152;
+constexpr int PAIR_THREADS = 64, PAIR_BLOCKS = 16 * SMS;
 // f(kind, pair) for every listed pair; a warp's pairs are of one kind
 template <class F>
 __device__ __forceinline__ void each_pair(const PairList& L, F f) {
@@ -1193,7 +1193,7 @@ static int broad_prepare(fipc_ctx* c, const double* x, const double* p, int quer
     b->qe = QueryView{b->qt.cell + c->nBT, b->qt.box + 2ll * c->nBT, b->n->mid_pairs + 1};
     FIPC_CUDA(cudaMemsetAsync(b->n, 0, sizeof(BroadCounters), s));
     const long long work = (long long)n + np, slots = (long long)(slots_p + slots_e);
-    const int grid = (int)std::max<long long>(nblk(work, 256), std::min<long long>(nblk(slots, 256), 1216));
+    const int grid = (int)std::max<long long>(nblk(work, 256), std::min<long long>(nblk(slots, 256), 8 * SMS));
     k_prepare<<<grid, 256, 0, s>>>(c->nBT, c->bt, c->nBE, c->be, b->gp, b->ge, x, p, c->dhat, g, b->qt, b->qe, c->prim_off,
                                    c->n_scenes, tri_size, tri_size + c->nBT, c->big_list.as<int>(), b->n);
     FIPC_LAUNCHED();

@@ -14,6 +14,10 @@
 
 namespace fipc {
 
+// SMs of a GB300.  A grid or a number of chunks that sets the order of a sum follows this constant, not the device's own
+// number, so that results do not depend on the device; the sizes at which kernels were measured do too.
+constexpr int SMS = 152;
+
 // number of kernels this library launched (reported by fipc_launch_count)
 extern std::atomic<long long> g_launches;
 
@@ -198,7 +202,7 @@ struct TypeTable {
     long long ent0[N_TYPES + 1];
 };
 
-constexpr int RED_BLOCKS = 304;     // 2 x 152 SMs: fixed reduction grid (deterministic sums)
+constexpr int RED_BLOCKS = 2 * SMS;   // fixed reduction grid (deterministic sums)
 constexpr int RED_THREADS = 256;
 
 // cell key of integer cell coordinates (21 bits per axis, offset 2^20)

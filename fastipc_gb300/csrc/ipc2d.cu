@@ -30,7 +30,7 @@ namespace {
 
 constexpr int T2 = 256;       // threads per CTA of the 2D kernels
 constexpr int TILE = 256;     // edges / triangles per shared-memory tile
-constexpr int P2_RED = 304;   // fixed reduction grid (2 x 152 SMs)
+constexpr int P2_RED = 2 * SMS;   // fixed reduction grid
 
 inline int nb2(long long n, int b) { return (int)((n + b - 1) / b); }
 

@@ -836,7 +836,7 @@ int mg_prepare(fipc_ctx* c, const unsigned char* fixed, PCGArgs& a, cudaStream_t
         const long long ne = 288ll * c->n_slots, nc = 9ll * c->c_nnzb;
         if (M->v32.ensure(4ull * (ne + nc) + 64) || M->z0f.ensure(16ull * nV + 64)) return FIPC_ERR_CUDA;
         float* v32 = M->v32.as<float>();
-        k_mg_to_f32<<<1216, 256, 0, s>>>(ne, c->sell_val, v32);
+        k_mg_to_f32<<<8 * SMS, 256, 0, s>>>(ne, c->sell_val, v32);
         FIPC_LAUNCHED();
         if (nc) {
             k_mg_to_f32<<<nblk_m(nc, 256), 256, 0, s>>>(nc, c->c_val.as<double>(), v32 + ne);

@@ -454,7 +454,7 @@ namespace fipc {
 static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
 // rows per tile: the largest that still gives every SM two CTAs (R = 128) or most SMs one (R = 64)
-static int tile_rows(int n) { return n >= 128 * 304 ? 128 : (n >= 64 * 96 ? 64 : 32); }
+static int tile_rows(int n) { return n >= 128 * 2 * SMS ? 128 : (n >= 64 * 96 ? 64 : 32); }
 
 template <int R>
 static int launch_forward(int n, const float* X, const float* P, float* Z, float* A, float* out, bool al, cudaStream_t s) {
@@ -484,7 +484,7 @@ template <int DIN>
 static void weight_grad(int n, const float* d, const float* in, float* scratch, float* G, bool al, cudaStream_t s) {
     constexpr int size = MLP_H * DIN + MLP_H;
     int nc = n / 192;
-    nc = nc < 1 ? 1 : (nc > 152 ? 152 : nc);
+    nc = nc < 1 ? 1 : (nc > SMS ? SMS : nc);
     const int chunk = (n + nc - 1) / nc;
     nc = nblk(n, chunk);
     k_mlp_weight_grad<DIN><<<dim3(nc, 2), MLP_THREADS, 0, s>>>(n, chunk, d, in, nc > 1 ? scratch : G, al);
@@ -530,7 +530,7 @@ int fipc_mlp_backward(int n, const float* X, const float* params, const float* Z
     float *d0 = dA, *d1 = dA + L;
     const bool al = aligned16({X, params, Z, A, dout, grads, dA});
     {   // layer 4 (linear): at least 64 rows a chunk (MLP_LAST / 64 < 8.1 floats a row)
-        const int chunk = n > 64 * 304 ? (n + 303) / 304 : 64, nc = nblk(n, chunk);
+        const int chunk = n > 64 * 2 * SMS ? nblk(n, 2 * SMS) : 64, nc = nblk(n, chunk);
         float* part = nc > 1 ? d1 : G + OFF_W4;
         k_mlp_last_grad<<<nc, MLP_THREADS, 0, s>>>(n, chunk, dout, P + OFF_W4, A + 2 * L, Z + 2 * L, d0, part, al);
         FIPC_LAUNCHED();

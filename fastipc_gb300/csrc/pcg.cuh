@@ -147,7 +147,7 @@ __device__ __forceinline__ void contact_rows(const int* __restrict__ crp, const 
 // with nothing to hide it.  (FP64 products are bound by the FP64 pipe and lose by the second part's adds.)
 // Up to two dozen slices per SM: 61,700 rows (13 per SM) res0 22 -> 16 us, post0 28 -> 17; 182,000 (37 per
 // SM) 23.5 -> 24.5 and 26.8 -> 27.1.
-inline int row_parts(int nV) { return nV <= 24 * 152 * 32 ? 2 : 1; }
+inline int row_parts(int nV) { return nV <= 24 * SMS * 32 ? 2 : 1; }
 template <int PARTS>
 struct RowPart {
     int i, part;
